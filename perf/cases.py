@@ -69,10 +69,10 @@ def _log(rng, lo, hi):
     return int(round(lo * (hi / lo) ** rng.random()))
 
 
-def _draw_pattern(rng, lo, hi):
+def _draw_pattern(rng, lo, hi, grids=False):
     """A pattern of about lo..hi block rows, ragged sides."""
     nb = _log(rng, lo, hi)
-    t = rng.randrange(5)
+    t = rng.randrange(1 if grids else 0, 5)
     if t == 0:
         return dict(powerlaw=max(64, min(nb, 62500)))
     if t <= 2:
@@ -93,8 +93,10 @@ def draw(rng):
         return dict(op=op, **_draw_pattern(rng, 1000, 200000 if bs == 4 else 80000), bs=bs,
                     prec=rng.choice(["fp64", "fp32"]), k=rng.choice([1, 2, 7, 16, 32, 33, 64]))
     if op == "convert":
-        return dict(op=op, **_draw_pattern(rng, 1000, 100000 if bs < 8 else 40000), bs=bs,
-                    fill=rng.choice([1.0, 0.8, 0.4]))
+        # files of assembled grids: a hub row of thousands of scalar entries
+        # takes seconds
+        return dict(op=op, **_draw_pattern(rng, 1000, 100000 if bs < 8 else 40000, grids=True),
+                    bs=bs, fill=rng.choice([1.0, 0.8, 0.4]))
     if op == "setup":
         level = rng.choice([1, 1, 2])
         p = _draw_pattern(rng, 500, 200000 if level == 1 else 30000)
