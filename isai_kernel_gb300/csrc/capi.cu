@@ -15,7 +15,7 @@ int transpose_pattern(int mb, int nbcol, const int* cptr, const int* cind, long 
 size_t syncfree_ws(int nb);
 int diag_positions(int nb, const int* row, const int* col, int* diag, int* h_bad, Carver& ws,
                    cudaStream_t st);
-size_t level_sched_ws(int nb, long long nnzb);
+size_t level_sched_ws(int nb);
 int sptrsv_level_impl(int nb, long long nnzb, int bs, const int* row, const int* col,
                       const int* diag, const double* val, int lower, int unit, const double* b,
                       double* x, Carver& ws, cudaStream_t st);
@@ -157,7 +157,7 @@ static size_t sptrsv_t_ws(int nb, long long nnzb, int bs) {
   return carve_size(sizeof(int) * (size_t)(nb + 1)) + carve_size(sizeof(int) * (size_t)nnzb) +
          carve_size(sizeof(double) * (size_t)nnzb * bs * bs) +
          std::max(bsr_transpose_ws(nb, nnzb),
-                  level_sched_ws(nb, nnzb) + carve_size(sizeof(int) * ((size_t)nb + 1)) +
+                  level_sched_ws(nb) + carve_size(sizeof(int) * ((size_t)nb + 1)) +
                       carve_size(sizeof(int) * 2));
 }
 

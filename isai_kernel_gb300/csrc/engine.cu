@@ -36,9 +36,9 @@ int reorder_impl(long long nnzb, int bs, const int* map, const double* src, doub
 size_t syncfree_ws(int nb);
 int diag_positions(int nb, const int* row, const int* col, int* diag, int* h_bad, Carver& ws,
                    cudaStream_t st);
-size_t level_sched_ws(int nb, long long nnzb);
+size_t level_sched_ws(int nb);
 size_t bilu0_ws(int nb, long long nnzb);
-size_t levels_ws(int nb, long long ndeps);
+size_t levels_ws(int nb);
 size_t pattern_product_ws(int n);
 int pattern_product_rowptr(int n, const int* Xrow, const int* Xcol, const int* Arow,
                            const int* Acol, int* Crow, int* h_nnz, int* h_bad, Carver& ws,
@@ -423,7 +423,7 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
   BILU_TRY_CUDA(cudaMemcpyAsync(c->Acol, d_col, sizeof(int) * nnzb, cudaMemcpyDeviceToDevice, st));
   // scratch shared by every step
   size_t wsb = std::max({isai_pattern_ws(nb, nnzb), bilu0_ws(nb, nnzb), pairs_ws(nnzb + nb),
-                         levels_ws(nb, nnzb), pattern_product_ws(nb),
+                         levels_ws(nb), pattern_product_ws(nb),
                          scan_ws_bytes(nnzb + nb + 1)}) + (1 << 16);
   void* wsp = nullptr;
   void* wsq = nullptr;  // a larger scratch for the pattern(A^k) steps

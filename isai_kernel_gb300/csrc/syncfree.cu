@@ -4,9 +4,9 @@
 //   spTrSolveL / spTrSolveU (cape_sptrsv.h:8,55)         -> k_sptrsv_levels,
 //                                                            k_sptrsv (sync-free)
 //
-// Level schedule (default): a breadth-first sweep (k_bfs_levels) groups the
-// block rows by dependency level; one cooperative launch then processes a
-// level with a group of bs lanes per row and meets at a bounded grid barrier.
+// Level schedule (default): the block rows are grouped by dependency level
+// (k_levels); one cooperative launch then processes a level with a group of
+// bs lanes per row and meets at a bounded grid barrier.
 //
 // Sync-free schedule (the reference's design, kept for the solve): a warp
 // owns one block row at a time.  Rows are handed out by an atomic ticket
@@ -361,173 +361,220 @@ __global__ void __launch_bounds__(128) k_sptrsv(int nb, const int* __restrict__ 
 }
 
 // ------------------------------------------------------------------ levels
-// Dependency level of every block row (1 + the deepest row it waits on),
-// thread per row, sync-free like the solves: rows are taken in ticket order,
-// a row waits (bounded) for the levels of its dependencies and publishes its
-// own.  The lower DAG follows the strictly lower blocks, the upper DAG the
-// strictly upper ones in reverse order.
+// The dependency DAG is cut into levels (level 0: rows without dependencies;
+// level l+1: rows whose dependencies all sit in levels <= l).  The lower DAG
+// follows the strictly lower blocks, the upper DAG the strictly upper ones in
+// reverse order.
+
+// rows with more dependencies than this make the level kernels give each
+// row a whole warp instead of a bs-lane group
+constexpr int kLongRow = 32;
+// Level analysis recommendations (measured on GB300, stencil and power-law
+// systems).  Solves: the level order (flow kernel) when no row has more than
+// kFlowMaxDeps dependencies, whatever the level width (it was 4-10x faster
+// than the sync-free kernel on 2D and 3D stencils down to 32 rows per
+// level), the sync-free kernel otherwise (a lane group walks a long row's
+// dependencies one after the other).  BILU(0): the level order (a barrier
+// per level) when a level holds at least kFactorLevelWidth rows on average
+// and no row has more than kLongRow dependencies, sync-free otherwise.
+constexpr int kFlowMaxDeps = 8;
+constexpr int kFactorLevelWidth = 4096;
+
+// Words of a level analysis on the device (zero before it starts).
+struct LevelWords {
+  int ticket, err;           // next 32 rows; 0 or a bilu_status
+  int maxdeg, nlev;          // largest dependency count of a row; levels
+  unsigned long long ndeps;  // dependencies of all rows
+};
+
+__device__ __forceinline__ void st_relaxed(int* p, int v) {
+  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// level[I] = 1 + the largest level of the rows I depends on (1 for none).
+// Sync-free: a warp takes the next 32 rows by ticket, a lane per row.  A round
+// polls the levels of the dependencies that are still missing (kLevelBatch of
+// them in flight a lane), hands the levels that became known to the lanes of
+// the same warp through shuffles (consecutive rows of a stencil depend on one
+// another: a chain through a warp costs shuffles instead of trips through the
+// L2), and stores them; the level is the only datum, so no fence is needed.
+// No lane ever waits inside a round.  Rows with more than 32 dependencies left
+// are walked by the whole warp, 32 at a time, also without waiting.  Tickets
+// ascend with the rows, so every row polled is finished, running or in the
+// same warp.
+//
+// What bounds it is the longest chain: one store-to-load hop through the L2
+// (0.35-0.6 us on GB300) where it leaves a warp, instead of the barrier, list
+// and append round trips a level of the breadth-first sweep it replaced (4-6 us
+// a level; in one 16-CTA cluster 3-4 us).  Whole analysis, before and after:
+// 64^3 7-point grid (190 levels) 1.35 -> 0.35 ms, 128^3 (382) 3.0 -> 1.6 ms,
+// 512 x 512 5-point grid (1023) 4.5 -> 0.74 ms, 33 x 9000 (9032) 36 -> 8.8 ms,
+// 62,500-row power-law pattern 1.46 -> 0.54 ms.
+constexpr int kLevelBatch = 4;
+constexpr int kLevelSpins = 64;      // polls of a waiting warp before it sleeps
+constexpr unsigned kLevelSleep = 32;  // ns between its polls then
+
 template <bool LOWER>
 __global__ void __launch_bounds__(256) k_levels(int nb, const int* __restrict__ row,
                                                 const int* __restrict__ col,
                                                 const int* __restrict__ diag, int* level,
-                                                int* ticket, int* err, long long spin) {
+                                                LevelWords* w, long long spin) {
+  const int lane = threadIdx.x & 31;
   while (true) {
-    int t = atomicAdd(ticket, 1);
-    if (t >= nb) return;
-    int I = LOWER ? t : nb - 1 - t;
-    int ps = LOWER ? __ldg(row + I) : __ldg(diag + I) + 1;
-    int pe = LOWER ? __ldg(diag + I) : __ldg(row + I + 1);
-    int lv = 0;
-    for (int p = ps; p < pe; ++p) {
-      const int* f = level + __ldg(col + p);
+    int t = 0;
+    if (lane == 0) t = atomicAdd(&w->ticket, 1);
+    const long long k0 = (long long)__shfl_sync(FULL, t, 0) * 32;
+    if (k0 >= nb) return;
+    const bool mine = k0 + lane < nb;
+    const int I = mine ? (LOWER ? (int)k0 + lane : nb - 1 - ((int)k0 + lane)) : 0;
+    int p = 0, pe = 0;
+    if (mine) {
+      p = LOWER ? __ldg(row + I) : __ldg(diag + I) + 1;
+      pe = LOWER ? __ldg(diag + I) : __ldg(row + I + 1);
+    }
+    const int deg = __reduce_max_sync(FULL, pe - p);
+    const unsigned deps = __reduce_add_sync(FULL, (unsigned)(pe - p));
+    if (lane == 0 && deg > 0) {
+      atomicMax(&w->maxdeg, deg);
+      atomicAdd(&w->ndeps, (unsigned long long)deps);
+    }
+    int c[kLevelBatch];
+#pragma unroll
+    for (int u = 0; u < kLevelBatch; ++u) c[u] = -1;
+    bool todo = mine;
+    int lv = 0, own = 0;  // largest level seen; this row's, once known
+    const int I0 = LOWER ? (int)k0 : nb - 1 - (int)k0;  // lane 0's row
+    auto lane_of = [&](int r) { return LOWER ? r - I0 : I0 - r; };
+    auto in_warp = [&](int r) { return (unsigned)lane_of(r) < 32u; };
+    while (__any_sync(FULL, todo)) {
+      bool moved = false;
+      unsigned lng = deg > 32 ? __ballot_sync(FULL, todo && pe - p > 32) : 0u;
+      while (lng) {
+        const int src = __ffs(lng) - 1;
+        lng &= lng - 1;
+        const int q = __shfl_sync(FULL, p, src);
+        const int v = ld_relaxed(level + __ldg(col + q + lane));
+        const unsigned wait = __ballot_sync(FULL, v == 0);
+        const int adv = wait ? __ffs(wait) - 1 : 32;
+        const int m = __reduce_max_sync(FULL, lane < adv ? v : 0);
+        if (lane == src) {
+          p += adv;
+          lv = max(lv, m);
+        }
+        moved |= adv > 0;
+      }
+      if (todo && pe - p <= 32) {
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < kLevelBatch; ++u) any |= c[u] >= 0;
+        if (!any) {  // the next few dependencies
+#pragma unroll
+          for (int u = 0; u < kLevelBatch; ++u) c[u] = p + u < pe ? __ldg(col + p + u) : -1;
+          p = min(p + kLevelBatch, pe);
+        }
+        int v[kLevelBatch];
+#pragma unroll
+        for (int u = 0; u < kLevelBatch; ++u)
+          v[u] = c[u] >= 0 && !in_warp(c[u]) ? ld_relaxed(level + c[u]) : 0;
+#pragma unroll
+        for (int u = 0; u < kLevelBatch; ++u)
+          if (v[u] != 0) {
+            lv = max(lv, v[u]);
+            c[u] = -1;
+            moved = true;
+          }
+      }
+      // rows that are now known, and through shuffles the rows of the same
+      // warp that waited for them
+      while (true) {
+        bool step = false, any = false;
+#pragma unroll
+        for (int u = 0; u < kLevelBatch; ++u) {
+          const bool in = c[u] >= 0 && in_warp(c[u]);
+          const int v = __shfl_sync(FULL, own, in ? lane_of(c[u]) : 0);
+          if (in && v != 0) {
+            lv = max(lv, v);
+            c[u] = -1;
+            moved = true;  // the row may have dependencies yet to load
+          }
+          any |= c[u] >= 0;
+        }
+        if (todo && !any && p >= pe) {
+          own = lv + 1;
+          st_relaxed(level + I, own);
+          todo = false;
+          step = moved = true;
+        }
+        if (!__any_sync(FULL, step)) break;
+      }
+      if (__any_sync(FULL, moved)) continue;
+      // Nothing moved.  The lanes that wait for no lane of this warp poll one
+      // dependency each until one of those is there.  (Every lane polling all
+      // of its own floods the L2 on large systems; a single word for the warp
+      // would hold up the lanes of another grid line.)
+      int wait = -1;
+      if (todo) {
+        bool inside = false;
+#pragma unroll
+        for (int u = 0; u < kLevelBatch; ++u)
+          if (c[u] >= 0) {
+            wait = c[u];
+            inside |= in_warp(c[u]);
+          }
+        if (pe - p > 32) wait = __ldg(col + p);
+        else if (inside) wait = -1;
+      }
       long long n = 0;
-      unsigned ns = 32;
-      int v;
-      while ((v = ld_relaxed(f)) == 0) {
-        if (ld_relaxed(err) != 0) return;
+      while (!__any_sync(FULL, wait >= 0 && ld_relaxed(level + max(wait, 0)) != 0)) {
         if (++n > spin) {
-          atomicCAS(err, 0, (int)BILU_ERR_TIMEOUT);
+          if (lane == 0) atomicCAS(&w->err, 0, (int)BILU_ERR_TIMEOUT);
           return;
         }
-        backoff(ns);
+        if ((n & 63) == 0 && __any_sync(FULL, ld_relaxed(&w->err) != 0)) return;
+        if (n > kLevelSpins) __nanosleep(kLevelSleep);
       }
-      lv = max(lv, v);  // the level value itself is the only datum read
     }
-    st_release(level + I, lv + 1);
+    const int top = __reduce_max_sync(FULL, own);
+    if (lane == 0) atomicMax(&w->nlev, top);
   }
 }
 
+// cnt[l] = rows of level l; one atomic per distinct level of a warp.  (Rows
+// without a level, after a timeout, are skipped: the host reports it.)
 __global__ void k_level_count(int nb, const int* __restrict__ level, int* cnt) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nb) atomicAdd(cnt + level[i] - 1, 1);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int l = i < nb ? level[i] - 1 : -1;
+  const unsigned same = __match_any_sync(FULL, l);
+  if (l >= 0 && (int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(cnt + l, __popc(same));
 }
 
-__global__ void k_level_scatter(int nb, const int* __restrict__ level, int* cursor, int* order) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nb) order[atomicAdd(cursor + level[i] - 1, 1)] = i;
-}
-
-// ------------------------------------------------------------------ level schedule
-// The dependency DAG is cut into levels (level 0: rows without dependencies;
-// level l+1: rows whose dependencies all sit in levels <= l).  A level
-// scheduled kernel is one cooperative launch (all CTAs co-resident) that
-// processes the rows of a level with one warp each and then meets at a
-// grid-wide barrier; no per-row flags are polled.
-
-// Dependencies of row I: lower -> columns in [row[I], diag[I]); upper ->
-// columns in (diag[I], row[I+1]).  cnt[K] += 1 per dependent of K.
-__global__ void k_dep_count(int nb, const int* __restrict__ row, const int* __restrict__ col,
-                            const int* __restrict__ diag, int lower, int* __restrict__ cnt,
-                            int* __restrict__ indeg, int* maxdeg) {
-  int I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= nb) return;
-  int ps = lower ? row[I] : diag[I] + 1, pe = lower ? diag[I] : row[I + 1];
-  indeg[I] = pe - ps;
-  if (pe - ps > 0) atomicMax(maxdeg, pe - ps);
-  for (int p = ps; p < pe; ++p) atomicAdd(cnt + col[p], 1);
-}
-
-// Successor lists: sidx[sptr[K] ...] = rows that depend on K (any order).
-__global__ void k_dep_fill(int nb, const int* __restrict__ row, const int* __restrict__ col,
-                           const int* __restrict__ diag, int lower, const int* __restrict__ sptr,
-                           int* __restrict__ cursor, int* __restrict__ sidx) {
-  int I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= nb) return;
-  int ps = lower ? row[I] : diag[I] + 1, pe = lower ? diag[I] : row[I + 1];
-  for (int p = ps; p < pe; ++p) {
-    int K = col[p];
-    sidx[sptr[K] + atomicAdd(cursor + K, 1)] = I;
-  }
-}
-
-// Appends the rows of the warp's ready lanes to order[base0 + ...] with one
-// atomic on the level's append counter per warp (ballot + prefix count).
-// Called by all 32 lanes.
-__device__ __forceinline__ void warp_append(bool ready, int J, int* order, int base0,
-                                            int* count) {
-  const unsigned m = __ballot_sync(FULL, ready);
-  if (!m) return;
-  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(count, __popc(m));
-  base = __shfl_sync(FULL, base, leader);
-  if (ready) order[base0 + base + __popc(m & ((1u << lane) - 1u))] = J;
-}
-
-// Breadth-first level sweep (Kahn's algorithm, one level per barrier):
-// order[] receives the rows level by level, lvl_ptr[l] the start of level l
-// (lvl_ptr[nlev] = nb), *nlev the number of levels.  Warps take 32
-// consecutive frontier rows, walk their successor lists in step (one slot
-// per lane and round), decrement in-degrees and append the rows that reach
-// zero with one atomic per warp.  The rows inside a level come in append
-// order (k_sort_levels orders them afterwards); the level sizes do not
-// depend on it.
-//
-// Every CTA must see the same frontier: after the barrier that closes
-// level l, each CTA reads how many rows level l appended, while the CTAs
-// that left the barrier first are already appending level l + 1's rows.
-// So the levels count their appends in three rotating counters (cnt[l % 3];
-// the rows of the initial frontier in cnt[2]): the one a CTA reads after
-// barrier l is not written again until level l + 3, and CTA 0 clears the
-// counter of level l + 1 while it works on level l, after every CTA has
-// read it at level l - 2 (barrier l - 1 orders the reads before the clear,
-// barrier l the clear before the appends).  Rows go to absolute positions
-// e + count, e being the end of the current frontier, which every CTA knows.
-__global__ void __launch_bounds__(256) k_bfs_levels(int nb, const int* __restrict__ sptr,
-                                                    const int* __restrict__ sidx, int* indeg,
-                                                    int* order, int* lvl_ptr, int* cnt,
-                                                    int* nlev, GridSync gs) {
-  __shared__ int end_s;
-  unsigned passed = 0;
+// order[lvl[l] ...] = the rows of level l, taking cnt back to 0; and the
+// analysis record: levels, largest dependency count, recommended schedules of
+// the solves and of BILU(0) (0 level order, 1 sync-free).
+__global__ void k_level_scatter(int nb, const int* __restrict__ level,
+                                const int* __restrict__ lvl, int* cnt, int* order,
+                                const LevelWords* w, int* rec) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long wbase = tid - lane;  // first position of this warp
-  const long long nthr = (long long)gridDim.x * blockDim.x;
-  for (long long I0 = wbase; I0 < nb; I0 += nthr) {
-    const long long I = I0 + lane;
-    warp_append(I < nb && indeg[I] == 0, (int)I, order, 0, cnt + 2);
-  }
-  if (!grid_sync_count(gs, passed)) return;
-  if (threadIdx.x == 0) end_s = ld_relaxed(cnt + 2);
-  __syncthreads();
-  int s = 0, e = end_s;
-  if (tid == 0) {
-    lvl_ptr[0] = 0;
-    lvl_ptr[1] = e;
-  }
-  for (int l = 0;; ++l) {
-    if (s == e) {
-      if (tid == 0) *nlev = l;
-      grid_exit_count(gs);
-      return;
-    }
-    if (tid == 0) atomicExch(cnt + (l + 1) % 3, 0);
-    int* count = cnt + l % 3;
-    for (long long q0 = s + wbase; q0 < e; q0 += nthr) {
-      const long long q = q0 + lane;
-      const int I = q < e ? __ldcg(order + q) : -1;
-      int p = I >= 0 ? __ldg(sptr + I) : 0;
-      const int pe = I >= 0 ? __ldg(sptr + I + 1) : 0;
-      while (__any_sync(FULL, p < pe)) {
-        bool ready = false;
-        int J = -1;
-        if (p < pe) {
-          J = __ldg(sidx + p);
-          ready = atomicSub(indeg + J, 1) == 1;
-          ++p;
-        }
-        warp_append(ready, J, order, e, count);
-      }
-    }
-    if (!grid_sync_count(gs, passed)) return;
-    if (threadIdx.x == 0) end_s = e + ld_relaxed(count);
-    __syncthreads();
-    s = e;
-    e = end_s;
-    if (tid == 0) lvl_ptr[l + 2] = e;
+  const int l = i < nb ? level[i] - 1 : -1;
+  const unsigned same = __match_any_sync(FULL, l);
+  const int lead = __ffs(same) - 1, n = __popc(same);
+  int left = 0;
+  if (l >= 0 && lane == lead) left = atomicSub(cnt + l, n);
+  left = __shfl_sync(FULL, left, lead);
+  if (l >= 0) order[lvl[l] + left - n + __popc(same & ((1u << lane) - 1u))] = i;
+  if (i == 0 && rec) {
+    rec[0] = w->nlev;
+    rec[1] = w->maxdeg;
+    rec[2] = w->maxdeg > kFlowMaxDeps ? 1 : 0;
+    rec[3] = ((long long)nb < (long long)kFactorLevelWidth * w->nlev || w->maxdeg > kLongRow) ? 1
+                                                                                            : 0;
   }
 }
 
+// A level scheduled kernel is one cooperative launch (all CTAs co-resident)
+// that processes the rows of a level and then meets at a grid-wide barrier;
+// no per-row flags are polled.
 constexpr int kLvlThreads = 256;
 
 // Warp rank for level work.  Consecutive ranks sit in different CTAs (the
@@ -558,20 +605,6 @@ __device__ __forceinline__ int spread_warp(int per_sm) {
   const int round = ((int)(threadIdx.x >> 5) - rot_s + nwc) % nwc;
   return (int)(round * gridDim.x + blockIdx.x);
 }
-// rows with more dependencies than this make the level kernels give each
-// row a whole warp instead of a bs-lane group
-constexpr int kLongRow = 32;
-// Level analysis recommendations (measured on GB300, stencil and power-law
-// systems).  Solves: the level order (flow kernel) when no row has more than
-// kFlowMaxDeps dependencies, whatever the level width (it was 4-10x faster
-// than the sync-free kernel on 2D and 3D stencils down to 32 rows per
-// level), the sync-free kernel otherwise (a lane group walks a long row's
-// dependencies one after the other).  BILU(0): the level order (a barrier
-// per level) when a level holds at least kFactorLevelWidth rows on average
-// and no row has more than kLongRow dependencies, sync-free otherwise.
-constexpr int kFlowMaxDeps = 8;
-constexpr int kFactorLevelWidth = 4096;
-
 // Rows of the flow schedule: a group of BS lanes per block row (32/BS rows
 // per warp; lane r of a group owns scalar row r).  On GB300 an FP64 warp
 // instruction costs the same whatever the number of active lanes, so packing
@@ -1575,36 +1608,47 @@ int sync_finish(const SyncState& ss, int* h_zp, cudaStream_t st) {
   return BILU_OK;
 }
 
+// Launches of a level analysis: the levels, their sizes, lvl[nb+1] (level l is
+// order[lvl[l]] .. order[lvl[l+1]-1]) and order[nb].  rec (optional): the
+// four words of the analysis record.  Returns the words' device copy.
+int level_sets(int nb, const int* row, const int* col, const int* diag, int lower, int* order,
+               int* lvl, int* rec, LevelWords** out, Carver& ws, cudaStream_t st) {
+  int* level = ws.take<int>((size_t)nb + 1);
+  int* cnt = ws.take<int>((size_t)nb + 1);
+  LevelWords* w = ws.take<LevelWords>(1);
+  if (!level || !cnt || !w) return BILU_ERR_WORKSPACE;
+  *out = w;
+  // level, cnt and the words are neighbours: one fill
+  BILU_TRY_CUDA(cudaMemsetAsync(level, 0, (char*)(w + 1) - (char*)level, st));
+  if (nb == 0) return BILU_OK;
+  const void* fn = lower ? (const void*)k_levels<true> : (const void*)k_levels<false>;
+  const int grid = (int)std::min<long long>(occupancy_grid(fn, 256), (nb + 255) / 256);
+  if (lower)
+    k_levels<true><<<grid, 256, 0, st>>>(nb, row, col, diag, level, w, kSpinLimit);
+  else
+    k_levels<false><<<grid, 256, 0, st>>>(nb, row, col, diag, level, w, kSpinLimit);
+  BILU_LAUNCH_CHECK();
+  k_level_count<<<ceil_div(nb, 256), 256, 0, st>>>(nb, level, cnt);
+  BILU_LAUNCH_CHECK();
+  BILU_TRY(scan_exclusive(cnt, lvl, nb, nullptr, ws, st));
+  k_level_scatter<<<ceil_div(nb, 256), 256, 0, st>>>(nb, level, lvl, cnt, order, w, rec);
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
+
 // Ticket order by dependency level (ascending).  Rows of one level are
 // independent, so consecutive tickets can run concurrently; every row's
 // dependencies sit at lower levels, i.e. at earlier tickets.
 int build_order(int nb, const int* row, const int* col, const int* diag, int lower, int* order,
                 Carver& ws, cudaStream_t st) {
-  int* level = ws.take<int>((size_t)nb + 1);
-  int* cnt = ws.take<int>((size_t)nb + 1);
-  int* misc = ws.take<int>(4);
-  if (!level || !cnt || !misc) return BILU_ERR_WORKSPACE;
-  BILU_TRY_CUDA(cudaMemsetAsync(level, 0, sizeof(int) * ((size_t)nb + 1), st));
-  BILU_TRY_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)nb + 1), st));
-  BILU_TRY_CUDA(cudaMemsetAsync(misc, 0, sizeof(int) * 4, st));
-  if (nb == 0) return BILU_OK;
-  const void* fn = lower ? (const void*)k_levels<true> : (const void*)k_levels<false>;
-  int grid = std::min<long long>(occupancy_grid(fn, 256), (nb + 255) / 256);
-  if (lower)
-    k_levels<true><<<grid, 256, 0, st>>>(nb, row, col, diag, level, misc, misc + 1, kSpinLimit);
-  else
-    k_levels<false><<<grid, 256, 0, st>>>(nb, row, col, diag, level, misc, misc + 1, kSpinLimit);
-  BILU_LAUNCH_CHECK();
+  int* lvl = ws.take<int>((size_t)nb + 1);
+  LevelWords* w = nullptr;
+  if (!lvl) return BILU_ERR_WORKSPACE;
+  BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl, nullptr, &w, ws, st));
   int herr = 0;
-  BILU_TRY_CUDA(cudaMemcpyAsync(&herr, misc + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaMemcpyAsync(&herr, &w->err, sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
-  if (herr != 0) return herr;
-  k_level_count<<<ceil_div(nb, 256), 256, 0, st>>>(nb, level, cnt);
-  BILU_LAUNCH_CHECK();
-  BILU_TRY(scan_exclusive(cnt, cnt, nb, nullptr, ws, st));
-  k_level_scatter<<<ceil_div(nb, 256), 256, 0, st>>>(nb, level, cnt, order);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  return herr;
 }
 
 template <int BS>
@@ -1814,7 +1858,7 @@ __global__ void __launch_bounds__(kLvlThreads, 3) k_bilu0_syncfree(
 // consecutive levels of a structured problem depend on rows of a few
 // neighbouring warps instead of rows all over the previous level, which
 // the flow schedule turns into shorter waits.  One CTA per level, bitonic
-// sort in shared memory; a level wider than kSortCap keeps its breadth-first
+// sort in shared memory; a level wider than kSortCap keeps its append
 // order (only the speed depends on it).
 constexpr int kSortCap = 16384;
 
@@ -1877,83 +1921,44 @@ int launch_coop(const void* fn, int grid, int threads, void** args, cudaStream_t
   return BILU_OK;
 }
 
-// Level analysis of the lower (or upper) dependency DAG: successor lists by
-// counting sort, then the breadth-first level sweep.  order[nb],
-// lvl_ptr[nb+2] and *nlev_d on the device; *h_nlev on the host.
+// Level analysis of the lower (or upper) dependency DAG: order[nb] (ascending
+// inside a level), lvl_ptr[nb+1] and nlev_d[4] (levels, largest dependency
+// count, recommended solve and factorisation schedules: 0 level order, 1
+// sync-free) on the device; the same words on the host.  One host
+// synchronisation.  ndeps_max: the dependencies the caller's block count
+// leaves room for (BILU_ERR_WORKSPACE beyond it).
 int build_levels(int nb, const int* row, const int* col, const int* diag, int lower,
                  long long ndeps_max, int* order, int* lvl_ptr, int* nlev_d, int* h_nlev,
                  Carver& ws, cudaStream_t st, int* h_sched = nullptr, int* h_maxdeg = nullptr,
                  int* h_fsched = nullptr) {
-  int* sptr = ws.take<int>((size_t)nb + 1);
-  int* cursor = ws.take<int>((size_t)nb + 1);
-  int* indeg = ws.take<int>((size_t)nb + 1);
-  int* sidx = ws.take<int>((size_t)std::max(ndeps_max, 1ll));
-  // tail[1]: the largest dependency count (k_dep_count); tail[4..6]: the
-  // breadth-first sweep's append counters
-  int* tail = ws.take<int>(8);
-  if (!sptr || !cursor || !indeg || !sidx || !tail) return BILU_ERR_WORKSPACE;
-  GridSync gs;
-  BILU_TRY(grid_sync_init(gs, ws, st));
-  BILU_TRY_CUDA(cudaMemsetAsync(sptr, 0, sizeof(int) * ((size_t)nb + 1), st));
-  BILU_TRY_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * ((size_t)nb + 1), st));
-  BILU_TRY_CUDA(cudaMemsetAsync(tail, 0, sizeof(int) * 8, st));
-  BILU_TRY_CUDA(cudaMemsetAsync(nlev_d, 0, sizeof(int) * 4, st));
-  BILU_TRY_CUDA(cudaMemsetAsync(lvl_ptr, 0, sizeof(int) * ((size_t)nb + 2), st));
   if (nb == 0) {
+    BILU_TRY_CUDA(cudaMemsetAsync(nlev_d, 0, sizeof(int) * 4, st));
+    BILU_TRY_CUDA(cudaMemsetAsync(lvl_ptr, 0, sizeof(int) * 2, st));
     if (h_nlev) *h_nlev = 0;
     if (h_maxdeg) *h_maxdeg = 0;
     return BILU_OK;
   }
-  k_dep_count<<<ceil_div(nb, 256), 256, 0, st>>>(nb, row, col, diag, lower, sptr, indeg,
-                                                  tail + 1);
-  BILU_LAUNCH_CHECK();
-  int total = 0;
-  BILU_TRY(scan_exclusive(sptr, sptr, nb, &total, ws, st));
-  if (total > ndeps_max) return BILU_ERR_WORKSPACE;
-  k_dep_fill<<<ceil_div(nb, 256), 256, 0, st>>>(nb, row, col, diag, lower, sptr, cursor, sidx);
-  BILU_LAUNCH_CHECK();
-  // two CTAs per SM at most: a level's frontier is small, the barrier's
-  // cost grows with the number of CTAs
-  int grid = std::min<long long>(std::min(coop_grid((const void*)k_bfs_levels, 256),
-                                          2 * sm_count()),
-                                 ceil_div(nb, 256));
-  int* cnt = tail + 4;
-  void* args[] = {&nb, &sptr, &sidx, &indeg, &order, &lvl_ptr, &cnt, &nlev_d, &gs};
-  BILU_TRY(launch_coop((const void*)k_bfs_levels, grid, 256, args, st));
-  int herr = grid_sync_finish(gs, st);
-  if (herr != 0) return herr;
-  int h[2] = {0, 0};
-  BILU_TRY_CUDA(cudaMemcpyAsync(&h[0], nlev_d, sizeof(int), cudaMemcpyDeviceToHost, st));
+  LevelWords *w = nullptr, hw;
+  BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st));
+  int rec[4];
+  BILU_TRY_CUDA(cudaMemcpyAsync(&hw, w, sizeof(hw), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaMemcpyAsync(rec, nlev_d, sizeof(rec), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
-  BILU_TRY_CUDA(cudaMemcpyAsync(&h[1], lvl_ptr + h[0], sizeof(int), cudaMemcpyDeviceToHost, st));
-  BILU_TRY_CUDA(cudaStreamSynchronize(st));
-  if (h[1] != nb) return BILU_ERR_PATTERN;  // a row was never reached
-  if (h_nlev) *h_nlev = h[0];
-  if (h[0] > 0) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      BILU_TRY_CUDA(cudaFuncSetAttribute((const void*)k_sort_levels,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kSortCap * sizeof(int))));
-      attr_set = true;
-    }
-    k_sort_levels<<<(unsigned)h[0], 512, kSortCap * sizeof(int), st>>>(order, lvl_ptr);
-    BILU_LAUNCH_CHECK();
+  if (hw.err != 0) return hw.err;
+  if (hw.ndeps > (unsigned long long)ndeps_max) return BILU_ERR_WORKSPACE;
+  if (h_nlev) *h_nlev = rec[0];
+  if (h_maxdeg) *h_maxdeg = rec[1];
+  if (h_sched) *h_sched = rec[2];
+  if (h_fsched) *h_fsched = rec[3];
+  static bool attr_set = false;
+  if (!attr_set) {
+    BILU_TRY_CUDA(cudaFuncSetAttribute((const void*)k_sort_levels,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kSortCap * sizeof(int))));
+    attr_set = true;
   }
-  // nlev_d[1] = the largest dependency count (picks warp or group rows);
-  // nlev_d[2] = the recommended schedule (0 level, 1 sync-free)
-  BILU_TRY_CUDA(cudaMemcpyAsync(nlev_d + 1, tail + 1, sizeof(int), cudaMemcpyDeviceToDevice, st));
-  int maxdeg = 0;
-  BILU_TRY_CUDA(cudaMemcpy(&maxdeg, tail + 1, sizeof(int), cudaMemcpyDeviceToHost));
-  // nlev_d[2] = the recommended solve schedule, nlev_d[3] the recommended
-  // factorisation schedule (0 level order, 1 sync-free)
-  int sched[2] = {maxdeg > kFlowMaxDeps ? 1 : 0,
-                  ((long long)nb < (long long)kFactorLevelWidth * h[0] || maxdeg > kLongRow) ? 1
-                                                                                            : 0};
-  BILU_TRY_CUDA(cudaMemcpy(nlev_d + 2, sched, sizeof(sched), cudaMemcpyHostToDevice));
-  if (h_sched) *h_sched = sched[0];
-  if (h_fsched) *h_fsched = sched[1];
-  if (h_maxdeg) *h_maxdeg = maxdeg;
+  k_sort_levels<<<(unsigned)rec[0], 512, kSortCap * sizeof(int), st>>>(order, lvl_ptr);
+  BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
 
@@ -2058,25 +2063,24 @@ size_t syncfree_ws(int nb) {
          carve_size(sizeof(int) * 2) + scan_ws_bytes(nb + 1);
 }
 
-// Level analysis scratch (successor lists of up to ndeps dependencies).
-size_t levels_ws(int nb, long long ndeps) {
-  return carve_size(sizeof(int) * ((size_t)nb + 1)) * 3 +
-         carve_size(sizeof(int) * (size_t)std::max(ndeps, 1ll)) + carve_size(sizeof(int) * 8) +
-         carve_size(sizeof(unsigned) * 4) + scan_ws_bytes(nb + 1);
+// Level analysis scratch: levels, level sizes, words, scan sums.
+size_t levels_ws(int nb) {
+  return carve_size(sizeof(int) * ((size_t)nb + 1)) * 2 + carve_size(sizeof(LevelWords)) +
+         scan_ws_bytes(nb + 1);
 }
 
 // Level-scheduled factor / solve scratch: the analysis output (order,
 // lvl_ptr, nlev), the analysis scratch, and the error / barrier words.
-size_t level_sched_ws(int nb, long long nnzb) {
+size_t level_sched_ws(int nb) {
   return carve_size(sizeof(int) * ((size_t)nb + 1)) + carve_size(sizeof(int) * ((size_t)nb + 2)) +
-         carve_size(sizeof(int) * 2) + levels_ws(nb, std::max(nnzb - nb, 0ll)) +
+         carve_size(sizeof(int) * 4) + levels_ws(nb) + carve_size(sizeof(int) * ((size_t)nb + 1)) +
          carve_size(sizeof(int) * 4) + carve_size(sizeof(unsigned) * 4);
 }
 
 // BILU(0) scratch: the level-scheduled one plus the sync-free schedule's
 // per-position match counts.
 size_t bilu0_ws(int nb, long long nnzb) {
-  return level_sched_ws(nb, nnzb) + carve_size(sizeof(int) * (size_t)std::max(nnzb, 1ll));
+  return level_sched_ws(nb) + carve_size(sizeof(int) * (size_t)std::max(nnzb, 1ll));
 }
 
 // diagonal positions (validates the pattern); returns BILU_ERR_PATTERN with
@@ -2406,7 +2410,7 @@ extern "C" size_t bilu_sptrsv_analysis_bytes(int nb) {
 
 extern "C" size_t bilu_sptrsv_analysis_ws_bytes(int nb, int nnzb) {
   if (nb < 0 || nnzb < 0) return 0;
-  return levels_ws(nb, std::max((long long)nnzb - nb, 0ll)) + carve_size(sizeof(int) * 2);
+  return levels_ws(nb) + carve_size(sizeof(int) * 2);
 }
 
 extern "C" size_t bilu_sptrsv_solve_ws_bytes(int nb) {
@@ -2511,7 +2515,7 @@ extern "C" int bilu_bsrilu0_ex(int nb, int nnzb, int bs, const int* d_row, const
 extern "C" size_t bilu_sptrsv_ws_bytes(int nb, int nnzb) {
   if (nb < 0 || nnzb < 0) return 0;
   return carve_size(sizeof(int) * ((size_t)nb + 1)) + carve_size(sizeof(int) * 2) +
-         level_sched_ws(nb, nnzb);
+         level_sched_ws(nb);
 }
 
 extern "C" int bilu_sptrsv(int nb, int nnzb, int bs, const int* d_row, const int* d_col,

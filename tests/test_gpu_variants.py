@@ -63,3 +63,78 @@ def test_csr_to_bsr_column_out_of_range(cuda, bad):
     col[50] = bad
     with pytest.raises(api.BiluError):
         api.csr_to_bsr5(40, 5, T(rp, cuda), T(col, cuda), T(np.ones(80), cuda))
+
+
+# ------------------------------------------------------------------ level analysis
+def pattern_of(rows):
+    """rowptr, col of a block pattern given as one set of columns per row."""
+    cols = [np.array(sorted(set(r) | {i}), np.int32) for i, r in enumerate(rows)]
+    rp = np.zeros(len(rows) + 1, np.int32)
+    np.cumsum([len(c) for c in cols], out=rp[1:])
+    return rp, np.concatenate(cols)
+
+
+def level_pattern(name):
+    rng = np.random.default_rng(11)
+    if name == "chain":  # every row waits for a row of its own warp
+        return pattern_of([[i - 1, i + 1] if 0 < i < 99 else [] for i in range(100)])
+    if name == "grid":  # grid lines that straddle the warps
+        A = gen.laplace2d(21, bs=4)
+        return A.rowptr, A.colind
+    if name == "dense":  # rows of more dependencies than a warp takes at once
+        return pattern_of([range(97) for _ in range(97)])
+    if name == "hubs":  # hub rows among short ones, hubs waiting for hubs
+        n = 333
+        return pattern_of([rng.integers(0, n, size=200 if i % 31 == 5 else 5) for i in range(n)])
+    if name == "diagonal":
+        return pattern_of([[] for _ in range(65)])
+    return pattern_of([rng.integers(0, 4000, size=9) for _ in range(4000)])  # "random"
+
+
+@pytest.mark.parametrize("lower", [1, 0])
+@pytest.mark.parametrize("name", ["chain", "grid", "dense", "hubs", "diagonal", "random"])
+def test_level_analysis(cuda, name, lower):
+    """The analysis record against longest paths on the host: the rows by
+    (level, index), the level bounds, the level count and the largest
+    dependency count."""
+    from isai_kernel_gb300 import _lib, api
+
+    rp, col = level_pattern(name)
+    nb, nnzb = len(rp) - 1, len(col)
+    level = np.zeros(nb, np.int64)
+    deg = 0
+    for i in (range(nb) if lower else range(nb - 1, -1, -1)):
+        c = col[rp[i]:rp[i + 1]]
+        c = c[c < i] if lower else c[c > i]
+        deg = max(deg, len(c))
+        level[i] = 1 + level[c].max() if len(c) else 0
+    L = _lib.lib()
+    info = api._ws(L.bilu_sptrsv_analysis_bytes(nb), cuda)
+    ws = api._ws(L.bilu_sptrsv_analysis_ws_bytes(nb, nnzb), cuda)
+    r, c = T(rp, cuda), T(col, cuda)
+    api.call("bilu_sptrsv_analysis", nb, nnzb, 4, api._p(r), api._p(c), lower, api._p(info),
+             api._p(ws), ws.numel(), api._s())
+    words = N(info).view(np.int32)
+    up = lambda k: (k + 63) // 64 * 64  # 256-byte steps in int32 words
+    o1 = up(nb + 1)
+    o2 = o1 + up(nb + 1)
+    o3 = o2 + up(nb + 2)
+    nlev = int(level.max()) + 1
+    assert words[o3] == nlev and words[o3 + 1] == deg
+    bounds = np.zeros(nlev + 1, np.int64)
+    np.cumsum(np.bincount(level, minlength=nlev), out=bounds[1:])
+    assert np.array_equal(words[o2:o2 + nlev + 1], bounds)
+    assert np.array_equal(words[o1:o1 + nb], np.lexsort((np.arange(nb), level)))
+    # one dependency more than the caller's block count leaves room for
+    st = L.bilu_sptrsv_analysis(nb, nnzb - 1, 4, api._p(r), api._p(c), lower, api._p(info),
+                                api._p(ws), ws.numel(), api._s())
+    deps = int(sum(((col[rp[i]:rp[i + 1]] < i) if lower else (col[rp[i]:rp[i + 1]] > i)).sum()
+                   for i in range(nb)))
+    assert st == (0 if nnzb - 1 >= nb and deps <= nnzb - 1 - nb else
+                  _lib_status("BILU_ERR_WORKSPACE" if nnzb - 1 >= nb else "BILU_ERR_ARG"))
+
+
+def _lib_status(name):
+    from isai_kernel_gb300 import _lib
+
+    return {v: k for k, v in _lib.STATUS.items()}[name]
