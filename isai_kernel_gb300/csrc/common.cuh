@@ -128,6 +128,10 @@ struct LevelOut {
   // positions mptr[p] .. mptr[p+1] of mpair for block position p
   const int* mptr = nullptr;
   const int2* mpair = nullptr;
+  // BILU(0)'s plan, one entry per stored block (k_bilu0_plan), and whether the
+  // pattern takes the row flow
+  int2* plan = nullptr;
+  int h_rowflow = 0;
 };
 
 }  // namespace bilu

@@ -1,6 +1,9 @@
 // BILU(0) and block triangular solves on the dependency DAG (sm_103a):
 //
-//   bsrilu02_inplace (bsrilu.h:20, cuSPARSE bsrilu02)   -> k_bilu0_levels
+//   bsrilu02_inplace (bsrilu.h:20, cuSPARSE bsrilu02)   -> k_bilu0_rowflow,
+//                                                            k_bilu0_blocks,
+//                                                            k_bilu0_levels,
+//                                                            k_bilu0_syncfree
 //   spTrSolveL / spTrSolveU (cape_sptrsv.h:8,55)         -> k_sptrsv_levels,
 //                                                            k_sptrsv (sync-free)
 //
@@ -385,6 +388,7 @@ struct LevelWords {
   int ticket, err;           // next 32 rows; 0 or a bilu_status
   int maxdeg, nlev;          // largest dependency count of a row; levels
   unsigned long long ndeps;  // dependencies of all rows
+  int other;                 // k_bilu0_plan: the pattern is not one for the row flow
 };
 
 __device__ __forceinline__ void st_relaxed(int* p, int v) {
@@ -1223,8 +1227,8 @@ __device__ __forceinline__ void bilu0_grow(const BRowPre& pr, const int* __restr
   }
 }
 
-// One block row with a whole warp (the sync-free factorisation, used for
-// matrices with long rows or narrow levels).  WAIT: the rows K it reads may
+// One block row with a whole warp (the sync-free factorisation of patterns with
+// triangles, narrow levels and no row of more than kLongRow dependencies).  WAIT: the rows K it reads may
 // still be in progress and are waited for through their flags.  Phase 1 by
 // the whole warp (PL lanes per row of L_IK), or for runs of dependencies
 // without updates by a lane group each; phase 2 with teams of lanes per
@@ -1514,6 +1518,438 @@ __device__ __forceinline__ bool bilu0_wrow(int I, const int* __restrict__ row,
   return true;
 }
 
+// ------------------------------------------------------------------ row flow
+// BILU(0) in level order without grid barriers, for patterns in which a
+// dependency K of row I updates the diagonal block of row I and nothing else
+// (k_bilu0_plan: 5- and 7-point stencils, any pattern without triangles).  The
+// dependencies of a row are then independent of one another, and a row is a
+// fixed sequence for a team of T lanes (16 at block size 4: two rows a warp;
+// else the warp):
+//   L_IK = A_IK U_KK^-1 for NQ = T / BS dependencies at once, lane (q, r)
+//     holding row r of the q-th block,
+//   A_II -= L_IK U_KI, a lane (or two slots of one) per element, K ascending,
+//   the LU of A_II on the same elements,
+//   U_IJ = L_II^-1 A_IJ for NQ blocks at once, lane (q, c) holding column c.
+// Every operation and its order per element are those of bilu0_grow.
+//
+// What bounds a row is its chain of FP64 warp instructions (about 64 cycles
+// each on GB300 whatever the lanes: 10 + 12 + ~40 + 6 at block size 4, half of
+// what a lane per matrix row takes) and one release-to-acquire hop, so the
+// split spends lanes, not instructions.  Rows are dealt statically in level
+// order as in k_sptrsv_flow (the rows of one warp sit in one level and never
+// wait for each other; all warps are resident, so every wait ends); the next
+// row's blocks and the structure of the one after it are loaded before the
+// current row waits.  A row's flag is released as soon as U_II, U_IJ and the
+// reciprocal pivots are stored; its L blocks, which no other row reads, follow.
+// Measured, analysis included, against the schedules before it
+// (block size 4): 64^3 7-point 4.3 -> 1.6 ms, 128^3 11.5 -> 6.6 ms, 256 x 256
+// 5-point 7.7 -> 2.8 ms; block size 8: 64^3 6.1 -> 4.2 ms.
+template <int BS>
+struct RowFlow {
+  static constexpr int T = BS == 4 ? 16 : 32;              // lanes per row
+  static constexpr int NR = 32 / T;                        // rows per warp
+  static constexpr int NQ = T / BS;                        // blocks at once
+  static constexpr int EPL = (BS * BS + T - 1) / T;        // diagonal elements per lane
+  int I, rs, re, dI;  // I < 0: no row
+  int K;              // this lane's dependency (q-th), -1: none
+  int2 pl;            // its plan: diagonal position of row K, position of U_KI (or < 0)
+  double a[BS];       // row r of A_IK
+  double u[BS];       // column r of the q-th block right of the diagonal
+  double d[EPL];      // elements of the diagonal block
+};
+
+// Lane (q, r)'s part of the dependencies [p0, p0 + NQ) of a row.
+template <int BS>
+__device__ __forceinline__ void rowflow_low(RowFlow<BS>& w, int p0, int q, int r, bool on,
+                                            const int* __restrict__ col,
+                                            const int2* __restrict__ plan, const double* val) {
+  const int p = w.rs + p0 + q;
+  const bool has = on && w.I >= 0 && p < w.dI;
+  w.K = has ? __ldg(col + p) : -1;
+  w.pl = has ? __ldg(plan + p) : make_int2(0, -1);
+  const double* b = val + ((long long)(has ? p : 0) * BS + r) * BS;
+#pragma unroll
+  for (int c = 0; c < BS; ++c) w.a[c] = has ? b[c] : 0.0;
+}
+
+template <int BS>
+__device__ __forceinline__ void rowflow_up(RowFlow<BS>& w, int p0, int q, int r, bool on,
+                                           const double* val) {
+  const int p = w.dI + 1 + p0 + q;
+  const bool has = on && w.I >= 0 && p < w.re;
+  const double* b = val + (long long)(has ? p : 0) * BS * BS + r;
+#pragma unroll
+  for (int k = 0; k < BS; ++k) w.u[k] = has ? b[k * BS] : 0.0;
+}
+
+template <int BS>
+__device__ __forceinline__ void rowflow_load(int I, const GRowMeta& m, RowFlow<BS>& w, int tl,
+                                             int q, int r, bool on, const int* __restrict__ col,
+                                             const int2* __restrict__ plan, const double* val) {
+  using F = RowFlow<BS>;
+  w.I = I;
+  w.rs = m.rs;
+  w.re = m.re;
+  w.dI = m.dI;
+  rowflow_low<BS>(w, 0, q, r, on, col, plan, val);
+  rowflow_up<BS>(w, 0, q, r, on, val);
+#pragma unroll
+  for (int x = 0; x < F::EPL; ++x) {
+    const int e = tl + x * F::T;
+    w.d[x] = I >= 0 && e < BS * BS ? val[(long long)m.dI * BS * BS + e]
+                                   : (e % (BS + 1) == 0 ? 1.0 : 0.0);
+  }
+}
+
+// One row per team; false (in every lane) if the launch aborted.
+template <int BS>
+__device__ __forceinline__ bool rowflow_finish(RowFlow<BS>& w, int tl, int tb, int q, int r,
+                                               bool on, const int* __restrict__ col,
+                                               const int2* __restrict__ plan, double* val,
+                                               const SyncState& ss) {
+  using F = RowFlow<BS>;
+  constexpr int T = F::T, NQ = F::NQ, EPL = F::EPL, BS2 = BS * BS;
+  int er[EPL], ec[EPL];
+#pragma unroll
+  for (int x = 0; x < EPL; ++x) {
+    const int e = tl + x * T;
+    er[x] = e < BS2 ? e / BS : 0;
+    ec[x] = e < BS2 ? e % BS : 0;
+  }
+  const int nlow = w.I >= 0 ? w.dI - w.rs : 0, nup = w.I >= 0 ? w.re - w.dI - 1 : 0;
+  const int most_low = __reduce_max_sync(FULL, nlow);
+  const int most_up = __reduce_max_sync(FULL, nup);
+  for (int p0 = 0; p0 < most_low; p0 += NQ) {
+    if (p0 > 0) rowflow_low<BS>(w, p0, q, r, on, col, plan, val);
+    // the rows this pass reads
+    bool wait = w.K >= 0;
+    long long n = 0;
+    unsigned ns = 32;
+    while (true) {
+      if (wait) wait = ld_relaxed(ss.flags + w.K) == 0;
+      if (!__any_sync(FULL, wait)) break;
+      if (++n > ss.spin) {
+        if ((threadIdx.x & 31) == 0) atomicCAS(ss.err, 0, (int)BILU_ERR_TIMEOUT);
+        return false;
+      }
+      if ((n & 31) == 0 && __any_sync(FULL, ld_relaxed(ss.err) != 0)) return false;
+      if (n > kFlowSpin) backoff(ns);
+    }
+    fence_acquire();
+    __syncwarp();  // every lane's reads after every lane's fence
+    // U_KI for the diagonal update: column ec of every dependency's block
+    // (every slot of a lane has the same column)
+    int pu[NQ];
+    double uk[NQ][BS];
+#pragma unroll
+    for (int x = 0; x < NQ; ++x) {
+      pu[x] = __shfl_sync(FULL, w.pl.y, tb + x * BS);
+      const double* b = val + (long long)max(pu[x], 0) * BS2 + ec[0];
+#pragma unroll
+      for (int k = 0; k < BS; ++k) uk[x][k] = pu[x] >= 0 ? __ldcg(b + k * BS) : 0.0;
+    }
+    if (w.K >= 0) {
+      const double* ukk = val + (long long)w.pl.x * BS2;
+      const double* rk = ss.rdiag + (long long)w.K * BS;
+#pragma unroll
+      for (int k = 0; k < BS; ++k) {
+        w.a[k] = w.a[k] * __ldcg(rk + k);
+#pragma unroll
+        for (int c = k + 1; c < BS; ++c) w.a[c] -= w.a[k] * __ldcg(ukk + k * BS + c);
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < NQ; ++x) {
+      if (!__any_sync(FULL, pu[x] >= 0)) continue;
+#pragma unroll
+      for (int m = 0; m < EPL; ++m) {
+        double v = w.d[m];
+#pragma unroll
+        for (int k = 0; k < BS; ++k) {
+          const double l = __shfl_sync(FULL, w.a[k], tb + x * BS + er[m]);
+          v -= l * uk[x][k];
+        }
+        if (pu[x] >= 0) w.d[m] = v;
+      }
+    }
+    if (p0 + NQ < most_low && w.K >= 0) {  // more passes: this one's L now
+      double* b = val + ((long long)(w.rs + p0 + q) * BS + r) * BS;
+#pragma unroll
+      for (int c = 0; c < BS; ++c) b[c] = w.a[c];
+      w.K = -1;
+    }
+  }
+  // LU of the diagonal block on its elements (bilu0_diag_lu's operations)
+  double rp = 0.0;
+#pragma unroll
+  for (int k = 0; k < BS; ++k) {
+    const double rk = 1.0 / __shfl_sync(FULL, w.d[k * (BS + 1) / T], tb + k * (BS + 1) % T);
+    if (tl == k * (BS + 1) % T) rp = rk;
+#pragma unroll
+    for (int m = 0; m < EPL; ++m)
+      if (ec[m] == k && er[m] > k) w.d[m] *= rk;
+    double ukc[EPL], lrk[EPL];
+#pragma unroll
+    for (int m = 0; m < EPL; ++m) {
+      // (k, ec) sits in slot k BS / T, (er, k) in this slot
+      ukc[m] = __shfl_sync(FULL, w.d[k * BS / T], tb + (k * BS + ec[m]) % T);
+      lrk[m] = __shfl_sync(FULL, w.d[m], tb + (er[m] * BS + k) % T);
+    }
+#pragma unroll
+    for (int m = 0; m < EPL; ++m)
+      if (er[m] > k && ec[m] > k) w.d[m] -= lrk[m] * ukc[m];
+  }
+  // columns right of the diagonal
+  for (int p0 = 0; p0 < most_up || p0 == 0; p0 += NQ) {
+    if (p0 > 0) rowflow_up<BS>(w, p0, q, r, on, val);
+#pragma unroll
+    for (int i = 1; i < BS; ++i)
+#pragma unroll
+      for (int k = 0; k < i; ++k)
+        w.u[i] -= __shfl_sync(FULL, w.d[(i * BS + k) / T], tb + (i * BS + k) % T) * w.u[k];
+    if (on && p0 + q < nup) {
+      double* b = val + (long long)(w.dI + 1 + p0 + q) * BS2 + r;
+#pragma unroll
+      for (int k = 1; k < BS; ++k) b[k * BS] = w.u[k];
+    }
+  }
+  if (w.I >= 0) {
+#pragma unroll
+    for (int m = 0; m < EPL; ++m) {
+      const int e = tl + m * T;
+      if (e < BS2) {
+        val[(long long)w.dI * BS2 + e] = w.d[m];
+        if (e % (BS + 1) == 0) {
+          ss.rdiag[(long long)w.I * BS + e / (BS + 1)] = rp;
+          if (w.d[m] == 0.0) atomicMin(ss.zp, w.I);
+        }
+      }
+    }
+  }
+  __syncwarp();  // the team's stores before its first lane's release
+  if (tl == 0 && w.I >= 0) st_release(ss.flags + w.I, 1);
+  if (w.K >= 0) {  // the last pass's L blocks
+    double* b = val + ((long long)(w.rs + (nlow - 1) / NQ * NQ + q) * BS + r) * BS;
+#pragma unroll
+    for (int c = 0; c < BS; ++c) b[c] = w.a[c];
+  }
+  return true;
+}
+
+template <int BS>
+__global__ void __launch_bounds__(kLvlThreads, BS == 4 ? 2 : 1) k_bilu0_rowflow(
+    const int* __restrict__ row, const int* __restrict__ col, const int* __restrict__ diag,
+    double* val, const int* __restrict__ order, const int* __restrict__ lvl_ptr,
+    const int* __restrict__ nlev_p, const int2* __restrict__ plan, SyncState ss, int per_sm) {
+  using F = RowFlow<BS>;
+  const int lane = threadIdx.x & 31, team = lane / F::T, tl = lane % F::T, tb = team * F::T;
+  const int q = tl / BS, r = tl % BS;
+  const bool on = q < F::NQ;
+  const int warp = spread_warp(per_sm);
+  const int nw = (int)(((long long)gridDim.x * blockDim.x) >> 5);
+  const long long ngrp = (long long)nw * F::NR, first = (long long)warp * F::NR;
+  const int nlev = __ldg(nlev_p);
+  if (nlev <= 0) return;
+  RowCursor c0{0, __ldg(lvl_ptr) + first}, c1 = c0;
+  cursor_next(c1, nlev, first, ngrp, lvl_ptr);
+  RowCursor c2 = c1;
+  cursor_next(c2, nlev, first, ngrp, lvl_ptr);
+  RowCursor c3 = c2;
+  cursor_next(c3, nlev, first, ngrp, lvl_ptr);
+  auto row_at = [&](const RowCursor& c) {
+    return cursor_row(c, team, true, nlev, order, lvl_ptr);
+  };
+  F cur;
+  {
+    GRowMeta m;
+    const int I = row_at(c0);
+    grow_meta(I, row, diag, m);
+    rowflow_load<BS>(I, m, cur, tl, q, r, on, col, plan, val);
+  }
+  int I1 = row_at(c1);
+  GRowMeta m1;
+  grow_meta(I1, row, diag, m1);
+  int I2 = row_at(c2);
+  while (c0.l < nlev) {
+    F nxt;
+    rowflow_load<BS>(I1, m1, nxt, tl, q, r, on, col, plan, val);
+    GRowMeta m2;
+    grow_meta(I2, row, diag, m2);
+    const int I3 = row_at(c3);
+    if (__any_sync(FULL, cur.I >= 0)) {
+      if (!rowflow_finish<BS>(cur, tl, tb, q, r, on, col, plan, val, ss)) return;
+    }
+    cur = nxt;
+    m1 = m2;
+    I1 = I2;
+    I2 = I3;
+    c0 = c1;
+    c1 = c2;
+    c2 = c3;
+    cursor_next(c3, nlev, first, ngrp, lvl_ptr);
+  }
+}
+
+// Sync-free BILU(0) over single blocks (patterns with rows of more than
+// kLongRow dependencies).  A task is one stored block (I, J), taken by a warp:
+//   A_IJ -= L_IK U_KJ for the K < min(I, J) stored in rows I and (as K, J) K,
+//     in ascending K,
+//   then L_IJ = A_IJ U_JJ^-1 (J < I), the LU of the diagonal block (J = I) or
+//   U_IJ = L_II^-1 A_IJ (J > I).
+// It waits for the blocks it reads through one ready flag per block (bounded
+// polls, one acquire fence), so the blocks of a row are as independent as the
+// arithmetic lets them be: a hub row of a power-law matrix has about a
+// thousand lower blocks of which a few hundred update another one, and a warp
+// (or CTA) that walks the row takes them one after another on the critical
+// path.  Tasks are dealt by ticket, rows in level order and a row's blocks in
+// column order, so every block a task reads belongs to an earlier ticket and
+// its warp is running.  tcnt[p] is the number of updates of block p
+// (structure only, k_bilu0_tcount): most blocks have none and search for
+// none; the others look J up in the rows K of the row's earlier blocks, 32 at a
+// time, until they have found tcnt.  The operations per element and their
+// order are those of bilu0_grow.  What bounds it is the chain of dependent
+// blocks (about 26 rows deep on the 20,011-row power-law pattern, 8x8 blocks):
+// 0.85 ms for the factorisation
+// (1.4 ms with its analysis), 6.5 ms (8.0) with a warp per block row.
+//
+// PL lanes per row (lower) or column (diagonal, upper) of the block, lane
+// (pr, pj) holding its elements pj + m PL.
+template <int BS>
+__global__ void __launch_bounds__(kLvlThreads, 3) k_bilu0_blocks(
+    int nb, const int* __restrict__ row, const int* __restrict__ col,
+    const int* __restrict__ diag, double* val, const int* __restrict__ order,
+    const int* __restrict__ tptr, const int* __restrict__ tcnt, int* flags, SyncState ss) {
+  constexpr int BS2 = BS * BS;
+  constexpr int PL = 32 / BS < BS ? 32 / BS : BS;
+  constexpr int PC = (BS + PL - 1) / PL;
+  const int lane = threadIdx.x & 31;
+  const int pr = lane / PL, pj = lane - pr * PL;
+  const bool p_on = pr < BS;
+  const int ntask = __ldg(tptr + nb);
+  while (true) {
+    int task = 0;
+    if (lane == 0) task = atomicAdd(ss.ticket, 1);
+    task = __shfl_sync(FULL, task, 0);
+    if (task >= ntask) return;
+    // the task's row: last t with tptr[t] <= task, 32 probes a round
+    int lo = 0, n = nb;
+    while (n > 1) {
+      const int step = (n + 31) / 32;
+      const int at = lo + lane * step;
+      const bool le = lane * step < n && __ldg(tptr + at) <= task;
+      const int k = 31 - __clz((int)__ballot_sync(FULL, le));
+      n = min(step, n - k * step);
+      lo += k * step;
+    }
+    const int I = __ldg(order + lo);
+    const int rs = __ldg(row + I), dI = __ldg(diag + I);
+    const int p = rs + task - __ldg(tptr + lo);
+    const int J = __ldg(col + p);
+    const bool low = p < dI;
+    // element (er, ec) of slot m
+    int er[PC], ec[PC];
+    bool on[PC];
+    double a[PC];
+    double* blk = val + (long long)p * BS2;
+#pragma unroll
+    for (int m = 0; m < PC; ++m) {
+      const int q = pj + m * PL;
+      on[m] = p_on && q < BS;
+      const int x = p_on ? pr : 0, y = q < BS ? q : 0;
+      er[m] = low ? x : y;
+      ec[m] = low ? y : x;
+      a[m] = on[m] ? blk[er[m] * BS + ec[m]] : 1.0;
+    }
+    int left = __ldg(tcnt + p);
+    const int pe = min(p, dI);
+    for (int c0 = rs; left > 0 && c0 < pe; c0 += 32) {
+      int at = -1;
+      if (c0 + lane < pe) {
+        const int K = __ldg(col + c0 + lane);
+        at = find_in_row(col, __ldg(diag + K) + 1, __ldg(row + K + 1), J);
+      }
+      unsigned found = __ballot_sync(FULL, at >= 0);
+      left -= __popc(found);
+      while (found) {
+        const int bit = __ffs(found) - 1;
+        found &= found - 1;
+        const int pk = c0 + bit, pu = __shfl_sync(FULL, at, bit);
+        if (!warp_wait(lane & 1 ? flags + pu : flags + pk, ss.err, ss.spin)) return;
+        const double* L = val + (long long)pk * BS2;
+        const double* U = val + (long long)pu * BS2;
+#pragma unroll
+        for (int m = 0; m < PC; ++m) {
+          double v = a[m];
+#pragma unroll
+          for (int k = 0; k < BS; ++k)
+            v -= __ldcg(L + er[m] * BS + k) * __ldcg(U + k * BS + ec[m]);
+          if (on[m]) a[m] = v;
+        }
+      }
+    }
+    if (low) {
+      const int dJ = __ldg(diag + J);
+      if (!warp_wait(flags + dJ, ss.err, ss.spin)) return;
+      // row pr of L_IJ = A_IJ U_JJ^-1: step k scales column k by the
+      // reciprocal pivot, broadcasts it along the row and updates the columns
+      // right of it (slots whose columns are all <= k are skipped at compile
+      // time); every operand is loaded up front, unpredicated
+      const double* Ujj = val + (long long)dJ * BS2;
+      const double* rJ = ss.rdiag + (long long)J * BS;
+      double rkv[PC], u[BS][PC];
+#pragma unroll
+      for (int m = 0; m < PC; ++m) {
+        rkv[m] = __ldcg(rJ + ec[m]);
+#pragma unroll
+        for (int k = 0; k < BS; ++k)
+          u[k][m] = m * PL + PL - 1 <= k ? 0.0 : __ldcg(Ujj + k * BS + ec[m]);
+      }
+#pragma unroll
+      for (int k = 0; k < BS; ++k) {
+        const int mk = k / PL, jk = k - mk * PL;
+        if (pj == jk) a[mk] = a[mk] * rkv[mk];
+        const double ak = __shfl_sync(FULL, a[mk], (pr * PL + jk) & 31);
+#pragma unroll
+        for (int m = 0; m < PC; ++m) {
+          if (m * PL + PL - 1 <= k) continue;  // every column of slot m is final
+          if (pj + m * PL > k) a[m] -= ak * u[k][m];
+        }
+      }
+    } else if (p == dI) {
+      double rp, piv;
+      bilu0_diag_lu_warp<BS, PL>(a, pr, pj, rp, piv);
+      if (pr < BS && pj == pr % PL) {
+        if (piv == 0.0) atomicMin(ss.zp, I);
+        ss.rdiag[(long long)I * BS + pr] = rp;
+      }
+    } else {
+      // column pr of U_IJ = L_II^-1 A_IJ
+      if (!warp_wait(flags + dI, ss.err, ss.spin)) return;
+      const double* D = val + (long long)dI * BS2;
+      double l[BS][PC];
+#pragma unroll
+      for (int m = 0; m < PC; ++m)
+#pragma unroll
+        for (int k = 0; k < BS - 1; ++k)
+          l[k][m] = m * PL + PL - 1 <= k ? 0.0 : __ldcg(D + er[m] * BS + k);
+#pragma unroll
+      for (int k = 0; k < BS - 1; ++k) {
+        const int mk = k / PL, jk = k - mk * PL;
+        const double uk = __shfl_sync(FULL, a[mk], (pr * PL + jk) & 31);
+#pragma unroll
+        for (int m = 0; m < PC; ++m) {
+          if (m * PL + PL - 1 <= k) continue;  // every row of slot m is final
+          if (pj + m * PL > k) a[m] -= l[k][m] * uk;
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < PC; ++m)
+      if (on[m]) blk[er[m] * BS + ec[m]] = a[m];
+    __syncwarp();  // the warp's stores before lane 0's release
+    if (lane == 0) st_release(flags + p, 1);
+  }
+}
 
 template <int BS>
 __global__ void __launch_bounds__(kLvlThreads, 2) k_bilu0_levels(
@@ -1673,8 +2109,8 @@ int launch_sptrsv(int nb, const int* row, const int* col, const int* diag, const
 // J > K present in both rows, i.e. the blocks dependency K updates in row I
 // (0 at the other positions).  Structure only and free of dependencies; the
 // same shorter-list searches as the factorisation.  On graphs with few
-// triangles most counts are 0, and the sync-free factorisation then skips
-// those searches inside its dependency chains.
+// triangles most counts are 0, and the sync-free factorisation by rows then
+// skips those searches inside its dependency chains.
 //
 // Pass 1: a thread per position (its block row found by binary search over
 // the row pointers, so that the thousand dependencies of a hub row spread
@@ -1711,33 +2147,46 @@ __device__ __forceinline__ MatchLists match_lists(long long pk, int nb,
   return m;
 }
 
+// TARGET false: nmatch[pk] = the count (the level-order factorisation's match
+// lists).  TARGET true: nmatch[p] += 1 for every updated block p (zeroed
+// before; the block-wise factorisation), and mark[pk] = 1 for the positions
+// left to pass 2.
+template <bool TARGET>
 __global__ void __launch_bounds__(256) k_bilu0_nmatch(int nb, long long nnzb,
                                                       const int* __restrict__ row,
                                                       const int* __restrict__ col,
                                                       const int* __restrict__ diag,
-                                                      int* __restrict__ nmatch) {
+                                                      int* __restrict__ nmatch,
+                                                      int* __restrict__ mark) {
   const long long pk = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (pk >= nnzb) return;
   int I;
   const MatchLists m = match_lists(pk, nb, row, col, diag, I);
-  if (m.ce - m.cs > kMatchSerial) {
-    nmatch[pk] = -1;
-    return;
-  }
+  const bool later = m.ce - m.cs > kMatchSerial;
+  if (TARGET) mark[pk] = later;
+  else if (later) nmatch[pk] = -1;
+  if (later) return;
   int n = 0;
-  for (int c = m.cs; c < m.ce; ++c) n += find_in_row(col, m.s, m.e, __ldg(col + c)) >= 0;
-  nmatch[pk] = n;
+  for (int c = m.cs; c < m.ce; ++c) {
+    const int o = find_in_row(col, m.s, m.e, __ldg(col + c));
+    n += o >= 0;
+    if (TARGET && o >= 0) atomicAdd(nmatch + (m.from_i ? c : o), 1);
+  }
+  if (!TARGET) nmatch[pk] = n;
 }
 
+template <bool TARGET>
 __global__ void __launch_bounds__(256) k_bilu0_nmatch_long(int nb, long long nnzb,
                                                            const int* __restrict__ row,
                                                            const int* __restrict__ col,
                                                            const int* __restrict__ diag,
-                                                           int* __restrict__ nmatch) {
+                                                           int* __restrict__ nmatch,
+                                                           const int* __restrict__ mark) {
   const long long p0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll;
   const int lane = threadIdx.x & 31;
   if (p0 >= nnzb) return;
-  unsigned todo = __ballot_sync(FULL, p0 + lane < nnzb && nmatch[p0 + lane] < 0);
+  unsigned todo = __ballot_sync(
+      FULL, p0 + lane < nnzb && (TARGET ? mark[p0 + lane] != 0 : nmatch[p0 + lane] < 0));
   while (todo) {
     const long long pk = p0 + __ffs(todo) - 1;
     todo &= todo - 1;
@@ -1746,11 +2195,49 @@ __global__ void __launch_bounds__(256) k_bilu0_nmatch_long(int nb, long long nnz
     int n = 0;
     for (int c0 = m.cs; c0 < m.ce; c0 += 32) {
       const int c = c0 + lane;
-      const bool hit = c < m.ce && find_in_row(col, m.s, m.e, __ldg(col + c)) >= 0;
-      n += __popc(__ballot_sync(FULL, hit));
+      const int o = c < m.ce ? find_in_row(col, m.s, m.e, __ldg(col + c)) : -1;
+      if (TARGET && o >= 0) atomicAdd(nmatch + (m.from_i ? c : o), 1);
+      n += __popc(__ballot_sync(FULL, o >= 0));
     }
-    if (lane == 0) nmatch[pk] = n;
+    if (!TARGET && lane == 0) nmatch[pk] = n;
   }
+}
+
+// len[t] = blocks of row order[t] (scanned into the tasks' row pointers)
+__global__ void k_order_len(int nb, const int* __restrict__ row, const int* __restrict__ order,
+                            int* __restrict__ len) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nb) return;
+  const int I = __ldg(order + t);
+  len[t] = __ldg(row + I + 1) - __ldg(row + I);
+}
+
+// The row flow's plan for every lower position pk = (I, K): the diagonal
+// position of row K and the position of U_KI in row K (-1: not stored).
+// *other is set when some dependency updates a block that is not the diagonal
+// of its row (or has a list too long to tell cheaply): the pattern then does
+// not take the row flow.
+__global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
+                                                    const int* __restrict__ row,
+                                                    const int* __restrict__ col,
+                                                    const int* __restrict__ diag,
+                                                    int2* __restrict__ plan, int* other) {
+  const long long pk = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pk >= nnzb) return;
+  int I;
+  const MatchLists m = match_lists(pk, nb, row, col, diag, I);
+  const int dI = __ldg(diag + I);
+  if (pk >= dI) return;
+  bool odd = m.ce - m.cs > kMatchSerial;
+  int at = -1;
+  for (int c = m.cs; c < m.ce && !odd; ++c) {
+    const int o = find_in_row(col, m.s, m.e, __ldg(col + c));
+    if (o < 0) continue;
+    odd = (m.from_i ? c : o) != dI;
+    at = m.from_i ? o : c;
+  }
+  plan[pk] = make_int2(__ldg(diag + __ldg(col + pk)), at);
+  if (odd) *other = 1;
 }
 
 // Total of the match counts in 64 bits (the caller decides from it whether
@@ -1827,10 +2314,9 @@ __global__ void __launch_bounds__(256) k_bilu0_match_fill_long(int nb, long long
   }
 }
 
-// Sync-free BILU(0) (matrices with narrow levels or long rows): block rows
-// taken by atomic tickets in level order, a warp per row, bounded waits on
-// the rows it reads, the row's flag released when it is final.  Hub rows of
-// a power-law matrix then no longer hold up a whole level.
+// Sync-free BILU(0) by block rows: rows taken by atomic tickets in level
+// order, a warp per row, bounded waits on the rows it reads, the row's flag
+// released when it is final.
 template <int BS>
 __global__ void __launch_bounds__(kLvlThreads, 3) k_bilu0_syncfree(
     int nb, const int* __restrict__ row, const int* __restrict__ col,
@@ -1847,8 +2333,7 @@ __global__ void __launch_bounds__(kLvlThreads, 3) k_bilu0_syncfree(
     const int I = __ldg(ss.order + t);
     if (__any_sync(FULL, ld_relaxed(ss.err) != 0)) return;
     if (!bilu0_wrow<BS, true>(I, row, col, diag, val, ss, stage)) return;
-    __threadfence();
-    __syncwarp();
+    __syncwarp();  // the warp's stores before lane 0's release
     if (lane == 0) st_release(ss.flags + I, 1);
   }
 }
@@ -1926,11 +2411,13 @@ int launch_coop(const void* fn, int grid, int threads, void** args, cudaStream_t
 // count, recommended solve and factorisation schedules: 0 level order, 1
 // sync-free) on the device; the same words on the host.  One host
 // synchronisation.  ndeps_max: the dependencies the caller's block count
-// leaves room for (BILU_ERR_WORKSPACE beyond it).
+// leaves room for (BILU_ERR_WORKSPACE beyond it).  plan (optional, lower DAG,
+// one entry per stored block): the row flow's plan; *h_rowflow whether the
+// pattern takes it.
 int build_levels(int nb, const int* row, const int* col, const int* diag, int lower,
                  long long ndeps_max, int* order, int* lvl_ptr, int* nlev_d, int* h_nlev,
                  Carver& ws, cudaStream_t st, int* h_sched = nullptr, int* h_maxdeg = nullptr,
-                 int* h_fsched = nullptr) {
+                 int* h_fsched = nullptr, int2* plan = nullptr, int* h_rowflow = nullptr) {
   if (nb == 0) {
     BILU_TRY_CUDA(cudaMemsetAsync(nlev_d, 0, sizeof(int) * 4, st));
     BILU_TRY_CUDA(cudaMemsetAsync(lvl_ptr, 0, sizeof(int) * 2, st));
@@ -1940,6 +2427,11 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
   }
   LevelWords *w = nullptr, hw;
   BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st));
+  if (plan) {
+    const long long nnzb = ndeps_max + nb;
+    k_bilu0_plan<<<ceil_div(nnzb, 256), 256, 0, st>>>(nb, nnzb, row, col, diag, plan, &w->other);
+    BILU_LAUNCH_CHECK();
+  }
   int rec[4];
   BILU_TRY_CUDA(cudaMemcpyAsync(&hw, w, sizeof(hw), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaMemcpyAsync(rec, nlev_d, sizeof(rec), cudaMemcpyDeviceToHost, st));
@@ -1950,6 +2442,7 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
   if (h_maxdeg) *h_maxdeg = rec[1];
   if (h_sched) *h_sched = rec[2];
   if (h_fsched) *h_fsched = rec[3];
+  if (h_rowflow) *h_rowflow = plan && !hw.other && rec[1] <= kLongRow ? 1 : 0;
   static bool attr_set = false;
   if (!attr_set) {
     BILU_TRY_CUDA(cudaFuncSetAttribute((const void*)k_sort_levels,
@@ -2044,6 +2537,34 @@ int launch_bilu0_syncfree(int nb, const int* row, const int* col, const int* dia
 }
 
 template <int BS>
+int launch_bilu0_rowflow(int nb, const int* row, const int* col, const int* diag, double* val,
+                         const int* order, const int* lvl_ptr, const int* nlev_d,
+                         const int2* plan, SyncState ss, cudaStream_t st) {
+  const void* fn = (const void*)k_bilu0_rowflow<BS>;
+  int grid = std::min<long long>(coop_grid(fn, kLvlThreads),
+                                 ceil_div(nb, (kLvlThreads / 32) * RowFlow<BS>::NR));
+  int per_sm = std::max(1, std::min(occupancy_per_sm(fn, kLvlThreads),
+                                    (int)ceil_div(grid, sm_count())));
+  void* args[] = {&row, &col, &diag, &val, &order, &lvl_ptr, &nlev_d, &plan, &ss, &per_sm};
+  return launch_coop(fn, grid, kLvlThreads, args, st);
+}
+
+template <int BS>
+int launch_bilu0_blocks(int nb, long long nnzb, const int* row, const int* col, const int* diag,
+                        double* val, const int* order, const int* tptr, const int* tcnt,
+                        int* flags, SyncState ss, cudaStream_t st) {
+  const void* fn = (const void*)k_bilu0_blocks<BS>;
+  // every warp resident at once is not required (tickets), but more warps
+  // than blocks would only spin
+  int grid = std::min<long long>(occupancy_grid(fn, kLvlThreads),
+                                 ceil_div(nnzb, kLvlThreads / 32));
+  k_bilu0_blocks<BS><<<grid, kLvlThreads, 0, st>>>(nb, row, col, diag, val, order, tptr, tcnt,
+                                                   flags, ss);
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
+
+template <int BS>
 int launch_bilu0_levels(int nb, const int* row, const int* col, const int* diag, double* val,
                         const int* order, const int* lvl_ptr, const int* nlev_d, SyncState ss,
                         GridSync gs, const int* mptr, const int2* mpair, cudaStream_t st) {
@@ -2077,10 +2598,11 @@ size_t level_sched_ws(int nb) {
          carve_size(sizeof(int) * 4) + carve_size(sizeof(unsigned) * 4);
 }
 
-// BILU(0) scratch: the level-scheduled one plus the sync-free schedule's
-// per-position match counts.
+// BILU(0) scratch: the level-scheduled one plus the row flow's plan (or the
+// block-wise schedule's update counts and ready flags) and task pointers.
 size_t bilu0_ws(int nb, long long nnzb) {
-  return level_sched_ws(nb) + carve_size(sizeof(int) * (size_t)std::max(nnzb, 1ll));
+  return level_sched_ws(nb) + carve_size(sizeof(int2) * (size_t)std::max(nnzb, 1ll)) +
+         carve_size(sizeof(int) * ((size_t)nb + 1)) + scan_ws_bytes(nb + 1);
 }
 
 // diagonal positions (validates the pattern); returns BILU_ERR_PATTERN with
@@ -2127,7 +2649,7 @@ int bilu0_analyze(int nb, long long nnzb, const int* row, const int* col, const 
   if (!keep.order || !keep.lvl || !keep.nlev) return BILU_ERR_WORKSPACE;
   return build_levels(nb, row, col, diag, 1, std::max(nnzb - nb, 0ll), keep.order, keep.lvl,
                       keep.nlev, &keep.h_nlev, ws, st, &keep.h_sched, &keep.h_maxdeg,
-                      &keep.h_fsched);
+                      &keep.h_fsched, keep.plan, &keep.h_rowflow);
 }
 
 // BILU(0)'s match lists from the pattern alone (a structure step, before
@@ -2143,9 +2665,9 @@ int bilu0_match_count(int nb, long long nnzb, const int* row, const int* col, co
   unsigned long long* tot = ws.take<unsigned long long>(1);
   if (!tot) return BILU_ERR_WORKSPACE;
   const unsigned grid = ceil_div(nnzb, 256);
-  k_bilu0_nmatch<<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, mptr);
+  k_bilu0_nmatch<false><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, mptr, nullptr);
   BILU_LAUNCH_CHECK();
-  k_bilu0_nmatch_long<<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, mptr);
+  k_bilu0_nmatch_long<false><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, mptr, nullptr);
   BILU_LAUNCH_CHECK();
   BILU_TRY_CUDA(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), st));
   k_match_total<<<std::min(grid, 1024u), 256, 0, st>>>(nnzb, mptr, tot);
@@ -2183,9 +2705,20 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
   if (!order || !lvl || !nlev_d || !rdiag) return BILU_ERR_WORKSPACE;
   int sched = keep.h_fsched;
   if (schedule == 0 || schedule == 1) sched = schedule;  // caller's choice
-  if (sched == 1) {
-    // narrow levels or long rows: sync-free, tickets in level order
-    int* nmatch = ws.take<int>((size_t)std::max(nnzb, 1ll));
+  if (keep.h_rowflow && schedule != 1) {
+    SyncState ss;
+    BILU_TRY(sync_init(ss, nb, ws, st));
+    ss.rdiag = rdiag;
+    if (nb > 0)
+      BILU_TRY(BILU_DISPATCH_BS(bs, launch_bilu0_rowflow, nb, row, col, diag, val, order, lvl,
+                                nlev_d, keep.plan, ss, st));
+    return sync_finish(ss, h_zp, st);
+  }
+  if (sched == 1 && keep.h_maxdeg <= kLongRow) {
+    // narrow levels: sync-free over rows.  (Block by block, below, a short row
+    // costs more hand-overs than it gains: 64^3 27-point pattern 104 ms against
+    // 15.6; with hub rows, 20,011-row power-law pattern, 1.4 ms against 8.0.)
+    int* nmatch = (int*)keep.plan;  // the plan is not read any more
     if (!nmatch) return BILU_ERR_WORKSPACE;
     SyncState ss;
     BILU_TRY(sync_init(ss, nb, ws, st));
@@ -2194,11 +2727,37 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
     ss.nmatch = nmatch;
     if (nb > 0) {
       const unsigned grid = ceil_div(std::max(nnzb, 1ll), 256);
-      k_bilu0_nmatch<<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, nmatch);
+      k_bilu0_nmatch<false><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, nmatch, nullptr);
       BILU_LAUNCH_CHECK();
-      k_bilu0_nmatch_long<<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, nmatch);
+      k_bilu0_nmatch_long<false><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, nmatch, nullptr);
       BILU_LAUNCH_CHECK();
       BILU_TRY(BILU_DISPATCH_BS(bs, launch_bilu0_syncfree, nb, row, col, diag, val, ss, st));
+    }
+    return sync_finish(ss, h_zp, st);
+  }
+  if (sched == 1) {
+    // long rows: sync-free over blocks, rows in level order
+    const size_t cnt = (size_t)std::max(nnzb, 1ll);
+    int* tcnt = (int*)keep.plan;  // not read any more: two ints a block
+    int* flags = tcnt + cnt;
+    int* tptr = ws.take<int>((size_t)nb + 1);
+    if (!tcnt || !tptr) return BILU_ERR_WORKSPACE;
+    SyncState ss;
+    BILU_TRY(sync_init_words(ss, ws, st));
+    ss.rdiag = rdiag;
+    if (nb > 0) {
+      const unsigned grid = ceil_div(nnzb, 256);
+      BILU_TRY_CUDA(cudaMemsetAsync(tcnt, 0, sizeof(int) * cnt, st));
+      k_bilu0_nmatch<true><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, tcnt, flags);
+      BILU_LAUNCH_CHECK();
+      k_bilu0_nmatch_long<true><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, tcnt, flags);
+      BILU_LAUNCH_CHECK();
+      BILU_TRY_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * cnt, st));
+      k_order_len<<<ceil_div(nb, 256), 256, 0, st>>>(nb, row, order, tptr);
+      BILU_LAUNCH_CHECK();
+      BILU_TRY(scan_exclusive(tptr, tptr, nb, nullptr, ws, st));
+      BILU_TRY(BILU_DISPATCH_BS(bs, launch_bilu0_blocks, nb, nnzb, row, col, diag, val, order,
+                                tptr, tcnt, flags, ss, st));
     }
     return sync_finish(ss, h_zp, st);
   }
@@ -2229,6 +2788,8 @@ int bilu0_impl(int nb, long long nnzb, int bs, const int* row, const int* col, c
     k.nlev = ws.take<int>(4);
     if (!k.order || !k.lvl || !k.nlev) return BILU_ERR_WORKSPACE;
   }
+  if (!k.plan) k.plan = ws.take<int2>((size_t)std::max(nnzb, 1ll));
+  if (!k.plan) return BILU_ERR_WORKSPACE;
   {
     Carver w2 = ws;
     BILU_TRY(bilu0_analyze(nb, nnzb, row, col, diag, k, w2, st));

@@ -138,3 +138,74 @@ def _lib_status(name):
     from isai_kernel_gb300 import _lib
 
     return {v: k for k, v in _lib.STATUS.items()}[name]
+
+
+# ------------------------------------------------------------------ BILU(0)
+def nine_point(side):
+    """2D 9-point pattern: neighbours of a row are neighbours of each other."""
+    at = lambda x, y: y * side + x
+    return pattern_of([[at(u, v) for u in range(max(x - 1, 0), min(x + 2, side))
+                        for v in range(max(y - 1, 0), min(y + 2, side))]
+                       for y in range(side) for x in range(side)])
+
+
+def bilu_pattern(name):
+    if name == "5-point":
+        A = gen.laplace2d(19, bs=4)
+        return A.rowptr, A.colind
+    if name == "7-point":
+        A = gen.convdiff3d(7, bs=4)
+        return A.rowptr, A.colind
+    if name == "bipartite":  # 13 dependencies or 13 blocks right of the diagonal
+        return pattern_of([range(13, 26) if i < 13 else range(13) for i in range(26)])
+    if name == "one-sided":  # no U_KI for most dependencies
+        rng = np.random.default_rng(3)
+        return pattern_of([rng.integers(0, 90, size=2) for _ in range(90)])
+    if name == "9-point":
+        return nine_point(11)
+    if name == "dense":
+        return pattern_of([range(37) for _ in range(37)])
+    if name == "diagonal":
+        return pattern_of([[] for _ in range(7)])
+    rng = np.random.default_rng(5)  # "hubs": rows of more than 32 dependencies
+    return pattern_of([rng.integers(0, 300, size=150 if i % 37 == 9 else 4) for i in range(300)])
+
+
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("name", ["5-point", "7-point", "bipartite", "one-sided", "9-point",
+                                  "dense", "diagonal", "hubs"])
+def test_bilu0_schedules(cuda, orc, name, bs):
+    """Every schedule's factor: the same bits, and the oracle's to 1e-12 of
+    the largest entry (diagonally dominant blocks: errors of a few ulps)."""
+    from isai_kernel_gb300 import api
+
+    rp, col = bilu_pattern(name)
+    nb, nnzb = len(rp) - 1, len(col)
+    rng = np.random.default_rng(bs)
+    val = rng.uniform(-1, 1, size=(nnzb, bs, bs))
+    rows = np.repeat(np.arange(nb), np.diff(rp))
+    diag = np.nonzero(rows == col)[0]
+    i = np.arange(bs)
+    val[diag[:, None], i, i] = 2.0 * bs * np.diff(rp)[:, None]
+    ref, _ = orc.bsrilu0(nb, bs, rp, col, val)
+    out = []
+    for schedule in (-1, 0, 1):
+        v = T(val, cuda)
+        assert api.bsrilu02_inplace(nb, nnzb, bs, T(rp, cuda), T(col, cuda), v, schedule) == -1
+        out.append(N(v))
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    assert np.max(np.abs(out[0] - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_bilu0_zero_pivot_row(cuda):
+    """The first row with a zero pivot is reported by every schedule."""
+    from isai_kernel_gb300 import api
+
+    A = gen.laplace2d(9, bs=4)
+    val = A.val.copy()
+    rows = np.repeat(np.arange(A.nb), np.diff(A.rowptr))
+    for bad in (70, 33):
+        val[rows == bad] = 0.0
+    for schedule in (-1, 0, 1):
+        assert api.bsrilu02_inplace(A.nb, A.nnzb, 4, T(A.rowptr, cuda), T(A.colind, cuda),
+                                    T(val, cuda), schedule) == 33
