@@ -148,18 +148,22 @@ int bilu_bcsc_to_bcsr(int mb, int nbcol, int bs, const int* d_cscPtr, const int*
 
 /* Replaces bsrilu02_inplace (bsrilu.h:20; cuSPARSE bsrilu02, row direction,
  * no level information): BILU(0) in place.  A level analysis of the lower
- * DAG picks the schedule: levels of at least 4096 block rows on average and
- * no row with more than 32 dependencies -> one cooperative launch with a
- * bounded grid barrier per level (a bs-lane group per row); otherwise
- * sync-free (warp per row, atomic tickets in level order, bounded waits on
- * ready flags).
+ * DAG picks the schedule.  Patterns in which a dependency updates nothing but
+ * its row's diagonal block (stencils without triangles), no row with more than
+ * 32 dependencies: rows in level order, each waiting for the rows it reads.
+ * Otherwise levels of at least 4096 block rows on average and no row with more
+ * than 32 dependencies -> one cooperative launch with a bounded grid barrier
+ * per level (a bs-lane group per row); else sync-free, atomic tickets in level
+ * order and bounded waits on ready flags: a warp per row, or per block where a
+ * row has more than 32 dependencies.
  * h_info[0] receives the first block row with a zero pivot (or -1);
  * BILU_ERR_ZERO_PIVOT then. */
 size_t bilu_bsrilu0_ws_bytes(int nb, int nnzb);
 int bilu_bsrilu0(int nb, int nnzb, int bs, const int* d_row, const int* d_col, double* d_val,
                  int* h_info, void* d_ws, size_t ws_bytes, bilu_stream_t stream);
 /* Same with the schedule chosen by the caller: -1 as recommended by the
- * analysis, 0 level schedule, 1 sync-free (both give identical factors). */
+ * analysis, 0 level schedule (level order or the barrier kernel), 1 sync-free
+ * (all give identical factors). */
 int bilu_bsrilu0_ex(int nb, int nnzb, int bs, const int* d_row, const int* d_col, double* d_val,
                     int schedule, int* h_info, void* d_ws, size_t ws_bytes, bilu_stream_t stream);
 

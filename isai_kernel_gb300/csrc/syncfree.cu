@@ -377,9 +377,10 @@ constexpr int kLongRow = 32;
 // kFlowMaxDeps dependencies, whatever the level width (it was 4-10x faster
 // than the sync-free kernel on 2D and 3D stencils down to 32 rows per
 // level), the sync-free kernel otherwise (a lane group walks a long row's
-// dependencies one after the other).  BILU(0): the level order (a barrier
-// per level) when a level holds at least kFactorLevelWidth rows on average
-// and no row has more than kLongRow dependencies, sync-free otherwise.
+// dependencies one after the other).  BILU(0) of patterns that do not take
+// the row flow: the barrier kernel when a level holds at least
+// kFactorLevelWidth rows on average and no row has more than kLongRow
+// dependencies, sync-free otherwise.
 constexpr int kFlowMaxDeps = 8;
 constexpr int kFactorLevelWidth = 4096;
 
