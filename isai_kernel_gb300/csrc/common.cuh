@@ -112,6 +112,28 @@ __device__ __forceinline__ float ld_stream(const float* p) {
   return v;
 }
 
+// The entries [s, e) of a pattern row per thread, f(row, p) for each: a thread
+// walks its own row, except that rows of more than kSharedRow entries are
+// walked by the whole warp, 32 entries at a time (one thread alone takes
+// hundreds of microseconds over a power-law hub row of 2000 entries with an
+// atomic each, while the rest of the GPU idles).  Called by all 32 lanes;
+// threads without a row pass s = e.
+constexpr int kSharedRow = 48;
+template <class F>
+__device__ __forceinline__ void for_row_entries(int row, int s, int e, F f) {
+  const bool shared = e - s > kSharedRow;
+  if (!shared)
+    for (int p = s; p < e; ++p) f(row, p);
+  unsigned todo = __ballot_sync(0xffffffffu, shared);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int r = __shfl_sync(0xffffffffu, row, src);
+    const int a = __shfl_sync(0xffffffffu, s, src), b = __shfl_sync(0xffffffffu, e, src);
+    for (int p = a + (int)(threadIdx.x & 31); p < b; p += 32) f(r, p);
+  }
+}
+
 // Bounded spin budget for sync-free kernels: after this many polls of a
 // dependency flag the waiter records BILU_ERR_TIMEOUT and returns.
 // Polls back off up to 256 ns, so the budget bounds a wait at a few seconds.

@@ -40,33 +40,37 @@ __global__ void k_fill_int(int* p, long long n, int v) {
 // the column counters (ISAI pattern) -- cnt[] preset to 1 for the diagonal.
 __global__ void k_isai_count(int nb, const int* __restrict__ row, const int* __restrict__ col,
                              int lower, int* cnt, int* err) {
-  int br = blockIdx.x * blockDim.x + threadIdx.x;
-  if (br >= nb) return;
-  int s = row[br], e = row[br + 1];
-  if (e < s) { report(err, br, 4); return; }
-  int prev = -1;
-  for (int p = s; p < e; ++p) {
-    int bc = col[p];
-    if (bc < 0 || bc >= nb) { report(err, br, 1); return; }
-    if (bc <= prev) { report(err, br, 2); return; }
-    prev = bc;
-    if (bc == br) continue;
-    if (lower ? (bc > br) : (bc < br)) continue;
-    atomicAdd(cnt + bc, 1);
+  const int br = blockIdx.x * blockDim.x + threadIdx.x;
+  int s = 0, e = 0;
+  if (br < nb) {
+    s = row[br];
+    e = row[br + 1];
+    if (e < s) report(err, br, 4);
   }
+  for_row_entries(br, s, max(s, e), [&](int r, int p) {
+    const int bc = col[p];
+    if (bc < 0 || bc >= nb) { report(err, r, 1); return; }
+    if (p > row[r] && bc <= col[p - 1]) { report(err, r, 2); return; }
+    if (bc == r || (lower ? bc > r : bc < r)) return;
+    atomicAdd(cnt + bc, 1);
+  });
 }
 
 __global__ void k_isai_scatter(int nb, const int* __restrict__ row, const int* __restrict__ col,
                                int lower, const int* __restrict__ Mptr, int* cursor, int* tmp) {
-  int br = blockIdx.x * blockDim.x + threadIdx.x;
-  if (br >= nb) return;
-  for (int p = row[br]; p < row[br + 1]; ++p) {
-    int bc = col[p];
-    if (bc == br || bc < 0 || bc >= nb) continue;
-    if (lower ? (bc > br) : (bc < br)) continue;
-    tmp[Mptr[bc] + atomicAdd(cursor + bc, 1)] = br;
+  const int br = blockIdx.x * blockDim.x + threadIdx.x;
+  int s = 0, e = 0;
+  if (br < nb) {
+    s = row[br];
+    e = row[br + 1];
+    tmp[Mptr[br] + atomicAdd(cursor + br, 1)] = br;
   }
-  tmp[Mptr[br] + atomicAdd(cursor + br, 1)] = br;
+  for_row_entries(br, s, max(s, e), [&](int r, int p) {
+    const int bc = col[p];
+    if (bc == r || bc < 0 || bc >= nb) return;
+    if (lower ? (bc > r) : (bc < r)) return;
+    tmp[Mptr[bc] + atomicAdd(cursor + bc, 1)] = r;
+  });
 }
 
 // Warp per segment: out[ptr[s] + rank(key)] = key (and payload), keys
@@ -86,22 +90,42 @@ __global__ void k_segment_rank_sort(int nseg, const int* __restrict__ ptr,
   }
 }
 
-__global__ void k_tri_count(int nb, const int* __restrict__ row, const int* __restrict__ col,
-                            int lower, int* cnt) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nb) return;
-  int c = 0;
-  for (int p = row[r]; p < row[r + 1]; ++p) c += lower ? (col[p] <= r) : (col[p] >= r);
-  cnt[r] = c;
-}
-
-__global__ void k_tri_fill(int nb, const int* __restrict__ row, const int* __restrict__ col,
-                           int lower, const int* __restrict__ Trow, int* __restrict__ Tcol) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nb) return;
-  int o = Trow[r];
-  for (int p = row[r]; p < row[r + 1]; ++p)
-    if (lower ? (col[p] <= r) : (col[p] >= r)) Tcol[o++] = col[p];
+// Rows of the lower (upper) triangle in their stored order: a thread per row,
+// the warp together on rows of more than kSharedRow entries (ballots keep the
+// order).  FILL false: out[r] = entries; true: Tcol at out[r] (= Trow).
+template <bool FILL>
+__global__ void k_tri(int nb, const int* __restrict__ row, const int* __restrict__ col, int lower,
+                      int* out, int* __restrict__ Tcol) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int s = r < nb ? row[r] : 0, e = r < nb ? row[r + 1] : 0;
+  const bool shared = e - s > kSharedRow;
+  if (r < nb && !shared) {
+    int o = FILL ? out[r] : 0;
+    for (int p = s; p < e; ++p) {
+      const int c = col[p];
+      if (!(lower ? (c <= r) : (c >= r))) continue;
+      if (FILL) Tcol[o] = c;
+      ++o;
+    }
+    if (!FILL) out[r] = o;
+  }
+  unsigned todo = __ballot_sync(0xffffffffu, shared);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int q = __shfl_sync(0xffffffffu, r, src);
+    const int a = __shfl_sync(0xffffffffu, s, src), b = __shfl_sync(0xffffffffu, e, src);
+    int o = FILL ? out[q] : 0;
+    for (int p0 = a; p0 < b; p0 += 32) {
+      const int c = p0 + lane < b ? col[p0 + lane] : 0;
+      const bool in = p0 + lane < b && (lower ? (c <= q) : (c >= q));
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (FILL && in) Tcol[o + __popc(m & ((1u << lane) - 1u))] = c;
+      o += __popc(m);
+    }
+    if (!FILL && lane == 0) out[q] = o;
+  }
 }
 
 // Thread per BCSC column: binary search of each entry in its BCSR row.
@@ -480,7 +504,7 @@ int isai_pattern_fill_impl(int nb, const int* row, const int* col, int lower, co
 int tri_pattern_rowptr_impl(int nb, const int* row, const int* col, int lower, int* Trow,
                             int* h_nnz, Carver& ws, cudaStream_t st) {
   if (nb > 0) {
-    k_tri_count<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, Trow);
+    k_tri<false><<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, Trow, nullptr);
     BILU_LAUNCH_CHECK();
   }
   return scan_exclusive(Trow, Trow, nb, h_nnz, ws, st);
@@ -489,7 +513,7 @@ int tri_pattern_rowptr_impl(int nb, const int* row, const int* col, int lower, i
 int tri_pattern_fill_impl(int nb, const int* row, const int* col, int lower, const int* Trow,
                           int* Tcol, cudaStream_t st) {
   if (nb == 0) return BILU_OK;
-  k_tri_fill<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, Trow, Tcol);
+  k_tri<true><<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, const_cast<int*>(Trow), Tcol);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }

@@ -98,20 +98,45 @@ __device__ __forceinline__ int find_in_row(const int* __restrict__ col, int s, i
   return -1;
 }
 
+// diag[i] = position of block (i, i), -1 where row i has none or is not
+// strictly ascending inside [0, nb); *bad: the first such row.
 __global__ void k_diag_pos(int nb, const int* __restrict__ row, const int* __restrict__ col,
                            int* __restrict__ diag, int* bad) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nb) return;
-  int s = row[i], e = row[i + 1];
-  int prev = -1;
-  for (int p = s; p < e; ++p) {
-    int c = col[p];
-    if (c <= prev || c < 0 || c >= nb) { atomicMin(bad, i); diag[i] = -1; return; }
-    prev = c;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = i < nb ? row[i] : 0, e = i < nb ? row[i + 1] : 0;
+  const bool shared = e - s > kSharedRow;
+  if (i < nb && !shared) {
+    int d = -1, prev = -1;
+    bool ok = true;
+    for (int p = s; p < e; ++p) {
+      const int c = col[p];
+      ok = ok && c > prev && c < nb;
+      if (c == i) d = p;
+      prev = c;
+    }
+    diag[i] = ok ? d : -1;
+    if (!ok || d < 0) atomicMin(bad, i);
   }
-  int d = find_in_row(col, s, e, i);
-  diag[i] = d;
-  if (d < 0) atomicMin(bad, i);
+  unsigned todo = __ballot_sync(FULL, shared);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int r = __shfl_sync(FULL, i, src);
+    const int a = __shfl_sync(FULL, s, src), b = __shfl_sync(FULL, e, src);
+    int d = -1;
+    bool ok = true;
+    for (int p = a + (int)(threadIdx.x & 31); p < b; p += 32) {
+      const int c = col[p];
+      ok = ok && c > (p > a ? col[p - 1] : -1) && c < nb;
+      if (c == r) d = p;
+    }
+    d = __reduce_max_sync(FULL, d);
+    ok = __all_sync(FULL, ok);
+    if ((int)(threadIdx.x & 31) == src) {
+      diag[r] = ok ? d : -1;
+      if (!ok || d < 0) atomicMin(bad, r);
+    }
+  }
 }
 
 // ------------------------------------------------------------------ SpTRSV

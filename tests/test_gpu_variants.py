@@ -209,3 +209,38 @@ def test_bilu0_zero_pivot_row(cuda):
     for schedule in (-1, 0, 1):
         assert api.bsrilu02_inplace(A.nb, A.nnzb, 4, T(A.rowptr, cuda), T(A.colind, cuda),
                                     T(val, cuda), schedule) == 33
+
+
+# ------------------------------------------------------------------ patterns with long rows
+@pytest.mark.parametrize("lower", [True, False])
+def test_patterns_rows_walked_by_a_warp(cuda, orc, lower):
+    """Rows just below, at and above the length from which a warp shares a
+    row, several of them in one warp, against the oracle (integers)."""
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(17)
+    n = 150
+    length = {3: 47, 4: 48, 5: 49, 6: 110, 40: 149, 149: 120}
+    rp, col = pattern_of([rng.choice(n, size=length.get(i, 3), replace=False) for i in range(n)])
+    r, c = T(rp, cuda), T(col, cuda)
+    mp, mi = api.build_bcsc_pattern_from_bsr_scalarILU(n, r, c, lower)
+    omp, omi = orc.isai_pattern(n, rp, col, int(lower))
+    assert np.array_equal(N(mp), omp) and np.array_equal(N(mi), omi)
+    tr, tc = api.build_triangular_bcsr_pattern_from_A(n, r, c, lower)
+    otr, otc = orc.tri_pattern(n, rp, col, int(lower))
+    assert np.array_equal(N(tr), otr) and np.array_equal(N(tc), otc)
+    # a long row out of order, and one without its diagonal block, are refused
+    bad = col.copy()
+    bad[rp[40] + 70], bad[rp[40] + 71] = col[rp[40] + 71], col[rp[40] + 70]
+    with pytest.raises(api.BiluError):
+        api.build_bcsc_pattern_from_bsr_scalarILU(n, r, T(bad, cuda), lower)
+    val = np.ones((len(col), 4, 4))
+    b = np.ones(4 * n)
+    with pytest.raises(api.BiluError):
+        api.sptrsv(n, 4, r, T(bad, cuda), T(val, cuda), T(b, cuda), lower)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    keep = ~((rows == 6) & (col == 6))
+    rp2 = np.zeros(n + 1, np.int32)
+    np.cumsum(np.bincount(rows[keep], minlength=n), out=rp2[1:])
+    with pytest.raises(api.BiluError):
+        api.sptrsv(n, 4, T(rp2, cuda), T(col[keep], cuda), T(val[keep], cuda), T(b, cuda), lower)
