@@ -73,20 +73,36 @@ __global__ void k_isai_scatter(int nb, const int* __restrict__ row, const int* _
   });
 }
 
-// Warp per segment: out[ptr[s] + rank(key)] = key (and payload), keys
-// distinct inside a segment.
-__global__ void k_segment_rank_sort(int nseg, const int* __restrict__ ptr,
-                                    const int* __restrict__ key, const int* __restrict__ pay,
-                                    int* __restrict__ key_out, int* __restrict__ pay_out) {
-  int lane = threadIdx.x & 31;
-  int sgi = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (sgi >= nseg) return;
-  int s = ptr[sgi], e = ptr[sgi + 1];
-  for (int i = s + lane; i < e; i += 32) {
-    int k = key[i], rank = 0;
-    for (int j = s; j < e; ++j) rank += key[j] < k;
-    key_out[s + rank] = k;
-    if (pay_out) pay_out[s + rank] = pay[i];
+// out[ptr[s] + rank(key)] = key (and payload), keys distinct inside a segment:
+// 8 lanes per segment (most hold a handful of keys), the warp together on
+// segments of more than kSharedRow keys.
+__device__ __forceinline__ void rank_one(int i, int s, int e, const int* __restrict__ key,
+                                         const int* __restrict__ pay, int* __restrict__ key_out,
+                                         int* __restrict__ pay_out) {
+  const int k = key[i];
+  int rank = 0;
+  for (int j = s; j < e; ++j) rank += key[j] < k;
+  key_out[s + rank] = k;
+  if (pay_out) pay_out[s + rank] = pay[i];
+}
+
+__global__ void __launch_bounds__(kT) k_segment_rank_sort(int nseg, const int* __restrict__ ptr,
+                                                          const int* __restrict__ key,
+                                                          const int* __restrict__ pay,
+                                                          int* __restrict__ key_out,
+                                                          int* __restrict__ pay_out) {
+  const int lane = threadIdx.x & 31, l = lane & 7;
+  const long long sg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int s = sg < nseg ? ptr[sg] : 0, e = sg < nseg ? ptr[sg + 1] : 0;
+  const bool shared = e - s > kSharedRow;
+  if (!shared)
+    for (int i = s + l; i < e; i += 8) rank_one(i, s, e, key, pay, key_out, pay_out);
+  unsigned todo = __ballot_sync(0xffffffffu, shared && l == 0);
+  while (todo) {
+    const int from = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int a = __shfl_sync(0xffffffffu, s, from), b = __shfl_sync(0xffffffffu, e, from);
+    for (int i = a + lane; i < b; i += 32) rank_one(i, a, b, key, pay, key_out, pay_out);
   }
 }
 
@@ -197,14 +213,39 @@ __global__ void k_count_rows(long long nnzb, const int* __restrict__ ind, int mb
 __global__ void k_csc_scatter(int nbcol, const int* __restrict__ cptr,
                               const int* __restrict__ cind, const int* __restrict__ rptr,
                               int* cursor, int* key, int* src) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nbcol) return;
-  for (int k = cptr[c]; k < cptr[c + 1]; ++k) {
-    int r = cind[k];
-    int d = rptr[r] + atomicAdd(cursor + r, 1);
-    key[d] = c;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = c < nbcol ? cptr[c] : 0, e = c < nbcol ? cptr[c + 1] : 0;
+  for_row_entries(c, s, max(s, e), [&](int q, int k) {
+    const int r = cind[k];
+    const int d = rptr[r] + atomicAdd(cursor + r, 1);
+    key[d] = q;
     src[d] = k;
+  });
+}
+
+// cnt[col[k]] += 1 over all blocks; words: 0 a column out of range, 1 the block
+// count (read on the device, so that the host need not wait for it).
+__global__ void __launch_bounds__(kT) k_count_cols(int mb, const int* __restrict__ row,
+                                                   const int* __restrict__ col, int* cnt,
+                                                   int* words) {
+  const int nnzb = __ldg(row + mb);
+  if (blockIdx.x == 0 && threadIdx.x == 0) words[1] = nnzb;
+  for (long long k = (long long)blockIdx.x * kT + threadIdx.x; k < nnzb;
+       k += (long long)gridDim.x * kT) {
+    const int c = col[k];
+    if (c < 0 || c >= mb) words[0] = 1;
+    else atomicAdd(cnt + c, 1);
   }
+}
+
+// words[2] = the longest segment
+__global__ void __launch_bounds__(kT) k_longest(int n, const int* __restrict__ ptr, int* words) {
+  int m = 0;
+  for (long long i = (long long)blockIdx.x * kT + threadIdx.x; i < n;
+       i += (long long)gridDim.x * kT)
+    m = max(m, ptr[i + 1] - ptr[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(words + 2, m);
 }
 
 __global__ void k_gather_blocks(long long nnzb, int bs2, const int* __restrict__ src,
@@ -495,7 +536,7 @@ int isai_pattern_fill_impl(int nb, const int* row, const int* col, int lower, co
   BILU_TRY_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * nb, st));
   k_isai_scatter<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, Mptr, cursor, tmp);
   BILU_LAUNCH_CHECK();
-  k_segment_rank_sort<<<ceil_div(nb, 8), 256, 0, st>>>(nb, Mptr, tmp, nullptr, Mind, nullptr);
+  k_segment_rank_sort<<<ceil_div((long long)nb * 8, kT), kT, 0, st>>>(nb, Mptr, tmp, nullptr, Mind, nullptr);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
@@ -563,15 +604,53 @@ size_t transpose_ws(int mb, long long nnzb) {
          3 * carve_size(sizeof(int) * (size_t)(nnzb + 1)) + scan_ws_bytes(mb + 1);
 }
 
+// The entries of a transposed pattern whose row pointer is known: rind
+// ascending inside a row, src[d] = index of entry d in the given pattern.
+int transpose_fill(int mb, int nbcol, const int* cptr, const int* cind, long long nnzb,
+                   const int* rptr, int* rind, int* src, Carver& ws, cudaStream_t st) {
+  int* cursor = ws.take<int>((size_t)mb + 1);
+  int* key = ws.take<int>((size_t)nnzb + 1);
+  int* pay = ws.take<int>((size_t)nnzb + 1);
+  if (!cursor || !key || !pay) return BILU_ERR_WORKSPACE;
+  if (mb == 0 || nnzb == 0) return BILU_OK;
+  BILU_TRY_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * mb, st));
+  k_csc_scatter<<<ceil_div(nbcol, kT), kT, 0, st>>>(nbcol, cptr, cind, rptr, cursor, key, pay);
+  BILU_LAUNCH_CHECK();
+  k_segment_rank_sort<<<ceil_div((long long)mb * 8, kT), kT, 0, st>>>(mb, rptr, key, pay, rind,
+                                                                      src);
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
+
+// Row pointer of the transpose of a square pattern, its block count and longest
+// row on the host (one synchronisation); BILU_ERR_PATTERN for a column out of
+// range.
+int transpose_count(int mb, const int* row, const int* col, int* trow, int* h_nnzb,
+                    int* h_longest, Carver& ws, cudaStream_t st) {
+  int* words = ws.take<int>(4);
+  if (!words) return BILU_ERR_WORKSPACE;
+  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * 4, st));
+  BILU_TRY_CUDA(cudaMemsetAsync(trow, 0, sizeof(int) * ((size_t)mb + 1), st));
+  k_count_cols<<<152 * 8, kT, 0, st>>>(mb, row, col, trow, words);
+  BILU_LAUNCH_CHECK();
+  BILU_TRY(scan_exclusive(trow, trow, mb, nullptr, ws, st));
+  k_longest<<<std::min<unsigned>(ceil_div(mb, kT), 152 * 8), kT, 0, st>>>(mb, trow, words);
+  BILU_LAUNCH_CHECK();
+  int h[4];
+  BILU_TRY_CUDA(cudaMemcpyAsync(h, words, sizeof(h), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaStreamSynchronize(st));
+  if (h[0]) return BILU_ERR_PATTERN;
+  *h_nnzb = h[1];
+  *h_longest = h[2];
+  return BILU_OK;
+}
+
 // BCSC (cptr over nbcol columns) -> BCSR pattern with ascending columns and
 // src[d] = BCSC index of BCSR entry d.
 int transpose_pattern(int mb, int nbcol, const int* cptr, const int* cind, long long nnzb,
                       int* rptr, int* rind, int* src, Carver& ws, cudaStream_t st) {
   int* err = ws.take<int>(2);
-  int* cursor = ws.take<int>((size_t)mb + 1);
-  int* key = ws.take<int>((size_t)nnzb + 1);
-  int* pay = ws.take<int>((size_t)nnzb + 1);
-  if (!err || !cursor || !key || !pay) return BILU_ERR_WORKSPACE;
+  if (!err) return BILU_ERR_WORKSPACE;
   BILU_TRY(init_err(err, st));
   BILU_TRY_CUDA(cudaMemsetAsync(rptr, 0, sizeof(int) * (mb + 1), st));
   if (nnzb > 0) {
@@ -582,13 +661,7 @@ int transpose_pattern(int mb, int nbcol, const int* cptr, const int* cind, long 
   int h_err[2];
   BILU_TRY(read_err(err, h_err, st));
   if (h_err[1] != 0) return BILU_ERR_PATTERN;
-  if (mb == 0 || nnzb == 0) return BILU_OK;
-  BILU_TRY_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * mb, st));
-  k_csc_scatter<<<ceil_div(nbcol, kT), kT, 0, st>>>(nbcol, cptr, cind, rptr, cursor, key, pay);
-  BILU_LAUNCH_CHECK();
-  k_segment_rank_sort<<<ceil_div(mb, 8), 256, 0, st>>>(mb, rptr, key, pay, rind, src);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  return transpose_fill(mb, nbcol, cptr, cind, nnzb, rptr, rind, src, ws, st);
 }
 
 int gather_blocks(long long nnzb, int bs, const int* src, const double* in, double* out,

@@ -91,6 +91,27 @@ __device__ __forceinline__ void load_row(const VT* __restrict__ val, long long p
   }
 }
 
+// Row r of the transpose of block p: its column r.  The BS lanes of a block row
+// read neighbouring columns, so each of the BS loads is one run of BS values.
+template <int BS, class VT, class AccT>
+__device__ __forceinline__ void load_col(const VT* __restrict__ val, long long p, int r, AccT* a) {
+  const VT* q = val + p * BS * BS + r;
+#pragma unroll
+  for (int c = 0; c < BS; ++c) a[c] = to_acc(__ldg(q + c * BS), AccT());
+}
+
+// Row r of entry p of the matrix: TR reads the transpose of block src[p] of
+// another matrix's values (the transposed product, without transposing them).
+template <int BS, bool TR, class VT, class AccT>
+__device__ __forceinline__ void load_entry(const VT* __restrict__ val,
+                                           const int* __restrict__ src, long long p, int r,
+                                           AccT* a) {
+  if constexpr (TR)
+    load_col<BS, VT, AccT>(val, __ldg(src + p), r, a);
+  else
+    load_row<BS, VT, AccT>(val, p, r, a);
+}
+
 // Rows with more blocks than this are worth the CTA's help: power-law hub
 // rows hold up to ~2000 blocks, and a lane group alone runs one dependent
 // FMA chain over all of them while the rest of the GPU idles.
@@ -100,9 +121,10 @@ constexpr int kLongSpmvRow = 64;
 // take the blocks g, g + NG, ... of each (two accumulators, even and odd
 // turns), the NG partials are added in group order.  Out of line so that
 // the short rows' loop keeps its registers.  Called by every thread.
-template <int BS, class VT, class XT, class YT, class AccT, int NSLOT, int NG>
+template <int BS, class VT, class XT, class YT, class AccT, int NSLOT, int NG, bool TR>
 __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __restrict__ row,
                                             const int* __restrict__ col,
+                                            const int* __restrict__ src,
                                             const VT* __restrict__ val,
                                             const XT* __restrict__ x, YT* __restrict__ y,
                                             float* __restrict__ y32, AccT* red, bool in_group,
@@ -116,8 +138,8 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
       int p = rs + cg;
       for (; p + NG < re; p += 2 * NG) {
         AccT v0[BS], v1[BS], x0[BS], x1[BS];
-        load_row<BS, VT, AccT>(val, p, r, v0);
-        load_row<BS, VT, AccT>(val, p + NG, r, v1);
+        load_entry<BS, TR, VT, AccT>(val, src, p, r, v0);
+        load_entry<BS, TR, VT, AccT>(val, src, p + NG, r, v1);
         load_x<BS, XT, AccT>(x, __ldg(col + p), x0);
         load_x<BS, XT, AccT>(x, __ldg(col + p + NG), x1);
 #pragma unroll
@@ -128,7 +150,7 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
       }
       if (p < re) {
         AccT v0[BS], x0[BS];
-        load_row<BS, VT, AccT>(val, p, r, v0);
+        load_entry<BS, TR, VT, AccT>(val, src, p, r, v0);
         load_x<BS, XT, AccT>(x, __ldg(col + p), x0);
 #pragma unroll
         for (int k = 0; k < BS; ++k) a0 = fma(v0[k], x0[k], a0);
@@ -161,9 +183,11 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
 // such a row is skipped by its group and summed after the short rows by
 // the whole CTA (dynamic shared memory: the CTA's long-row slots and the
 // group partials); the other instance has no CTA barrier at all.
-template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool LONG>
+template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool LONG,
+          bool TR>
 __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __restrict__ row,
                                                      const int* __restrict__ col,
+                                                     const int* __restrict__ src,
                                                      const VT* __restrict__ val,
                                                      const XT* __restrict__ x,
                                                      YT* __restrict__ y,
@@ -215,7 +239,7 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (c[q][u] >= 0) {
-          load_row<BS, VT, AccT>(val, s[q] + off + u, r, a[q][u]);
+          load_entry<BS, TR, VT, AccT>(val, src, s[q] + off + u, r, a[q][u]);
         } else {
 #pragma unroll
           for (int k = 0; k < BS; ++k) a[q][u][k] = 0;
@@ -244,8 +268,8 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
     constexpr int NSLOT = 8 * G * RPG;
     // one CTA barrier, which also says whether the CTA holds a long row
     if (__syncthreads_or(mine_long))
-      spmv_long_rows<BS, VT, XT, YT, AccT, NSLOT, 8 * G>(
-          long_slots, row, col, val, x, y, y32,
+      spmv_long_rows<BS, VT, XT, YT, AccT, NSLOT, 8 * G, TR>(
+          long_slots, row, col, src, val, x, y, y32,
           reinterpret_cast<AccT*>(long_slots + ((NSLOT + 1) & ~1)), g < G, cg, r);
   }
 }
@@ -260,9 +284,10 @@ constexpr int kLayoutLong = 1;
 constexpr int kLayoutWide = 2;
 constexpr int kWideSpmvRow = 5;
 
-template <int BS, class VT, class XT, class YT, int RPG, int U, int MINB, bool LONG>
+template <int BS, class VT, class XT, class YT, int RPG, int U, int MINB, bool LONG,
+          bool TR = false>
 int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
-                    cudaStream_t st, float* y32) {
+                    cudaStream_t st, float* y32, const int* src = nullptr) {
   using AccT = VT;
   constexpr int G = 32 / BS;
   long long groups = (mb + RPG - 1) / RPG;
@@ -271,11 +296,11 @@ int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const
   if constexpr (LONG) {
     constexpr int NSLOT = 8 * G * RPG;
     const size_t smem = sizeof(int) * ((NSLOT + 1) & ~1) + sizeof(AccT) * 8 * G * BS;
-    k_bsr_spmv<BS, VT, XT, YT, AccT, RPG, U, MINB, true><<<grid, 256, smem, st>>>(
-        mb, row, col, val, x, y, y32);
+    k_bsr_spmv<BS, VT, XT, YT, AccT, RPG, U, MINB, true, TR><<<grid, 256, smem, st>>>(
+        mb, row, col, src, val, x, y, y32);
   } else {
-    k_bsr_spmv<BS, VT, XT, YT, AccT, RPG, U, MINB, false><<<grid, 256, 0, st>>>(
-        mb, row, col, val, x, y, y32);
+    k_bsr_spmv<BS, VT, XT, YT, AccT, RPG, U, MINB, false, TR><<<grid, 256, 0, st>>>(
+        mb, row, col, src, val, x, y, y32);
   }
   BILU_LAUNCH_CHECK();
   return BILU_OK;
@@ -315,6 +340,24 @@ int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT*
       return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8, false>(mb, row, col, val, x, y, st, y32);
     return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4, false>(mb, row, col, val, x, y, st, y32);
   }
+}
+
+// y = M^T x from M's values and the transposed pattern (launch_spmv's FP64
+// configurations, so the sums run in the order of a product with the
+// transposed matrix: the same bits).
+template <int BS>
+int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, const double* val,
+                  const double* x, double* y, cudaStream_t st, int layout) {
+  using D = double;
+  if (layout & kLayoutLong)
+    return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, true, true>(mb, trow, tcol, val, x, y, st,
+                                                             nullptr, src);
+  if constexpr (BS <= 5)
+    return launch_spmv_cfg<BS, D, D, D, 2, 1, 4, false, true>(mb, trow, tcol, val, x, y, st,
+                                                              nullptr, src);
+  else
+    return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, false, true>(mb, trow, tcol, val, x, y, st,
+                                                              nullptr, src);
 }
 
 // Multi-RHS: Y[n,k] = M X[n,k], row-major with ld = k.  One warp per block
@@ -509,6 +552,15 @@ int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const voi
                             (double*)y, st, lr);
   }
   return BILU_DISPATCH_BS(bs, spmv_f32, mb, row, col, (const float*)val, x, x32, y, y32, st, lr);
+}
+
+// y = M^T x: trow / tcol the transposed pattern, src the block of M each of its
+// entries stands for, longest its longest row.
+int spmv_gather_t(int mb, int bs, const int* trow, const int* tcol, const int* src,
+                  const double* val, const double* x, double* y, int longest,
+                  cudaStream_t st) {
+  const int layout = longest > kLongSpmvRow ? kLayoutLong : 0;
+  return BILU_DISPATCH_BS(bs, launch_spmv_t, mb, trow, tcol, src, val, x, y, st, layout);
 }
 
 int convert_f64_f32(size_t count, const double* src, float* dst, cudaStream_t st) {

@@ -253,3 +253,64 @@ def test_patterns_rows_walked_by_a_warp(cuda, orc, lower):
     np.cumsum(np.bincount(rows[keep], minlength=n), out=rp2[1:])
     with pytest.raises(api.BiluError):
         api.sptrsv(n, 4, T(rp2, cuda), T(col[keep], cuda), T(val[keep], cuda), T(b, cuda), lower)
+
+
+# ------------------------------------------------------------------ adjoint products
+def sparse_rows(name):
+    """rowptr, col (no diagonal needed): hub rows and columns, empty rows."""
+    rng = np.random.default_rng(23)
+    n = 260
+    if name == "empty":
+        return np.zeros(n + 1, np.int32), np.zeros(0, np.int32)
+    if name == "gaps":  # stored rows a long way apart
+        rows = [[0, 3, 259] if i in (0, 1, 100, 258) else [] for i in range(n)]
+    elif name == "hub column":  # column 7 in every row, columns of 63 to 66 rows
+        rows = [[7] + [20 + k for k in range(4) if i < 63 + k] for i in range(n)]
+    else:  # "hub row"
+        rows = [rng.integers(0, n, size=200 if i == 31 else 3) for i in range(n)]
+    cols = [np.unique(np.array(r, np.int32)) for r in rows]
+    rp = np.zeros(n + 1, np.int32)
+    np.cumsum([len(c) for c in cols], out=rp[1:])
+    return rp, np.concatenate(cols).astype(np.int32)
+
+
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("name", ["gaps", "hub column", "hub row"])
+def test_transposed_product(cuda, name, bs):
+    """M^T x against dense FP64: sums of up to 260 bs products of numbers in
+    [-1, 1], so 1e-13 of the number of terms."""
+    from isai_kernel_gb300 import api
+
+    rp, col = sparse_rows(name)
+    nb = len(rp) - 1
+    rng = np.random.default_rng(bs)
+    val, x = rng.uniform(-1, 1, size=(len(col), bs, bs)), rng.uniform(-1, 1, size=nb * bs)
+    y = N(api.bcsr_spmv_transpose(nb, bs, T(rp, cuda), T(col, cuda), T(val, cuda), T(x, cuda)))
+    D = np.zeros((nb, bs, nb, bs))
+    D[np.repeat(np.arange(nb), np.diff(rp)), :, col, :] = val
+    assert np.max(np.abs(y - D.reshape(nb * bs, -1).T @ x)) <= 1e-13 * 260 * bs
+    bad = col.copy()
+    bad[-1] = nb
+    with pytest.raises(api.BiluError):
+        api.bcsr_spmv_transpose(nb, bs, T(rp, cuda), T(bad, cuda), T(val, cuda), T(x, cuda))
+
+
+@pytest.mark.parametrize("scale", [1.0, -1.0, 2.5])
+@pytest.mark.parametrize("bs", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("name", ["empty", "gaps", "hub column", "hub row"])
+def test_masked_outer_runs(cuda, name, bs, scale):
+    """Bit for bit: (scale u) v is one rounding (two for a general scale, in
+    the same order), adding to G one more."""
+    from isai_kernel_gb300 import api
+
+    rp, col = sparse_rows(name)
+    nb = len(rp) - 1
+    rng = np.random.default_rng(bs)
+    u, v = rng.uniform(-1, 1, size=nb * bs), rng.uniform(-1, 1, size=nb * bs)
+    G0 = rng.uniform(-1, 1, size=(len(col), bs, bs))
+    rows = np.repeat(np.arange(nb), np.diff(rp))
+    ref = (scale * u.reshape(nb, bs)[rows])[:, :, None] * v.reshape(nb, bs)[col][:, None, :]
+    args = (nb, bs, T(rp, cuda), T(col, cuda), T(u, cuda), T(v, cuda), scale)
+    assert np.array_equal(N(api.masked_outer(*args)), ref)
+    added = N(api.masked_outer(*args, G=T(G0, cuda)))
+    assert np.max(np.abs(added - (G0 + ref)), initial=0.0) <= 2.0 ** -52 * 3  # fused or not
