@@ -12,6 +12,9 @@
 #include <algorithm>
 
 #include <mutex>
+#include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 
@@ -121,10 +124,9 @@ constexpr int kLongSpmvRow = 64;
 // take the blocks g, g + NG, ... of each (two accumulators, even and odd
 // turns), the NG partials are added in group order.  Out of line so that
 // the short rows' loop keeps its registers.  Called by every thread.
-template <int BS, class VT, class XT, class YT, class AccT, int NSLOT, int NG, bool TR>
+template <int BS, class VT, class XT, class YT, class AccT, int NSLOT, int NG>
 __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __restrict__ row,
                                             const int* __restrict__ col,
-                                            const int* __restrict__ src,
                                             const VT* __restrict__ val,
                                             const XT* __restrict__ x, YT* __restrict__ y,
                                             float* __restrict__ y32, AccT* red, bool in_group,
@@ -136,21 +138,29 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
     AccT a0 = 0, a1 = 0;
     if (in_group) {
       int p = rs + cg;
-      for (; p + NG < re; p += 2 * NG) {
-        AccT v0[BS], v1[BS], x0[BS], x1[BS];
-        load_entry<BS, TR, VT, AccT>(val, src, p, r, v0);
-        load_entry<BS, TR, VT, AccT>(val, src, p + NG, r, v1);
-        load_x<BS, XT, AccT>(x, __ldg(col + p), x0);
-        load_x<BS, XT, AccT>(x, __ldg(col + p + NG), x1);
+      // F blocks' loads in flight; even turns go to a0, odd ones to a1
+      auto turns = [&](auto f) {
+        constexpr int F = decltype(f)::value;
+        for (; p + (F - 1) * NG < re; p += F * NG) {
+          AccT v[F][BS], xv[F][BS];
 #pragma unroll
-        for (int k = 0; k < BS; ++k) {
-          a0 = fma(v0[k], x0[k], a0);
-          a1 = fma(v1[k], x1[k], a1);
+          for (int t = 0; t < F; ++t) load_row<BS, VT, AccT>(val, p + t * NG, r, v[t]);
+#pragma unroll
+          for (int t = 0; t < F; ++t) load_x<BS, XT, AccT>(x, __ldg(col + p + t * NG), xv[t]);
+#pragma unroll
+          for (int t = 0; t < F; t += 2)
+#pragma unroll
+            for (int k = 0; k < BS; ++k) {
+              a0 = fma(v[t][k], xv[t][k], a0);
+              a1 = fma(v[t + 1][k], xv[t + 1][k], a1);
+            }
         }
-      }
+      };
+      turns(std::integral_constant<int, 4>());
+      turns(std::integral_constant<int, 2>());
       if (p < re) {
         AccT v0[BS], x0[BS];
-        load_entry<BS, TR, VT, AccT>(val, src, p, r, v0);
+        load_row<BS, VT, AccT>(val, p, r, v0);
         load_x<BS, XT, AccT>(x, __ldg(col + p), x0);
 #pragma unroll
         for (int k = 0; k < BS; ++k) a0 = fma(v0[k], x0[k], a0);
@@ -179,12 +189,9 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
 // 0.40 ms on the 7-point FP64 operator, the same on the triangle); FP32
 // values U = 4 with RPG = 1 for wider rows (0.199 -> 0.176 ms on the FP32
 // operator), RPG = 1 at 8 CTAs per SM for bs 4 rows of ~4 blocks, else
-// RPG = 2.  LONG (matrices with rows of more than kLongSpmvRow blocks):
-// such a row is skipped by its group and summed after the short rows by
-// the whole CTA (dynamic shared memory: the CTA's long-row slots and the
-// group partials); the other instance has no CTA barrier at all.
-template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool LONG,
-          bool TR>
+// RPG = 2.  Patterns with rows of more than kLongSpmvRow blocks take
+// k_bsr_spmv_balanced (FP64) or k_bsr_spmv_uneven (FP32).
+template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool TR>
 __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __restrict__ row,
                                                      const int* __restrict__ col,
                                                      const int* __restrict__ src,
@@ -196,31 +203,20 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
   int lane = threadIdx.x & 31;
   int g = lane / BS, r = lane - g * BS;
   long long base = (((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + g) * RPG;
-  const bool active = g < G && base < mb;
-  if (!LONG && !active) return;
+  if (g >= G || base >= mb) return;
   int s[RPG], e[RPG];
-  bool skip[RPG], mine_long = false;
-  extern __shared__ int long_slots[];  // LONG: [8*G*RPG] slots, then the partials
-  const int cg = (threadIdx.x >> 5) * G + g;
 #pragma unroll
   for (int q = 0; q < RPG; ++q) {
-    bool ok = active && base + q < mb;
+    bool ok = base + q < mb;
     s[q] = ok ? __ldg(row + base + q) : 0;
     e[q] = ok ? __ldg(row + base + q + 1) : 0;
-    skip[q] = false;
-    if constexpr (LONG) {
-      skip[q] = e[q] - s[q] > kLongSpmvRow;
-      if (g < G && r == 0) long_slots[cg * RPG + q] = skip[q] ? (int)(base + q) : -1;
-      if (skip[q]) e[q] = s[q];
-      mine_long |= skip[q];
-    }
   }
   AccT acc[RPG];
 #pragma unroll
   for (int q = 0; q < RPG; ++q) acc[q] = 0;
   // batches of U blocks per row; every load of a batch (column indices,
   // block rows, x segments) is issued before its FMAs
-  for (int off = 0; active; off += U) {
+  for (int off = 0;; off += U) {
     bool any = false;
 #pragma unroll
     for (int q = 0; q < RPG; ++q) any |= s[q] + off < e[q];
@@ -260,104 +256,338 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
   }
 #pragma unroll
   for (int q = 0; q < RPG; ++q)
-    if (active && base + q < mb && !skip[q]) {
+    if (base + q < mb) {
       y[(base + q) * BS + r] = (YT)acc[q];
       if (y32) y32[(base + q) * BS + r] = (float)acc[q];  // optional FP32 copy
     }
-  if constexpr (LONG) {
-    constexpr int NSLOT = 8 * G * RPG;
-    // one CTA barrier, which also says whether the CTA holds a long row
-    if (__syncthreads_or(mine_long))
-      spmv_long_rows<BS, VT, XT, YT, AccT, NSLOT, 8 * G, TR>(
-          long_slots, row, col, src, val, x, y, y32,
-          reinterpret_cast<AccT*>(long_slots + ((NSLOT + 1) & ~1)), g < G, cg, r);
+}
+
+// The same product with FP32 values for patterns with rows of more than
+// kLongSpmvRow blocks (power-law: rows of ~7 blocks on average, many of one or
+// two, hubs of up to 2000).  A group that walks a row alone waits for memory
+// about once a batch, so the batches are deep; a warp owns `rw` consecutive
+// rows and its lane groups take them one after another as they finish (the row
+// pointers sit in the lanes' registers: taking a row is a ballot and two
+// shuffles).  Rows of more than kLongSpmvRow blocks are summed by the CTA at
+// the end.  Every sum runs in the order of a row per group.  62,500-row
+// power-law ISAI factors, the apply: 8x8 blocks 151 -> 122 us, 4x4 92 -> 72 us.
+constexpr int kUnevenMaxRows = 16;
+
+template <int BS, class VT, class XT, class YT, class AccT, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_bsr_spmv_uneven(int mb, int rw,
+                                                               const int* __restrict__ row,
+                                                               const int* __restrict__ col,
+                                                               const VT* __restrict__ val,
+                                                               const XT* __restrict__ x,
+                                                               YT* __restrict__ y,
+                                                               float* __restrict__ y32) {
+  constexpr int G = 32 / BS;
+  constexpr int NSLOT = 8 * kUnevenMaxRows;
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ int long_slots[];  // [NSLOT] slots, then the partials
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane / BS, r = lane - g * BS;
+  const long long r0 = ((long long)blockIdx.x * 8 + warp) * rw;
+  const int nrow = (int)max(0ll, min((long long)rw, mb - r0));
+  int sl = 0, el = 0;  // lane l < nrow: row r0 + l
+  if (lane < nrow) {
+    sl = __ldg(row + r0 + lane);
+    el = __ldg(row + r0 + lane + 1);
   }
+  const bool lng = el - sl > kLongSpmvRow;
+  if (lane < kUnevenMaxRows) long_slots[warp * kUnevenMaxRows + lane] = lng ? (int)(r0 + lane) : -1;
+  const unsigned skip = __ballot_sync(kAll, lng);
+  if (lng) el = sl;
+  int next = 0, cur = -1, p = 0, e = 0;
+  AccT acc = 0;
+  bool on = g < G;
+  while (true) {
+    const bool need = on && p >= e;
+    if (need && cur >= 0 && !((skip >> cur) & 1u)) {
+      y[(r0 + cur) * BS + r] = (YT)acc;
+      if (y32) y32[(r0 + cur) * BS + r] = (float)acc;
+    }
+    const unsigned want = __ballot_sync(kAll, need && r == 0);
+    const int idx = next + __popc(want & ((1u << (g * BS)) - 1u));
+    next += __popc(want);
+    const int from = min(idx, kUnevenMaxRows - 1);
+    const int ps = __shfl_sync(kAll, sl, from), pe = __shfl_sync(kAll, el, from);
+    if (need) {
+      on = idx < nrow;
+      cur = idx;
+      p = ps;
+      e = on ? pe : ps;
+      acc = 0;
+    }
+    if (!__any_sync(kAll, on)) break;
+    int c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = p + u < e ? __ldg(col + p + u) : -1;
+    AccT a[U][BS];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0) load_row<BS, VT, AccT>(val, p + u, r, a[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0) {
+        AccT xv[BS];
+        load_x<BS, XT, AccT>(x, c[u], xv);
+#pragma unroll
+        for (int k = 0; k < BS; ++k) acc = fma(a[u][k], xv[k], acc);
+      }
+    p += U;
+  }
+  // one CTA barrier, which also says whether the CTA holds a long row
+  if (__syncthreads_or(skip != 0))
+    spmv_long_rows<BS, VT, XT, YT, AccT, NSLOT, 8 * G>(
+        long_slots, row, col, val, x, y, y32, reinterpret_cast<AccT*>(long_slots + NSLOT),
+        g < G, warp * G + g, r);
+}
+
+// The same product with FP64 values for those patterns, bound by the FP64 pipe
+// (an FP64 warp instruction costs the same with one lane group active as with
+// all, and a row per group left half of them idle; one SM alone takes 30 us for
+// a hub of 1900 8x8 blocks).  A cluster of kBalCluster CTAs owns `rows`
+// consecutive rows and splits their blocks, not their rows, evenly among all
+// its lane groups: a group streams its run of blocks, storing a row's sum where
+// the row ends inside the run.  A row that goes on into the next groups' runs is
+// finished by the group it starts in, which adds the others' heads in order:
+// those of its CTA from shared memory, one sum of each later CTA's (so a sum's
+// order depends on the pattern alone).  62,500-row power-law ISAI factors, 8x8
+// blocks (the apply: two products, 88 us of DFMA): 320 -> 152 us; 4x4 151 -> 69.
+constexpr int kBalCluster = 8;
+constexpr int kBalMaxRows = 1024;
+
+template <int BS, int U, int MINB, bool TR>
+__global__ void __launch_bounds__(256, MINB) k_bsr_spmv_balanced(
+    int mb, int rows, const int* __restrict__ row, const int* __restrict__ col,
+    const int* __restrict__ src, const double* __restrict__ val, const double* __restrict__ x,
+    double* __restrict__ y, float* __restrict__ y32) {
+  namespace cgr = cooperative_groups;
+  constexpr int G = 32 / BS, NG = 8 * G, NGC = NG * kBalCluster;
+  __shared__ int rp[kBalMaxRows + 1];
+  __shared__ double head_s[NG][BS];
+  __shared__ double chead_s[BS];
+  cgr::cluster_group cl = cgr::this_cluster();
+  const int rank = (int)cl.block_rank();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane / BS, r = lane - g * BS;
+  const long long r0 = (long long)(blockIdx.x / kBalCluster) * rows;
+  const int n = (int)min((long long)rows, mb - r0);
+  for (int t = threadIdx.x; t <= n; t += 256) rp[t] = __ldg(row + r0 + t);
+  __syncthreads();
+  for (int t = rank * 256 + threadIdx.x; t < n * BS; t += 256 * kBalCluster)
+    if (rp[t / BS] == rp[t / BS + 1]) {  // empty rows
+      y[r0 * BS + t] = 0.0;
+      if (y32) y32[r0 * BS + t] = 0.f;
+    }
+  const int b0 = rp[0];
+  const long long T = rp[n] - b0;
+  auto start = [&](int q) { return b0 + (int)(T * q / NGC); };  // group q's run
+  auto row_at = [&](int p) {  // last row starting at or before p: the one holding block p
+    int lo = 0, up = n - 1;
+    while (lo < up) {
+      const int m = (lo + up + 1) >> 1;
+      if (rp[m] <= p) lo = m; else up = m - 1;
+    }
+    return lo;
+  };
+  const int q0 = rank * NG, gi = q0 + warp * G + g;
+  int p = g < G ? start(gi) : 0;
+  const int hi = g < G ? start(gi + 1) : 0;
+  double acc = 0.0;
+  int cur = 0, e = 0;
+  bool head = false, open = false;  // the row started before this run; acc is of a row
+  if (p < hi) {
+    cur = row_at(p);
+    e = rp[cur + 1];
+    head = rp[cur] < p;
+    open = true;
+  }
+  while (p < hi) {
+    int c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = p + u < hi ? __ldg(col + p + u) : -1;
+    double a[U][BS];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0) load_entry<BS, TR, double, double>(val, src, p + u, r, a[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0) {
+        double xv[BS];
+        load_x<BS, double, double>(x, c[u], xv);
+#pragma unroll
+        for (int k = 0; k < BS; ++k) acc = fma(a[u][k], xv[k], acc);
+        if (p + u + 1 == e) {  // the row ends here
+          if (head) {
+            head_s[gi - q0][r] = acc;
+          } else {
+            y[(r0 + cur) * BS + r] = acc;
+            if (y32) y32[(r0 + cur) * BS + r] = (float)acc;
+          }
+          head = false;
+          acc = 0.0;
+          open = e < hi;
+          if (open) {
+            do e = rp[++cur + 1];
+            while (e == p + u + 1);
+          }
+        }
+      }
+    p += U;
+  }
+  if (open && head) head_s[gi - q0][r] = acc;  // a row that fills the whole run
+  __syncthreads();
+  bool more = false;  // the row goes on in the next CTA
+  if (open && !head) {
+    for (int q = gi + 1; q < q0 + NG; ++q) {
+      const int s = start(q);
+      if (s >= e) break;
+      if (s < start(q + 1)) acc += head_s[q - q0][r];
+    }
+    more = start(q0 + NG) < e;
+    if (!more) {
+      y[(r0 + cur) * BS + r] = acc;
+      if (y32) y32[(r0 + cur) * BS + r] = (float)acc;
+    }
+  }
+  // this CTA's part of a row that started in an earlier one
+  const int cs = start(q0), ce = start(q0 + NG);
+  if (threadIdx.x < BS && cs < ce) {
+    const int k = row_at(cs), end = rp[k + 1];
+    if (rp[k] < cs) {
+      double t = 0.0;
+      for (int q = q0; q < q0 + NG; ++q) {
+        const int s = start(q);
+        if (s >= end) break;
+        if (s < start(q + 1)) t += head_s[q - q0][threadIdx.x];
+      }
+      chead_s[threadIdx.x] = t;
+    }
+  }
+  cl.sync();
+  if (more) {
+    for (int c = rank + 1; c < kBalCluster; ++c) {
+      const int s = start(c * NG);
+      if (s >= e) break;
+      if (s < start((c + 1) * NG)) acc += cl.map_shared_rank(chead_s, c)[r];
+    }
+    y[(r0 + cur) * BS + r] = acc;
+    if (y32) y32[(r0 + cur) * BS + r] = (float)acc;
+  }
+  cl.sync();  // nobody leaves while its sums may be read
 }
 
 // Layout word of a matrix for the SpMV: bit 0 = rows of more than
-// kLongSpmvRow blocks present (the LONG instance); bit 1 = more than
+// kLongSpmvRow blocks present (k_bsr_spmv_balanced, _uneven); bit 1 = more than
 // kWideSpmvRow blocks a row on average (FP32 values: one row per lane
-// group).  (Taking several blocks of a row side by side, or rows in length
-// order, was measured slower on the power-law patterns: the product is
-// latency-bound there, not bound by the lanes an uneven warp leaves idle.)
+// group).
 constexpr int kLayoutLong = 1;
 constexpr int kLayoutWide = 2;
 constexpr int kWideSpmvRow = 5;
 
-template <int BS, class VT, class XT, class YT, int RPG, int U, int MINB, bool LONG,
-          bool TR = false>
+template <int BS, class VT, class XT, class YT, int RPG, int U, int MINB, bool TR = false>
 int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
                     cudaStream_t st, float* y32, const int* src = nullptr) {
-  using AccT = VT;
   constexpr int G = 32 / BS;
   long long groups = (mb + RPG - 1) / RPG;
   long long warps = (groups + G - 1) / G;
-  unsigned grid = ceil_div(warps, 8);
-  if constexpr (LONG) {
-    constexpr int NSLOT = 8 * G * RPG;
-    const size_t smem = sizeof(int) * ((NSLOT + 1) & ~1) + sizeof(AccT) * 8 * G * BS;
-    k_bsr_spmv<BS, VT, XT, YT, AccT, RPG, U, MINB, true, TR><<<grid, 256, smem, st>>>(
-        mb, row, col, src, val, x, y, y32);
-  } else {
-    k_bsr_spmv<BS, VT, XT, YT, AccT, RPG, U, MINB, false, TR><<<grid, 256, 0, st>>>(
-        mb, row, col, src, val, x, y, y32);
-  }
+  k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR><<<ceil_div(warps, 8), 256, 0, st>>>(
+      mb, row, col, src, val, x, y, y32);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
 
-// Patterns with long rows (power-law: rows of ~12 blocks on average, hubs
-// of up to 2000) are latency-bound per lane group and keep two blocks a
-// batch (FP64) or two rows a group (FP32); the configurations measured
-// faster on the stencil patterns (above) apply to patterns without long
-// rows, FP64 at block sizes 4 and 5.
+// Rows per warp: as many as leave two warps for every one that can be resident
+// (balance), at least one per lane group, at most kUnevenMaxRows.
+template <int BS, class XT, class YT, int U, int MINB>
+int launch_spmv_uneven(int mb, const int* row, const int* col, const float* val, const XT* x,
+                       YT* y, cudaStream_t st, float* y32) {
+  const int rw = std::max(32 / BS, std::min(kUnevenMaxRows, mb / (152 * 8 * MINB * 2)));
+  constexpr size_t smem = sizeof(int) * 8 * kUnevenMaxRows + sizeof(float) * 8 * (32 / BS) * BS;
+  k_bsr_spmv_uneven<BS, float, XT, YT, float, U, MINB>
+      <<<ceil_div(mb, 8ll * rw), 256, smem, st>>>(mb, rw, row, col, val, x, y, y32);
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
+
+// Rows per cluster: as many as leave one CTA (8x8 blocks: two) for every one that
+// can be resident -- the two barriers of a cluster cost more than a second wave
+// balances while the blocks are small (62,500 rows, the apply, 1 / 2 / 3 / 6
+// waves: 4x4 69 / 77 / 92 / 141 us, 8x8 163 / 152 / 155 / 185 us) -- at least 64,
+// at most kBalMaxRows.
+
+template <int BS, int U, int MINB, bool TR>
+int launch_spmv_balanced(int mb, const int* row, const int* col, const int* src,
+                         const double* val, const double* x, double* y, cudaStream_t st,
+                         float* y32) {
+  const long long per = (long long)mb * kBalCluster / (152 * MINB * (BS == 8 ? 2 : 1));
+  const int rows = (int)std::max(64ll, std::min((long long)kBalMaxRows, per));
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kBalCluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div(mb, rows) * kBalCluster);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  BILU_TRY_CUDA(cudaLaunchKernelEx(&cfg, k_bsr_spmv_balanced<BS, U, MINB, TR>, mb, rows, row, col,
+                                   src, val, x, y, y32));
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
+
+// The configurations measured faster on the stencil patterns (k_bsr_spmv)
+// apply to patterns without long rows, FP64 at block sizes 4 and 5.
 template <int BS, class VT, class XT, class YT>
 int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
                 cudaStream_t st, int layout, float* y32 = nullptr) {
   if (mb == 0) return BILU_OK;
-  const bool lng = (layout & kLayoutLong) != 0;
-  if constexpr (sizeof(VT) == 8) {
-    if (lng)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 2, 2, true>(mb, row, col, val, x, y, st, y32);
-    if constexpr (BS <= 5)
-      return launch_spmv_cfg<BS, VT, XT, YT, 2, 1, 4, false>(mb, row, col, val, x, y, st, y32);
+  if (layout & kLayoutLong) {
+    if constexpr (sizeof(VT) == 8)
+      return launch_spmv_balanced<BS, 2, 4, false>(mb, row, col, nullptr, val, x, y, st, y32);
     else
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 2, 2, false>(mb, row, col, val, x, y, st, y32);
+      return launch_spmv_uneven<BS, XT, YT, BS == 4 ? 4 : 8, BS == 4 ? 4 : 2>(mb, row, col, val, x,
+                                                                             y, st, y32);
+  }
+  if constexpr (sizeof(VT) == 8) {
+    if constexpr (BS <= 5)
+      return launch_spmv_cfg<BS, VT, XT, YT, 2, 1, 4>(mb, row, col, val, x, y, st, y32);
+    else
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 2, 2>(mb, row, col, val, x, y, st, y32);
   } else if constexpr (BS == 8 && sizeof(XT) == 8) {
     // two rows of 8x8 blocks with FP64 x segments spill at 64 registers
-    if (lng)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4, true>(mb, row, col, val, x, y, st, y32);
-    return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4, false>(mb, row, col, val, x, y, st, y32);
+    return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32);
   } else {
-    if (lng)
-      return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4, true>(mb, row, col, val, x, y, st, y32);
     if (layout & kLayoutWide)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4, false>(mb, row, col, val, x, y, st, y32);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32);
     // bs 4 rows of ~4 blocks (the ISAI triangles of a 7-point pattern): one
     // row per group at 32 registers, 8 CTAs per SM (0.2214 -> 0.2185 ms
     // for the 128^3 inner apply)
     if constexpr (BS == 4)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8, false>(mb, row, col, val, x, y, st, y32);
-    return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4, false>(mb, row, col, val, x, y, st, y32);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8>(mb, row, col, val, x, y, st, y32);
+    return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4>(mb, row, col, val, x, y, st, y32);
   }
 }
 
 // y = M^T x from M's values and the transposed pattern (launch_spmv's FP64
-// configurations, so the sums run in the order of a product with the
-// transposed matrix: the same bits).
+// kernels, so the sums run in the order of a product with the transposed
+// matrix).
 template <int BS>
 int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, const double* val,
                   const double* x, double* y, cudaStream_t st, int layout) {
   using D = double;
   if (layout & kLayoutLong)
-    return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, true, true>(mb, trow, tcol, val, x, y, st,
-                                                             nullptr, src);
+    return launch_spmv_balanced<BS, 2, 4, true>(mb, trow, tcol, src, val, x, y, st, nullptr);
   if constexpr (BS <= 5)
-    return launch_spmv_cfg<BS, D, D, D, 2, 1, 4, false, true>(mb, trow, tcol, val, x, y, st,
-                                                              nullptr, src);
+    return launch_spmv_cfg<BS, D, D, D, 2, 1, 4, true>(mb, trow, tcol, val, x, y, st, nullptr,
+                                                       src);
   else
-    return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, false, true>(mb, trow, tcol, val, x, y, st,
-                                                              nullptr, src);
+    return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, true>(mb, trow, tcol, val, x, y, st, nullptr,
+                                                       src);
 }
 
 // Multi-RHS: Y[n,k] = M X[n,k], row-major with ld = k.  One warp per block

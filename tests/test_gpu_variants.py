@@ -314,3 +314,50 @@ def test_masked_outer_runs(cuda, name, bs, scale):
     assert np.array_equal(N(api.masked_outer(*args)), ref)
     added = N(api.masked_outer(*args, G=T(G0, cuda)))
     assert np.max(np.abs(added - (G0 + ref)), initial=0.0) <= 2.0 ** -52 * 3  # fused or not
+
+
+# ------------------------------------------------------------------ uneven rows
+def uneven_pattern(name):
+    """Row lengths around the splits: (nb, longest) per name."""
+    rng = np.random.default_rng(29)
+    n = {"one hub": 70, "hubs": 1500, "all long": 66, "big": 9000}[name]
+    length = rng.integers(0, 5, size=n)
+    if name == "one hub":
+        length[33] = 70
+    elif name == "all long":
+        length[:] = 66
+    else:
+        length[rng.integers(0, n, size=n // 60)] = rng.integers(40, 100, size=n // 60)
+        length[[0, n // 2, n - 1]] = min(n, 1400)
+    cols = [np.sort(rng.choice(n, size=k, replace=False)) for k in length]
+    rp = np.zeros(n + 1, np.int32)
+    np.cumsum(length, out=rp[1:])
+    return rp, np.concatenate(cols).astype(np.int32)
+
+
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("name", ["one hub", "hubs", "all long", "big"])
+def test_uneven_rows_product(cuda, orc, name, bs):
+    """Products over rows of 0 to 1400 blocks (empty rows among them).  FP64:
+    a sum of N products of numbers in [-1, 1] is within N 2^-53 (N of them) of
+    any other order.  FP32: against the same bound at 2^-24; the same call
+    twice gives the same bits."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    rp, col = uneven_pattern(name)
+    nb = len(rp) - 1
+    rng = np.random.default_rng(bs)
+    val, x = rng.uniform(-1, 1, size=(len(col), bs, bs)), rng.uniform(-1, 1, size=nb * bs)
+    terms = np.repeat(np.diff(rp) * bs, bs).astype(float)
+    ref = orc.bcsr_spmv(nb, bs, rp, col, val, x)
+    r, c, v, xd = T(rp, cuda), T(col, cuda), T(val, cuda), T(x, cuda)
+    y = api.bcsr_spmv(nb, bs, r, c, v, xd)
+    assert torch.equal(y, api.bcsr_spmv(nb, bs, r, c, v, xd))
+    assert np.all(np.abs(N(y) - ref) <= terms * terms * 2.0 ** -53)
+    v32 = v.float()
+    ref32 = orc.bcsr_spmv(nb, bs, rp, col, N(v32).astype(np.float64), N(xd.float()).astype(np.float64))
+    y32 = api.bcsr_spmv(nb, bs, r, c, v32, xd.float())
+    assert torch.equal(y32, api.bcsr_spmv(nb, bs, r, c, v32, xd.float()))
+    assert np.all(np.abs(N(y32) - ref32) <= terms * terms * 2.0 ** -24)
