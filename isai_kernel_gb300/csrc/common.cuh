@@ -112,6 +112,58 @@ __device__ __forceinline__ float ld_stream(const float* p) {
   return v;
 }
 
+// The bits of a double (hi, lo) whose rounding to FP32 is a normal number or
+// infinity, rounded.
+__device__ __forceinline__ float narrow_normal(unsigned hi, unsigned lo) {
+  // nine exponent bits and the first 23 of the fraction; the exponents in
+  // question, 897 to 1150, differ from FP32's by 384 modulo 512
+  const unsigned m = __funnelshift_l(lo, hi, 3);
+  // the 29 bits left over against one half, ties to even (a carry may run into
+  // the exponent, up to infinity)
+  const unsigned up = ((lo << 3) | (m & 1u)) > 0x80000000u ? 1u : 0u;
+  return __uint_as_float((m - (384u << 23) + up) | (hi & 0x80000000u));
+}
+
+// double -> float, round to nearest even, on the integer pipe: the same bits as
+// the conversion instruction, which runs at the FP64 rate on GB300 (64 cycles a
+// warp instruction per SM sub-partition against about 9 for this).  A value
+// whose result is neither zero nor a normal float (subnormal, overflow, NaN)
+// takes the instruction.
+__device__ __forceinline__ float narrow(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  if ((hi & 0x7fffffffu) - (897u << 20) >= (254u << 20)) {
+    if (((hi << 1) | lo) == 0) return __uint_as_float(hi);
+    return __double2float_rn(d);
+  }
+  return narrow_normal(hi, lo);
+}
+
+// narrow() of N values with one branch for all of them.
+template <int N>
+__device__ __forceinline__ void narrow_all(const double (&d)[N], float (&f)[N]) {
+  unsigned worst = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const unsigned hi = (unsigned)__double2hiint(d[i]), lo = (unsigned)__double2loint(d[i]);
+    worst = max(worst, (hi & 0x7fffffffu) - (897u << 20));
+    f[i] = narrow_normal(hi, lo);
+  }
+  if (worst >= (254u << 20)) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = narrow(d[i]);
+  }
+}
+
+// float -> double (exact), likewise on the integer pipe.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+  if (a - 0x00800000u >= 0x7f000000u) {  // zero, subnormal, infinity, NaN
+    if (a == 0) return __hiloint2double((int)u, 0);
+    return (double)f;
+  }
+  return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + (896u << 20))), (int)(u << 29));
+}
+
 // The entries [s, e) of a pattern row per thread, f(row, p) for each: a thread
 // walks its own row, except that rows of more than kSharedRow entries are
 // walked by the whole warp, 32 entries at a time (one thread alone takes

@@ -590,63 +590,242 @@ int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, cons
                                                        src);
 }
 
-// Multi-RHS: Y[n,k] = M X[n,k], row-major with ld = k.  One warp per block
-// row; lane c (and c+32) owns right-hand side c; blocks are broadcast reads.
-template <int BS, class VT, int KW>
-__global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k, const int* __restrict__ row,
+// Multi-RHS: Y[n,k] = M X[n,k], row-major with ld = k.  LPR lanes per block row
+// (32 / LPR rows a warp), lane l owning right-hand sides l, l + LPR, ... (KW of
+// them); every block is read by its lanes at once, row by row.  The FP64 product
+// is bound by the FP64 pipe, whose warp instructions cost the same whatever the
+// lanes, so LPR and KW are chosen to leave few of them without a right-hand
+// side (launch_spmm).  With FP32 values X is rounded to FP32 where it is read
+// and the sums are widened where they are stored, on the integer pipe: the
+// conversion instructions run on the FP64 pipe and were the bound (512 x 512
+// 5-point grid, 4x4 blocks, k 32: 342 -> 220 us, 92 us of HBM, bound by issue and L1).  Sums run in
+// block order, then column order, whatever LPR and KW are.
+// Rows of more than kLongSpmvRow blocks (a group alone takes ~0.5 us a block, a
+// millisecond for a hub of 2000) are left to k_spmm_hubs.
+// vec: val starts on a 16-byte boundary (else blocks are read element by element)
+template <int BS, class VT>
+__device__ __forceinline__ void spmm_row(const VT* __restrict__ val, long long p, int r, int vec,
+                                         VT* a) {
+  if (vec) {
+    load_row<BS, VT, VT>(val, p, r, a);
+  } else {
+#pragma unroll
+    for (int kk = 0; kk < BS; ++kk) a[kk] = __ldg(val + (p * BS + r) * BS + kk);
+  }
+}
+
+// X in the precision of the product
+template <int N>
+__device__ __forceinline__ void spmm_in(const double (&d)[N], double (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = d[i];
+}
+template <int N>
+__device__ __forceinline__ void spmm_in(const double (&d)[N], float (&v)[N]) {
+  if constexpr (N == 1) v[0] = narrow(d[0]);
+  else narrow_all<N>(d, v);
+}
+// what a lane without a right-hand side works on (1: a zero would send its warp
+// down narrow()'s branch)
+constexpr double kNoRhs = 1.0;
+
+template <class VT>
+__device__ __forceinline__ double spmm_out(VT v) {
+  if constexpr (sizeof(VT) == 4) return widen(v);
+  else return v;
+}
+
+// The long rows of the product, a CTA per kHubRows block rows, which looks for
+// them (most CTAs find none; a launch of its own so that the short rows' kernel
+// keeps its registers).  With FP64 values the CTA's groups of LPR lanes share a
+// row's blocks, U in flight each; FP32 sums keep their order, so there a group
+// takes one scalar row of the block row.  20,000-row power-law pattern, 4x4
+// blocks, k 32, the whole product: FP64 2461 -> 590 us, FP32 1023 -> 470 us.
+constexpr int kHubRows = 64;
+
+template <int BS, class VT, int LPR>
+__global__ void __launch_bounds__(256) k_spmm_hubs(int mb, int k, int vec,
+                                                   const int* __restrict__ row,
+                                                   const int* __restrict__ col,
+                                                   const VT* __restrict__ val,
+                                                   const double* __restrict__ X,
+                                                   double* __restrict__ Y) {
+  constexpr bool SHARE = sizeof(VT) == 8;
+  constexpr int GW = 32 / LPR, NG = 8 * GW;
+  constexpr int U = SHARE ? (BS <= 5 ? 4 : 2) : 8;
+  __shared__ double part_s[SHARE ? 8 * BS * LPR : 1];
+  __shared__ int list_s[kHubRows];
+  const int lane = threadIdx.x & 31, l = lane & (LPR - 1), warp = threadIdx.x >> 5;
+  const int gi = warp * GW + lane / LPR;
+  bool lng = false;
+  if (threadIdx.x < kHubRows) {
+    const long long i = (long long)blockIdx.x * kHubRows + threadIdx.x;
+    lng = i < mb && __ldg(row + i + 1) - __ldg(row + i) > kLongSpmvRow;
+    list_s[threadIdx.x] = lng ? (int)i : -1;
+  }
+  if (!__syncthreads_or(lng)) return;
+  for (int h = 0; h < kHubRows; ++h) {
+    const int hub = list_s[h];
+    if (hub < 0) continue;  // uniform across the CTA
+    const int hs = __ldg(row + hub), he = __ldg(row + hub + 1);
+    for (int k0 = 0; k0 < k; k0 += LPR) {
+      const bool in = k0 + l < k;
+      const double* Xc = X + k0 + l;
+      if constexpr (SHARE) {
+        double acc[BS];
+#pragma unroll
+        for (int r = 0; r < BS; ++r) acc[r] = 0;
+        for (int q = hs + gi; q < he; q += NG * U) {
+          double xv[U][BS];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const double* xb = Xc + (long long)__ldg(col + min(q + u * NG, he - 1)) * BS * k;
+#pragma unroll
+            for (int kk = 0; kk < BS; ++kk) xv[u][kk] = in ? __ldg(xb + (long long)kk * k) : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (q + u * NG >= he) break;
+#pragma unroll
+            for (int r = 0; r < BS; ++r) {
+              double a[BS];
+              spmm_row<BS, double>(val, q + u * NG, r, vec, a);
+#pragma unroll
+              for (int kk = 0; kk < BS; ++kk) acc[r] = fma(a[kk], xv[u][kk], acc[r]);
+            }
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < BS; ++r) {
+#pragma unroll
+          for (int o = LPR; o < 32; o <<= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+          if (lane < LPR) part_s[(warp * BS + r) * LPR + l] = acc[r];
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < BS * LPR; t += 256) {
+          const int r = t / LPR, c = k0 + t % LPR;
+          double sum = 0.0;
+#pragma unroll
+          for (int w = 0; w < 8; ++w) sum += part_s[(w * BS + r) * LPR + t % LPR];
+          if (c < k) Y[((long long)hub * BS + r) * k + c] = sum;
+        }
+        __syncthreads();
+      } else if (gi < BS) {
+        VT t = 0;
+        for (int q = hs; q < he; q += U) {
+          double xd[U][BS];
+          VT a[U][BS];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int p = min(q + u, he - 1);
+            const double* xb = Xc + (long long)__ldg(col + p) * BS * k;
+#pragma unroll
+            for (int kk = 0; kk < BS; ++kk)
+              xd[u][kk] = in ? __ldg(xb + (long long)kk * k) : kNoRhs;
+            spmm_row<BS, VT>(val, p, gi, vec, a[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (q + u < he) {
+              VT xv[BS];
+              spmm_in<BS>(xd[u], xv);
+#pragma unroll
+              for (int kk = 0; kk < BS; ++kk) t = fma(a[u][kk], xv[kk], t);
+            }
+        }
+        if (in) Y[((long long)hub * BS + gi) * k + k0 + l] = spmm_out(t);
+      }
+    }
+  }
+}
+
+// FULL: k is LPR KW and val is aligned, known to the compiler (immediate offsets,
+// no predicates or branches).
+template <int BS, class VT, int LPR, int KW, bool FULL>
+__global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any,
+                                                  const int* __restrict__ row,
                                                   const int* __restrict__ col,
                                                   const VT* __restrict__ val,
                                                   const double* __restrict__ X,
                                                   double* __restrict__ Y) {
-  using AccT = VT;
-  int lane = threadIdx.x & 31;
-  long long br = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int k = FULL ? LPR * KW : k_any, vec = FULL ? 1 : vec_any;
+  const int lane = threadIdx.x & 31, l = lane & (LPR - 1);
+  const long long br =
+      ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / LPR) + lane / LPR;
   if (br >= mb) return;
-  AccT acc[KW][BS];
+  const int e = __ldg(row + br + 1);
+  int p = __ldg(row + br);
+  if (e - p > kLongSpmvRow) return;
+  VT acc[KW][BS];
 #pragma unroll
   for (int w = 0; w < KW; ++w)
 #pragma unroll
     for (int r = 0; r < BS; ++r) acc[w][r] = 0;
-  int s = row[br], e = row[br + 1];
-  for (int p = s; p < e; ++p) {
-    long long bc = col[p];
-    const VT* blk = val + (long long)p * BS * BS;
+  int bc = p < e ? __ldg(col + p) : 0;
+  for (; p < e; ++p) {
+    const double* xb = X + (long long)bc * BS * k + l;
+    double xd[BS * KW];
 #pragma unroll
-    for (int kk = 0; kk < BS; ++kk) {
-      AccT xv[KW];
+    for (int kk = 0; kk < BS; ++kk)
 #pragma unroll
-      for (int w = 0; w < KW; ++w) {
-        int c = lane + 32 * w;
-        xv[w] = c < k ? (AccT)X[(bc * BS + kk) * k + c] : (AccT)0;
-      }
+      for (int w = 0; w < KW; ++w)
+        xd[kk * KW + w] = l + LPR * w < k ? __ldg(xb + kk * k + LPR * w) : kNoRhs;
+    if (p + 1 < e) bc = __ldg(col + p + 1);
+    // FP32: the next block's X on its way (250 -> 220 us on the grid above; the
+    // FP64 product has the time)
+    if (sizeof(VT) == 4 && p + 1 < e)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(X + (long long)bc * BS * k + l));
+    VT xv[BS * KW];
 #pragma unroll
-      for (int r = 0; r < BS; ++r) {
-        AccT a = (AccT)blk[r * BS + kk];
+    for (int i = 0; i < BS * KW; ++i) spmm_in<1>({xd[i]}, reinterpret_cast<VT(&)[1]>(xv[i]));
 #pragma unroll
-        for (int w = 0; w < KW; ++w) acc[w][r] = fma(a, xv[w], acc[w][r]);
-      }
+    for (int r = 0; r < BS; ++r) {
+      VT a[BS];
+      spmm_row<BS, VT>(val, p, r, vec, a);
+#pragma unroll
+      for (int kk = 0; kk < BS; ++kk)
+#pragma unroll
+        for (int w = 0; w < KW; ++w) acc[w][r] = fma(a[kk], xv[kk * KW + w], acc[w][r]);
     }
   }
 #pragma unroll
-  for (int w = 0; w < KW; ++w) {
-    int c = lane + 32 * w;
-    if (c < k)
+  for (int w = 0; w < KW; ++w)
+    if (l + LPR * w < k)
 #pragma unroll
-      for (int r = 0; r < BS; ++r) Y[(br * BS + r) * k + c] = (double)acc[w][r];
-  }
+      for (int r = 0; r < BS; ++r) Y[(br * BS + r) * k + l + LPR * w] = spmm_out(acc[w][r]);
 }
 
+template <int BS, class VT, int LPR, int KW>
+int launch_spmm_cfg(int mb, int k, const int* row, const int* col, const VT* val, const double* X,
+                    double* Y, cudaStream_t st) {
+  const int vec = (uintptr_t)val % 16 == 0;
+  const unsigned grid = ceil_div(mb, 8 * (32 / LPR));
+  if (k == LPR * KW && vec)
+    k_bsr_spmm<BS, VT, LPR, KW, true><<<grid, 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
+  else
+    k_bsr_spmm<BS, VT, LPR, KW, false><<<grid, 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
+  BILU_LAUNCH_CHECK();
+  if (mb > kLongSpmvRow) {  // as many blocks in a row need as many columns
+    k_spmm_hubs<BS, VT, sizeof(VT) == 8 ? LPR : 32>
+        <<<ceil_div(mb, kHubRows), 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
+    BILU_LAUNCH_CHECK();
+  }
+  return BILU_OK;
+}
+
+// The lanes' padding decides: k right-hand sides take ceil(k / LPR) LPR slots.
 template <int BS, class VT>
 int launch_spmm(int mb, int k, const int* row, const int* col, const VT* val, const double* X,
                 double* Y, cudaStream_t st) {
   if (mb == 0) return BILU_OK;
-  unsigned grid = ceil_div(mb, 8);
-  if (k <= 32)
-    k_bsr_spmm<BS, VT, 1><<<grid, 256, 0, st>>>(mb, k, row, col, val, X, Y);
-  else
-    k_bsr_spmm<BS, VT, 2><<<grid, 256, 0, st>>>(mb, k, row, col, val, X, Y);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  if (k <= 4) return launch_spmm_cfg<BS, VT, 4, 1>(mb, k, row, col, val, X, Y, st);
+  if (k <= 8) return launch_spmm_cfg<BS, VT, 8, 1>(mb, k, row, col, val, X, Y, st);
+  if (k <= 16) return launch_spmm_cfg<BS, VT, 16, 1>(mb, k, row, col, val, X, Y, st);
+  if (k <= 24) return launch_spmm_cfg<BS, VT, 8, 3>(mb, k, row, col, val, X, Y, st);
+  if (k <= 32) return launch_spmm_cfg<BS, VT, 32, 1>(mb, k, row, col, val, X, Y, st);
+  if (k <= 48) return launch_spmm_cfg<BS, VT, 16, 3>(mb, k, row, col, val, X, Y, st);
+  return launch_spmm_cfg<BS, VT, 32, 2>(mb, k, row, col, val, X, Y, st);
 }
 
 __global__ void k_f64_to_f32(size_t n, const double* __restrict__ s, float* __restrict__ d) {

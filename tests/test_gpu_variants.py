@@ -361,3 +361,51 @@ def test_uneven_rows_product(cuda, orc, name, bs):
     y32 = api.bcsr_spmv(nb, bs, r, c, v32, xd.float())
     assert torch.equal(y32, api.bcsr_spmv(nb, bs, r, c, v32, xd.float()))
     assert np.all(np.abs(N(y32) - ref32) <= terms * terms * 2.0 ** -24)
+
+
+# ------------------------------------------------------------------ several right-hand sides
+@pytest.mark.parametrize("k", [1, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("bs", [4, 5, 8])
+def test_spmm_splits(cuda, orc, bs, k):
+    """Every lane split at its edges, over rows of 0 to 70 blocks, against the
+    column-by-column product: N products of numbers in [-1, 1] are within
+    N 2^-53 (2^-24 for FP32-stored values) of any order, N of them.  A
+    right-hand side of zeros, infinities and subnormals converts as IEEE says."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    rp, col = uneven_pattern("one hub")
+    nb = len(rp) - 1
+    rng = np.random.default_rng(100 * bs + k)
+    val, X = rng.uniform(-1, 1, size=(len(col), bs, bs)), rng.uniform(-1, 1, size=(nb * bs, k))
+    terms = (np.repeat(np.diff(rp) * bs, bs).astype(float) ** 2)[:, None]
+    r, c, v = T(rp, cuda), T(col, cuda), T(val, cuda)
+    D = np.zeros((nb, bs, nb, bs))
+    rows = np.repeat(np.arange(nb), np.diff(rp))
+    D[rows, :, col, :] = val
+    Y = N(api.bcsr_spmm(nb, bs, r, c, v, T(X, cuda)))
+    assert np.all(np.abs(Y - D.reshape(nb * bs, -1) @ X) <= terms * 2.0 ** -53 * 2)
+    v32 = v.float()
+    D[rows, :, col, :] = N(v32)
+    Y32 = N(api.bcsr_spmm(nb, bs, r, c, v32, T(X, cuda)))
+    ref = D.reshape(nb * bs, -1) @ X.astype(np.float32).astype(np.float64)
+    assert np.all(np.abs(Y32 - ref) <= terms * 2.0 ** -24 * 2)
+    # values that start off a 16-byte boundary
+    odd = torch.empty(v32.numel() + 1, dtype=torch.float32, device=cuda)[1:].view_as(v32)
+    odd.copy_(v32)
+    assert np.array_equal(N(api.bcsr_spmm(nb, bs, r, c, odd, T(X, cuda))), Y32)
+    # one identity block per row: Y is X rounded to FP32
+    n = nb * bs
+    special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 1e-40, -1e-45, 1e39, 3.4028235677973366e38,
+                        1.1754943508222875e-38, 1.0 + 2.0 ** -24, 1.0 + 3 * 2.0 ** -24, -1e-310])
+    Xs = np.resize(special, (n, 1)).repeat(k, axis=1)
+    eye = np.zeros((nb, 1, 1)) + np.eye(bs)
+    # (0 * inf: keep one special value per block row)
+    Xs[np.arange(n) % bs != 0] = 0.0
+    got = N(api.bcsr_spmm(nb, bs, T(np.arange(nb + 1, dtype=np.int32), cuda),
+                          T(np.arange(nb, dtype=np.int32), cuda), T(eye, cuda).float(),
+                          T(Xs, cuda)))[::bs]
+    with np.errstate(over="ignore"):
+        want = Xs[::bs].astype(np.float32).astype(np.float64)
+    assert np.array_equal(got, want, equal_nan=True)
