@@ -20,17 +20,12 @@ thread_local int g_last_cuda_error = 0;
 unsigned long long g_launches = 0;
 
 // implemented in the other translation units
-size_t isai_pattern_ws(int nb, long long nnzb);
-int isai_pattern_colptr_impl(int nb, const int* row, const int* col, int lower, int* Mptr,
-                             int* h_nnz, Carver& ws, cudaStream_t st);
-int isai_pattern_fill_impl(int nb, const int* row, const int* col, int lower, const int* Mptr,
-                           int* Mind, int mnnz, Carver& ws, cudaStream_t st);
-int tri_pattern_rowptr_impl(int nb, const int* row, const int* col, int lower, int* Trow,
-                            int* h_nnz, Carver& ws, cudaStream_t st);
-int tri_pattern_fill_impl(int nb, const int* row, const int* col, int lower, const int* Trow,
-                          int* Tcol, cudaStream_t st);
-int map_impl(int nb, const int* cptr, const int* cind, const int* rrow, const int* rcol, int* map,
-             int* h_bad, Carver& ws, cudaStream_t st);
+size_t isai_both_ws(int nb, long long nnz);
+int isai_both_count(int nb, const int* row, const int* col, int* mL, int* mU, int* tL, int* tU,
+                    int* h_nnz, int* h_longest, Carver& ws, cudaStream_t st);
+int isai_both_fill(int nb, const int* row, const int* col, const int* mL, const int* mU,
+                   const int* tL, const int* tU, int nL, int nU, int* indL, int* indU,
+                   int* tcolL, int* tcolU, int* mapL, int* mapU, Carver& ws, cudaStream_t st);
 int reorder_impl(long long nnzb, int bs, const int* map, const double* src, double* dst,
                  cudaStream_t st, float* dst32);
 size_t syncfree_ws(int nb);
@@ -75,10 +70,10 @@ int bilu0_match_fill(int nb, long long nnzb, const int* row, const int* col, con
                      const int* mptr, int2* mpair, cudaStream_t st);
 int dinv_impl(int nb, int bs, const int* row, const int* col, const double* val, int lower,
               double* Dinv, int* d_fail, cudaStream_t st);
-size_t pairs_ws(long long mnnz);
-int pairs_ptr_impl(int nb, const int* Arow, const int* Acol, const int* Mptr, const int* Mind,
-                   int lower, int* PairPtr, int mnnz, int* h_total, int* h_nmax, Carver& ws,
-                   cudaStream_t st);
+size_t pairs_both_ws(long long mnnz);
+int pairs_both_ptr(int nb, const int* Arow, const int* Acol, const int* const* Mptr,
+                   const int* const* Mind, int* const* PairPtr, const int* mnnz, int* h_total,
+                   Carver& ws, cudaStream_t st);
 int pairs_fill_impl(int nb, const int* Arow, const int* Acol, const int* Mptr, const int* Mind,
                     int lower, const int* PairPtr, int mnnz, int* PL, int* PS, cudaStream_t st);
 int isai_impl(int nb, int bs, const double* Aval, const int* Mptr, const int* Mind, int lower,
@@ -88,6 +83,7 @@ int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const voi
              const void* x, int x32, void* y, int y32, cudaStream_t st, int layout);
 int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t st,
                    int* h_layout);
+int spmv_layout_word(int mb, long long nnzb, int longest);
 int isai_apply_impl(int nb, int bs, int prec, const int* Lrow, const int* Lcol, const void* Lval,
                     const int* Urow, const int* Ucol, const void* Uval, const double* b,
                     void* tmp, double* x, cudaStream_t st, int longL, int longU);
@@ -275,7 +271,7 @@ extern "C" int bilu_ctx_destroy(bilu_ctx* ctx) {
 namespace {
 
 struct Timer {
-  cudaEvent_t e[6];
+  cudaEvent_t e[10];
   cudaStream_t st;
   explicit Timer(cudaStream_t s) : st(s) {
     for (auto& x : e) cudaEventCreate(&x);
@@ -300,69 +296,64 @@ struct IsaiSym {
   int mnnz = 0;
 };
 
-// Structure only (A's pattern, or pattern(A^k) for ISAI(k)): may run before
-// the values are on the device.
-int build_isai_sym(bilu_ctx* c, int lower, Carver& ws, IsaiSym& y, double* t_pattern) {
+// Structure only (A's pattern, or pattern(A^k) for ISAI(k)), both sides: may run
+// before the values are on the device.  Two host synchronisations: the sizes of
+// M_L and M_U, then of their pair lists.
+int build_isai_sym(bilu_ctx* c, Carver& ws, IsaiSym& L, IsaiSym& U, int* h_longest) {
   cudaStream_t st = c->st;
   int nb = c->nb;
   // the M patterns come from pattern(A^k) for ISAI(k); the pair lists, Dinv
   // and the column solves still read the factor on A's pattern
   const int* pr = c->Prow ? c->Prow : c->Arow;
   const int* pc = c->Pcol ? c->Pcol : c->Acol;
-  Timer tm(st);
-  tm.mark(0);
-  BILU_TRY(c->alloc(&y.Mptr, nb + 1));
-  BILU_TRY(c->alloc(&y.Trow, nb + 1));
-  int mnnz = 0, tnnz = 0;
-  {
-    Carver w2 = ws;
-    BILU_TRY(isai_pattern_colptr_impl(nb, pr, pc, lower, y.Mptr, &mnnz, w2, st));
+  for (IsaiSym* y : {&L, &U}) {
+    BILU_TRY(c->alloc(&y->Mptr, nb + 1));
+    BILU_TRY(c->alloc(&y->Trow, nb + 1));
   }
+  int nnz[4];  // M_L, M_U, lower and upper triangle
   {
     Carver w2 = ws;
-    BILU_TRY(tri_pattern_rowptr_impl(nb, pr, pc, lower, y.Trow, &tnnz, w2, st));
+    BILU_TRY(isai_both_count(nb, pr, pc, L.Mptr, U.Mptr, L.Trow, U.Trow, nnz, h_longest, w2, st));
   }
   // the reference's guard (main.cu:537-546): both views must hold the same
   // blocks, i.e. every diagonal block is stored
-  if (mnnz != tnnz) return BILU_ERR_PATTERN;
-  BILU_TRY(c->alloc(&y.Mind, mnnz));
-  BILU_TRY(c->alloc(&y.Tcol, tnnz));
-  BILU_TRY(c->alloc(&y.map, mnnz));
+  if (nnz[0] != nnz[2] || nnz[1] != nnz[3]) return BILU_ERR_PATTERN;
+  L.mnnz = nnz[0];
+  U.mnnz = nnz[1];
+  for (IsaiSym* y : {&L, &U}) {
+    BILU_TRY(c->alloc(&y->Mind, y->mnnz));
+    BILU_TRY(c->alloc(&y->Tcol, y->mnnz));
+    BILU_TRY(c->alloc(&y->map, y->mnnz));
+    BILU_TRY(c->alloc(&y->pp, (size_t)y->mnnz + 1));
+  }
   {
     Carver w2 = ws;
-    if (!w2.take<int>(2)) return BILU_ERR_WORKSPACE;
-    BILU_TRY(isai_pattern_fill_impl(nb, pr, pc, lower, y.Mptr, y.Mind, mnnz, w2, st));
+    BILU_TRY(isai_both_fill(nb, pr, pc, L.Mptr, U.Mptr, L.Trow, U.Trow, L.mnnz, U.mnnz, L.Mind,
+                            U.Mind, L.Tcol, U.Tcol, L.map, U.map, w2, st));
   }
-  BILU_TRY(tri_pattern_fill_impl(nb, pr, pc, lower, y.Trow, y.Tcol, st));
+  int total[2];
   {
     Carver w2 = ws;
-    BILU_TRY(map_impl(nb, y.Mptr, y.Mind, y.Trow, y.Tcol, y.map, nullptr, w2, st));
+    const int *mp[2] = {L.Mptr, U.Mptr}, *mi[2] = {L.Mind, U.Mind};
+    int* pp[2] = {L.pp, U.pp};
+    BILU_TRY(pairs_both_ptr(nb, c->Arow, c->Acol, mp, mi, pp, nnz, total, w2, st));
   }
-  BILU_TRY(c->alloc(&y.pp, (size_t)mnnz + 1));
-  int total = 0;
-  {
-    Carver w2 = ws;
-    BILU_TRY(pairs_ptr_impl(nb, c->Arow, c->Acol, y.Mptr, y.Mind, lower, y.pp, mnnz, &total,
-                            nullptr, w2, st));
+  for (int i = 0; i < 2; ++i) {
+    IsaiSym& y = i == 0 ? L : U;
+    BILU_TRY(c->alloc(&y.pl, total[i]));
+    BILU_TRY(c->alloc(&y.ps, total[i]));
+    BILU_TRY(pairs_fill_impl(nb, c->Arow, c->Acol, y.Mptr, y.Mind, i == 0, y.pp, y.mnnz, y.pl,
+                             y.ps, st));
   }
-  BILU_TRY(c->alloc(&y.pl, total));
-  BILU_TRY(c->alloc(&y.ps, total));
-  BILU_TRY(pairs_fill_impl(nb, c->Arow, c->Acol, y.Mptr, y.Mind, lower, y.pp, mnnz, y.pl, y.ps,
-                           st));
-  y.mnnz = mnnz;
-  tm.mark(1);
-  *t_pattern += tm.ms(0, 1);
   return BILU_OK;
 }
 
 // The values of one ISAI side on the factor: Dinv, the column solves into
 // BCSC and the reorder into BCSR (with the FP32 copy when asked for).
 int build_isai_num(bilu_ctx* c, int lower, const IsaiSym& y, int** orow, int** ocol,
-                   double** oval, int* onnz, double* t_isai, float** oval32) {
+                   double** oval, int* onnz, float** oval32) {
   cudaStream_t st = c->st;
   int nb = c->nb, bs = c->bs, bs2 = bs * bs;
-  Timer tm(st);
-  tm.mark(0);
   double *Dinv, *Mcsc, *Mcsr;
   BILU_TRY(c->alloc(&Dinv, (size_t)nb * bs2));
   BILU_TRY(c->alloc(&Mcsc, (size_t)y.mnnz * bs2));
@@ -376,8 +367,6 @@ int build_isai_num(bilu_ctx* c, int lower, const IsaiSym& y, int** orow, int** o
   if (oval32) *oval32 = M32;
   c->release(Mcsc);
   c->release(Dinv);
-  tm.mark(1);
-  *t_isai += tm.ms(0, 1);
   *orow = y.Trow;
   *ocol = y.Tcol;
   *oval = Mcsr;
@@ -422,9 +411,8 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
   BILU_TRY_CUDA(cudaMemcpyAsync(c->Arow, d_row, sizeof(int) * (nb + 1), cudaMemcpyDeviceToDevice, st));
   BILU_TRY_CUDA(cudaMemcpyAsync(c->Acol, d_col, sizeof(int) * nnzb, cudaMemcpyDeviceToDevice, st));
   // scratch shared by every step
-  size_t wsb = std::max({isai_pattern_ws(nb, nnzb), bilu0_ws(nb, nnzb), pairs_ws(nnzb + nb),
-                         levels_ws(nb), pattern_product_ws(nb),
-                         scan_ws_bytes(nnzb + nb + 1)}) + (1 << 16);
+  size_t wsb = std::max({isai_both_ws(nb, nnzb), bilu0_ws(nb, nnzb), pairs_both_ws(nnzb + nb),
+                         levels_ws(nb), pattern_product_ws(nb)}) + (1 << 16);
   void* wsp = nullptr;
   void* wsq = nullptr;  // a larger scratch for the pattern(A^k) steps
   BILU_TRY(c->alloc((char**)&wsp, wsb));
@@ -476,7 +464,6 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
     }
   }
   tm.mark(2);
-  double t_pat = 0, t_isai = 0;
   // a mask of exact-ILU modes alone builds no ISAI
   const bool isai = (prec_mask & ~ilu_bits) != 0 || (prec_mask & ilu_bits) == 0;
   if (isai && c->isai_level > 1) {
@@ -502,28 +489,26 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
     }
     // the pattern steps below scale with nnz(pattern(A^k))
     long long np = c->nnzP;
-    size_t need = std::max({isai_pattern_ws(nb, np), pairs_ws(np + nb),
-                            scan_ws_bytes(np + nb + 1)}) + (1 << 16);
+    size_t need = std::max(isai_both_ws(nb, np), pairs_both_ws(np + nb)) + (1 << 16);
     if (need > wsb) {
       BILU_TRY(c->alloc((char**)&wsq, need));
       ws = Carver(wsq, need);
     }
   }
   IsaiSym symL, symU;
-  if (isai) {
-    BILU_TRY(build_isai_sym(c, 1, ws, symL, &t_pat));
-    BILU_TRY(build_isai_sym(c, 0, ws, symU, &t_pat));
-  }
-  {
+  int longest[3] = {0, 0, 0};  // the pattern's longest row, its triangles'
+  tm.mark(6);
+  if (isai) BILU_TRY(build_isai_sym(c, ws, symL, symU, longest));
+  tm.mark(7);
+  c->spmv_layout[1] = spmv_layout_word(nb, symL.mnnz, longest[1]);
+  c->spmv_layout[2] = spmv_layout_word(nb, symU.mnnz, longest[2]);
+  if (isai && !c->Prow) {
+    c->spmv_layout[0] = spmv_layout_word(nb, nnzb, longest[0]);
+  } else {  // not counted with the ISAI patterns
     Carver w2 = ws;
     int* words = w2.take<int>(1);
     if (!words) return BILU_ERR_WORKSPACE;
     BILU_TRY(spmv_layout_of(nb, bs, c->Arow, words, st, &c->spmv_layout[0]));
-    c->spmv_layout[1] = c->spmv_layout[2] = 0;
-    if (isai) {
-      BILU_TRY(spmv_layout_of(nb, bs, symL.Trow, words, st, &c->spmv_layout[1]));
-      BILU_TRY(spmv_layout_of(nb, bs, symU.Trow, words, st, &c->spmv_layout[2]));
-    }
   }
   if (ilu) {
     // level analyses of both triangles of the packed factor for the exact
@@ -573,11 +558,12 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
   if (isai) {
     const bool want32 =
         (prec_mask & ((1 << BILU_FP32) | (1 << BILU_FP32_INNER) | (1 << BILU_NESTED))) != 0;
-    BILU_TRY(build_isai_num(c, 1, symL, &c->Lrow, &c->Lcol, &c->Lval, &c->nnzL, &t_isai,
+    BILU_TRY(build_isai_num(c, 1, symL, &c->Lrow, &c->Lcol, &c->Lval, &c->nnzL,
                             want32 ? &c->Lval32 : nullptr));
-    BILU_TRY(build_isai_num(c, 0, symU, &c->Urow, &c->Ucol, &c->Uval, &c->nnzU, &t_isai,
+    BILU_TRY(build_isai_num(c, 0, symU, &c->Urow, &c->Ucol, &c->Uval, &c->nnzU,
                             want32 ? &c->Uval32 : nullptr));
   }
+  tm.mark(9);
   if (prec_mask & ((1 << BILU_FP32_INNER) | (1 << BILU_NESTED))) {
     BILU_TRY(c->alloc(&c->Aval32, (size_t)nnzb * bs2));
     BILU_TRY(bilu_convert_f64_to_f32((size_t)nnzb * bs2, c->Aval, c->Aval32, st));
@@ -606,7 +592,8 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
   c->release(wsq);
   tm.mark(5);
   // factor: BILU(0)'s analysis and factorisation
-  double t_factor = tm.ms(1, 2) + tm.ms(3, 4), t_total = tm.ms(0, 5);
+  const double t_total = tm.ms(0, 5), t_factor = tm.ms(1, 2) + tm.ms(3, 4),
+               t_pat = tm.ms(6, 7), t_isai = tm.ms(4, 9);
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
   if (h_times) {
     h_times[0] = t_factor;

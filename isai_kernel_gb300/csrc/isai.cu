@@ -364,6 +364,30 @@ int pairs_ptr_impl(int nb, const int* Arow, const int* Acol, const int* Mptr, co
   return BILU_OK;
 }
 
+// Pair pointers of both sides with one host synchronisation (h_total[2]).
+size_t pairs_both_ws(long long mnnz) {
+  return carve_size(sizeof(int) * 4) + scan_multi_ws_bytes(mnnz + 1);
+}
+
+int pairs_both_ptr(int nb, const int* Arow, const int* Acol, const int* const* Mptr,
+                   const int* const* Mind, int* const* PairPtr, const int* mnnz, int* h_total,
+                   Carver& ws, cudaStream_t st) {
+  int* words = ws.take<int>(4);  // totals, then the longest columns (not read)
+  if (!words) return BILU_ERR_WORKSPACE;
+  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * 4, st));
+  for (int i = 0; i < 2; ++i) {  // M_L, M_U
+    k_pairs<false><<<ceil_div(std::max(mnnz[i], 1), 256), 256, 0, st>>>(
+        nb, mnnz[i], Arow, Acol, Mptr[i], Mind[i], i == 0, PairPtr[i], nullptr, nullptr,
+        words + 2 + i);
+    BILU_LAUNCH_CHECK();
+  }
+  const ScanSets sets = {{PairPtr[0], PairPtr[1]}, {mnnz[0], mnnz[1]}};
+  BILU_TRY(scan_exclusive_multi(2, sets, words, ws, st));
+  BILU_TRY_CUDA(cudaMemcpyAsync(h_total, words, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaStreamSynchronize(st));
+  return BILU_OK;
+}
+
 int pairs_fill_impl(int nb, const int* Arow, const int* Acol, const int* Mptr, const int* Mind,
                     int lower, const int* PairPtr, int mnnz, int* PL, int* PS, cudaStream_t st) {
   if (nb == 0 || mnnz == 0) return BILU_OK;

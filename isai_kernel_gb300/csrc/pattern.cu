@@ -489,6 +489,83 @@ __global__ void k_b2c_fill(int mb, int bs, long long nnzb, const int* __restrict
   }
 }
 
+// Structure of both ISAI sides of a pattern in one pass each (the setup's form of
+// k_isai_count / k_tri: the counts of M_L and M_U, of both triangles, and the
+// longest rows together, so that the host waits once).  Column counters cL, cU,
+// row counters tL, tU; words: 0 error kind, 1 longest row of the pattern, 2 / 3
+// of its lower / upper triangle.
+__global__ void __launch_bounds__(kT) k_isai_both_count(int nb, const int* __restrict__ row,
+                                                        const int* __restrict__ col, int* cL,
+                                                        int* cU, int* __restrict__ tL,
+                                                        int* __restrict__ tU, int* words) {
+  const int br = blockIdx.x * blockDim.x + threadIdx.x;
+  int s = 0, e = 0, nL = 0, nU = 0;
+  if (br < nb) {
+    s = row[br];
+    e = row[br + 1];
+    if (e < s) {
+      atomicMax(words, 4);
+      e = s;
+    }
+    int lo = s, hi = e;  // first column >= br (rows in order; checked below)
+    while (lo < hi) {
+      const int m = (lo + hi) >> 1;
+      if (col[m] < br) lo = m + 1; else hi = m;
+    }
+    nL = lo - s + (lo < e && col[lo] == br);
+    nU = e - lo;
+    tL[br] = nL;
+    tU[br] = nU;
+    atomicAdd(cL + br, 1);  // the diagonal block of the column
+    atomicAdd(cU + br, 1);
+  }
+  for_row_entries(br, s, e, [&](int r, int p) {
+    const int bc = col[p];
+    if (bc < 0 || bc >= nb) { atomicMax(words, 1); return; }
+    if (p > row[r] && bc <= col[p - 1]) { atomicMax(words, 2); return; }
+    if (bc < r) atomicAdd(cL + bc, 1);
+    else if (bc > r) atomicAdd(cU + bc, 1);
+  });
+  const int a = __reduce_max_sync(0xffffffffu, e - s), b = __reduce_max_sync(0xffffffffu, nL),
+            c = __reduce_max_sync(0xffffffffu, nU);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(words + 1, a);
+    atomicMax(words + 2, b);
+    atomicMax(words + 3, c);
+  }
+}
+
+// Both triangles' columns (BCSR order) and, per column, the rows of M_L / M_U
+// with their BCSR positions (in any order: k_segment_rank_sort follows).  The
+// BCSR position of an entry is known here, so the BCSC -> BCSR map is a payload
+// of that sort instead of a search.
+__global__ void __launch_bounds__(kT) k_isai_both_fill(
+    int nb, const int* __restrict__ row, const int* __restrict__ col,
+    const int* __restrict__ mL, const int* __restrict__ mU, const int* __restrict__ tL,
+    const int* __restrict__ tU, int* curL, int* curU, int* __restrict__ tcolL,
+    int* __restrict__ tcolU, int* __restrict__ keyL, int* __restrict__ payL,
+    int* __restrict__ keyU, int* __restrict__ payU) {
+  const int br = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = br < nb ? row[br] : 0, e = br < nb ? row[br + 1] : 0;
+  for_row_entries(br, s, e, [&](int r, int p) {
+    const int c = col[p];
+    if (c <= r) {
+      const int t = tL[r] + (p - row[r]);
+      tcolL[t] = c;
+      const int d = mL[c] + atomicAdd(curL + c, 1);
+      keyL[d] = r;
+      payL[d] = t;
+    }
+    if (c >= r) {
+      const int t = tU[r + 1] - (row[r + 1] - p);
+      tcolU[t] = c;
+      const int d = mU[c] + atomicAdd(curU + c, 1);
+      keyU[d] = r;
+      payU[d] = t;
+    }
+  });
+}
+
 int read_err(int* d_err, int* h_err, cudaStream_t st) {
   BILU_TRY_CUDA(cudaMemcpyAsync(h_err, d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
@@ -537,6 +614,59 @@ int isai_pattern_fill_impl(int nb, const int* row, const int* col, int lower, co
   k_isai_scatter<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, Mptr, cursor, tmp);
   BILU_LAUNCH_CHECK();
   k_segment_rank_sort<<<ceil_div((long long)nb * 8, kT), kT, 0, st>>>(nb, Mptr, tmp, nullptr, Mind, nullptr);
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
+
+// --------------------------------------------------------------- both ISAI sides
+size_t isai_both_ws(int nb, long long nnz) {
+  return carve_size(sizeof(int) * 8) + scan_multi_ws_bytes(nb + 1) +
+         2 * carve_size(sizeof(int) * ((size_t)nb + 1)) +
+         4 * carve_size(sizeof(int) * (size_t)(nnz + 1));
+}
+
+// Column pointers of M_L and M_U and row pointers of the triangles of pattern
+// (row, col); h_nnz: blocks of M_L, M_U, the lower and the upper triangle;
+// h_longest: longest row of the pattern and of its triangles.  One host
+// synchronisation.
+int isai_both_count(int nb, const int* row, const int* col, int* mL, int* mU, int* tL, int* tU,
+                    int* h_nnz, int* h_longest, Carver& ws, cudaStream_t st) {
+  int* words = ws.take<int>(8);
+  if (!words) return BILU_ERR_WORKSPACE;
+  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * 8, st));
+  BILU_TRY_CUDA(cudaMemsetAsync(mL, 0, sizeof(int) * nb, st));
+  BILU_TRY_CUDA(cudaMemsetAsync(mU, 0, sizeof(int) * nb, st));
+  k_isai_both_count<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, mL, mU, tL, tU, words);
+  BILU_LAUNCH_CHECK();
+  const ScanSets sets = {{mL, mU, tL, tU}, {nb, nb, nb, nb}};
+  BILU_TRY(scan_exclusive_multi(4, sets, words + 4, ws, st));
+  int h[8];
+  BILU_TRY_CUDA(cudaMemcpyAsync(h, words, sizeof(h), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaStreamSynchronize(st));
+  if (h[0] != 0) return BILU_ERR_PATTERN;
+  for (int i = 0; i < 4; ++i) h_nnz[i] = h[4 + i];
+  for (int i = 0; i < 3; ++i) h_longest[i] = h[1 + i];
+  return BILU_OK;
+}
+
+// Mind / Tcol / map of both sides (nL, nU blocks), after isai_both_count.
+int isai_both_fill(int nb, const int* row, const int* col, const int* mL, const int* mU,
+                   const int* tL, const int* tU, int nL, int nU, int* indL, int* indU,
+                   int* tcolL, int* tcolU, int* mapL, int* mapU, Carver& ws, cudaStream_t st) {
+  int* cur = ws.take<int>(2 * (size_t)nb);
+  int* keyL = ws.take<int>((size_t)nL);
+  int* payL = ws.take<int>((size_t)nL);
+  int* keyU = ws.take<int>((size_t)nU);
+  int* payU = ws.take<int>((size_t)nU);
+  if (!cur || !keyL || !payL || !keyU || !payU) return BILU_ERR_WORKSPACE;
+  BILU_TRY_CUDA(cudaMemsetAsync(cur, 0, sizeof(int) * 2 * nb, st));
+  k_isai_both_fill<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, mL, mU, tL, tU, cur, cur + nb,
+                                                    tcolL, tcolU, keyL, payL, keyU, payU);
+  BILU_LAUNCH_CHECK();
+  const unsigned grid = ceil_div((long long)nb * 8, kT);
+  k_segment_rank_sort<<<grid, kT, 0, st>>>(nb, mL, keyL, payL, indL, mapL);
+  BILU_LAUNCH_CHECK();
+  k_segment_rank_sort<<<grid, kT, 0, st>>>(nb, mU, keyU, payU, indU, mapU);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }

@@ -86,7 +86,93 @@ __global__ void k_tile_scan(const int* in, int* out, long long n, const int* __r
   }
 }
 
+// The three passes for set blockIdx.y, its tile sums at sums + y * stride.
+__global__ void k_tile_sums_multi(ScanSets ss, int* __restrict__ sums, long long stride) {
+  const int* in = ss.p[blockIdx.y];
+  const long long n = ss.n[blockIdx.y], base = (long long)blockIdx.x * kScanTile;
+  if (base >= n) return;
+  int s = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    const long long idx = base + (long long)i * kScanThreads + threadIdx.x;
+    if (idx < n) s += in[idx];
+  }
+  __shared__ int tot;
+  block_exclusive_scan(s, &tot);
+  if (threadIdx.x == 0) sums[blockIdx.y * stride + blockIdx.x] = tot;
+}
+
+__global__ void k_scan_sums_multi(ScanSets ss, int* sums, long long stride, int* totals) {
+  __shared__ int carry_s;
+  __shared__ int tot;
+  int* my = sums + blockIdx.x * stride;
+  const long long n = ss.n[blockIdx.x], ntiles = (n + kScanTile - 1) / kScanTile;
+  if (threadIdx.x == 0) carry_s = 0;
+  __syncthreads();
+  for (long long base = 0; base < ntiles; base += kScanThreads) {
+    const long long idx = base + threadIdx.x;
+    const int v = idx < ntiles ? my[idx] : 0;
+    const int ex = block_exclusive_scan(v, &tot);
+    const int carry = carry_s;
+    if (idx < ntiles) my[idx] = ex + carry;
+    __syncthreads();
+    if (threadIdx.x == 0) carry_s = carry + tot;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    ss.p[blockIdx.x][n] = carry_s;  // past the items: no tile reads it
+    if (totals) totals[blockIdx.x] = carry_s;
+  }
+}
+
+__global__ void k_tile_scan_multi(ScanSets ss, const int* __restrict__ sums, long long stride) {
+  int* io = ss.p[blockIdx.y];
+  const long long n = ss.n[blockIdx.y];
+  if ((long long)blockIdx.x * kScanTile >= n) return;
+  const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
+  int v[kScanItems];
+  int s = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    v[i] = base + i < n ? io[base + i] : 0;
+    s += v[i];
+  }
+  __shared__ int tot;
+  int ex = block_exclusive_scan(s, &tot) + sums[blockIdx.y * stride + blockIdx.x];
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    if (base + i < n) io[base + i] = ex;
+    ex += v[i];
+  }
+}
+
 }  // namespace
+
+size_t scan_multi_ws_bytes(long long n_max) {
+  return carve_size(sizeof(int) * kScanSets * (size_t)(n_max / kScanTile + 2));
+}
+
+int scan_exclusive_multi(int sets, const ScanSets& ss, int* d_totals, Carver& ws,
+                         cudaStream_t st) {
+  long long most = 0;
+  for (int i = 0; i < sets; ++i) most = ss.n[i] > most ? ss.n[i] : most;
+  const long long tiles = (most + kScanTile - 1) / kScanTile, stride = tiles + 1;
+  int* sums = ws.take<int>((size_t)(stride * sets));
+  if (!sums) return BILU_ERR_WORKSPACE;
+  if (tiles > 0) {
+    k_tile_sums_multi<<<dim3((unsigned)tiles, (unsigned)sets), kScanThreads, 0, st>>>(ss, sums,
+                                                                                      stride);
+    BILU_LAUNCH_CHECK();
+  }
+  k_scan_sums_multi<<<(unsigned)sets, kScanThreads, 0, st>>>(ss, sums, stride, d_totals);
+  BILU_LAUNCH_CHECK();
+  if (tiles > 0) {
+    k_tile_scan_multi<<<dim3((unsigned)tiles, (unsigned)sets), kScanThreads, 0, st>>>(ss, sums,
+                                                                                      stride);
+    BILU_LAUNCH_CHECK();
+  }
+  return BILU_OK;
+}
 
 size_t scan_ws_bytes(long long n) {
   long long tiles = (n + kScanTile - 1) / kScanTile;

@@ -885,6 +885,12 @@ int spmm_f32(int mb, int k, const int* row, const int* col, const float* val, co
 
 }  // namespace
 
+// The layout word of a pattern of mb rows and nnzb blocks, its longest row given.
+int spmv_layout_word(int mb, long long nnzb, int longest) {
+  return (longest > kLongSpmvRow ? kLayoutLong : 0) |
+         (nnzb > (long long)kWideSpmvRow * mb ? kLayoutWide : 0);
+}
+
 // SpMV layout word of a block pattern (see kLayoutLong): one reduction
 // over the row pointers into d_words (one device int), then a synchronising
 // read of it and of the block count row[mb].  The engine calls it once per
@@ -903,8 +909,7 @@ int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t s
   BILU_TRY_CUDA(cudaMemcpyAsync(&h[0], d, sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaMemcpyAsync(&h[1], row + mb, sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
-  *h_layout = (h[0] > kLongSpmvRow ? kLayoutLong : 0) |
-              ((long long)h[1] > (long long)kWideSpmvRow * mb ? kLayoutWide : 0);
+  *h_layout = spmv_layout_word(mb, h[1], h[0]);
   return BILU_OK;
 }
 

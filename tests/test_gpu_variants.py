@@ -255,6 +255,46 @@ def test_patterns_rows_walked_by_a_warp(cuda, orc, lower):
         api.sptrsv(n, 4, T(rp2, cuda), T(col[keep], cuda), T(val[keep], cuda), T(b, cuda), lower)
 
 
+@pytest.mark.parametrize("level", [1, 2])
+@pytest.mark.parametrize("n", [1, 33, 2048, 2049, 5000])
+def test_setup_builds_the_step_by_step_factors(cuda, n, level):
+    """The setup builds both sides' patterns and pair lists together: the same
+    structure as the entry points give one side at a time, and the same values
+    (the same kernel on the same pair order).  Sizes around a scan tile."""
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(n)
+    length = {5: 47, 6: 48, 7: 49, 20: 110}
+    rp, col = pattern_of([rng.choice(n, size=min(length.get(i, 2), n), replace=False)
+                          for i in range(n)])
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    val = rng.standard_normal((len(col), 4, 4))
+    i4 = np.arange(4)
+    val[np.nonzero(rows == col)[0][:, None], i4, i4] = 8.0 * np.diff(rp)[:, None]
+    r, c, v = T(rp, cuda), T(col, cuda), T(val, cuda)
+    p = api.Preconditioner(n, 4, r, c, v, fp32=False, isai_level=level)
+    lu, L, U = p.factors()
+    pr, pc = (r, c) if level == 1 else api.pattern_product(n, r, c, r, c)
+    for got, lower in ((L, True), (U, False)):
+        mp, mi = api.build_bcsc_pattern_from_bsr_scalarILU(n, pr, pc, lower)
+        tr, tc = api.build_triangular_bcsr_pattern_from_A(n, pr, pc, lower)
+        assert np.array_equal(N(got[0]), N(tr)) and np.array_equal(N(got[1]), N(tc))
+        pp, pl, ps, _ = api.build_pairs(n, r, c, mp, mi, lower)
+        m = api.isai_compute(n, 4, lu, mp, mi, pp, pl, ps, api.build_Dinv(n, 4, r, c, lu, lower),
+                             lower)
+        m = api.reorder_bcsc_val_to_bcsr(api.build_map_bcsc2bcsr_host(n, mp, mi, tr, tc), m)
+        assert np.array_equal(N(got[2]), N(m).reshape(-1, 4, 4))
+    p.close()
+    # a diagonal block that is not stored is refused
+    if n > 1:
+        keep = ~((rows == n - 1) & (col == n - 1))
+        rp2 = np.zeros(n + 1, np.int32)
+        np.cumsum(np.bincount(rows[keep], minlength=n), out=rp2[1:])
+        with pytest.raises(api.BiluError):
+            api.Preconditioner(n, 4, T(rp2, cuda), T(col[keep], cuda), T(val[keep], cuda),
+                               isai_level=level)
+
+
 # ------------------------------------------------------------------ adjoint products
 def sparse_rows(name):
     """rowptr, col (no diagonal needed): hub rows and columns, empty rows."""
