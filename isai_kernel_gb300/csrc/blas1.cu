@@ -80,12 +80,20 @@ __global__ void __launch_bounds__(kRedThreads) k_multiaxpy_norm(
   }
 }
 
-__global__ void k_reduce(const double* __restrict__ partial, int nout, double* __restrict__ out) {
-  int i = threadIdx.x;
-  if (i >= nout) return;
-  double s = 0.0;
-  for (int c = 0; c < kRedCTAs; ++c) s += partial[(long long)c * kPartStride + i];
-  out[i] = s;
+// A warp per output, lane l adding partials l, l + 32, ... and a shuffle tree
+// (a thread per output added 608 one after the other: 47 us a launch, now 4).
+__global__ void __launch_bounds__(512) k_reduce(const double* __restrict__ partial, int nout,
+                                                double* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  static_assert(kRedCTAs % 32 == 0, "whole rounds of a warp");
+  for (int i = threadIdx.x >> 5; i < nout; i += blockDim.x >> 5) {
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kRedCTAs; c += 32) s += partial[(long long)(c + lane) * kPartStride + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[i] = s;
+  }
 }
 
 __global__ void k_scale_rsqrt(long long n, const double* __restrict__ x,
@@ -248,22 +256,34 @@ void launch_combine(long long n, const float* Q, long long ldq, const double* y,
 // Whole modified Gram-Schmidt step in one cooperative launch: sweeps
 // i = 0 .. j+1 over the same slice of w per CTA, sweep i applying
 // h_{i-1} v_{i-1} and taking v_i . w (the last one w . w), then
-// v_{j+1} = w / ||w|| (and its FP32 copy).  Between sweeps
-// a counting grid barrier replaces the kernel boundary: each CTA writes its
-// partial sum, meets the others at the barrier, and then every CTA adds all
-// partials in index order (warp 0, fixed lane strides and shuffle tree), so
-// every CTA holds the same h_i bit for bit and the result does not depend on
-// timing.  The partials alternate between two halves of the buffer: a CTA
-// writes sweep i+1's partial only after barrier i, and sweep i+2 (same half
-// as i) only after barrier i+1, which every CTA reaches after it has read
-// sweep i's partials.  A barrier that times out sets the error word and
-// every CTA returns.  Memory traffic at 128^3 (ncu, one step of 17 sweeps):
+// v_{j+1} = w / ||w|| (and its FP32 copy).  No CTA reads another's part of w:
+// all that crosses between CTAs is one partial sum each a sweep and the total
+// back, and both carry their own flag, the sweep's tag in the same 64-bit
+// words.  CTA 0 reads the sums until all hold the tag, adds them in index
+// order and stores the total once for every kStepFan CTAs, in lines of their
+// own: two store-to-load hops, in place of an atomic arrival, a poll of the
+// count and a read of the sums (1 M elements, a sweep: FP32 4.3 -> 3.6 us, FP64
+// 9.9 -> 9.3).  All CTAs reading all the sums is one hop, and 8.3 us: 304
+// CTAs polling the same 19 lines.  The result does not depend on timing.  A
+// CTA writes the next sweep's sum after the total of this one, which CTA 0
+// stores after it has read the sums; CTA 0 writes the next total after the
+// next sums, which each CTA stores after it has read this total: one slot each
+// is enough.  Tags count on from launch to launch (words[3]), so nothing is
+// cleared between launches.  A wait that runs out sets the error word and
+// every CTA returns.
+//
+// KR = 0, streaming: memory traffic at 128^3 (ncu, one step of 17 sweeps):
 // FP32 reads each basis vector once from DRAM (w and the previous basis
 // vector are L2 hits); FP64 moves ~2.8 vectors a sweep (3.17 GB a step):
 // w (67 MB) does not stay fully in the L2 beside the streamed basis
 // vectors, even with evict-last hints on w; held there by an L2 persisting
 // window it costs 3% less a sweep, which is then bound by the DFMA pipe's
 // issue and the per-sweep synchronisation rather than by HBM.
+// KR > 0, resident: the grid holds the step on the chip, each thread its KR
+// vectors of w in registers and those of v_{i-1} and v_i in shared memory
+// (its own slots only), v_{i+1} on its way while the sums of sweep i cross.
+// A sweep then reads one basis vector and writes nothing.  Same elements per
+// thread and same order of additions as the streaming form: the same bits.
 template <class T>
 struct MgsVec;
 template <>
@@ -348,6 +368,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* g, unsigned l
                "l"(pol)
                : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(g) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -356,12 +380,57 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// A CTA's sum with its tag: FP32 {tag, bits} in one 64-bit word, FP64
+// {tag, high half}, {tag, low half} in two.  Each word is single-copy atomic
+// and carries the tag, so no order between the words is needed.
+__device__ __forceinline__ void store_tagged(unsigned long long* p, unsigned tag, float v) {
+  const unsigned long long x = (unsigned long long)tag << 32 | __float_as_uint(v);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+}
+__device__ __forceinline__ void store_tagged(unsigned long long* p, unsigned tag, double v) {
+  const unsigned long long t = (unsigned long long)tag << 32,
+                           hi = t | (unsigned)__double2hiint(v),
+                           lo = t | (unsigned)__double2loint(v);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(hi) : "memory");
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p + 1), "l"(lo) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool load_tagged(const unsigned long long* p, unsigned tag, float& v) {
+  const unsigned long long x = ld_relaxed_u64(p);
+  v = __uint_as_float((unsigned)x);
+  return (unsigned)(x >> 32) == tag;
+}
+__device__ __forceinline__ bool load_tagged(const unsigned long long* p, unsigned tag,
+                                            double& v) {
+  const unsigned long long hi = ld_relaxed_u64(p), lo = ld_relaxed_u64(p + 1);
+  v = __hiloint2double((int)(unsigned)hi, (int)(unsigned)lo);
+  return (unsigned)(hi >> 32) == tag && (unsigned)(lo >> 32) == tag;
+}
+// Waits, kSpinLimit polls at most, for the tagged sum at p; false when the wait
+// ran out here or elsewhere (the error word is set).
 template <class T>
+__device__ __forceinline__ bool wait_tagged(const unsigned long long* p, unsigned tag, int* err,
+                                            T& v) {
+  for (long long k = 0; !load_tagged(p, tag, v);) {
+    if ((++k & 63) == 0 && ld_relaxed(err) != 0) return false;
+    if (k > kSpinLimit) {
+      atomicCAS(err, 0, (int)BILU_ERR_TIMEOUT);
+      return false;
+    }
+  }
+  return true;
+}
+
+template <class T, int KR>
 __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     long long n, const T* __restrict__ V, long long ldv, int j, T* __restrict__ w,
     double* __restrict__ hout, int hstride, double* __restrict__ wwout,
-    double* __restrict__ partial, GridSync gs, T* __restrict__ vnext,
-    float* __restrict__ vnext32) {
+    unsigned* __restrict__ words, T* __restrict__ vnext, float* __restrict__ vnext32) {
+  constexpr bool kResident = KR > 0;
   using M = MgsVec<T>;
   using VT = typename M::V;
   constexpr int W = M::W;
@@ -369,8 +438,13 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
   // every FP32 <-> FP64 conversion) takes the FP64 pipe, which the FP64
   // kernel needs for its DFMAs and the FP32 kernel should not touch
   __shared__ T red_s[kStepThreads];
+  __shared__ T sum_s[sizeof(T) == 8 ? kStepMaxCTAs : kStepThreads / 32];
   __shared__ T h_s;
-  unsigned passed = 0;
+  __shared__ unsigned epoch_s;
+  int* err = reinterpret_cast<int*>(words + kStepErrWord);
+  constexpr int PW = sizeof(T) / 4;  // 64-bit words of a tagged value
+  unsigned long long* sums = reinterpret_cast<unsigned long long*>(words + 32);
+  unsigned long long* totals = sums + (size_t)kStepMaxCTAs * 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int G = (int)gridDim.x;
   const long long stride = (long long)G * blockDim.x;
@@ -381,9 +455,41 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
   // FP64 staging: w kept in the L2 as long as it fits, the basis vectors
   // streamed through
   unsigned long long pol_w = 0, pol_v = 0;
-  if constexpr (sizeof(T) == 8) {
+  extern __shared__ __align__(16) unsigned char step_stage[];
+  VT* const stage = reinterpret_cast<VT*>(step_stage);
+  VT wr[KR > 0 ? KR : 1];
+  // resident: this thread's k-th vector of v_b in slot [b & 1][k]
+  auto slot = [&](int b, int k) {
+    return stage + ((b & 1) * KR + k) * kStepThreads + threadIdx.x;
+  };
+  auto fetch = [&](int b) {
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      const long long e = tid + k * stride;
+      if (e < nv) cp_async16(slot(b, k), reinterpret_cast<const VT*>(V + b * ldv) + e);
+    }
+    cp_async_commit();
+  };
+  if constexpr (kResident) {
+    fetch(0);
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      const long long e = tid + k * stride;
+      if (e < nv) wr[k] = M::ldcg(wv + e);
+    }
+  } else if constexpr (sizeof(T) == 8) {
     pol_w = l2_policy_evict_last();
     pol_v = l2_policy_evict_first();
+  }
+  if (threadIdx.x == 0) {
+    epoch_s = ld_relaxed_u(words + 3);  // before this CTA's exit, so before it changes
+    h_s = ld_relaxed(err) != 0 ? T(1) : T(0);
+  }
+  __syncthreads();
+  const unsigned epoch = epoch_s;
+  if (h_s != T(0)) {  // an earlier launch gave up
+    if constexpr (kResident) cp_async_wait<0>();
+    return;
   }
   T h = T(0);
   for (int i = 0; i <= j + 1; ++i) {
@@ -393,12 +499,20 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     T a[4] = {T(0), T(0), T(0), T(0)};
     const VT* vpv = reinterpret_cast<const VT*>(vp);
     const VT* vnv = reinterpret_cast<const VT*>(vn);
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (kResident) {
+      cp_async_wait<0>();  // v_i is here
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        if (tid + k * stride >= nv) continue;
+        if (i > 0) M::axpy(hn, *slot(i - 1, k), wr[k]);
+        M::dot(i <= j ? *slot(i, k) : wr[k], wr[k], a);
+      }
+      if (i < j) fetch(i + 1);  // over v_{i-1}, read above by this thread alone
+    } else if constexpr (sizeof(T) == 8) {
       // iteration k of this thread: element tid + k * stride; slot k % S of
       // the thread's w, v_{i-1} and v_i stages, loaded S - 1 iterations ahead
       constexpr int S = kStepStages;
-      extern __shared__ __align__(16) unsigned char step_stage[];
-      VT* stage = reinterpret_cast<VT*>(step_stage);  // [S][3][kStepThreads]
+      // stage[S][3][kStepThreads]
       const long long K = tid < nv ? (nv - tid + stride - 1) / stride : 0;
       auto issue = [&](long long k) {
         const long long e = tid + k * stride;
@@ -458,57 +572,58 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     }
     // CTA partial, fixed order: the threads' sums through shared memory,
     // warp 0 adds eight per lane and then the lanes by a shuffle tree
-    red_s[threadIdx.x] = (a[0] + a[1]) + (a[2] + a[3]);
+    // (an FP64 dot has two sums: the others' adds would cost the FP64 pipe
+    // 0.5 us a sweep)
+    red_s[threadIdx.x] = sizeof(T) == 8 ? a[0] + a[1] : (a[0] + a[1]) + (a[2] + a[3]);
     __syncthreads();
-    T* part = reinterpret_cast<T*>(partial) + (long long)(i & 1) * kStepMaxCTAs;
+    const unsigned tag = epoch + (unsigned)i + 1u;
     if (warp == 0) {
-      T t = T(0);
+      T t = red_s[lane];
 #pragma unroll
-      for (int q = 0; q < kStepThreads / 32; ++q) t += red_s[lane + 32 * q];
+      for (int q = 1; q < kStepThreads / 32; ++q) t += red_s[lane + 32 * q];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) part[blockIdx.x] = t;  // lane 0 of warp 0 arrives at the barrier
+      if (lane == 0) store_tagged(sums + (size_t)blockIdx.x * PW, tag, t);
     }
-    if (!grid_sync_count(gs, passed)) return;
-    // every CTA adds all partials in the same order
-    if constexpr (sizeof(T) == 8) {
-      // FP64: warp 0 alone (the adds take the FP64 pipe), lane l taking
-      // partials l, l + 32, ... in ascending order, eight loads in flight,
-      // then the shuffle tree
-      if (warp == 0) {
-        T t = T(0);
-        for (int c0 = 0; c0 < G; c0 += 8 * 32) {
-          T v[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int c = c0 + lane + 32 * u;
-            v[u] = c < G ? __ldcg(part + c) : T(0);
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u) t += v[u];
-        }
+    bool ok = true;
+    if (blockIdx.x == 0) {
+      T t = T(0);
+      for (int c = threadIdx.x; c < G; c += kStepThreads) {
+        T v = T(0);
+        ok = ok && wait_tagged(sums + (size_t)c * PW, tag, err, v);
+        if constexpr (sizeof(T) == 8) sum_s[c] = v; else t += v;
+      }
+      __syncwarp();
+      if constexpr (sizeof(T) == 4) {  // the warps' trees
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sum_s[warp] = t;
+      }
+      ok = __syncthreads_and(ok) != 0;
+      if (ok && warp == 0) {
+        if constexpr (sizeof(T) == 8) {
+          // lane l adds sums l, l + 32, ... in ascending order, then the tree
+          for (int c = lane; c < G; c += 32) t += sum_s[c];
+          __syncwarp();
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        } else {  // the warp sums
+          t = T(0);
+#pragma unroll
+          for (int q = 0; q < kStepThreads / 32; ++q) t += sum_s[q];
+        }
+        for (int f = lane; f * kStepFan < G; f += 32) store_tagged(totals + f * 16, tag, t);
         if (lane == 0) h_s = t;
       }
-    } else {
-      // FP32: every thread loads its few partials at once (one L2 round
-      // trip), the warps' trees, then warp 0 adds the eight warp sums
-      T t = T(0);
-      for (int c = threadIdx.x; c < G; c += kStepThreads) t += __ldcg(part + c);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      __syncthreads();  // red_s is free again (warp 0 read it before the barrier)
-      if (lane == 0) red_s[warp] = t;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        T u = T(0);
-#pragma unroll
-        for (int q = 0; q < kStepThreads / 32; ++q) u += red_s[q];
-        h_s = u;
-      }
+    } else if (threadIdx.x == 0) {
+      T v = T(0);
+      ok = wait_tagged(totals + (size_t)(blockIdx.x / kStepFan) * 16, tag, err, v);
+      h_s = v;
     }
-    __syncthreads();
+    if (!__syncthreads_and(ok)) {
+      if constexpr (kResident) cp_async_wait<0>();
+      return;
+    }
     h = h_s;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       if (i <= j) hout[(long long)i * hstride] = (double)h;
@@ -519,8 +634,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
   if (vnext) {
     const T s = h > T(0) ? T(1) / sqrt(h) : T(0);
     VT* out = reinterpret_cast<VT*>(vnext);
-    for (long long e = tid; e < nv; e += stride) {
-      VT v = M::ldcg(wv + e);
+    auto put = [&](long long e, VT v) {
       M::scale(v, s);
       out[e] = v;
       if (vnext32) {
@@ -528,6 +642,15 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
 #pragma unroll
         for (int q = 0; q < W; ++q) vnext32[e * W + q] = (float)vs[q];
       }
+    };
+    if constexpr (kResident) {
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        const long long e = tid + k * stride;
+        if (e < nv) put(e, wr[k]);
+      }
+    } else {
+      for (long long e = tid; e < nv; e += stride) put(e, M::ldcg(wv + e));
     }
     if (tid < n - tail) {
       const long long e = tail + tid;
@@ -536,7 +659,12 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       if (vnext32) vnext32[e] = (float)v;
     }
   }
-  grid_exit_count(gs);
+  // every CTA has read the epoch before it arrives here: the last one leaves
+  // the words as the next launch needs them
+  if (threadIdx.x == 0 && atomicAdd(words + 1, 1u) == gridDim.x - 1u) {
+    atomicExch(words + 1, 0u);
+    atomicExch(words + 3, epoch + (unsigned)j + 2u);
+  }
 }
 }  // namespace
 
@@ -557,7 +685,7 @@ int multiaxpy_norm(long long n, const double* V, long long ldv, int nv, const do
 
 int reduce_partials(const double* partial, int nout, double* out, cudaStream_t st) {
   if (nout < 1 || nout > kPartStride) return BILU_ERR_ARG;
-  k_reduce<<<1, 64, 0, st>>>(partial, nout, out);
+  k_reduce<<<1, 512, 0, st>>>(partial, nout, out);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
@@ -569,48 +697,77 @@ int scale_rsqrt(long long n, const double* x, const double* nrm2, double* y, cud
   return BILU_OK;
 }
 
-template <class T>
-int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout, int hstride,
-               double* wwout, double* partial, unsigned* words, T* vnext, float* vnext32,
+// The grid of the k_mgs_step forms: one CTA count for all of them, so that a
+// vector is cut alike whichever form runs.
+template <class T, int KR>
+int mgs_prepare(int* grid) {
+  const size_t smem = KR > 0 ? (size_t)2 * KR * kStepThreads * 16
+                             : (sizeof(T) == 8 ? kStepStageBytes : 0);
+  int per = 0, dev = 0, sms = 0;
+  BILU_TRY_CUDA(cudaGetDevice(&dev));
+  BILU_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (smem)
+    BILU_TRY_CUDA(cudaFuncSetAttribute(k_mgs_step<T, KR>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  BILU_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mgs_step<T, KR>,
+                                                              kStepThreads, smem));
+  *grid = std::max(1, std::min(per, kStepPerSM)) * sms;
+  return BILU_OK;
+}
+
+template <class T, int KR>
+int mgs_launch(int grid, long long n, const T* V, long long ldv, int j, T* w, double* hout,
+               int hstride, double* wwout, unsigned* words, T* vnext, float* vnext32,
                cudaStream_t st) {
-  static int grid = 0;
-  const size_t smem = sizeof(T) == 8 ? kStepStageBytes : 0;
-  if (!grid) {
-    int per = 0, dev = 0, sms = 0;
-    BILU_TRY_CUDA(cudaGetDevice(&dev));
-    BILU_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (smem)
-      BILU_TRY_CUDA(cudaFuncSetAttribute(k_mgs_step<T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    BILU_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mgs_step<T>,
-                                                                kStepThreads, smem));
-    grid = std::max(1, std::min(per, kStepPerSM)) * sms;
-  }
-  if (grid > kStepMaxCTAs) return BILU_ERR_UNSUPPORTED;
-  GridSync gs;
-  gs.count = words;
-  gs.gen = words + 1;
-  gs.err = reinterpret_cast<int*>(words + 2);
-  gs.spin = kSpinLimit;
-  void* args[] = {&n, &V, &ldv, &j, &w, &hout, &hstride, &wwout, &partial, &gs, &vnext, &vnext32};
-  BILU_TRY_CUDA(cudaLaunchCooperativeKernel((const void*)k_mgs_step<T>, dim3(grid),
+  const size_t smem = KR > 0 ? (size_t)2 * KR * kStepThreads * 16
+                             : (sizeof(T) == 8 ? kStepStageBytes : 0);
+  void* args[] = {&n, &V, &ldv, &j, &w, &hout, &hstride, &wwout, &words, &vnext, &vnext32};
+  BILU_TRY_CUDA(cudaLaunchCooperativeKernel((const void*)k_mgs_step<T, KR>, dim3(grid),
                                             dim3(kStepThreads), args, smem, st));
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
 
+template <class T>
+int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout, int hstride,
+               double* wwout, unsigned* words, T* vnext, float* vnext32, cudaStream_t st) {
+  static int grid = 0, resident = 0;
+  if (!grid) {
+    int g0 = 0, g2 = 0, g4 = 0, g6 = 0;
+    BILU_TRY((mgs_prepare<T, 0>(&g0)));
+    BILU_TRY((mgs_prepare<T, 2>(&g2)));
+    BILU_TRY((mgs_prepare<T, 4>(&g4)));
+    BILU_TRY((mgs_prepare<T, 6>(&g6)));
+    // a resident form whose CTAs do not all fit at once is not used
+    resident = g6 >= g0 ? 6 : g4 >= g0 ? 4 : g2 >= g0 ? 2 : 0;
+    grid = g0;
+  }
+  if (grid > kStepMaxCTAs) return BILU_ERR_UNSUPPORTED;
+  // Vectors a thread has to hold: up to 6 of w fit its 64 registers, and twice
+  // that two CTAs' shared memory (196 of 227 KB), i.e. n up to 1.87 M in FP64,
+  // 3.7 M in FP32.  Measured a sweep, streaming / resident: 1 M FP64
+  // 9.3 / 7.7 us (3.6 of it DFMA), FP32 3.6 / 2.6; 1.8 M FP64 12.1 / 10.5;
+  // 3.6 M FP32 7.0 / 4.8; 65 k FP64 4.9 / 4.4, FP32 2.5 / 1.9.
+  const long long threads = (long long)grid * kStepThreads, nv = n / MgsVec<T>::W;
+  const long long need = (nv + threads - 1) / threads;
+#define BILU_MGS(KR) \
+  mgs_launch<T, KR>(grid, n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, st)
+  if (need > resident) return BILU_MGS(0);
+  if (need <= 2) return BILU_MGS(2);
+  if (need <= 4) return BILU_MGS(4);
+  return BILU_MGS(6);
+#undef BILU_MGS
+}
+
 int mgs_step(long long n, const double* V, long long ldv, int j, double* w, double* hout,
-             int hstride, double* wwout, double* partial, unsigned* words, double* vnext,
-             float* vnext32, cudaStream_t st) {
-  return mgs_step_t<double>(n, V, ldv, j, w, hout, hstride, wwout, partial, words, vnext,
-                            vnext32, st);
+             int hstride, double* wwout, unsigned* words, double* vnext, float* vnext32,
+             cudaStream_t st) {
+  return mgs_step_t<double>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, st);
 }
 
 int mgs_step_f32(long long n, const float* V, long long ldv, int j, float* w, double* hout,
-                 int hstride, double* wwout, double* partial, unsigned* words, float* vnext,
-                 cudaStream_t st) {
-  return mgs_step_t<float>(n, V, ldv, j, w, hout, hstride, wwout, partial, words, vnext,
-                           nullptr, st);
+                 int hstride, double* wwout, unsigned* words, float* vnext, cudaStream_t st) {
+  return mgs_step_t<float>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, nullptr, st);
 }
 
 int inner_lsq(int k, const double* H, const double* ww, double* y, cudaStream_t st) {
@@ -642,7 +799,7 @@ using namespace bilu;
 // Test and measurement hook: one modified Gram-Schmidt step (mgs_step or
 // its FP32 form) on caller vectors.
 extern "C" size_t bilu_debug_mgs_step_ws_bytes(void) {
-  return sizeof(double) * 2 * kStepMaxCTAs + 256 + sizeof(unsigned) * 4;
+  return kStepWordsBytes + 256;
 }
 
 extern "C" int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long long ldv, int j,
@@ -656,16 +813,15 @@ extern "C" int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long 
       (d_vnext && (uintptr_t)d_vnext % 16 != 0))
     return BILU_ERR_ARG;
   cudaStream_t st = S(stream);
-  double* partial = (double*)d_ws;
-  unsigned* words = (unsigned*)((char*)d_ws + sizeof(double) * 2 * kStepMaxCTAs + 256);
-  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, sizeof(unsigned) * 4, st));
+  unsigned* words = (unsigned*)(((uintptr_t)d_ws + 255) & ~(uintptr_t)255);
+  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, kStepWordsBytes, st));
   int rc = fp32 ? mgs_step_f32(n, (const float*)d_V, ldv, j, (float*)d_w, d_h, 1, d_h + j + 1,
-                               partial, words, (float*)d_vnext, st)
+                               words, (float*)d_vnext, st)
                 : mgs_step(n, (const double*)d_V, ldv, j, (double*)d_w, d_h, 1, d_h + j + 1,
-                           partial, words, (double*)d_vnext, nullptr, st);
+                           words, (double*)d_vnext, nullptr, st);
   if (rc != BILU_OK) return rc;
   int err = 0;
-  BILU_TRY_CUDA(cudaMemcpyAsync(&err, words + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaMemcpyAsync(&err, words + kStepErrWord, sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
   return err;
 }

@@ -46,24 +46,29 @@ int combine_f32(long long n, const float* Q, long long ldq, int k, const double*
 
 // Whole modified Gram-Schmidt step of Arnoldi step j in one cooperative
 // launch: j+2 fused sweeps (sweep i applies w -= h_{i-1} v_{i-1} and takes
-// h_i = v_i . w; the last one w . w) with a counting grid barrier between
-// them: h_i into hout[i * hstride]
+// h_i = v_i . w; the last one w . w) with an exchange of tagged CTA sums
+// between them: h_i into hout[i * hstride]
 // (i <= j), ||w||^2 into *wwout, then vnext = w / ||w|| (and vnext32, its
-// FP32 copy, when given; zeros when ||w|| = 0).  Sums are in the vectors'
-// precision and in a fixed order (warp 0 of every CTA adds all CTA
-// partials alike).  partial holds 2 * kStepMaxCTAs doubles; words are the barrier's count, exit count and
-// error word (zero before the first launch; every launch leaves them zero
-// unless a barrier timed out, which sets the error word to
-// BILU_ERR_TIMEOUT).
+// FP32 copy, when given; zeros when ||w|| = 0).  w is used up (its contents
+// afterwards are unspecified).  Sums are in the vectors' precision and in a
+// fixed order (CTA 0 adds the CTA sums by their index).  words holds
+// kStepWordsBytes: zero before the first launch; after a wait that ran out its
+// error word (kStepErrWord) holds BILU_ERR_TIMEOUT, launches return at once,
+// and all of it is zeroed before the next use.
 constexpr int kStepMaxCTAs = 152 * 8;
+constexpr int kStepErrWord = 2;
+// 32 words (2: error, others the launch's), the CTAs' tagged sums, and the
+// tagged total in a 128-byte line for every kStepFan CTAs
+constexpr int kStepFan = 8;
+constexpr size_t kStepWordsBytes =
+    128 + (size_t)kStepMaxCTAs * 16 + (size_t)kStepMaxCTAs / kStepFan * 128;
 int mgs_step(long long n, const double* V, long long ldv, int j, double* w, double* hout,
-             int hstride, double* wwout, double* partial, unsigned* words, double* vnext,
-             float* vnext32, cudaStream_t st);
+             int hstride, double* wwout, unsigned* words, double* vnext, float* vnext32,
+             cudaStream_t st);
 // The FP32 form for the nested mode's inner solver: FP32 products and FP32
-// sums throughout (the CTA partials and their sum too; the FP64 pipe is
+// sums throughout (the CTA sums and their sum too; the FP64 pipe is
 // left alone), h and ||w||^2 written as FP64.
 int mgs_step_f32(long long n, const float* V, long long ldv, int j, float* w, double* hout,
-                 int hstride, double* wwout, double* partial, unsigned* words, float* vnext,
-                 cudaStream_t st);
+                 int hstride, double* wwout, unsigned* words, float* vnext, cudaStream_t st);
 
 }  // namespace bilu

@@ -181,7 +181,7 @@ struct bilu_ctx {
   double* hpin = nullptr;  // pinned host mirror of dscal
   cudaEvent_t ev = nullptr;
   unsigned* counter = nullptr;  // arrival counter of the MGS sweep reductions
-  unsigned* step_words = nullptr;  // barrier count, exit count, error word of mgs_step
+  unsigned* step_words = nullptr;  // kStepWordsBytes of mgs_step: error word, tagged sums
   long long steps = 0, restarts = 0;  // Arnoldi steps and cycles of the last solve
   // nested (GMRES-IR) mode: FP32 inner GMRES of inner_k steps per outer
   // step; its basis U32 ((k+1) vectors, U32[0] = the outer basis vector in
@@ -671,8 +671,8 @@ int ensure_solver(bilu_ctx* c, int m) {
   BILU_TRY_CUDA(cudaMallocHost(&c->hpin, sizeof(double) * 6 * kPartStride));
   BILU_TRY_CUDA(get(&c->counter, sizeof(unsigned)));
   BILU_TRY_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->st));
-  BILU_TRY_CUDA(get(&c->step_words, sizeof(unsigned) * 4));
-  BILU_TRY_CUDA(cudaMemsetAsync(c->step_words, 0, sizeof(unsigned) * 4, c->st));
+  BILU_TRY_CUDA(get(&c->step_words, kStepWordsBytes));
+  BILU_TRY_CUDA(cudaMemsetAsync(c->step_words, 0, kStepWordsBytes, c->st));
   c->m_alloc = m;
   return BILU_OK;
 }
@@ -762,8 +762,8 @@ int inner_solve(bilu_ctx* c, double* z) {
     BILU_TRY(spmv_any(c->nb, c->bs, BILU_FP32, c->Arow, c->Acol, c->Aval32, qj, 1, c->w32, 1, st,
                       c->spmv_layout[0]));
     // the j+2 FP32 sweeps and u_{j+1} = w / ||w|| in one cooperative launch
-    BILU_TRY(mgs_step_f32(n, c->U32, (long long)ld, j, c->w32, H + j, k, ww + j, c->partial,
-                          c->step_words, j + 1 < k ? c->U32 + ld * (j + 1) : nullptr, st));
+    BILU_TRY(mgs_step_f32(n, c->U32, (long long)ld, j, c->w32, H + j, k, ww + j, c->step_words,
+                          j + 1 < k ? c->U32 + ld * (j + 1) : nullptr, st));
   }
   BILU_TRY(inner_lsq(k, H, ww, y, st));
   return combine_f32(n, c->Q32, (long long)ld, k, y, z, st);
@@ -848,12 +848,12 @@ int arnoldi_back(bilu_ctx* c, int j, int prec) {
   size_t ld = (size_t)c->ldv;
   double* s = c->dscal;
   const double* V = c->V;
-  BILU_TRY(mgs_step(n, V, (long long)ld, j, c->w, s, 1, s + kPartStride, c->partial,
-                    c->step_words, c->V + ld * (j + 1), v32_of(c, prec), st));
+  BILU_TRY(mgs_step(n, V, (long long)ld, j, c->w, s, 1, s + kPartStride, c->step_words,
+                    c->V + ld * (j + 1), v32_of(c, prec), st));
   BILU_TRY_CUDA(cudaMemcpyAsync(c->hpin, s, sizeof(double) * (kPartStride + 1),
                                 cudaMemcpyDeviceToHost, st));
-  // the barrier error word of this step's (and the inner solver's) launches
-  BILU_TRY_CUDA(cudaMemcpyAsync(c->hpin + kPartStride + 1, c->step_words + 2, sizeof(unsigned),
+  // the error word of this step's (and the inner solver's) launches
+  BILU_TRY_CUDA(cudaMemcpyAsync(c->hpin + kPartStride + 1, c->step_words + kStepErrWord, sizeof(unsigned),
                                 cudaMemcpyDeviceToHost, st));
   return BILU_OK;
 }
@@ -875,7 +875,7 @@ extern "C" int bilu_ctx_solve(bilu_ctx* c, int prec, const double* d_b, double* 
   cudaStream_t st = c->st;
   const bool ilu_mode = prec == BILU_ILU || prec == BILU_ILU_FP32;
   if (ilu_mode) BILU_TRY_CUDA(cudaMemsetAsync(c->ilu_words, 0, sizeof(unsigned) * 4, st));
-  BILU_TRY_CUDA(cudaMemsetAsync(c->step_words, 0, sizeof(unsigned) * 4, st));
+  BILU_TRY_CUDA(cudaMemsetAsync(c->step_words, 0, kStepWordsBytes, st));
   const int m = restart;
   const long long n = c->n;
   double* s = c->dscal;
@@ -917,9 +917,9 @@ extern "C" int bilu_ctx_solve(bilu_ctx* c, int prec, const double* d_b, double* 
       BILU_TRY_CUDA(cudaEventSynchronize(c->ev));
       unsigned step_err = 0;
       std::memcpy(&step_err, hp + kPartStride + 1, sizeof(unsigned));
-      if (step_err != 0) {  // a grid barrier of the orthogonalisation timed out
+      if (step_err != 0) {  // a wait of the orthogonalisation ran out
         cudaStreamSynchronize(st);
-        cudaMemsetAsync(c->step_words, 0, sizeof(unsigned) * 4, st);
+        cudaMemsetAsync(c->step_words, 0, kStepWordsBytes, st);
         cudaStreamSynchronize(st);
         return (int)step_err;
       }

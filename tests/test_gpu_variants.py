@@ -449,3 +449,48 @@ def test_spmm_splits(cuda, orc, bs, k):
     with np.errstate(over="ignore"):
         want = Xs[::bs].astype(np.float32).astype(np.float64)
     assert np.array_equal(got, want, equal_nan=True)
+
+
+# ------------------------------------------------------------------ orthogonalisation
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("per_thread", [0, 2, 4, 6, 7])
+def test_mgs_step_forms(cuda, fp32, per_thread):
+    """n one element below, at and above what fills 2, 4 and 6 vectors a thread
+    of two 512-thread CTAs per SM (where the kernel's form changes), against
+    the same Gram-Schmidt in FP64: v_{j+1} within 1e-12 (FP32 2e-5) of its
+    largest element.  (h_i carries the rounding of a sum of |v_i| |w|: some
+    50 eps sqrt(n), that is 50 eps of an element of w after h_i v_i.)"""
+    import torch
+
+    from isai_kernel_gb300 import _lib, api
+
+    L = _lib.lib()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    full = sms * 1024 * (4 if fp32 else 2) * max(per_thread, 1)
+    dt, tol = (torch.float32, 2e-5) if fp32 else (torch.float64, 1e-12)
+    j = 2
+    for n in ((1, 7, 513) if per_thread == 0 else (full - 1, full, full + 5)):
+        gen_ = torch.Generator(device=cuda).manual_seed(n)
+        j = min(2, n - 1)
+        B = torch.randn(n, j + 1, dtype=torch.float64, device=cuda, generator=gen_)
+        Q = torch.linalg.qr(B)[0].T.contiguous()
+        ldv = (n + 31) // 32 * 32
+        V = torch.zeros(j + 1, ldv, dtype=dt, device=cuda)
+        V[:, :n] = Q.to(dt)
+        w = torch.zeros(ldv, dtype=dt, device=cuda)
+        w[:n] = torch.randn(n, dtype=torch.float64, device=cuda, generator=gen_).to(dt)
+        wr, Vr = w[:n].double().clone(), V[:, :n].double()  # the kernel uses w up
+        h = torch.empty(j + 2, dtype=torch.float64, device=cuda)
+        vn = torch.zeros_like(w)
+        ws = torch.empty(L.bilu_debug_mgs_step_ws_bytes(), dtype=torch.uint8, device=cuda)
+        assert L.bilu_debug_mgs_step(n, fp32, api._p(V), ldv, j, api._p(w), api._p(h),
+                                     api._p(vn), api._p(ws), ws.numel(), api._s()) == 0
+        for i in range(j + 1):
+            hi = Vr[i] @ wr
+            assert abs(hi - h[i]) <= tol * n ** 0.5
+            wr = wr - hi * Vr[i]
+        if n == 1:  # nothing is left but rounding
+            continue
+        ref = wr / wr.norm()
+        assert (vn[:n].double() - ref).abs().max() <= tol * ref.abs().max()
+        assert torch.all(vn[n:] == 0)
