@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(kRedThreads) k_combine_f32(long long n,
                                                              long long ldq,
                                                              const double* __restrict__ y,
                                                              double* __restrict__ z) {
+  dependents_launch();
   __shared__ float ys[K > 0 ? K : 1];
   if (threadIdx.x < K) ys[threadIdx.x] = (float)y[threadIdx.x];
   __syncthreads();
@@ -431,6 +432,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     double* __restrict__ hout, int hstride, double* __restrict__ wwout,
     unsigned* __restrict__ words, T* __restrict__ vnext, float* __restrict__ vnext32) {
   constexpr bool kResident = KR > 0;
+  dependents_launch();  // the next product may read its matrix during the sweeps
   using M = MgsVec<T>;
   using VT = typename M::V;
   constexpr int W = M::W;

@@ -27,7 +27,8 @@ int transpose_fill(int mb, int nbcol, const int* cptr, const int* cind, long lon
 int spmv_gather_t(int mb, int bs, const int* trow, const int* tcol, const int* src,
                   const double* val, const double* x, double* y, int longest, cudaStream_t st);
 int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const void* val,
-             const void* x, int x32, void* y, int y32, cudaStream_t st, int layout);
+             const void* x, int x32, void* y, int y32, cudaStream_t st, int layout,
+             bool dep = false);
 
 namespace {
 

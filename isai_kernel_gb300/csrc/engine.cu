@@ -80,7 +80,8 @@ int isai_impl(int nb, int bs, const double* Aval, const int* Mptr, const int* Mi
               const int* pp, const int* pl, const int* ps, const double* Dinv, double* Mval,
               cudaStream_t st);
 int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const void* val,
-             const void* x, int x32, void* y, int y32, cudaStream_t st, int layout);
+             const void* x, int x32, void* y, int y32, cudaStream_t st, int layout,
+             bool dep = false);
 int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t st,
                    int* h_layout);
 int spmv_layout_word(int mb, long long nnzb, int longest);
@@ -756,11 +757,11 @@ int inner_solve(bilu_ctx* c, double* z) {
     const float* uj = c->U32 + ld * j;
     float* qj = c->Q32 + ld * j;
     BILU_TRY(spmv_any(c->nb, c->bs, BILU_FP32, c->Lrow, c->Lcol, c->Lval32, uj, 1, t32, 1, st,
-                      c->spmv_layout[1]));
+                      c->spmv_layout[1], true));
     BILU_TRY(spmv_any(c->nb, c->bs, BILU_FP32, c->Urow, c->Ucol, c->Uval32, t32, 1, qj, 1, st,
-                      c->spmv_layout[2]));
+                      c->spmv_layout[2], true));
     BILU_TRY(spmv_any(c->nb, c->bs, BILU_FP32, c->Arow, c->Acol, c->Aval32, qj, 1, c->w32, 1, st,
-                      c->spmv_layout[0]));
+                      c->spmv_layout[0], true));
     // the j+2 FP32 sweeps and u_{j+1} = w / ||w|| in one cooperative launch
     BILU_TRY(mgs_step_f32(n, c->U32, (long long)ld, j, c->w32, H + j, k, ww + j, c->step_words,
                           j + 1 < k ? c->U32 + ld * (j + 1) : nullptr, st));
@@ -829,11 +830,13 @@ int arnoldi_front(bilu_ctx* c, int prec, int j) {
   size_t ld = (size_t)c->ldv;
   double* zj = c->Z + ld * j;
   BILU_TRY(apply_prec(c, prec, c->V + ld * j, zj));
+  // z_j is the last launch's result, but for the triangular solves and the copy
+  const bool dep = prec >= 0 && prec != BILU_ILU && prec != BILU_ILU_FP32;
   if (prec == BILU_FP32_INNER)  // FP32-stored A and z (written by the apply), FP64 w
     return spmv_any(c->nb, c->bs, BILU_FP32, c->Arow, c->Acol, c->Aval32, c->z32, 1, c->w, 0,
-                    c->st, c->spmv_layout[0]);
+                    c->st, c->spmv_layout[0], dep);
   return spmv_any(c->nb, c->bs, BILU_FP64, c->Arow, c->Acol, c->Aval, zj, 0, c->w, 0, c->st,
-                  c->spmv_layout[0]);
+                  c->spmv_layout[0], dep);
 }
 
 // Orthogonalises w against V_0..V_j by modified Gram-Schmidt: j+2 fused

@@ -40,9 +40,45 @@ __device__ __forceinline__ double to_acc(float v, double) { return (double)v; }
 __device__ __forceinline__ float to_acc(double v, float) { return (float)v; }
 __device__ __forceinline__ float to_acc(float v, float) { return v; }
 
+// Reads of x where the launch before may still have been writing it when this
+// one started: not the read-only path.  They cannot move above dependency_wait
+// because the pointer comes out of after_wait.
+template <class T>
+__device__ __forceinline__ const T* after_wait(const T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+__device__ __forceinline__ double ld_dep(const double* p) {
+  double v;
+  asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_dep(const float* p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_dep(const double2* p) {
+  double2 v;
+  asm("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_dep(const float4* p) {
+  float4 v;
+  asm("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(p));
+  return v;
+}
+template <bool DEP, class T>
+__device__ __forceinline__ T ld_x(const T* p) {
+  if constexpr (DEP) return ld_dep(p);
+  else return __ldg(p);
+}
+
 // Load the BS-long x segment of block column bc into registers (AccT).
-template <int BS, class XT, class AccT>
-__device__ __forceinline__ void load_x(const XT* __restrict__ x, long long bc, AccT* xr) {
+template <int BS, class XT, class AccT, bool DEP = false>
+__device__ __forceinline__ void load_x(const XT* x, long long bc, AccT* xr) {
   const XT* p = x + bc * BS;
   constexpr int W = Vec<XT>::W;
   if constexpr (BS % W == 0) {
@@ -51,7 +87,7 @@ __device__ __forceinline__ void load_x(const XT* __restrict__ x, long long bc, A
     using V = typename Vec<XT>::V;
 #pragma unroll
     for (int c = 0; c < BS / W; ++c) {
-      V v = __ldg(reinterpret_cast<const V*>(p) + c);
+      V v = ld_x<DEP>(reinterpret_cast<const V*>(p) + c);
       if constexpr (W == 2) {
         xr[2 * c] = to_acc(v.x, AccT());
         xr[2 * c + 1] = to_acc(v.y, AccT());
@@ -64,7 +100,7 @@ __device__ __forceinline__ void load_x(const XT* __restrict__ x, long long bc, A
     }
   } else {
 #pragma unroll
-    for (int c = 0; c < BS; ++c) xr[c] = to_acc(__ldg(p + c), AccT());
+    for (int c = 0; c < BS; ++c) xr[c] = to_acc(ld_x<DEP>(p + c), AccT());
   }
 }
 
@@ -191,7 +227,16 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
 // operator), RPG = 1 at 8 CTAs per SM for bs 4 rows of ~4 blocks, else
 // RPG = 2.  Patterns with rows of more than kLongSpmvRow blocks take
 // k_bsr_spmv_balanced (FP64) or k_bsr_spmv_uneven (FP32).
-template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool TR>
+// DEP, for a product whose x is the result of the launch before it (U after L,
+// A after U): started by programmatic dependent launch while that one drains,
+// it reads its row pointers, columns and first blocks, none of which the launch
+// before writes, and waits before its first read of x and before any write.
+// The launch before must itself have been ordered after whatever wrote the
+// matrix.  It hides the tail of one product and the three dependent DRAM
+// latencies at the start of the next (64^3 7-point, 4x4 blocks, the FP32 apply
+// 33.7 -> 28.9 us, FP64 71.2 -> 67.9; 128^3 FP32 249 -> 224).
+template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool TR,
+          bool DEP>
 __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __restrict__ row,
                                                      const int* __restrict__ col,
                                                      const int* __restrict__ src,
@@ -200,6 +245,7 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
                                                      YT* __restrict__ y,
                                                      float* __restrict__ y32) {
   constexpr int G = 32 / BS;  // lane groups per warp
+  dependents_launch();
   int lane = threadIdx.x & 31;
   int g = lane / BS, r = lane - g * BS;
   long long base = (((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + g) * RPG;
@@ -214,6 +260,9 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
   AccT acc[RPG];
 #pragma unroll
   for (int q = 0; q < RPG; ++q) acc[q] = 0;
+  const XT* xp = x;
+  // DEP: the first blocks wait in registers, or where these are too many in the L2
+  constexpr bool kHold = RPG * U * BS * sizeof(AccT) <= 128;
   // batches of U blocks per row; every load of a batch (column indices,
   // block rows, x segments) is issued before its FMAs
   for (int off = 0;; off += U) {
@@ -229,18 +278,38 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
         int p = s[q] + off + u;
         c[q][u] = p < e[q] ? __ldg(col + p) : -1;
       }
+    if constexpr (DEP && !kHold) {
+      if (off == 0) {
+#pragma unroll
+        for (int q = 0; q < RPG; ++q)
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (s[q] + u < e[q])
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                  val + ((long long)(s[q] + u) * BS + r) * BS));
+        dependency_wait();
+        xp = after_wait(x);
+      }
+    }
     AccT a[RPG][U][BS], xv[RPG][U][BS];
 #pragma unroll
     for (int q = 0; q < RPG; ++q)
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        if (c[q][u] >= 0) {
+        // FP32, DEP: not on c, so that both loads go out before the wait
+        if (DEP && sizeof(VT) == 4 ? s[q] + off + u < e[q] : c[q][u] >= 0) {
           load_entry<BS, TR, VT, AccT>(val, src, s[q] + off + u, r, a[q][u]);
         } else {
 #pragma unroll
           for (int k = 0; k < BS; ++k) a[q][u][k] = 0;
         }
       }
+    if constexpr (DEP && kHold) {
+      if (off == 0) {
+        dependency_wait();
+        xp = after_wait(x);
+      }
+    }
     // x segments (mostly L2 hits) are consumed as they arrive, which keeps
     // the register footprint low enough for 4 CTAs per SM with FP32 values
 #pragma unroll
@@ -248,12 +317,13 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (c[q][u] >= 0) {
-          load_x<BS, XT, AccT>(x, c[q][u], xv[q][u]);
+          load_x<BS, XT, AccT, DEP>(xp, c[q][u], xv[q][u]);
 #pragma unroll
           for (int k = 0; k < BS; ++k) acc[q] = fma(a[q][u][k], xv[q][u][k], acc[q]);
         }
       }
   }
+  if constexpr (DEP) dependency_wait();  // rows without blocks
 #pragma unroll
   for (int q = 0; q < RPG; ++q)
     if (base + q < mb) {
@@ -489,11 +559,28 @@ constexpr int kWideSpmvRow = 5;
 
 template <int BS, class VT, class XT, class YT, int RPG, int U, int MINB, bool TR = false>
 int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
-                    cudaStream_t st, float* y32, const int* src = nullptr) {
+                    cudaStream_t st, float* y32, bool dep, const int* src = nullptr) {
   constexpr int G = 32 / BS;
   long long groups = (mb + RPG - 1) / RPG;
   long long warps = (groups + G - 1) / G;
-  k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR><<<ceil_div(warps, 8), 256, 0, st>>>(
+  if constexpr (!TR) {
+    if (dep) {
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(ceil_div(warps, 8));
+      cfg.blockDim = dim3(256);
+      cfg.stream = st;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      BILU_TRY_CUDA(cudaLaunchKernelEx(&cfg, k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR, true>,
+                                       mb, row, col, src, val, x, y, y32));
+      BILU_LAUNCH_CHECK();
+      return BILU_OK;
+    }
+  }
+  k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR, false><<<ceil_div(warps, 8), 256, 0, st>>>(
       mb, row, col, src, val, x, y, y32);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
@@ -544,7 +631,7 @@ int launch_spmv_balanced(int mb, const int* row, const int* col, const int* src,
 // apply to patterns without long rows, FP64 at block sizes 4 and 5.
 template <int BS, class VT, class XT, class YT>
 int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
-                cudaStream_t st, int layout, float* y32 = nullptr) {
+                cudaStream_t st, int layout, float* y32, bool dep) {
   if (mb == 0) return BILU_OK;
   if (layout & kLayoutLong) {
     if constexpr (sizeof(VT) == 8)
@@ -555,21 +642,24 @@ int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT*
   }
   if constexpr (sizeof(VT) == 8) {
     if constexpr (BS <= 5)
-      return launch_spmv_cfg<BS, VT, XT, YT, 2, 1, 4>(mb, row, col, val, x, y, st, y32);
+      return launch_spmv_cfg<BS, VT, XT, YT, 2, 1, 4>(mb, row, col, val, x, y, st, y32, dep);
     else
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 2, 2>(mb, row, col, val, x, y, st, y32);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 2, 2>(mb, row, col, val, x, y, st, y32, dep);
   } else if constexpr (BS == 8 && sizeof(XT) == 8) {
     // two rows of 8x8 blocks with FP64 x segments spill at 64 registers
-    return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32);
+    return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
   } else {
-    if (layout & kLayoutWide)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32);
+    // one row per group also where the first blocks are to wait in registers
+    // for the launch before (two rows / one, the 512^2 5-point apply: bs 5 54.3
+    // / 45.2 us, bs 8 80.4 / 68.9)
+    if ((layout & kLayoutWide) || (BS != 4 && dep))
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
     // bs 4 rows of ~4 blocks (the ISAI triangles of a 7-point pattern): one
     // row per group at 32 registers, 8 CTAs per SM (0.2214 -> 0.2185 ms
     // for the 128^3 inner apply)
     if constexpr (BS == 4)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8>(mb, row, col, val, x, y, st, y32);
-    return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4>(mb, row, col, val, x, y, st, y32);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8>(mb, row, col, val, x, y, st, y32, dep);
+    return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
   }
 }
 
@@ -584,10 +674,10 @@ int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, cons
     return launch_spmv_balanced<BS, 2, 4, true>(mb, trow, tcol, src, val, x, y, st, nullptr);
   if constexpr (BS <= 5)
     return launch_spmv_cfg<BS, D, D, D, 2, 1, 4, true>(mb, trow, tcol, val, x, y, st, nullptr,
-                                                       src);
+                                                       false, src);
   else
     return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, true>(mb, trow, tcol, val, x, y, st, nullptr,
-                                                       src);
+                                                       false, src);
 }
 
 // Multi-RHS: Y[n,k] = M X[n,k], row-major with ld = k.  LPR lanes per block row
@@ -829,6 +919,7 @@ int launch_spmm(int mb, int k, const int* row, const int* col, const VT* val, co
 }
 
 __global__ void k_f64_to_f32(size_t n, const double* __restrict__ s, float* __restrict__ d) {
+  dependents_launch();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (; i < n; i += stride) d[i] = __double2float_rn(s[i]);
@@ -836,31 +927,31 @@ __global__ void k_f64_to_f32(size_t n, const double* __restrict__ s, float* __re
 
 template <int BS>
 int spmv_f64(int mb, const int* row, const int* col, const double* val, const double* x,
-             double* y, cudaStream_t st, int lr) {
-  return launch_spmv<BS, double, double, double>(mb, row, col, val, x, y, st, lr);
+             double* y, cudaStream_t st, int lr, bool dep) {
+  return launch_spmv<BS, double, double, double>(mb, row, col, val, x, y, st, lr, nullptr, dep);
 }
 
 template <int BS>
 int spmv_f32(int mb, const int* row, const int* col, const float* val, const void* x, int x32,
-             void* y, int y32, cudaStream_t st, int lr) {
+             void* y, int y32, cudaStream_t st, int lr, bool dep) {
   if (x32 && y32)
     return launch_spmv<BS, float, float, float>(mb, row, col, val, (const float*)x, (float*)y, st,
-                                                lr);
+                                                lr, nullptr, dep);
   if (x32)
     return launch_spmv<BS, float, float, double>(mb, row, col, val, (const float*)x, (double*)y,
-                                                 st, lr);
+                                                 st, lr, nullptr, dep);
   if (y32)
     return launch_spmv<BS, float, double, float>(mb, row, col, val, (const double*)x, (float*)y,
-                                                 st, lr);
+                                                 st, lr, nullptr, dep);
   return launch_spmv<BS, float, double, double>(mb, row, col, val, (const double*)x, (double*)y,
-                                                st, lr);
+                                                st, lr, nullptr, dep);
 }
 
 // FP32 values and x, FP64 y plus its FP32 copy y32
 template <int BS>
 int spmv_f32_dual(int mb, const int* row, const int* col, const float* val, const float* x,
-                  double* y, float* y32, cudaStream_t st, int lr) {
-  return launch_spmv<BS, float, float, double>(mb, row, col, val, x, y, st, lr, y32);
+                  double* y, float* y32, cudaStream_t st, int lr, bool dep) {
+  return launch_spmv<BS, float, float, double>(mb, row, col, val, x, y, st, lr, y32, dep);
 }
 
 __global__ void k_row_len_max(int mb, const int* __restrict__ row, int* out) {
@@ -957,15 +1048,16 @@ int layout_cached(int mb, int bs, const int* row, cudaStream_t st, int* out) {
 // internal entry point used by the solver; layout: the pattern's layout
 // word when the caller knows it (spmv_layout_of), -1 to look it up
 int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const void* val,
-             const void* x, int x32, void* y, int y32, cudaStream_t st, int layout) {
+             const void* x, int x32, void* y, int y32, cudaStream_t st, int layout, bool dep) {
   int lr = layout;
   if (layout < 0) BILU_TRY(layout_cached(mb, bs, row, st, &lr));
   if (prec == BILU_FP64) {
     if (x32 || y32) return BILU_ERR_ARG;
     return BILU_DISPATCH_BS(bs, spmv_f64, mb, row, col, (const double*)val, (const double*)x,
-                            (double*)y, st, lr);
+                            (double*)y, st, lr, dep);
   }
-  return BILU_DISPATCH_BS(bs, spmv_f32, mb, row, col, (const float*)val, x, x32, y, y32, st, lr);
+  return BILU_DISPATCH_BS(bs, spmv_f32, mb, row, col, (const float*)val, x, x32, y, y32, st, lr,
+                          dep);
 }
 
 // y = M^T x: trow / tcol the transposed pattern, src the block of M each of its
@@ -995,11 +1087,11 @@ int isai_apply_impl(int nb, int bs, int prec, const int* Lrow, const int* Lcol, 
   if (prec == BILU_FP32) {
     float* b32 = reinterpret_cast<float*>(x);
     BILU_TRY(convert_f64_f32((size_t)nb * bs, b, b32, st));
-    BILU_TRY(spmv_any(nb, bs, prec, Lrow, Lcol, Lval, b32, 1, tmp, 1, st, longL));
-    return spmv_any(nb, bs, prec, Urow, Ucol, Uval, tmp, 1, x, 0, st, longU);
+    BILU_TRY(spmv_any(nb, bs, prec, Lrow, Lcol, Lval, b32, 1, tmp, 1, st, longL, true));
+    return spmv_any(nb, bs, prec, Urow, Ucol, Uval, tmp, 1, x, 0, st, longU, true);
   }
-  BILU_TRY(spmv_any(nb, bs, prec, Lrow, Lcol, Lval, b, 0, tmp, 0, st, longL));
-  return spmv_any(nb, bs, prec, Urow, Ucol, Uval, tmp, 0, x, 0, st, longU);
+  BILU_TRY(spmv_any(nb, bs, prec, Lrow, Lcol, Lval, b, 0, tmp, 0, st, longL, false));
+  return spmv_any(nb, bs, prec, Urow, Ucol, Uval, tmp, 0, x, 0, st, longU, true);
 }
 
 // Solver form: the FP32 copy of the input is already there (written by the
@@ -1008,13 +1100,14 @@ int isai_apply_f32_staged(int nb, int bs, const int* Lrow, const int* Lcol, cons
                           const int* Urow, const int* Ucol, const float* Uval, const float* b32,
                           float* tmp, double* x, cudaStream_t st, float* x32, int longL,
                           int longU) {
-  BILU_TRY(spmv_any(nb, bs, BILU_FP32, Lrow, Lcol, Lval, b32, 1, tmp, 1, st, longL));
+  BILU_TRY(spmv_any(nb, bs, BILU_FP32, Lrow, Lcol, Lval, b32, 1, tmp, 1, st, longL, false));
   if (x32) {  // x also in FP32 (input of an FP32 operator product)
     int lr = longU;
     if (longU < 0) BILU_TRY(layout_cached(nb, bs, Urow, st, &lr));
-    return BILU_DISPATCH_BS(bs, spmv_f32_dual, nb, Urow, Ucol, Uval, tmp, x, x32, st, lr);
+    return BILU_DISPATCH_BS(bs, spmv_f32_dual, nb, Urow, Ucol, Uval, tmp, x, x32, st, lr,
+                            true);
   }
-  return spmv_any(nb, bs, BILU_FP32, Urow, Ucol, Uval, tmp, 1, x, 0, st, longU);
+  return spmv_any(nb, bs, BILU_FP32, Urow, Ucol, Uval, tmp, 1, x, 0, st, longU, true);
 }
 
 }  // namespace bilu
@@ -1026,7 +1119,7 @@ extern "C" int bilu_bcsr_spmv(int mb, int bs, const int* d_row, const int* d_col
                               bilu_stream_t stream) {
   if (mb < 0 || (mb > 0 && (!d_row || !d_col || !d_val || !d_x || !d_y))) return BILU_ERR_ARG;
   if (!bs_supported(bs)) return BILU_ERR_UNSUPPORTED;
-  return spmv_any(mb, bs, BILU_FP64, d_row, d_col, d_val, d_x, 0, d_y, 0, S(stream), -1);
+  return spmv_any(mb, bs, BILU_FP64, d_row, d_col, d_val, d_x, 0, d_y, 0, S(stream), -1, false);
 }
 
 extern "C" int bilu_spmv_layout(int mb, int bs, const int* d_row, bilu_stream_t stream,
@@ -1056,7 +1149,7 @@ extern "C" int bilu_bcsr_spmv_f32(int mb, int bs, const int* d_row, const int* d
   if (mb < 0 || (mb > 0 && (!d_row || !d_col || !d_val || !d_x || !d_y))) return BILU_ERR_ARG;
   if (!bs_supported(bs)) return BILU_ERR_UNSUPPORTED;
   return spmv_any(mb, bs, BILU_FP32, d_row, d_col, d_val, d_x, x_fp32 != 0, d_y, y_fp32 != 0,
-                  S(stream), -1);
+                  S(stream), -1, false);
 }
 
 extern "C" int bilu_bcsr_spmm(int mb, int bs, int k, const int* d_row, const int* d_col,

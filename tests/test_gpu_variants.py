@@ -451,6 +451,58 @@ def test_spmm_splits(cuda, orc, bs, k):
     assert np.array_equal(got, want, equal_nan=True)
 
 
+# ------------------------------------------------------------------ products one after another
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("name", ["gaps", "hub row", "grid"])
+def test_apply_starts_before_the_first_product_ends(cuda, name, bs, fp32):
+    """The second product of the apply is started while the first one drains:
+    it has to give the bits of two separate products, with rows without blocks,
+    when the matrices, b and the buffers change right before the call, on a side
+    stream, and replayed from a graph."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    if name == "grid":
+        A = gen.convdiff3d(23, bs=4)
+        rp, col, n = A.rowptr, A.colind, A.nb
+    else:
+        rp, col = sparse_rows(name)
+        n = len(rp) - 1
+    dt = torch.float32 if fp32 else torch.float64
+    r, c = T(rp, cuda), T(col, cuda)
+    g = torch.Generator(device=cuda).manual_seed(5)
+    rand = lambda *s: torch.randn(*s, dtype=torch.float64, device=cuda, generator=g)
+    vl, vu, b = rand(len(col), bs, bs).to(dt), rand(len(col), bs, bs).to(dt), rand(n * bs)
+    prec = api.BILU_FP32 if fp32 else api.BILU_FP64
+
+    def both():
+        got = api.isai_apply(n, bs, (r, c, vl), (r, c, vu), b, prec)
+        y = api.bcsr_spmv(n, bs, r, c, vl, b.to(dt))
+        x = torch.empty_like(b)
+        return got, api.bcsr_spmv(n, bs, r, c, vu, y, x)
+
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for _ in range(8):
+                vl.mul_(-0.5)
+                vu.add_(vl)
+                b.neg_()
+                got, ref = both()
+                assert torch.equal(got, ref)
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = api.isai_apply(n, bs, (r, c, vl), (r, c, vu), b, prec)
+    for _ in range(3):
+        vu.mul_(-0.25)
+        b.add_(1.0)
+        graph.replay()
+        assert torch.equal(got, both()[1])
+
+
 # ------------------------------------------------------------------ orthogonalisation
 @pytest.mark.parametrize("fp32", [0, 1])
 @pytest.mark.parametrize("per_thread", [0, 2, 4, 6, 7])
