@@ -2702,11 +2702,14 @@ size_t level_sched_ws(int nb) {
          carve_size(sizeof(int) * 4) + carve_size(sizeof(unsigned) * 4);
 }
 
-// BILU(0) scratch: the level-scheduled one plus the row flow's plan (or the
-// block-wise schedule's update counts and ready flags) and task pointers.
+// BILU(0) scratch: the analysis output, the row flow's plan (or the block-wise
+// schedule's update counts and ready flags), then the analysis scratch or, after
+// it, the factorisation's (row flags or task pointers, words, scan sums).
 size_t bilu0_ws(int nb, long long nnzb) {
-  return level_sched_ws(nb) + carve_size(sizeof(int2) * (size_t)std::max(nnzb, 1ll)) +
-         carve_size(sizeof(int) * ((size_t)nb + 1)) + scan_ws_bytes(nb + 1);
+  const size_t rows = carve_size(sizeof(int) * ((size_t)nb + 1));
+  return rows + carve_size(sizeof(int) * ((size_t)nb + 2)) + carve_size(sizeof(int) * 4) +
+         carve_size(sizeof(int2) * (size_t)std::max(nnzb, 1ll)) +
+         std::max(levels_ws(nb), rows + 3 * carve_size(sizeof(int) * 4) + scan_ws_bytes(nb + 1));
 }
 
 // diagonal positions (validates the pattern); returns BILU_ERR_PATTERN with
@@ -3075,7 +3078,10 @@ extern "C" size_t bilu_sptrsv_analysis_bytes(int nb) {
 
 extern "C" size_t bilu_sptrsv_analysis_ws_bytes(int nb, int nnzb) {
   if (nb < 0 || nnzb < 0) return 0;
-  return levels_ws(nb) + carve_size(sizeof(int) * 2);
+  // more than the analysis takes: the size callers have planned with holds a list
+  // of the dependencies
+  return levels_ws(nb) + carve_size(sizeof(int) * 2) +
+         carve_size(sizeof(int) * (size_t)std::max((long long)nnzb - nb, 1ll));
 }
 
 extern "C" size_t bilu_sptrsv_solve_ws_bytes(int nb) {
