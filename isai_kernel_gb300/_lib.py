@@ -109,4 +109,7 @@ def check(func: str, status: int, ok=(0,)) -> int:
 
 def call(name: str, *args, ok=(0,)):
     """Call an int-returning entry point and raise BiluError on failure."""
-    return check(name, getattr(lib(), name)(*args), ok)
+    status = getattr(_LIB or lib(), name)(*args)
+    if status not in ok:
+        raise BiluError(name, status)
+    return status
