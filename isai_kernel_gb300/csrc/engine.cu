@@ -26,8 +26,6 @@ int isai_both_count(int nb, const int* row, const int* col, int* mL, int* mU, in
 int isai_both_fill(int nb, const int* row, const int* col, const int* mL, const int* mU,
                    const int* tL, const int* tU, int nL, int nU, int* indL, int* indU,
                    int* tcolL, int* tcolU, int* mapL, int* mapU, Carver& ws, cudaStream_t st);
-int reorder_impl(long long nnzb, int bs, const int* map, const double* src, double* dst,
-                 cudaStream_t st, float* dst32);
 size_t syncfree_ws(int nb);
 int diag_positions(int nb, const int* row, const int* col, int* diag, int* h_bad, Carver& ws,
                    cudaStream_t st);
@@ -78,7 +76,7 @@ int pairs_fill_impl(int nb, const int* Arow, const int* Acol, const int* Mptr, c
                     int lower, const int* PairPtr, int mnnz, int* PL, int* PS, cudaStream_t st);
 int isai_impl(int nb, int bs, const double* Aval, const int* Mptr, const int* Mind, int lower,
               const int* pp, const int* pl, const int* ps, const double* Dinv, double* Mval,
-              cudaStream_t st);
+              cudaStream_t st, const int* map, float* M32);
 int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const void* val,
              const void* x, int x32, void* y, int y32, cudaStream_t st, int layout,
              bool dep = false);
@@ -355,18 +353,16 @@ int build_isai_num(bilu_ctx* c, int lower, const IsaiSym& y, int** orow, int** o
                    double** oval, int* onnz, float** oval32) {
   cudaStream_t st = c->st;
   int nb = c->nb, bs = c->bs, bs2 = bs * bs;
-  double *Dinv, *Mcsc, *Mcsr;
+  double *Dinv, *Mcsr;
   BILU_TRY(c->alloc(&Dinv, (size_t)nb * bs2));
-  BILU_TRY(c->alloc(&Mcsc, (size_t)y.mnnz * bs2));
   BILU_TRY(c->alloc(&Mcsr, (size_t)y.mnnz * bs2));
   BILU_TRY(dinv_impl(nb, bs, c->Arow, c->Acol, c->LU, lower, Dinv, nullptr, st));
-  BILU_TRY(isai_impl(nb, bs, c->LU, y.Mptr, y.Mind, lower, y.pp, y.pl, y.ps, Dinv, Mcsc, st));
-  // the FP32 copy of the mixed apply is written by the same pass
+  // row order and the FP32 copy of the mixed apply come out of the column solves
   float* M32 = nullptr;
   if (oval32) BILU_TRY(c->alloc(&M32, (size_t)y.mnnz * bs2));
-  BILU_TRY(reorder_impl(y.mnnz, bs, y.map, Mcsc, Mcsr, st, M32));
+  BILU_TRY(isai_impl(nb, bs, c->LU, y.Mptr, y.Mind, lower, y.pp, y.pl, y.ps, Dinv, Mcsr, st, y.map,
+                     M32));
   if (oval32) *oval32 = M32;
-  c->release(Mcsc);
   c->release(Dinv);
   *orow = y.Trow;
   *ocol = y.Tcol;

@@ -11,9 +11,10 @@
 // the elements of the current block (EPL elements each): bs=4 packs two
 // columns per warp, bs=8 gives each lane two elements of one column.  The
 // pair lists are built for M_U as well, so ISAI-U does no binary searches in
-// its inner loop.  Products keep the reference's order (sum over k, then
-// subtract) and run on the DFMA pipe: DMMA m8n8k4 measured slower than DFMA
-// on GB300 (1.05 vs 1.2 TFLOP/s) and a 4x4 block fills 1/8 of its tile.
+// its inner loop.  Products are subtracted term by term, in the reference's
+// order of pairs and k (one FP64 instruction a term, no sum to subtract), on the
+// DFMA pipe: DMMA m8n8k4 measured slower than DFMA on GB300 (1.05 vs 1.2
+// TFLOP/s) and a 4x4 block fills 1/8 of its tile.
 #include "common.cuh"
 #include "scan.cuh"
 
@@ -195,7 +196,10 @@ __global__ void __launch_bounds__(256) k_pairs(int nb, long long mnnz,
 // rhs -= A(t,p) Y_p over the pairs, Y_idx = Dinv[t] rhs.  M_U: idx
 // descending with the upper pair list.  The first kCache blocks of a column
 // stay in shared memory; later ones are re-read from Mval (written by this
-// team and ordered by __syncwarp).
+// team and ordered by __syncwarp).  Block q of a column goes to Mval[q], or with
+// map to Mval[map[q]] (row order) and, rounded, to M32: the setup's form, which
+// needs no pass of its own to put the blocks in row order (64^3 bs 4, both
+// sides: 477 us and 96 of the pass -> 475; DFMA bound, 350 us of them).
 template <int BS>
 struct IsaiCfg {
   static constexpr int kCache = BS == 8 ? 12 : 24;
@@ -210,7 +214,9 @@ __global__ void __launch_bounds__(256) k_isai(int nb, const double* __restrict__
                                               const int* __restrict__ PairPL,
                                               const int* __restrict__ PairSrc,
                                               const double* __restrict__ Dinv,
-                                              double* __restrict__ Mval) {
+                                              double* __restrict__ Mval,
+                                              const int* __restrict__ map,
+                                              float* __restrict__ M32) {
   using T = Team<BS>;
   constexpr int BS2 = T::BS2, EPL = T::EPL, TL = T::TL, TPW = T::TPW, SPAN = T::SPAN;
   constexpr int CACHE = IsaiCfg<BS>::kCache;
@@ -240,8 +246,9 @@ __global__ void __launch_bounds__(256) k_isai(int nb, const double* __restrict__
   for (int step = 0; step < Nw; ++step) {
     bool on = col_on && lane_on && step < N;
     int idx = lower ? step : N - 1 - step;
-    int t = 0, qb = 0, qe = 0;
+    int t = 0, qb = 0, qe = 0, to = start + idx;
     if (col_on && step < N) {
+      if (map) to = map[to];
       t = Mind[start + idx];
       qb = PairPtr[start + idx];
       qe = PairPtr[start + idx + 1];
@@ -252,15 +259,16 @@ __global__ void __launch_bounds__(256) k_isai(int nb, const double* __restrict__
     for (int qq = qb; qq < qe; ++qq) {
       int pl = PairPL[qq];
       const double* Ab = Aval + (long long)PairSrc[qq] * BS2;
-      const double* Yp = pl < CACHE ? sY + (size_t)pl * BS2 : Mval + (long long)(start + pl) * BS2;
+      const double* Yp =
+          pl < CACHE ? sY + (size_t)pl * BS2
+                     : Mval + (long long)(map ? map[start + pl] : start + pl) * BS2;
       if (on) {
 #pragma unroll
         for (int q = 0; q < EPL; ++q) {
           if (tl * EPL + q >= BS2) continue;
-          double s = 0.0;
 #pragma unroll
-          for (int k = 0; k < BS; ++k) s = fma(__ldg(Ab + er[q] * BS + k), Yp[k * BS + ec[q]], s);
-          rhs[q] -= s;
+          for (int k = 0; k < BS; ++k)
+            rhs[q] = fma(-__ldg(Ab + er[q] * BS + k), Yp[k * BS + ec[q]], rhs[q]);
         }
       }
     }
@@ -295,7 +303,9 @@ __global__ void __launch_bounds__(256) k_isai(int nb, const double* __restrict__
       for (int q = 0; q < EPL; ++q) {
         int e = tl * EPL + q;
         if (e >= BS2) continue;
-        Mval[(long long)(start + idx) * BS2 + e] = y[q];
+        Mval[(long long)to * BS2 + e] = y[q];
+        // on the integer pipe: the conversion instruction takes the FP64 pipe
+        if (M32) M32[(long long)to * BS2 + e] = narrow(y[q]);
         if (idx < CACHE) sY[(size_t)idx * BS2 + e] = y[q];
       }
     }
@@ -318,7 +328,7 @@ int launch_dinv(int nb, const int* row, const int* col, const double* val, int l
 template <int BS>
 int launch_isai(int nb, const double* Aval, const int* Mptr, const int* Mind, int lower,
                 const int* pp, const int* pl, const int* ps, const double* Dinv, double* Mval,
-                cudaStream_t st) {
+                const int* map, float* M32, cudaStream_t st) {
   if (nb == 0) return BILU_OK;
   using T = Team<BS>;
   constexpr int W = IsaiCfg<BS>::kWarps;
@@ -331,7 +341,7 @@ int launch_isai(int nb, const double* Aval, const int* Mptr, const int* Mind, in
   }
   long long warps = (nb + T::TPW - 1) / T::TPW;
   k_isai<BS><<<ceil_div(warps, W), 32 * W, smem, st>>>(nb, Aval, Mptr, Mind, lower, pp, pl, ps,
-                                                       Dinv, Mval);
+                                                       Dinv, Mval, map, M32);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
@@ -399,9 +409,9 @@ int pairs_fill_impl(int nb, const int* Arow, const int* Acol, const int* Mptr, c
 
 int isai_impl(int nb, int bs, const double* Aval, const int* Mptr, const int* Mind, int lower,
               const int* pp, const int* pl, const int* ps, const double* Dinv, double* Mval,
-              cudaStream_t st) {
+              cudaStream_t st, const int* map = nullptr, float* M32 = nullptr) {
   return BILU_DISPATCH_BS(bs, launch_isai, nb, Aval, Mptr, Mind, lower, pp, pl, ps, Dinv, Mval,
-                          st);
+                          map, M32, st);
 }
 
 }  // namespace bilu
