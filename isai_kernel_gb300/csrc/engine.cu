@@ -83,6 +83,8 @@ int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const voi
 int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t st,
                    int* h_layout);
 int spmv_layout_word(int mb, long long nnzb, int longest);
+int copy_values(size_t count, const double* src, double* d0, double* d1, float* d32,
+                cudaStream_t st);
 int isai_apply_impl(int nb, int bs, int prec, const int* Lrow, const int* Lcol, const void* Lval,
                     const int* Urow, const int* Ucol, const void* Uval, const double* b,
                     void* tmp, double* x, cudaStream_t st, int longL, int longU);
@@ -528,17 +530,19 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
   // the values
   if (values_ready) BILU_TRY_CUDA(cudaStreamWaitEvent(st, values_ready, 0));
   tm.mark(3);
+  BILU_TRY(c->alloc(&c->LU, nnzb * bs2));
+  BILU_TRY(c->alloc(&c->rdiag, (size_t)nb * bs + 1));
+  if (prec_mask & ((1 << BILU_FP32_INNER) | (1 << BILU_NESTED)))
+    BILU_TRY(c->alloc(&c->Aval32, nnzb * bs2));
+  // the values are read once: the factor's copy, A's and its FP32 form
   if (adopt_val) {
     c->Aval = const_cast<double*>(d_val);
     c->setup_bufs.push_back(c->Aval);
+    BILU_TRY(copy_values(nnzb * bs2, d_val, c->LU, nullptr, c->Aval32, st));
   } else {
     BILU_TRY(c->alloc(&c->Aval, nnzb * bs2));
-    BILU_TRY_CUDA(cudaMemcpyAsync(c->Aval, d_val, sizeof(double) * nnzb * bs2,
-                                  cudaMemcpyDeviceToDevice, st));
+    BILU_TRY(copy_values(nnzb * bs2, d_val, c->LU, c->Aval, c->Aval32, st));
   }
-  BILU_TRY(c->alloc(&c->LU, nnzb * bs2));
-  BILU_TRY(c->alloc(&c->rdiag, (size_t)nb * bs + 1));
-  BILU_TRY_CUDA(cudaMemcpyAsync(c->LU, d_val, sizeof(double) * nnzb * bs2, cudaMemcpyDeviceToDevice, st));
   {
     Carver w2 = ws;
     int zp = -1;
@@ -561,10 +565,6 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
                             want32 ? &c->Uval32 : nullptr));
   }
   tm.mark(9);
-  if (prec_mask & ((1 << BILU_FP32_INNER) | (1 << BILU_NESTED))) {
-    BILU_TRY(c->alloc(&c->Aval32, (size_t)nnzb * bs2));
-    BILU_TRY(bilu_convert_f64_to_f32((size_t)nnzb * bs2, c->Aval, c->Aval32, st));
-  }
   if (ilu) {
     BILU_TRY(c->alloc(&c->ilu_flags, (size_t)nb + 2));
     BILU_TRY(c->alloc(&c->ilu_words, 4));

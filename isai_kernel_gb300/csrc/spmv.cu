@@ -918,11 +918,43 @@ int launch_spmm(int mb, int k, const int* row, const int* col, const VT* val, co
   return launch_spmm_cfg<BS, VT, 32, 2>(mb, k, row, col, val, X, Y, st);
 }
 
-__global__ void k_f64_to_f32(size_t n, const double* __restrict__ s, float* __restrict__ d) {
+// d32 = s rounded to FP32, d0 and d1 (optional) copies of s.  Bound by HBM: four
+// elements a thread in 16-byte accesses, rounded on the integer pipe (the
+// conversion instruction runs on the FP64 pipe, 14 us for 8.4 M elements
+// beside 15 of HBM).  vec: every pointer is on a 16-byte boundary.
+__global__ void __launch_bounds__(256) k_copy_values(size_t n, int vec,
+                                                     const double* __restrict__ s,
+                                                     double* __restrict__ d0,
+                                                     double* __restrict__ d1,
+                                                     float* __restrict__ d32) {
   dependents_launch();
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) d[i] = __double2float_rn(s[i]);
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t n4 = vec ? n / 4 : 0;
+  for (size_t i = t; i < n4; i += stride) {
+    const double2 a = ld_stream(reinterpret_cast<const double2*>(s) + 2 * i),
+                  b = ld_stream(reinterpret_cast<const double2*>(s) + 2 * i + 1);
+    if (d0) {
+      reinterpret_cast<double2*>(d0)[2 * i] = a;
+      reinterpret_cast<double2*>(d0)[2 * i + 1] = b;
+    }
+    if (d1) {
+      reinterpret_cast<double2*>(d1)[2 * i] = a;
+      reinterpret_cast<double2*>(d1)[2 * i + 1] = b;
+    }
+    if (d32) {
+      const double v[4] = {a.x, a.y, b.x, b.y};
+      float f[4];
+      narrow_all<4>(v, f);
+      reinterpret_cast<float4*>(d32)[i] = make_float4(f[0], f[1], f[2], f[3]);
+    }
+  }
+  for (size_t i = 4 * n4 + t; i < n; i += stride) {
+    const double v = s[i];
+    if (d0) d0[i] = v;
+    if (d1) d1[i] = v;
+    if (d32) d32[i] = narrow(v);
+  }
 }
 
 template <int BS>
@@ -1069,10 +1101,13 @@ int spmv_gather_t(int mb, int bs, const int* trow, const int* tcol, const int* s
   return BILU_DISPATCH_BS(bs, launch_spmv_t, mb, trow, tcol, src, val, x, y, st, layout);
 }
 
-int convert_f64_f32(size_t count, const double* src, float* dst, cudaStream_t st) {
+int copy_values(size_t count, const double* src, double* d0, double* d1, float* d32,
+                cudaStream_t st) {
   if (count == 0) return BILU_OK;
-  unsigned grid = (unsigned)std::min<size_t>((count + 255) / 256, 152 * 16);
-  k_f64_to_f32<<<grid, 256, 0, st>>>(count, src, dst);
+  const int vec = ((uintptr_t)src | (uintptr_t)d0 | (uintptr_t)d1 | (uintptr_t)d32) % 16 == 0;
+  const size_t threads = vec ? (count + 3) / 4 : count;
+  k_copy_values<<<(unsigned)std::min<size_t>((threads + 255) / 256, 152 * 16), 256, 0, st>>>(
+      count, vec, src, d0, d1, d32);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
@@ -1086,7 +1121,7 @@ int isai_apply_impl(int nb, int bs, int prec, const int* Lrow, const int* Lcol, 
                     void* tmp, double* x, cudaStream_t st, int longL, int longU) {
   if (prec == BILU_FP32) {
     float* b32 = reinterpret_cast<float*>(x);
-    BILU_TRY(convert_f64_f32((size_t)nb * bs, b, b32, st));
+    BILU_TRY(copy_values((size_t)nb * bs, b, nullptr, nullptr, b32, st));
     BILU_TRY(spmv_any(nb, bs, prec, Lrow, Lcol, Lval, b32, 1, tmp, 1, st, longL, true));
     return spmv_any(nb, bs, prec, Urow, Ucol, Uval, tmp, 1, x, 0, st, longU, true);
   }
@@ -1172,10 +1207,7 @@ extern "C" int bilu_convert_f64_to_f32(size_t count, const double* d_src, float*
                                        bilu_stream_t stream) {
   if (count == 0) return BILU_OK;
   if (!d_src || !d_dst) return BILU_ERR_ARG;
-  unsigned grid = (unsigned)std::min<size_t>((count + 255) / 256, 152 * 16);
-  k_f64_to_f32<<<grid, 256, 0, S(stream)>>>(count, d_src, d_dst);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  return copy_values(count, d_src, nullptr, nullptr, d_dst, S(stream));
 }
 
 extern "C" int bilu_isai_apply(int nb, int bs, int prec, const int* d_Lrow, const int* d_Lcol,

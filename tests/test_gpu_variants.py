@@ -546,3 +546,31 @@ def test_mgs_step_forms(cuda, fp32, per_thread):
         ref = wr / wr.norm()
         assert (vn[:n].double() - ref).abs().max() <= tol * ref.abs().max()
         assert torch.all(vn[n:] == 0)
+
+
+# ------------------------------------------------------------------ conversion
+@pytest.mark.parametrize("shift_in, shift_out", [(0, 0), (1, 0), (0, 1), (2, 4)])
+def test_values_to_fp32(cuda, shift_in, shift_out):
+    """bilu_convert_f64_to_f32 on sizes and starts with and without whole
+    16-byte groups, bit for bit the rounding of the type conversion (zeros,
+    subnormals, overflow, infinities and NaN included)."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    g = torch.Generator(device=cuda).manual_seed(1)
+    special = torch.tensor([0.0, -0.0, 1e-310, 1e-46, 1.4e-45, -3e-39, 3.5e38, -1e300, float("inf"),
+                            float("-inf"), float("nan"), 1 + 2.0 ** -24, 1 + 3 * 2.0 ** -24],
+                           dtype=torch.float64, device=cuda)
+    for n in (1, 3, 4, 5, 1021, 300000):
+        src = torch.randn(n + shift_in, dtype=torch.float64, device=cuda, generator=g)
+        k = min(n, len(special))
+        src[shift_in:shift_in + k] = special[:k]
+        out = torch.full((n + shift_out + 3,), 7.0, dtype=torch.float32, device=cuda)
+        api.call("bilu_convert_f64_to_f32", n, src.data_ptr() + 8 * shift_in,
+                 out.data_ptr() + 4 * shift_out, api._s())
+        ref = src[shift_in:].float()
+        got = out[shift_out:shift_out + n]
+        same = (got.view(torch.int32) == ref.view(torch.int32)) | (got.isnan() & ref.isnan())
+        assert bool(same.all())
+        assert bool((out[:shift_out] == 7).all()) and bool((out[shift_out + n:] == 7).all())
