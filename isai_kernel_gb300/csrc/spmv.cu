@@ -215,17 +215,22 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
 }
 
 // y = M x: lane group of BS lanes per block row, lane r owns scalar row r.
-// A group handles RPG consecutive block rows and issues the loads of the
-// next U blocks of all of them before any arithmetic, so a warp keeps
-// RPG*U independent block loads per lane in flight; each row's sum runs in
-// block order whatever U and RPG are (the same bits).  Chosen by
-// launch_spmv from measurements on the 128^3 7-point pattern (7 blocks a
-// row) and its triangle (4 a row): FP64 values U = 1, RPG = 2 (two
-// independent DFMA chains per lane; one chain is latency-bound: 0.48 ->
-// 0.40 ms on the 7-point FP64 operator, the same on the triangle); FP32
-// values U = 4 with RPG = 1 for wider rows (0.199 -> 0.176 ms on the FP32
-// operator), RPG = 1 at 8 CTAs per SM for bs 4 rows of ~4 blocks, else
-// RPG = 2.  Patterns with rows of more than kLongSpmvRow blocks take
+// FP64: bound by the FP64 pipe, where an instruction takes as long with lanes
+// off, and as long predicated off.  So a warp's groups take one block each a turn
+// and go on together until the longest row ends: no place past a row's end that
+// all the groups have reached is issued, and the warps of a full SM cover the
+// latency (two rows a group of the 4- and 5-blocks, two blocks a batch of the
+// 8-blocks before; the apply, before -> now: 64^3 7-point 4x4 67.8 -> 63.7 us,
+// 47x43x41 5x5 41.3 -> 38.9, 512^2 5-point 5x5 81.8 -> 77.9, 8x8 249 -> 172 of
+// 174 at 0.58 TDFMA/s).
+// FP32: bound by memory.  A group handles RPG consecutive block rows and issues
+// the loads of the next U blocks of all of them before any arithmetic, so a warp
+// keeps RPG*U independent block loads per lane in flight; each row's sum runs in
+// block order whatever U and RPG are (the same bits).  Chosen by launch_spmv from
+// measurements on the 128^3 7-point pattern (7 blocks a row) and its triangle (4
+// a row): U = 4 with RPG = 1 for wider rows (0.199 -> 0.176 ms on the operator),
+// RPG = 1 at 8 CTAs per SM for bs 4 rows of ~4 blocks, else RPG = 2.
+// Patterns with rows of more than kLongSpmvRow blocks take
 // k_bsr_spmv_balanced (FP64) or k_bsr_spmv_uneven (FP32).
 // DEP, for a product whose x is the result of the launch before it (U after L,
 // A after U): started by programmatic dependent launch while that one drains,
@@ -249,6 +254,7 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
   int lane = threadIdx.x & 31;
   int g = lane / BS, r = lane - g * BS;
   long long base = (((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G + g) * RPG;
+  const unsigned live = __ballot_sync(0xffffffffu, g < G && base < mb);
   if (g >= G || base >= mb) return;
   int s[RPG], e[RPG];
 #pragma unroll
@@ -261,67 +267,75 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
 #pragma unroll
   for (int q = 0; q < RPG; ++q) acc[q] = 0;
   const XT* xp = x;
-  // DEP: the first blocks wait in registers, or where these are too many in the L2
-  constexpr bool kHold = RPG * U * BS * sizeof(AccT) <= 128;
-  // batches of U blocks per row; every load of a batch (column indices,
-  // block rows, x segments) is issued before its FMAs
-  for (int off = 0;; off += U) {
-    bool any = false;
-#pragma unroll
-    for (int q = 0; q < RPG; ++q) any |= s[q] + off < e[q];
-    if (!any) break;
-    int c[RPG][U];
-#pragma unroll
-    for (int q = 0; q < RPG; ++q)
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        int p = s[q] + off + u;
-        c[q][u] = p < e[q] ? __ldg(col + p) : -1;
-      }
-    if constexpr (DEP && !kHold) {
-      if (off == 0) {
-#pragma unroll
-        for (int q = 0; q < RPG; ++q)
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (s[q] + u < e[q])
-              asm volatile("prefetch.global.L2 [%0];" ::"l"(
-                  val + ((long long)(s[q] + u) * BS + r) * BS));
-        dependency_wait();
-        xp = after_wait(x);
-      }
-    }
-    AccT a[RPG][U][BS], xv[RPG][U][BS];
-#pragma unroll
-    for (int q = 0; q < RPG; ++q)
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        // FP32, DEP: not on c, so that both loads go out before the wait
-        if (DEP && sizeof(VT) == 4 ? s[q] + off + u < e[q] : c[q][u] >= 0) {
-          load_entry<BS, TR, VT, AccT>(val, src, s[q] + off + u, r, a[q][u]);
-        } else {
-#pragma unroll
-          for (int k = 0; k < BS; ++k) a[q][u][k] = 0;
+  if constexpr (sizeof(AccT) == 8) {
+    // one block at a time, the warp's groups together until the longest row ends
+    static_assert(RPG == 1 && U == 1);
+    int c = s[0] < e[0] ? __ldg(col + s[0]) : -1;
+    for (int p = s[0]; __any_sync(live, p < e[0]); ++p) {
+      AccT a[BS], xv[BS];
+      if (c >= 0) load_entry<BS, TR, VT, AccT>(val, src, p, r, a);
+      const int next = p + 1 < e[0] ? __ldg(col + p + 1) : -1;
+      if constexpr (DEP) {
+        if (p == s[0]) {
+          dependency_wait();
+          xp = after_wait(x);
         }
       }
-    if constexpr (DEP && kHold) {
-      if (off == 0) {
-        dependency_wait();
-        xp = after_wait(x);
+      if (c >= 0) {
+        load_x<BS, XT, AccT, DEP>(xp, c, xv);
+#pragma unroll
+        for (int k = 0; k < BS; ++k) acc[0] = fma(a[k], xv[k], acc[0]);
       }
+      c = next;
     }
-    // x segments (mostly L2 hits) are consumed as they arrive, which keeps
-    // the register footprint low enough for 4 CTAs per SM with FP32 values
+  } else {
+    // batches of U blocks per row; every load of a batch (column indices,
+    // block rows, x segments) is issued before its FMAs
+    for (int off = 0;; off += U) {
+      bool any = false;
 #pragma unroll
-    for (int q = 0; q < RPG; ++q)
+      for (int q = 0; q < RPG; ++q) any |= s[q] + off < e[q];
+      if (!any) break;
+      int c[RPG][U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (c[q][u] >= 0) {
-          load_x<BS, XT, AccT, DEP>(xp, c[q][u], xv[q][u]);
+      for (int q = 0; q < RPG; ++q)
 #pragma unroll
-          for (int k = 0; k < BS; ++k) acc[q] = fma(a[q][u][k], xv[q][u][k], acc[q]);
+        for (int u = 0; u < U; ++u) {
+          int p = s[q] + off + u;
+          c[q][u] = p < e[q] ? __ldg(col + p) : -1;
+        }
+      AccT a[RPG][U][BS], xv[RPG][U][BS];
+#pragma unroll
+      for (int q = 0; q < RPG; ++q)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          // DEP: not on c, so that both loads go out before the wait
+          if (DEP ? s[q] + off + u < e[q] : c[q][u] >= 0) {
+            load_entry<BS, TR, VT, AccT>(val, src, s[q] + off + u, r, a[q][u]);
+          } else {
+#pragma unroll
+            for (int k = 0; k < BS; ++k) a[q][u][k] = 0;
+          }
+        }
+      if constexpr (DEP) {  // the first blocks wait in registers
+        if (off == 0) {
+          dependency_wait();
+          xp = after_wait(x);
         }
       }
+      // x segments (mostly L2 hits) are consumed as they arrive, which keeps
+      // the register footprint low enough for 4 CTAs per SM with FP32 values
+#pragma unroll
+      for (int q = 0; q < RPG; ++q)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (c[q][u] >= 0) {
+            load_x<BS, XT, AccT, DEP>(xp, c[q][u], xv[q][u]);
+#pragma unroll
+            for (int k = 0; k < BS; ++k) acc[q] = fma(a[q][u][k], xv[q][u][k], acc[q]);
+          }
+        }
+    }
   }
   if constexpr (DEP) dependency_wait();  // rows without blocks
 #pragma unroll
@@ -563,7 +577,7 @@ int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const
   constexpr int G = 32 / BS;
   long long groups = (mb + RPG - 1) / RPG;
   long long warps = (groups + G - 1) / G;
-  if constexpr (!TR) {
+  if constexpr (!TR && RPG == 1) {
     if (dep) {
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -628,7 +642,7 @@ int launch_spmv_balanced(int mb, const int* row, const int* col, const int* src,
 }
 
 // The configurations measured faster on the stencil patterns (k_bsr_spmv)
-// apply to patterns without long rows, FP64 at block sizes 4 and 5.
+// apply to patterns without long rows.
 template <int BS, class VT, class XT, class YT>
 int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
                 cudaStream_t st, int layout, float* y32, bool dep) {
@@ -642,9 +656,9 @@ int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT*
   }
   if constexpr (sizeof(VT) == 8) {
     if constexpr (BS <= 5)
-      return launch_spmv_cfg<BS, VT, XT, YT, 2, 1, 4>(mb, row, col, val, x, y, st, y32, dep);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 1, 6>(mb, row, col, val, x, y, st, y32, dep);
     else
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 2, 2>(mb, row, col, val, x, y, st, y32, dep);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 1, 5>(mb, row, col, val, x, y, st, y32, dep);
   } else if constexpr (BS == 8 && sizeof(XT) == 8) {
     // two rows of 8x8 blocks with FP64 x segments spill at 64 registers
     return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
@@ -673,10 +687,10 @@ int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, cons
   if (layout & kLayoutLong)
     return launch_spmv_balanced<BS, 2, 4, true>(mb, trow, tcol, src, val, x, y, st, nullptr);
   if constexpr (BS <= 5)
-    return launch_spmv_cfg<BS, D, D, D, 2, 1, 4, true>(mb, trow, tcol, val, x, y, st, nullptr,
+    return launch_spmv_cfg<BS, D, D, D, 1, 1, 6, true>(mb, trow, tcol, val, x, y, st, nullptr,
                                                        false, src);
   else
-    return launch_spmv_cfg<BS, D, D, D, 1, 2, 2, true>(mb, trow, tcol, val, x, y, st, nullptr,
+    return launch_spmv_cfg<BS, D, D, D, 1, 1, 5, true>(mb, trow, tcol, val, x, y, st, nullptr,
                                                        false, src);
 }
 

@@ -451,6 +451,36 @@ def test_spmm_splits(cuda, orc, bs, k):
     assert np.array_equal(got, want, equal_nan=True)
 
 
+# ------------------------------------------------------------------ rows of mixed lengths
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("n", [1, 6, 31, 1000])
+def test_fp64_product_mixed_rows(cuda, n, bs):
+    """The FP64 product and its transpose with rows of 0 to 9 blocks side by
+    side in a warp, the last warp partly filled, against numpy: at most 72
+    products a sum, so 72 eps of the sum of their magnitudes."""
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(n)
+    cols = [np.sort(rng.choice(n, size=min(n, int(rng.integers(0, 10))), replace=False))
+            for _ in range(n)]
+    cols[0] = np.arange(min(n, 3))
+    rp = np.zeros(n + 1, np.int32)
+    np.cumsum([len(c) for c in cols], out=rp[1:])
+    col = np.concatenate(cols).astype(np.int32)
+    val, x = rng.standard_normal((len(col), bs, bs)), rng.standard_normal((n, bs))
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    for transpose in (False, True):
+        ref, mag = np.zeros((n, bs)), np.zeros((n, bs))
+        to, at = (col, rows) if transpose else (rows, col)
+        v = val.transpose(0, 2, 1) if transpose else val
+        np.add.at(ref, to, np.einsum("pij,pj->pi", v, x[at]))
+        np.add.at(mag, to, np.einsum("pij,pj->pi", np.abs(v), np.abs(x[at])))
+        f = api.bcsr_spmv_transpose if transpose else api.bcsr_spmv
+        got = N(f(n, bs, T(rp, cuda), T(col, cuda), T(val, cuda), T(x.ravel(), cuda)))
+        most = max(int(np.bincount(to, minlength=n).max()) * bs, 72)
+        assert np.all(np.abs(got.reshape(n, bs) - ref) <= 2 * most * 1.2e-16 * mag + 1e-300)
+
+
 # ------------------------------------------------------------------ products one after another
 @pytest.mark.parametrize("fp32", [False, True])
 @pytest.mark.parametrize("bs", [4, 5, 8])
