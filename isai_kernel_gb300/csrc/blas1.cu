@@ -338,7 +338,7 @@ struct MgsVec<float> {
   }
 };
 
-// 512 threads, two CTAs per SM: half the partials and barrier arrivals of
+// 512 threads, two CTAs per SM: half the partial sums of
 // 256-thread CTAs at the same occupancy (measured 3-6% faster a sweep at
 // 128^3, FP64 and FP32)
 constexpr int kStepThreads = 512;
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       }
       cp_async_wait<0>();
       // the next sweep's first stages read v_i (as v_{i-1}) and v_{i+1}: start
-      // those lines towards the L2 before the grid barrier (1-2% a sweep)
+      // those lines towards the L2 while the sums cross (1-2% a sweep)
       for (long long k = 0; k < S - 1 && k < K; ++k) {
         const long long e = tid + k * stride;
         if (vnv) asm volatile("prefetch.global.L2 [%0];" ::"l"(vnv + e));

@@ -349,8 +349,8 @@ int build_isai_sym(bilu_ctx* c, Carver& ws, IsaiSym& L, IsaiSym& U, int* h_longe
   return BILU_OK;
 }
 
-// The values of one ISAI side on the factor: Dinv, the column solves into
-// BCSC and the reorder into BCSR (with the FP32 copy when asked for).
+// The values of one ISAI side on the factor: Dinv, the column solves, stored
+// in BCSR order (with the FP32 copy when asked for).
 int build_isai_num(bilu_ctx* c, int lower, const IsaiSym& y, int** orow, int** ocol,
                    double** oval, int* onnz, float** oval32) {
   cudaStream_t st = c->st;
@@ -382,7 +382,7 @@ namespace {
 // ISAI patterns and pair lists of both sides, the SpMV layouts and the upper
 // level analysis of the exact-ILU modes.  Then, after values_ready (an event
 // the caller records when d_val is on the device; null: already there), the
-// values: BILU(0), Dinv, the ISAI column solves, the reorders and the FP32
+// values: BILU(0), Dinv, the ISAI column solves and the FP32
 // copies.  The structure phase thus overlaps a host-to-device copy of the
 // values that the caller issues on another stream.
 // adopt_val: d_val is a buffer of the library's pool that the handle takes
@@ -967,7 +967,7 @@ extern "C" int bilu_ctx_solve(bilu_ctx* c, int prec, const double* d_b, double* 
       BILU_TRY_CUDA(cudaMemcpyAsync(&ilu_err, c->ilu_words + 2, sizeof(int),
                                     cudaMemcpyDeviceToHost, st));
     BILU_TRY_CUDA(cudaStreamSynchronize(st));
-    if (ilu_err != 0) return ilu_err;  // a triangular-solve barrier timed out
+    if (ilu_err != 0) return ilu_err;  // a triangular solve's wait ran out
     beta = std::sqrt(rr);
     res = beta / bnorm;
     if (res <= tol) status = BILU_OK;

@@ -1,7 +1,6 @@
 // Grid-wide synchronisation for cooperative launches (sm_103a): bounded
 // polling with back-off and a counting grid barrier.  Shared by the level
-// kernels (BILU(0), triangular solves, level analysis) and the Krylov
-// solver's orthogonalisation kernels.
+// kernels (BILU(0), triangular solves) and the batch solver's step kernels.
 #pragma once
 
 #include "common.cuh"
