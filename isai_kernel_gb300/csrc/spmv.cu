@@ -10,7 +10,7 @@
 // (bs*bs*8 bytes) is fetched in whole 32-byte sectors by one group, and the x
 // segment is a broadcast within the group.
 #include <algorithm>
-
+#include <climits>
 #include <mutex>
 #include <type_traits>
 
@@ -704,8 +704,8 @@ int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, cons
 // conversion instructions run on the FP64 pipe and were the bound (512 x 512
 // 5-point grid, 4x4 blocks, k 32: 342 -> 220 us, 92 us of HBM, bound by issue and L1).  Sums run in
 // block order, then column order, whatever LPR and KW are.
-// Rows of more than kLongSpmvRow blocks (a group alone takes ~0.5 us a block, a
-// millisecond for a hub of 2000) are left to k_spmm_hubs.
+// Rows of more than `most` blocks (kLongSpmvRow: a group alone takes ~0.5 us a
+// block, a millisecond for a hub of 2000) are left to k_spmm_hubs.
 // vec: val starts on a 16-byte boundary (else blocks are read element by element)
 template <int BS, class VT>
 __device__ __forceinline__ void spmm_row(const VT* __restrict__ val, long long p, int r, int vec,
@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(256) k_spmm_hubs(int mb, int k, int vec,
 // FULL: k is LPR KW and val is aligned, known to the compiler (immediate offsets,
 // no predicates or branches).
 template <int BS, class VT, int LPR, int KW, bool FULL>
-__global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any,
+__global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any, int most,
                                                   const int* __restrict__ row,
                                                   const int* __restrict__ col,
                                                   const VT* __restrict__ val,
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any
   if (br >= mb) return;
   const int e = __ldg(row + br + 1);
   int p = __ldg(row + br);
-  if (e - p > kLongSpmvRow) return;
+  if (e - p > most) return;
   VT acc[KW][BS];
 #pragma unroll
   for (int w = 0; w < KW; ++w)
@@ -905,12 +905,17 @@ int launch_spmm_cfg(int mb, int k, const int* row, const int* col, const VT* val
                     double* Y, cudaStream_t st) {
   const int vec = (uintptr_t)val % 16 == 0;
   const unsigned grid = ceil_div(mb, 8 * (32 / LPR));
+  // A few rows are not worth a second launch for the long ones among them: a
+  // square matrix without repeated columns has none there, and a slice of a
+  // wider one keeps a group per row whatever its rows hold.
+  const bool hubs = mb > kLongSpmvRow;
+  const int most = hubs ? kLongSpmvRow : INT_MAX;
   if (k == LPR * KW && vec)
-    k_bsr_spmm<BS, VT, LPR, KW, true><<<grid, 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
+    k_bsr_spmm<BS, VT, LPR, KW, true><<<grid, 256, 0, st>>>(mb, k, vec, most, row, col, val, X, Y);
   else
-    k_bsr_spmm<BS, VT, LPR, KW, false><<<grid, 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
+    k_bsr_spmm<BS, VT, LPR, KW, false><<<grid, 256, 0, st>>>(mb, k, vec, most, row, col, val, X, Y);
   BILU_LAUNCH_CHECK();
-  if (mb > kLongSpmvRow) {  // as many blocks in a row need as many columns
+  if (hubs) {
     k_spmm_hubs<BS, VT, sizeof(VT) == 8 ? LPR : 32>
         <<<ceil_div(mb, kHubRows), 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
     BILU_LAUNCH_CHECK();

@@ -451,6 +451,39 @@ def test_spmm_splits(cuda, orc, bs, k):
     assert np.array_equal(got, want, equal_nan=True)
 
 
+@pytest.mark.parametrize("k", [1, 33])
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("mb, ncol, repeated", [(3, 200, False), (64, 65, False), (65, 300, False),
+                                                (16, 16, True)])
+def test_spmm_few_rows_of_many_blocks(cuda, bs, k, mb, ncol, repeated):
+    """Slices with more block columns than block rows, and rows that hold a
+    column several times: every row of Y is written, by the sum of its blocks
+    (bounds as in test_spmm_splits)."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(1000 * mb + 10 * bs + k)
+    cols = [np.sort(rng.integers(0, ncol, size=90)) if repeated else np.arange(ncol)
+            for _ in range(mb)]
+    rp = np.zeros(mb + 1, np.int32)
+    np.cumsum([len(c) for c in cols], out=rp[1:])
+    col = np.concatenate(cols).astype(np.int32)
+    val, X = rng.uniform(-1, 1, size=(len(col), bs, bs)), rng.uniform(-1, 1, size=(ncol * bs, k))
+    rows = np.repeat(np.arange(mb), np.diff(rp))
+    r, c, x = T(rp, cuda), T(col, cuda), T(X, cuda)
+    bound = 2 * (np.repeat(np.diff(rp) * bs, bs).astype(float) ** 2)[:, None]
+    for dtype, eps in ((torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)):
+        v = T(val, cuda).to(dtype)
+        D = np.zeros((mb, bs, ncol, bs))
+        np.add.at(D, (rows, slice(None), col, slice(None)), N(v).astype(np.float64))
+        Xr = X if dtype == torch.float64 else X.astype(np.float32).astype(np.float64)
+        Y = torch.full((mb * bs, k), float("nan"), dtype=torch.float64, device=cuda)
+        api.call("bilu_bcsr_spmm" if dtype == torch.float64 else "bilu_bcsr_spmm_f32", mb, bs, k,
+                 api._p(r), api._p(c), api._p(v), api._p(x), api._p(Y), api._s())
+        assert np.all(np.abs(N(Y) - D.reshape(mb * bs, -1) @ Xr) <= bound * eps)
+
+
 # ------------------------------------------------------------------ rows of mixed lengths
 @pytest.mark.parametrize("bs", [4, 5, 8])
 @pytest.mark.parametrize("n", [1, 6, 31, 1000])
