@@ -10,7 +10,6 @@
 // (bs*bs*8 bytes) is fetched in whole 32-byte sectors by one group, and the x
 // segment is a broadcast within the group.
 #include <algorithm>
-#include <climits>
 #include <mutex>
 #include <type_traits>
 
@@ -702,10 +701,11 @@ int launch_spmv_t(int mb, const int* trow, const int* tcol, const int* src, cons
 // side (launch_spmm).  With FP32 values X is rounded to FP32 where it is read
 // and the sums are widened where they are stored, on the integer pipe: the
 // conversion instructions run on the FP64 pipe and were the bound (512 x 512
-// 5-point grid, 4x4 blocks, k 32: 342 -> 220 us, 92 us of HBM, bound by issue and L1).  Sums run in
-// block order, then column order, whatever LPR and KW are.
-// Rows of more than `most` blocks (kLongSpmvRow: a group alone takes ~0.5 us a
-// block, a millisecond for a hub of 2000) are left to k_spmm_hubs.
+// 5-point grid, 4x4 blocks, k 32: 342 -> 213 us, 92 us of HBM, bound by issue and
+// L1).  Sums run in block order, then column order, whatever LPR and KW are (but
+// for hub rows).
+// With `hubs`, hub rows (spmm_hub: a group alone takes ~0.5 us a block, a
+// millisecond for a hub of 2000) are left to k_spmm_hubs.
 // vec: val starts on a 16-byte boundary (else blocks are read element by element)
 template <int BS, class VT>
 __device__ __forceinline__ void spmm_row(const VT* __restrict__ val, long long p, int r, int vec,
@@ -739,63 +739,84 @@ __device__ __forceinline__ double spmm_out(VT v) {
   else return v;
 }
 
-// The long rows of the product, a CTA per kHubRows block rows, which looks for
-// them (most CTAs find none; a launch of its own so that the short rows' kernel
-// keeps its registers).  With FP64 values the CTA's groups of LPR lanes share a
-// row's blocks, U in flight each; FP32 sums keep their order, so there a group
-// takes one scalar row of the block row.  20,000-row power-law pattern, 4x4
-// blocks, k 32, the whole product: FP64 2461 -> 590 us, FP32 1023 -> 470 us.
-constexpr int kHubRows = 64;
+// A row that is summed apart: long, and much longer than the rows are on average.
+// Where many rows are long a group per row fills the chip, and a CTA per row only
+// adds barriers (20,000 rows of 67 4x4 blocks, FP32, k 32: 165 us with a group per
+// row, 1845 with a CTA).  With few rows it does not: up to kHubFewRows every
+// long row is a hub (a wave of CTAs; 300 rows of 300 8x8 blocks, FP64, k 1: 1455 us
+// with a group per row, 50 so), and FP32 rows of twice that length up to 4096 rows
+// (2000 rows of 201 8x8 blocks, k 1: 350 / 214).
+constexpr int kHubFewRows = 152 * 4;
+constexpr int kHubCtas = 2 * kHubFewRows;
+template <class VT>
+__device__ __forceinline__ bool spmm_hub(int len, int mb, const int* __restrict__ row) {
+  if (len <= kLongSpmvRow) return false;
+  if (mb <= kHubFewRows || (sizeof(VT) == 4 && mb <= 4096 && len > 2 * kLongSpmvRow)) return true;
+  return (long long)len * mb > 4ll * (__ldg(row + mb) - __ldg(row));
+}
 
+// The hub rows of the product, a CTA each: its groups of LPR lanes share the row's
+// blocks, U in flight each, and add their sums in a fixed order.  The CTAs look
+// for hubs in turn, CH rows (a sector of row pointers on large matrices) at a
+// time, so that neighbouring hubs go to different CTAs.  Started by programmatic
+// dependent launch beside the other rows' kernel, whose rows of Y it does not
+// touch, it ends after that one.  20,000-row power-law pattern, 4x4 blocks, k 32,
+// the whole product, a warp per row / so: FP64 2507 / 530 us, FP32 1065 / 158.
 template <int BS, class VT, int LPR>
-__global__ void __launch_bounds__(256) k_spmm_hubs(int mb, int k, int vec,
-                                                   const int* __restrict__ row,
-                                                   const int* __restrict__ col,
-                                                   const VT* __restrict__ val,
-                                                   const double* __restrict__ X,
-                                                   double* __restrict__ Y) {
-  constexpr bool SHARE = sizeof(VT) == 8;
+__global__ void __launch_bounds__(256, BS <= 5 ? 3 : 2)
+    k_spmm_hubs(int mb, int k, int vec, int ch, const int* __restrict__ row,
+                const int* __restrict__ col, const VT* __restrict__ val,
+                const double* __restrict__ X, double* __restrict__ Y) {
   constexpr int GW = 32 / LPR, NG = 8 * GW;
-  constexpr int U = SHARE ? (BS <= 5 ? 4 : 2) : 8;
-  __shared__ double part_s[SHARE ? 8 * BS * LPR : 1];
-  __shared__ int list_s[kHubRows];
+  constexpr int U = BS <= 5 ? 4 : 2;
+  __shared__ VT part_s[8 * BS * LPR];
+  __shared__ int list_s[256];
   const int lane = threadIdx.x & 31, l = lane & (LPR - 1), warp = threadIdx.x >> 5;
   const int gi = warp * GW + lane / LPR;
-  bool lng = false;
-  if (threadIdx.x < kHubRows) {
-    const long long i = (long long)blockIdx.x * kHubRows + threadIdx.x;
-    lng = i < mb && __ldg(row + i + 1) - __ldg(row + i) > kLongSpmvRow;
-    list_s[threadIdx.x] = lng ? (int)i : -1;
-  }
-  if (!__syncthreads_or(lng)) return;
-  for (int h = 0; h < kHubRows; ++h) {
-    const int hub = list_s[h];
-    if (hub < 0) continue;  // uniform across the CTA
-    const int hs = __ldg(row + hub), he = __ldg(row + hub + 1);
-    for (int k0 = 0; k0 < k; k0 += LPR) {
-      const bool in = k0 + l < k;
-      const double* Xc = X + k0 + l;
-      if constexpr (SHARE) {
-        double acc[BS];
+  const int per = 256 / ch;  // this CTA's turns looked through at once
+  const int off = threadIdx.x % ch;
+  for (long long t0 = 0; (t0 * gridDim.x + blockIdx.x) * ch < mb; t0 += per) {
+    const long long i = ((t0 + threadIdx.x / ch) * gridDim.x + blockIdx.x) * ch + off;
+    const bool hub = i < mb && spmm_hub<VT>(__ldg(row + i + 1) - __ldg(row + i), mb, row);
+    if (!__syncthreads_or(hub)) continue;
+    list_s[threadIdx.x] = hub ? (int)i : -1;
+    __syncthreads();
+    unsigned todo = 0;  // of the list's next 32 entries, the same in every warp
+    for (int h = 0; h < 256 || todo;) {
+      if (!todo) {
+        todo = __ballot_sync(0xffffffffu, list_s[h + lane] >= 0);
+        h += 32;
+        continue;
+      }
+      const int br = list_s[h - 33 + __ffs(todo)];
+      todo &= todo - 1;
+      const int hs = __ldg(row + br), he = __ldg(row + br + 1);
+      for (int k0 = 0; k0 < k; k0 += LPR) {
+        const bool in = k0 + l < k;
+        const double* Xc = X + k0 + l;
+        VT acc[BS];
 #pragma unroll
         for (int r = 0; r < BS; ++r) acc[r] = 0;
         for (int q = hs + gi; q < he; q += NG * U) {
-          double xv[U][BS];
+          double xd[U][BS];
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const double* xb = Xc + (long long)__ldg(col + min(q + u * NG, he - 1)) * BS * k;
 #pragma unroll
-            for (int kk = 0; kk < BS; ++kk) xv[u][kk] = in ? __ldg(xb + (long long)kk * k) : 0.0;
+            for (int kk = 0; kk < BS; ++kk)
+              xd[u][kk] = in ? __ldg(xb + (long long)kk * k) : kNoRhs;
           }
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             if (q + u * NG >= he) break;
+            VT xv[BS];
+            spmm_in<BS>(xd[u], xv);
 #pragma unroll
             for (int r = 0; r < BS; ++r) {
-              double a[BS];
-              spmm_row<BS, double>(val, q + u * NG, r, vec, a);
+              VT a[BS];
+              spmm_row<BS, VT>(val, q + u * NG, r, vec, a);
 #pragma unroll
-              for (int kk = 0; kk < BS; ++kk) acc[r] = fma(a[kk], xv[u][kk], acc[r]);
+              for (int kk = 0; kk < BS; ++kk) acc[r] = fma(a[kk], xv[kk], acc[r]);
             }
           }
         }
@@ -809,50 +830,29 @@ __global__ void __launch_bounds__(256) k_spmm_hubs(int mb, int k, int vec,
         __syncthreads();
         for (int t = threadIdx.x; t < BS * LPR; t += 256) {
           const int r = t / LPR, c = k0 + t % LPR;
-          double sum = 0.0;
+          VT sum = 0;
 #pragma unroll
           for (int w = 0; w < 8; ++w) sum += part_s[(w * BS + r) * LPR + t % LPR];
-          if (c < k) Y[((long long)hub * BS + r) * k + c] = sum;
+          if (c < k) Y[((long long)br * BS + r) * k + c] = spmm_out(sum);
         }
         __syncthreads();
-      } else if (gi < BS) {
-        VT t = 0;
-        for (int q = hs; q < he; q += U) {
-          double xd[U][BS];
-          VT a[U][BS];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int p = min(q + u, he - 1);
-            const double* xb = Xc + (long long)__ldg(col + p) * BS * k;
-#pragma unroll
-            for (int kk = 0; kk < BS; ++kk)
-              xd[u][kk] = in ? __ldg(xb + (long long)kk * k) : kNoRhs;
-            spmm_row<BS, VT>(val, p, gi, vec, a[u]);
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (q + u < he) {
-              VT xv[BS];
-              spmm_in<BS>(xd[u], xv);
-#pragma unroll
-              for (int kk = 0; kk < BS; ++kk) t = fma(a[u][kk], xv[kk], t);
-            }
-        }
-        if (in) Y[((long long)hub * BS + gi) * k + k0 + l] = spmm_out(t);
       }
     }
+    __syncthreads();  // the list is written again
   }
+  dependency_wait();  // what follows in the stream comes after both kernels
 }
 
 // FULL: k is LPR KW and val is aligned, known to the compiler (immediate offsets,
 // no predicates or branches).
+// (8x8 blocks, FP64: 6 CTAs per SM, not the 4 of 56 registers: 5000 rows of 41
+// blocks, k 32, 1023 -> 890 us.)
 template <int BS, class VT, int LPR, int KW, bool FULL>
-__global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any, int most,
-                                                  const int* __restrict__ row,
-                                                  const int* __restrict__ col,
-                                                  const VT* __restrict__ val,
-                                                  const double* __restrict__ X,
-                                                  double* __restrict__ Y) {
+__global__ void __launch_bounds__(256, sizeof(VT) == 8 && BS == 8 && KW == 1 && FULL ? 6 : 0)
+    k_bsr_spmm(int mb, int k_any, int vec_any, int hubs, const int* __restrict__ row,
+               const int* __restrict__ col, const VT* __restrict__ val,
+               const double* __restrict__ X, double* __restrict__ Y) {
+  dependents_launch();  // k_spmm_hubs
   const int k = FULL ? LPR * KW : k_any, vec = FULL ? 1 : vec_any;
   const int lane = threadIdx.x & 31, l = lane & (LPR - 1);
   const long long br =
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any
   if (br >= mb) return;
   const int e = __ldg(row + br + 1);
   int p = __ldg(row + br);
-  if (e - p > most) return;
+  if (hubs && spmm_hub<VT>(e - p, mb, row)) return;
   VT acc[KW][BS];
 #pragma unroll
   for (int w = 0; w < KW; ++w)
@@ -876,10 +876,17 @@ __global__ void __launch_bounds__(256) k_bsr_spmm(int mb, int k_any, int vec_any
       for (int w = 0; w < KW; ++w)
         xd[kk * KW + w] = l + LPR * w < k ? __ldg(xb + kk * k + LPR * w) : kNoRhs;
     if (p + 1 < e) bc = __ldg(col + p + 1);
-    // FP32: the next block's X on its way (250 -> 220 us on the grid above; the
+    // FP32: the next block's X and values on their way (the grid above 250 -> 213 us;
+    // 2000 rows of 67 blocks, where every block waited for its values, 50 -> 41; the
     // FP64 product has the time)
     if (sizeof(VT) == 4 && p + 1 < e)
       asm volatile("prefetch.global.L1 [%0];" ::"l"(X + (long long)bc * BS * k + l));
+    {
+      constexpr int LW = 128 / (int)sizeof(VT);  // a line a lane, and the block's last element
+      if (sizeof(VT) == 4 && p + 1 < e && (l - 1) * LW < BS * BS)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(val + (long long)(p + 1) * BS * BS +
+                                                      min(l * LW, BS * BS - 1)));
+    }
     VT xv[BS * KW];
 #pragma unroll
     for (int i = 0; i < BS * KW; ++i) spmm_in<1>({xd[i]}, reinterpret_cast<VT(&)[1]>(xv[i]));
@@ -908,18 +915,29 @@ int launch_spmm_cfg(int mb, int k, const int* row, const int* col, const VT* val
   // A few rows are not worth a second launch for the long ones among them: a
   // square matrix without repeated columns has none there, and a slice of a
   // wider one keeps a group per row whatever its rows hold.
-  const bool hubs = mb > kLongSpmvRow;
-  const int most = hubs ? kLongSpmvRow : INT_MAX;
+  const int hubs = mb > kLongSpmvRow;
   if (k == LPR * KW && vec)
-    k_bsr_spmm<BS, VT, LPR, KW, true><<<grid, 256, 0, st>>>(mb, k, vec, most, row, col, val, X, Y);
+    k_bsr_spmm<BS, VT, LPR, KW, true><<<grid, 256, 0, st>>>(mb, k, vec, hubs, row, col, val, X, Y);
   else
-    k_bsr_spmm<BS, VT, LPR, KW, false><<<grid, 256, 0, st>>>(mb, k, vec, most, row, col, val, X, Y);
+    k_bsr_spmm<BS, VT, LPR, KW, false><<<grid, 256, 0, st>>>(mb, k, vec, hubs, row, col, val, X, Y);
   BILU_LAUNCH_CHECK();
-  if (hubs) {
-    k_spmm_hubs<BS, VT, sizeof(VT) == 8 ? LPR : 32>
-        <<<ceil_div(mb, kHubRows), 256, 0, st>>>(mb, k, vec, row, col, val, X, Y);
-    BILU_LAUNCH_CHECK();
-  }
+  if (!hubs) return BILU_OK;
+  // a row a CTA and turn up to kHubCtas, then runs of up to a sector of row
+  // pointers
+  int ch = 1;
+  while (ch < 8 && mb > ch * kHubCtas) ch *= 2;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min<unsigned>(ceil_div(mb, ch), kHubCtas));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  BILU_TRY_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_hubs<BS, VT, LPR>, mb, k, vec, ch, row, col, val,
+                                   X, Y));
+  BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
 

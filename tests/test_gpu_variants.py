@@ -484,6 +484,39 @@ def test_spmm_few_rows_of_many_blocks(cuda, bs, k, mb, ncol, repeated):
         assert np.all(np.abs(N(Y) - D.reshape(mb * bs, -1) @ Xr) <= bound * eps)
 
 
+@pytest.mark.parametrize("k", [1, 6, 33])
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("mb, hubs, ln", [(65, 65, 65), (608, 9, 64), (608, 9, 65), (609, 9, 65),
+                                          (1217, 1217, 67), (1300, 1300, 131), (5000, 20, 300)])
+def test_spmm_hub_rows(cuda, bs, k, mb, hubs, ln):
+    """Neighbouring rows of `ln` blocks among rows of two: as ordinary rows (64
+    blocks; rows all alike) and each by a CTA, on matrices around the sizes where
+    a CTA looks through one, two and more rows at a time (bounds as in
+    test_spmm_splits)."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(mb + 10 * bs + k + ln)
+    n = np.full(mb, 2)
+    n[mb - hubs:] = ln
+    rp = np.zeros(mb + 1, np.int32)
+    np.cumsum(n, out=rp[1:])
+    rows = np.repeat(np.arange(mb), n)
+    col = rng.integers(0, mb, size=len(rows)).astype(np.int32)
+    val, X = rng.uniform(-1, 1, size=(len(col), bs, bs)), rng.uniform(-1, 1, size=(mb * bs, k))
+    r, c = T(rp, cuda), T(col, cuda)
+    bound = 2 * ((n * bs).astype(float) ** 2)[:, None, None]
+    for dtype, eps in ((torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)):
+        v = T(val, cuda).to(dtype)
+        Xr = X if dtype == torch.float64 else X.astype(np.float32).astype(np.float64)
+        ref = np.zeros((mb, bs, k))
+        np.add.at(ref, rows, np.einsum("pij,pjk->pik", N(v).astype(np.float64),
+                                       Xr.reshape(mb, bs, k)[col]))
+        Y = N(api.bcsr_spmm(mb, bs, r, c, v, T(X, cuda))).reshape(mb, bs, k)
+        assert np.all(np.abs(Y - ref) <= bound * eps)
+
+
 # ------------------------------------------------------------------ rows of mixed lengths
 @pytest.mark.parametrize("bs", [4, 5, 8])
 @pytest.mark.parametrize("n", [1, 6, 31, 1000])
