@@ -553,6 +553,15 @@ int bilu_debug_sptrsv_withhold_flow(int nb, int nnzb, int bs, const int* d_row, 
                                     const double* d_val, int lower, const double* d_b,
                                     double* d_x, int withhold_row, long long spin_limit,
                                     void* d_ws, size_t ws_bytes, bilu_stream_t stream);
+/* bilu_bsrilu0_ex with block row withhold_row never publishing (-1: every row
+ * does) and a spin budget of spin_limit polls: the rows that depend on it give
+ * up, BILU_ERR_TIMEOUT.  Workspace bilu_bsrilu0_ws_bytes(nb, nnzb).  The row
+ * flow's waits give up when no row has been finished for spin_limit polls; the
+ * barrier kernel has no such wait and ignores both. */
+int bilu_debug_bsrilu0_withhold(int nb, int nnzb, int bs, const int* d_row, const int* d_col,
+                                double* d_val, int schedule, int withhold_row,
+                                long long spin_limit, void* d_ws, size_t ws_bytes,
+                                bilu_stream_t stream);
 /* Sets the SpMV layout word (0 to 3, see bilu_spmv_layout) the entry
  * points use for the pattern (d_row, mb, bs), replacing the one they found.
  * Every layout gives the product to within rounding for any pattern; this

@@ -215,6 +215,10 @@ struct LevelOut {
   // pattern takes the row flow
   int2* plan = nullptr;
   int h_rowflow = 0;
+  // test hook: polls before a wait of the factorisation gives up, and a row that
+  // never publishes (-1: none)
+  long long spin = kSpinLimit;
+  int withhold = -1;
 };
 
 }  // namespace bilu

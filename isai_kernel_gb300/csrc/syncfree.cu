@@ -1572,11 +1572,17 @@ __device__ __forceinline__ bool bilu0_wrow(int I, const int* __restrict__ row,
 // order as in k_sptrsv_flow (the rows of one warp sit in one level and never
 // wait for each other; all warps are resident, so every wait ends); the next
 // row's blocks and the structure of the one after it are loaded before the
-// current row waits.  A row's flag is released as soon as U_II, U_IJ and the
-// reciprocal pivots are stored; its L blocks, which no other row reads, follow.
+// current row waits.  With that deal warps may stand at a late level while one
+// warp alone walks a long path up to it: a wait gives up when no row at all has
+// been reported for ss.spin polls (ss.ticket names the last one; a warp reports a
+// row about every kTellCycles), not after ss.spin polls of its own row.  A row's
+// flag is released as soon as U_II, U_IJ and the reciprocal pivots are stored; its
+// L blocks, which no other row reads, follow.
 // Measured, analysis included, against the schedules before it
 // (block size 4): 64^3 7-point 4.3 -> 1.6 ms, 128^3 11.5 -> 6.6 ms, 256 x 256
 // 5-point 7.7 -> 2.8 ms; block size 8: 64^3 6.1 -> 4.2 ms.
+constexpr unsigned kTellCycles = 1u << 20;  // half a millisecond
+
 template <int BS>
 struct RowFlow {
   static constexpr int T = BS == 4 ? 16 : 32;              // lanes per row
@@ -1634,12 +1640,13 @@ __device__ __forceinline__ void rowflow_load(int I, const GRowMeta& m, RowFlow<B
   }
 }
 
-// One row per team; false (in every lane) if the launch aborted.
+// One row per team; false (in every lane) if the launch aborted.  tell: the row is
+// reported in ss.ticket.
 template <int BS>
 __device__ __forceinline__ bool rowflow_finish(RowFlow<BS>& w, int tl, int tb, int q, int r,
                                                bool on, const int* __restrict__ col,
                                                const int2* __restrict__ plan, double* val,
-                                               const SyncState& ss) {
+                                               bool tell, const SyncState& ss) {
   using F = RowFlow<BS>;
   constexpr int T = F::T, NQ = F::NQ, EPL = F::EPL, BS2 = BS * BS;
   int er[EPL], ec[EPL];
@@ -1658,12 +1665,18 @@ __device__ __forceinline__ bool rowflow_finish(RowFlow<BS>& w, int tl, int tb, i
     bool wait = w.K >= 0;
     long long n = 0;
     unsigned ns = 32;
+    int seen = -1;
     while (true) {
       if (wait) wait = ld_relaxed(ss.flags + w.K) == 0;
       if (!__any_sync(FULL, wait)) break;
       if (++n > ss.spin) {
-        if ((threadIdx.x & 31) == 0) atomicCAS(ss.err, 0, (int)BILU_ERR_TIMEOUT);
-        return false;
+        const int last = __shfl_sync(FULL, ld_relaxed(ss.ticket), 0);
+        if (last == seen) {
+          if ((threadIdx.x & 31) == 0) atomicCAS(ss.err, 0, (int)BILU_ERR_TIMEOUT);
+          return false;
+        }
+        seen = last;  // a row writes its own number, once
+        n = 0;
       }
       if ((n & 31) == 0 && __any_sync(FULL, ld_relaxed(ss.err) != 0)) return false;
       if (n > kFlowSpin) backoff(ns);
@@ -1760,7 +1773,10 @@ __device__ __forceinline__ bool rowflow_finish(RowFlow<BS>& w, int tl, int tb, i
     }
   }
   __syncwarp();  // the team's stores before its first lane's release
-  if (tl == 0 && w.I >= 0) st_release(ss.flags + w.I, 1);
+  if (tl == 0 && w.I >= 0 && w.I != ss.withhold) {
+    st_release(ss.flags + w.I, 1);
+    if (tell) st_relaxed(ss.ticket, w.I + 1);
+  }
   if (w.K >= 0) {  // the last pass's L blocks
     double* b = val + ((long long)(w.rs + (nlow - 1) / NQ * NQ + q) * BS + r) * BS;
 #pragma unroll
@@ -1803,6 +1819,7 @@ __global__ void __launch_bounds__(kLvlThreads, BS == 4 ? 2 : 1) k_bilu0_rowflow(
   GRowMeta m1;
   grow_meta(I1, row, diag, m1);
   int I2 = row_at(c2);
+  unsigned told = (unsigned)clock(), visits = 0;  // when it last reported a row; rows
   while (c0.l < nlev) {
     F nxt;
     rowflow_load<BS>(I1, m1, nxt, tl, q, r, on, col, plan, val);
@@ -1810,7 +1827,15 @@ __global__ void __launch_bounds__(kLvlThreads, BS == 4 ? 2 : 1) k_bilu0_rowflow(
     grow_meta(I2, row, diag, m2);
     const int I3 = row_at(c3);
     if (__any_sync(FULL, cur.I >= 0)) {
-      if (!rowflow_finish<BS>(cur, tl, tb, q, r, on, col, plan, val, ss)) return;
+      // (one store per row: 64^3 1.6 -> 5 ms, all go to one address; the clock is
+      // read every 16 rows, each time it cost a path 2%)
+      bool tell = false;
+      if ((++visits & 15u) == 0) {
+        const unsigned now = (unsigned)clock();
+        tell = now - told > kTellCycles;
+        if (tell) told = now;
+      }
+      if (!rowflow_finish<BS>(cur, tl, tb, q, r, on, col, plan, val, tell, ss)) return;
     }
     cur = nxt;
     m1 = m2;
@@ -2814,7 +2839,7 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
   if (schedule == 0 || schedule == 1) sched = schedule;  // caller's choice
   if (keep.h_rowflow && schedule != 1) {
     SyncState ss;
-    BILU_TRY(sync_init(ss, nb, ws, st));
+    BILU_TRY(sync_init(ss, nb, ws, st, keep.spin, keep.withhold));
     ss.rdiag = rdiag;
     if (nb > 0)
       BILU_TRY(BILU_DISPATCH_BS(bs, launch_bilu0_rowflow, nb, row, col, diag, val, order, lvl,
@@ -2888,6 +2913,7 @@ int bilu0_impl(int nb, long long nnzb, int bs, const int* row, const int* col, c
                double* rdiag, LevelOut* keep) {
   const bool kept = keep && keep->order && keep->lvl && keep->nlev;
   LevelOut local;
+  if (keep && !kept) local = *keep;  // the test hook's limits
   LevelOut& k = kept ? *keep : local;
   if (!kept) {
     k.order = ws.take<int>((size_t)nb + 1);
@@ -3209,6 +3235,30 @@ extern "C" int bilu_sptrsv_ex(int nb, int nnzb, int bs, const int* d_row, const 
   BILU_TRY(diag_positions(nb, d_row, d_col, diag, nullptr, ws, S(stream)));
   return sptrsv_level_impl(nb, nnzb, bs, d_row, d_col, diag, d_val, lower != 0, unit != 0, d_b,
                            d_x, ws, S(stream));
+}
+
+// Test hook: BILU(0) (bilu_bsrilu0_ex) with block row `withhold_row` never
+// publishing (-1: every row does) and a spin budget of spin_limit polls, so the
+// rows that depend on it give up and the call returns BILU_ERR_TIMEOUT (the others
+// see the error word and leave).  Every wait is bounded; the launch ends by itself
+// and the context stays usable.
+extern "C" int bilu_debug_bsrilu0_withhold(int nb, int nnzb, int bs, const int* d_row,
+                                           const int* d_col, double* d_val, int schedule,
+                                           int withhold_row, long long spin_limit, void* d_ws,
+                                           size_t ws_bytes, bilu_stream_t stream) {
+  if (nb < 1 || nnzb < nb || !d_row || !d_col || !d_val || schedule < -1 || schedule > 1 ||
+      spin_limit < 1 || spin_limit > kSpinLimit)
+    return BILU_ERR_ARG;
+  if (!bs_supported(bs)) return BILU_ERR_UNSUPPORTED;
+  Carver ws(d_ws, ws_bytes);
+  int* diag = ws.take<int>((size_t)nb + 1);
+  if (!diag) return BILU_ERR_WORKSPACE;
+  BILU_TRY(diag_positions(nb, d_row, d_col, diag, nullptr, ws, S(stream)));
+  LevelOut hook;
+  hook.spin = spin_limit;
+  hook.withhold = withhold_row;
+  return bilu0_impl(nb, nnzb, bs, d_row, d_col, diag, d_val, nullptr, ws, S(stream), schedule,
+                    nullptr, &hook);
 }
 
 // Test hook: the sync-free solve with block row `withhold_row` never

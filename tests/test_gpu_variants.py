@@ -206,6 +206,40 @@ def test_bilu0_schedules(cuda, orc, name, bs):
     assert np.max(np.abs(out[0] - ref)) <= 1e-12 * np.max(np.abs(ref))
 
 
+def withheld(cuda, A, schedule, row, polls):
+    """Status and factor of BILU(0) with `row` never publishing."""
+    from isai_kernel_gb300 import _lib, api
+
+    lu = T(A.val, cuda)
+    r, c = T(A.rowptr, cuda), T(A.colind, cuda)
+    L = _lib.lib()
+    ws = api._ws(L.bilu_bsrilu0_ws_bytes(A.nb, A.nnzb), cuda)
+    st = L.bilu_debug_bsrilu0_withhold(A.nb, A.nnzb, A.bs, api._p(r), api._p(c), api._p(lu),
+                                       schedule, row, polls, api._p(ws), ws.numel(), api._s())
+    return st, N(lu)
+
+
+@pytest.mark.parametrize("bs", [4, 8])
+def test_row_flow_waits_for_a_long_path(cuda, orc, bs):
+    """A path of 3000 rows, walked by one warp, in front of 2000 rows that wait
+    for its end: their waits last many times the limit, but rows keep finishing.
+    With a row of the path withheld they give up."""
+    n, fan = 3000, 2000
+    rp, col = pattern_of([{max(i - 1, 0), i + 1} if i < n - 1 else
+                          {n - 2, *range(n, n + 50)} if i < n else {n - 1}
+                          for i in range(n + fan)])
+    rng = np.random.default_rng(bs)
+    val = rng.uniform(-1, 1, size=(len(col), bs, bs))
+    val[np.repeat(np.arange(n + fan), np.diff(rp)) == col] += 8 * bs * np.eye(bs)
+    A = gen.BSRMatrix(n + fan, bs, rp, col, val)
+    st, lu = withheld(cuda, A, -1, -1, 4000)
+    assert st == 0
+    LU, _ = orc.bsrilu0(A.nb, bs, rp, col, val)
+    assert np.max(np.abs(lu - LU)) <= 1e-12 * np.max(np.abs(LU))
+    assert withheld(cuda, A, -1, n // 2, 4000)[0] == -4  # BILU_ERR_TIMEOUT
+    assert withheld(cuda, A, -1, -1, 1 << 20)[0] == 0
+
+
 def test_bilu0_zero_pivot_row(cuda):
     """The first row with a zero pivot is reported by every schedule."""
     from isai_kernel_gb300 import api
