@@ -215,6 +215,7 @@ struct LevelOut {
   // pattern takes the row flow
   int2* plan = nullptr;
   int h_rowflow = 0;
+  int h_counted = 0;  // the caller's block count covers the stored blocks
   // test hook: polls before a wait of the factorisation gives up, and a row that
   // never publishes (-1: none)
   long long spin = kSpinLimit;

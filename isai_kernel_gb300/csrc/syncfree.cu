@@ -417,6 +417,7 @@ struct LevelWords {
   unsigned long long ndeps;  // dependencies of all rows
   int other;                 // k_bilu0_plan: the pattern is not one for the row flow
   int widest;                // rows of the widest level of at most kSortCap rows
+  int blocks;                // k_bilu0_plan: the blocks the row pointers hold
 };
 
 __device__ __forceinline__ void st_relaxed(int* p, int v) {
@@ -2272,15 +2273,16 @@ __global__ void k_order_len(int nb, const int* __restrict__ row, const int* __re
 
 // The row flow's plan for every lower position pk = (I, K): the diagonal
 // position of row K and the position of U_KI in row K (-1: not stored).
-// *other is set when some dependency updates a block that is not the diagonal
+// w->other is set when some dependency updates a block that is not the diagonal
 // of its row (or has a list too long to tell cheaply): the pattern then does
 // not take the row flow.
 __global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
                                                     const int* __restrict__ row,
                                                     const int* __restrict__ col,
                                                     const int* __restrict__ diag,
-                                                    int2* __restrict__ plan, int* other) {
+                                                    int2* __restrict__ plan, LevelWords* w) {
   const long long pk = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (pk == 0) w->blocks = __ldg(row + nb);
   if (pk >= nnzb) return;
   int I;
   const MatchLists m = match_lists(pk, nb, row, col, diag, I);
@@ -2295,7 +2297,7 @@ __global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
     at = m.from_i ? o : c;
   }
   plan[pk] = make_int2(__ldg(diag + __ldg(col + pk)), at);
-  if (odd) *other = 1;
+  if (odd) w->other = 1;
 }
 
 // Total of the match counts in 64 bits (the caller decides from it whether
@@ -2536,12 +2538,13 @@ int launch_coop(const void* fn, int grid, int threads, void** args, cudaStream_t
 // sync-free) on the device; the same words on the host.  One host
 // synchronisation.  ndeps_max: the dependencies the caller's block count
 // leaves room for (BILU_ERR_WORKSPACE beyond it).  plan (optional, lower DAG,
-// one entry per stored block): the row flow's plan; *h_rowflow whether the
-// pattern takes it.
+// nplan entries, one per stored block): the row flow's plan; *h_rowflow whether
+// the pattern takes it, *h_counted whether nplan covers the stored blocks.
 int build_levels(int nb, const int* row, const int* col, const int* diag, int lower,
                  long long ndeps_max, int* order, int* lvl_ptr, int* nlev_d, int* h_nlev,
                  Carver& ws, cudaStream_t st, int* h_sched = nullptr, int* h_maxdeg = nullptr,
-                 int* h_fsched = nullptr, int2* plan = nullptr, int* h_rowflow = nullptr) {
+                 int* h_fsched = nullptr, int2* plan = nullptr, long long nplan = 0,
+                 int* h_rowflow = nullptr, int* h_counted = nullptr) {
   if (nb == 0) {
     BILU_TRY_CUDA(cudaMemsetAsync(nlev_d, 0, sizeof(int) * 4, st));
     BILU_TRY_CUDA(cudaMemsetAsync(lvl_ptr, 0, sizeof(int) * 2, st));
@@ -2552,8 +2555,8 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
   LevelWords *w = nullptr, hw;
   BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st));
   if (plan) {
-    const long long nnzb = ndeps_max + nb;
-    k_bilu0_plan<<<ceil_div(nnzb, 256), 256, 0, st>>>(nb, nnzb, row, col, diag, plan, &w->other);
+    k_bilu0_plan<<<ceil_div(std::max(nplan, 1ll), 256), 256, 0, st>>>(nb, nplan, row, col, diag,
+                                                                       plan, w);
     BILU_LAUNCH_CHECK();
   }
   int rec[4];
@@ -2566,7 +2569,9 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
   if (h_maxdeg) *h_maxdeg = rec[1];
   if (h_sched) *h_sched = rec[2];
   if (h_fsched) *h_fsched = rec[3];
-  if (h_rowflow) *h_rowflow = plan && !hw.other && rec[1] <= kLongRow ? 1 : 0;
+  const bool counted = plan && hw.blocks <= nplan;
+  if (h_rowflow) *h_rowflow = counted && !hw.other && rec[1] <= kLongRow ? 1 : 0;
+  if (h_counted) *h_counted = counted ? 1 : 0;
   if (hw.widest > 1) {
     static bool attr_set = false;
     if (!attr_set) {
@@ -2781,7 +2786,7 @@ int bilu0_analyze(int nb, long long nnzb, const int* row, const int* col, const 
   if (!keep.order || !keep.lvl || !keep.nlev) return BILU_ERR_WORKSPACE;
   return build_levels(nb, row, col, diag, 1, std::max(nnzb - nb, 0ll), keep.order, keep.lvl,
                       keep.nlev, &keep.h_nlev, ws, st, &keep.h_sched, &keep.h_maxdeg,
-                      &keep.h_fsched, keep.plan, &keep.h_rowflow);
+                      &keep.h_fsched, keep.plan, nnzb, &keep.h_rowflow, &keep.h_counted);
 }
 
 // BILU(0)'s match lists from the pattern alone (a structure step, before
@@ -2846,25 +2851,28 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
                                 nlev_d, keep.plan, ss, st));
     return sync_finish(ss, h_zp, st);
   }
-  if (sched == 1 && keep.h_maxdeg <= kLongRow) {
+  // A caller's block count that holds the dependencies but not every block is
+  // enough for the schedules that keep nothing per block: the barrier kernel and
+  // the rows without match counts.
+  if (sched == 1 && (keep.h_maxdeg <= kLongRow || !keep.h_counted)) {
     // narrow levels: sync-free over rows.  (Block by block, below, a short row
     // costs more hand-overs than it gains: 64^3 27-point pattern 104 ms against
     // 15.6; with hub rows, 20,011-row power-law pattern, 1.4 ms against 8.0.)
-    int* nmatch = (int*)keep.plan;  // the plan is not read any more
-    if (!nmatch) return BILU_ERR_WORKSPACE;
+    int* nmatch = keep.h_counted ? (int*)keep.plan : nullptr;  // the plan is not read any more
     SyncState ss;
     BILU_TRY(sync_init(ss, nb, ws, st));
     ss.order = order;
     ss.rdiag = rdiag;
     ss.nmatch = nmatch;
-    if (nb > 0) {
+    if (nb > 0 && nmatch) {
       const unsigned grid = ceil_div(std::max(nnzb, 1ll), 256);
       k_bilu0_nmatch<false><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, nmatch, nullptr);
       BILU_LAUNCH_CHECK();
       k_bilu0_nmatch_long<false><<<grid, 256, 0, st>>>(nb, nnzb, row, col, diag, nmatch, nullptr);
       BILU_LAUNCH_CHECK();
-      BILU_TRY(BILU_DISPATCH_BS(bs, launch_bilu0_syncfree, nb, row, col, diag, val, ss, st));
     }
+    if (nb > 0)
+      BILU_TRY(BILU_DISPATCH_BS(bs, launch_bilu0_syncfree, nb, row, col, diag, val, ss, st));
     return sync_finish(ss, h_zp, st);
   }
   if (sched == 1) {

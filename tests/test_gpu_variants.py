@@ -206,6 +206,32 @@ def test_bilu0_schedules(cuda, orc, name, bs):
     assert np.max(np.abs(out[0] - ref)) <= 1e-12 * np.max(np.abs(ref))
 
 
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("name", ["5-point", "7-point", "bipartite", "9-point", "dense", "hubs"])
+def test_bilu0_block_count_of_the_dependencies(cuda, name, bs):
+    """A block count that holds the diagonal and the dependencies, not the blocks
+    right of the diagonal, is accepted: the same factor, and one block less is
+    refused as long as the level analysis can see it."""
+    from isai_kernel_gb300 import api
+
+    rp, col = bilu_pattern(name)
+    nb, nnzb = len(rp) - 1, len(col)
+    rows = np.repeat(np.arange(nb), np.diff(rp))
+    rng = np.random.default_rng(bs)
+    val = rng.uniform(-1, 1, size=(nnzb, bs, bs))
+    val[rows == col] += 2.0 * bs * np.diff(rp)[:, None, None] * np.eye(bs)
+    low = nb + int((col < rows).sum())
+    assert low < nnzb
+    for schedule in (-1, 0, 1):
+        want, got = T(val, cuda), T(val, cuda)
+        assert api.bsrilu02_inplace(nb, nnzb, bs, T(rp, cuda), T(col, cuda), want, schedule) == -1
+        assert api.bsrilu02_inplace(nb, low, bs, T(rp, cuda), T(col, cuda), got, schedule) == -1
+        assert np.array_equal(N(want), N(got))
+    with pytest.raises(api.BiluError) as e:
+        api.bsrilu02_inplace(nb, low - 1, bs, T(rp, cuda), T(col, cuda), T(val, cuda))
+    assert e.value.status == _lib_status("BILU_ERR_WORKSPACE")
+
+
 def withheld(cuda, A, schedule, row, polls):
     """Status and factor of BILU(0) with `row` never publishing."""
     from isai_kernel_gb300 import _lib, api
