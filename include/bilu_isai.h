@@ -150,12 +150,13 @@ int bilu_bcsc_to_bcsr(int mb, int nbcol, int bs, const int* d_cscPtr, const int*
  * no level information): BILU(0) in place.  A level analysis of the lower
  * DAG picks the schedule.  Patterns in which a dependency updates nothing but
  * its row's diagonal block (stencils without triangles), no row with more than
- * 32 dependencies: rows in level order, each waiting for the rows it reads.
- * Otherwise levels of at least 4096 block rows on average and no row with more
- * than 32 dependencies -> one cooperative launch with a bounded grid barrier
- * per level (a bs-lane group per row); else sync-free, atomic tickets in level
- * order and bounded waits on ready flags: a warp per row, or per block where a
- * row has more than 32 dependencies.
+ * 32 dependencies: rows in level order, each waiting for the rows it reads, unless
+ * the levels are very wide.  Otherwise levels of at least 4096 block rows on
+ * average and no row with more than 32 dependencies -> one cooperative launch with
+ * a bounded grid barrier per level (a bs-lane group per row); else sync-free,
+ * atomic tickets in level order and bounded waits on ready flags: a warp per row,
+ * or per block where rows of more than 32 dependencies hold a good part of the
+ * blocks.
  * h_info[0] receives the first block row with a zero pivot (or -1);
  * BILU_ERR_ZERO_PIVOT then. */
 size_t bilu_bsrilu0_ws_bytes(int nb, int nnzb);

@@ -215,6 +215,7 @@ struct LevelOut {
   // pattern takes the row flow
   int2* plan = nullptr;
   int h_rowflow = 0;
+  int h_blocks = 0;   // long rows hold enough to take the factorisation by blocks
   int h_counted = 0;  // the caller's block count covers the stored blocks
   // test hook: polls before a wait of the factorisation gives up, and a row that
   // never publishes (-1: none)

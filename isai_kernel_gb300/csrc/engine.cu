@@ -57,7 +57,7 @@ int sptrsv_levels_async(int nb, int bs, const int* row, const int* col, const in
 int bilu0_impl(int nb, long long nnzb, int bs, const int* row, const int* col, const int* diag,
                double* val, int* h_zp, Carver& ws, cudaStream_t st, int schedule,
                double* rdiag, LevelOut* keep);
-int bilu0_analyze(int nb, long long nnzb, const int* row, const int* col, const int* diag,
+int bilu0_analyze(int nb, long long nnzb, int bs, const int* row, const int* col, const int* diag,
                   LevelOut& keep, Carver& ws, cudaStream_t st);
 int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
                  const int* diag, double* val, int* h_zp, Carver& ws, cudaStream_t st,
@@ -435,7 +435,7 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
   tm.mark(1);
   {
     Carver w2 = ws;
-    BILU_TRY(bilu0_analyze(nb, nnzb, c->Arow, c->Acol, c->diag, keepL, w2, st));
+    BILU_TRY(bilu0_analyze(nb, nnzb, bs, c->Arow, c->Acol, c->diag, keepL, w2, st));
   }
   // the barrier factorisation's match lists (which A_IJ each L_IK updates,
   // with U_KJ), built here from the pattern instead of searched for inside

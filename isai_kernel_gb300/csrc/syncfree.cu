@@ -415,6 +415,7 @@ struct LevelWords {
   int ticket, err;           // next 32 rows; 0 or a bilu_status
   int maxdeg, nlev;          // largest dependency count of a row; levels
   unsigned long long ndeps;  // dependencies of all rows
+  unsigned long long hubdeps;  // of the rows with more than kLongRow
   int other;                 // k_bilu0_plan: the pattern is not one for the row flow
   int widest;                // rows of the widest level of at most kSortCap rows
   int blocks;                // k_bilu0_plan: the blocks the row pointers hold
@@ -470,6 +471,10 @@ __global__ void __launch_bounds__(256) k_levels(int nb, const int* __restrict__ 
     if (lane == 0 && deg > 0) {
       atomicMax(&w->maxdeg, deg);
       atomicAdd(&w->ndeps, (unsigned long long)deps);
+    }
+    if (deg > kLongRow) {
+      const unsigned h = __reduce_add_sync(FULL, pe - p > kLongRow ? (unsigned)(pe - p) : 0u);
+      if (lane == 0) atomicAdd(&w->hubdeps, (unsigned long long)h);
     }
     int c[kLevelBatch];
 #pragma unroll
@@ -1262,8 +1267,8 @@ __device__ __forceinline__ void bilu0_grow(const BRowPre& pr, const int* __restr
 }
 
 // One block row with a whole warp (the sync-free factorisation of patterns with
-// triangles, narrow levels and no row of more than kLongRow dependencies).  WAIT: the rows K it reads may
-// still be in progress and are waited for through their flags.  Phase 1 by
+// triangles and narrow levels, or with few long rows).  WAIT: the rows K it reads
+// may still be in progress and are waited for through their flags.  Phase 1 by
 // the whole warp (PL lanes per row of L_IK), or for runs of dependencies
 // without updates by a lane group each; phase 2 with teams of lanes per
 // updated block; the diagonal LU by the whole warp; U blocks with 32/BS
@@ -1849,8 +1854,8 @@ __global__ void __launch_bounds__(kLvlThreads, BS == 4 ? 2 : 1) k_bilu0_rowflow(
   }
 }
 
-// Sync-free BILU(0) over single blocks (patterns with rows of more than
-// kLongRow dependencies).  A task is one stored block (I, J), taken by a warp:
+// Sync-free BILU(0) over single blocks (patterns with enough of their blocks in
+// rows of more than kLongRow dependencies: blocks_instead).  A task is one stored block (I, J), taken by a warp:
 //   A_IJ -= L_IK U_KJ for the K < min(I, J) stored in rows I and (as K, J) K,
 //     in ascending K,
 //   then L_IJ = A_IJ U_JJ^-1 (J < I), the LU of the diagonal block (J = I) or
@@ -2532,19 +2537,44 @@ int launch_coop(const void* fn, int grid, int threads, void** args, cudaStream_t
   return BILU_OK;
 }
 
+// Levels so wide that a row's latency does not count: the barrier kernel, whose
+// lane group per row spends fewer FP64 instructions a row than the row flow's team
+// of a half or whole warp.  Rows per level, dependencies a row: barrier / row flow
+// in us, block sizes 4, 5 and 8 --
+// 8000, 1: 484 / 508, 598 / 1048, 1052 / 1717; 8000, 3: 831 / 670, 990 / 1227,
+// 1827 / 2168; 16000, 1: 660 / 835, 999 / 1939, 1772 / 3264; 32000, 3 (bs 4):
+// 1631 / 1619; 16000, 12 (bs 4): 3972 / 2581; no dependencies at all, 300,000 rows:
+// 261 / 458, 328 / 972, 640 / 1767.
+bool barrier_instead(int bs, int nb, int nlev, unsigned long long ndeps) {
+  if (bs == 4) return nb >= 2ll * kFactorLevelWidth * nlev && 2 * ndeps < 5ull * nb;
+  return 2ll * nb >= 3ll * kFactorLevelWidth * nlev;
+}
+
+// Block tasks cost each block a few microseconds of a warp, and cut the chain
+// through long rows into its blocks: they pay where enough of the blocks are
+// dependencies of long rows.  That share of all blocks, 40^3 grids with long rows
+// (128^2: *), rows / blocks in ms, block sizes 4 and 8 --
+// 0.1%*: 2.4 / 5.6, 3.2 / 4.0; 0.2%: 2.2 / 4.2, 3.6 / 4.1; 0.4%: 4.4 / 7.5,
+// 7.2 / 6.3; 1.1%*: 7.0 / 8.6, 11.3 / 7.9; 3.8%: 17.9 / 23.9, 28 / 17; 8.4%*:
+// 18.8 / 11.1, 33 / 10; 8.7%: 25.9 / 27.2, 42 / 27; 19% (power law): 2.6 / 1.0,
+// 5.8 / 1.3.
+bool blocks_instead(int bs, long long nnzb, unsigned long long hubdeps) {
+  return hubdeps * (bs <= 5 ? 20 : 400) > (unsigned long long)nnzb;
+}
+
 // Level analysis of the lower (or upper) dependency DAG: order[nb] (ascending
 // inside a level), lvl_ptr[nb+1] and nlev_d[4] (levels, largest dependency
 // count, recommended solve and factorisation schedules: 0 level order, 1
 // sync-free) on the device; the same words on the host.  One host
 // synchronisation.  ndeps_max: the dependencies the caller's block count
-// leaves room for (BILU_ERR_WORKSPACE beyond it).  plan (optional, lower DAG,
-// nplan entries, one per stored block): the row flow's plan; *h_rowflow whether
-// the pattern takes it, *h_counted whether nplan covers the stored blocks.
+// leaves room for (BILU_ERR_WORKSPACE beyond it).  plan and out (optional, lower
+// DAG, nplan entries, one per stored block; bs the block size): the row flow's plan,
+// and which of BILU(0)'s schedules the pattern takes.
 int build_levels(int nb, const int* row, const int* col, const int* diag, int lower,
                  long long ndeps_max, int* order, int* lvl_ptr, int* nlev_d, int* h_nlev,
                  Carver& ws, cudaStream_t st, int* h_sched = nullptr, int* h_maxdeg = nullptr,
-                 int* h_fsched = nullptr, int2* plan = nullptr, long long nplan = 0,
-                 int* h_rowflow = nullptr, int* h_counted = nullptr) {
+                 int* h_fsched = nullptr, int2* plan = nullptr, long long nplan = 0, int bs = 0,
+                 LevelOut* out = nullptr) {
   if (nb == 0) {
     BILU_TRY_CUDA(cudaMemsetAsync(nlev_d, 0, sizeof(int) * 4, st));
     BILU_TRY_CUDA(cudaMemsetAsync(lvl_ptr, 0, sizeof(int) * 2, st));
@@ -2569,9 +2599,13 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
   if (h_maxdeg) *h_maxdeg = rec[1];
   if (h_sched) *h_sched = rec[2];
   if (h_fsched) *h_fsched = rec[3];
-  const bool counted = plan && hw.blocks <= nplan;
-  if (h_rowflow) *h_rowflow = counted && !hw.other && rec[1] <= kLongRow ? 1 : 0;
-  if (h_counted) *h_counted = counted ? 1 : 0;
+  if (out) {
+    const bool counted = plan && hw.blocks <= nplan;
+    out->h_counted = counted;
+    out->h_rowflow = counted && !hw.other && rec[1] <= kLongRow &&
+                     !barrier_instead(bs, nb, rec[0], hw.ndeps);
+    out->h_blocks = counted && rec[1] > kLongRow && blocks_instead(bs, nplan, hw.hubdeps);
+  }
   if (hw.widest > 1) {
     static bool attr_set = false;
     if (!attr_set) {
@@ -2781,12 +2815,12 @@ int sync_init_words(SyncState& ss, Carver& ws, cudaStream_t st) {
 // Level analysis of BILU(0)'s lower DAG into keep (order, lvl, nlev on the
 // device; level count, schedules and largest dependency count on the host).
 // Structure only: it may run before the values are on the device.
-int bilu0_analyze(int nb, long long nnzb, const int* row, const int* col, const int* diag,
+int bilu0_analyze(int nb, long long nnzb, int bs, const int* row, const int* col, const int* diag,
                   LevelOut& keep, Carver& ws, cudaStream_t st) {
   if (!keep.order || !keep.lvl || !keep.nlev) return BILU_ERR_WORKSPACE;
   return build_levels(nb, row, col, diag, 1, std::max(nnzb - nb, 0ll), keep.order, keep.lvl,
                       keep.nlev, &keep.h_nlev, ws, st, &keep.h_sched, &keep.h_maxdeg,
-                      &keep.h_fsched, keep.plan, nnzb, &keep.h_rowflow, &keep.h_counted);
+                      &keep.h_fsched, keep.plan, nnzb, bs, &keep);
 }
 
 // BILU(0)'s match lists from the pattern alone (a structure step, before
@@ -2854,10 +2888,10 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
   // A caller's block count that holds the dependencies but not every block is
   // enough for the schedules that keep nothing per block: the barrier kernel and
   // the rows without match counts.
-  if (sched == 1 && (keep.h_maxdeg <= kLongRow || !keep.h_counted)) {
+  if (sched == 1 && !keep.h_blocks) {
     // narrow levels: sync-free over rows.  (Block by block, below, a short row
     // costs more hand-overs than it gains: 64^3 27-point pattern 104 ms against
-    // 15.6; with hub rows, 20,011-row power-law pattern, 1.4 ms against 8.0.)
+    // 15.6.)
     int* nmatch = keep.h_counted ? (int*)keep.plan : nullptr;  // the plan is not read any more
     SyncState ss;
     BILU_TRY(sync_init(ss, nb, ws, st));
@@ -2876,7 +2910,7 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
     return sync_finish(ss, h_zp, st);
   }
   if (sched == 1) {
-    // long rows: sync-free over blocks, rows in level order
+    // many dependencies in long rows: sync-free over blocks, rows in level order
     const size_t cnt = (size_t)std::max(nnzb, 1ll);
     int* tcnt = (int*)keep.plan;  // not read any more: two ints a block
     int* flags = tcnt + cnt;
@@ -2933,7 +2967,7 @@ int bilu0_impl(int nb, long long nnzb, int bs, const int* row, const int* col, c
   if (!k.plan) return BILU_ERR_WORKSPACE;
   {
     Carver w2 = ws;
-    BILU_TRY(bilu0_analyze(nb, nnzb, row, col, diag, k, w2, st));
+    BILU_TRY(bilu0_analyze(nb, nnzb, bs, row, col, diag, k, w2, st));
   }
   return bilu0_factor(nb, nnzb, bs, row, col, diag, val, h_zp, ws, st, schedule, rdiag, k);
 }

@@ -206,6 +206,50 @@ def test_bilu0_schedules(cuda, orc, name, bs):
     assert np.max(np.abs(out[0] - ref)) <= 1e-12 * np.max(np.abs(ref))
 
 
+def rule_pattern(name):
+    """Patterns on either side of the lines between BILU(0)'s schedules."""
+    if name == "two wide levels":  # 8192 rows a level, one dependency
+        return pattern_of([[i - 8192] if i >= 8192 else [] for i in range(2 * 8192)])
+    if name == "a little narrower":
+        return pattern_of([[i - 6000] if i >= 6000 else [] for i in range(2 * 6000)])
+    if name == "wide, six dependencies":
+        return pattern_of([[(i * 7 + k * 31) % 8192 for k in range(6)] if i >= 8192 else []
+                           for i in range(2 * 8192)])
+    if name == "wide, a triangle":
+        return pattern_of([[] if i < 8192 else [0, 1, i - 8192] if i > 16383 else [i - 8192]
+                           for i in range(16385)] + [[8192, 0]])
+    A = gen.laplace2d(30, bs=4)
+    rows = [set(A.colind[A.rowptr[i]:A.rowptr[i + 1]].tolist()) for i in range(A.nb)]
+    n = {"one row of 33": 1, "long rows, 2%": 2, "long rows, 10%": 12}[name]
+    for q in range(n):
+        rows[A.nb - 1 - 5 * q] |= set(range(3 + q, 3 + q + 33 * 3, 3)) if n == 1 else \
+            set(range(q, q + 45 * 3, 3))
+    return pattern_of(rows)
+
+
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("name", ["two wide levels", "a little narrower",
+                                  "wide, six dependencies", "wide, a triangle",
+                                  "one row of 33", "long rows, 2%", "long rows, 10%"])
+def test_bilu0_rule_between_schedules(cuda, orc, name, bs):
+    """As test_bilu0_schedules, on both sides of each line of the rule."""
+    from isai_kernel_gb300 import api
+
+    rp, col = rule_pattern(name)
+    nb, nnzb = len(rp) - 1, len(col)
+    rows = np.repeat(np.arange(nb), np.diff(rp))
+    val = np.random.default_rng(bs).uniform(-1, 1, size=(nnzb, bs, bs))
+    val[rows == col] += 2.0 * bs * np.diff(rp)[:, None, None] * np.eye(bs)
+    ref, _ = orc.bsrilu0(nb, bs, rp, col, val)
+    out = []
+    for schedule in (-1, 0, 1):
+        v = T(val, cuda)
+        assert api.bsrilu02_inplace(nb, nnzb, bs, T(rp, cuda), T(col, cuda), v, schedule) == -1
+        out.append(N(v))
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    assert np.max(np.abs(out[0] - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
 @pytest.mark.parametrize("bs", [4, 5, 8])
 @pytest.mark.parametrize("name", ["5-point", "7-point", "bipartite", "9-point", "dense", "hubs"])
 def test_bilu0_block_count_of_the_dependencies(cuda, name, bs):
