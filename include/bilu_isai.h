@@ -204,21 +204,21 @@ int bilu_isai_compute(int nb, int bs, const double* d_Aval, const int* d_Mptr, c
 /* ------------------------------------------------------------------ */
 
 /* Replaces bcsr_spmv (bcsc2bcsrAndSpMV.h:49) and bsr_SpMV_tensorcore
- * (bsr_tensor_SpMV.h:402): y = M x.  FP64 values and vectors.  Rows of more
- * than 64 blocks are summed by a whole CTA instead of one lane group; the
- * first call with a given d_row array (and mb, bs) finds out whether there
- * are such rows with a synchronising reduction over d_row, later calls
- * reuse the answer (a stale answer after reusing d_row for another pattern
- * only costs speed).  The same holds for bilu_bcsr_spmv_f32 and
- * bilu_isai_apply. */
+ * (bsr_tensor_SpMV.h:402): y = M x.  FP64 values and vectors.  Patterns with
+ * rows of more than 64 blocks are not left to one lane group a row: a CTA takes
+ * each of a few such rows, else a cluster splits the blocks (FP64) or a CTA
+ * sums the long ones of its rows (FP32).  The first call with a given d_row
+ * array (and mb, bs) finds out what the rows are like with a synchronising
+ * reduction over d_row, later calls reuse the answer (a stale answer after
+ * reusing d_row for another pattern only costs speed).  The same holds for
+ * bilu_bcsr_spmv_f32 and bilu_isai_apply. */
 int bilu_bcsr_spmv(int mb, int bs, const int* d_row, const int* d_col, const double* d_val,
                    const double* d_x, double* d_y, bilu_stream_t stream);
 /* The SpMV layout word of a pattern, as cached by the entry points above:
- * bit 0 (1) when rows of more than 64 blocks are present (the kernel in
- * which the CTA shares such rows); bit 1 (2) when rows hold more than 5
- * blocks on average (FP32-stored values: one block row per lane group
- * instead of two).  Synchronises the stream on the first query of a
- * pattern. */
+ * bit 0 (1) when rows of more than 64 blocks are present; bit 1 (2) when rows
+ * hold more than 5 blocks on average (FP32-stored values: one block row per
+ * lane group instead of two).  Synchronises the stream on the first query of
+ * a pattern. */
 int bilu_spmv_layout(int mb, int bs, const int* d_row, bilu_stream_t stream, int* h_layout);
 /* FP32-stored values, FP32 accumulation; x and y each FP64 or FP32
  * (x_fp32 / y_fp32 flags). */

@@ -173,6 +173,11 @@ __device__ __forceinline__ double widen(float f) {
   return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + (896u << 20))), (int)(u << 29));
 }
 
+// Rows of a product with more blocks than this are long: power-law hub rows hold
+// up to ~2000, and a lane group alone runs one dependent FMA chain over all of
+// them while the rest of the GPU idles.
+constexpr int kLongSpmvRow = 64;
+
 // The entries [s, e) of a pattern row per thread, f(row, p) for each: a thread
 // walks its own row, except that rows of more than kSharedRow entries are
 // walked by the whole warp, 32 entries at a time (one thread alone takes

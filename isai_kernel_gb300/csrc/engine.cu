@@ -82,7 +82,7 @@ int spmv_any(int mb, int bs, int prec, const int* row, const int* col, const voi
              bool dep = false);
 int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t st,
                    int* h_layout);
-int spmv_layout_word(int mb, long long nnzb, int longest);
+int spmv_layout_word(int mb, long long nnzb, int longest, long long hubs);
 int copy_values(size_t count, const double* src, double* d0, double* d1, float* d32,
                 cudaStream_t st);
 int isai_apply_impl(int nb, int bs, int prec, const int* Lrow, const int* Lcol, const void* Lval,
@@ -495,17 +495,17 @@ int ctx_setup(bilu_ctx* c, int nb, int nnzb, int bs, const int* d_row, const int
     }
   }
   IsaiSym symL, symU;
-  int longest[3] = {0, 0, 0};  // the pattern's longest row, its triangles'
+  int longest[6] = {};  // longest row: the pattern's, its triangles'; blocks in long rows
   tm.mark(6);
   if (isai) BILU_TRY(build_isai_sym(c, ws, symL, symU, longest));
   tm.mark(7);
-  c->spmv_layout[1] = spmv_layout_word(nb, symL.mnnz, longest[1]);
-  c->spmv_layout[2] = spmv_layout_word(nb, symU.mnnz, longest[2]);
+  c->spmv_layout[1] = spmv_layout_word(nb, symL.mnnz, longest[1], longest[4]);
+  c->spmv_layout[2] = spmv_layout_word(nb, symU.mnnz, longest[2], longest[5]);
   if (isai && !c->Prow) {
-    c->spmv_layout[0] = spmv_layout_word(nb, nnzb, longest[0]);
+    c->spmv_layout[0] = spmv_layout_word(nb, nnzb, longest[0], longest[3]);
   } else {  // not counted with the ISAI patterns
     Carver w2 = ws;
-    int* words = w2.take<int>(1);
+    int* words = w2.take<int>(2);
     if (!words) return BILU_ERR_WORKSPACE;
     BILU_TRY(spmv_layout_of(nb, bs, c->Arow, words, st, &c->spmv_layout[0]));
   }

@@ -483,7 +483,7 @@ __global__ void k_b2c_fill(int mb, int bs, long long nnzb, const int* __restrict
 // k_isai_count / k_tri: the counts of M_L and M_U, of both triangles, and the
 // longest rows together, so that the host waits once).  Column counters cL, cU,
 // row counters tL, tU; words: 0 error kind, 1 longest row of the pattern, 2 / 3
-// of its lower / upper triangle.
+// of its lower / upper triangle, 8 to 10 the blocks in long rows of the three.
 __global__ void __launch_bounds__(kT) k_isai_both_count(int nb, const int* __restrict__ row,
                                                         const int* __restrict__ col, int* cL,
                                                         int* cU, int* __restrict__ tL,
@@ -522,6 +522,15 @@ __global__ void __launch_bounds__(kT) k_isai_both_count(int nb, const int* __res
     atomicMax(words + 1, a);
     atomicMax(words + 2, b);
     atomicMax(words + 3, c);
+  }
+  if (a > kLongSpmvRow) {  // the triangles' rows are no longer than the pattern's
+    auto add = [&](int n, int* to) {
+      const int h = __reduce_add_sync(0xffffffffu, n > kLongSpmvRow ? n : 0);
+      if ((threadIdx.x & 31) == 0 && h > 0) atomicAdd(to, h);
+    };
+    add(e - s, words + 8);
+    add(nL, words + 9);
+    add(nU, words + 10);
   }
 }
 
@@ -610,32 +619,35 @@ int isai_pattern_fill_impl(int nb, const int* row, const int* col, int lower, co
 
 // --------------------------------------------------------------- both ISAI sides
 size_t isai_both_ws(int nb, long long nnz) {
-  return carve_size(sizeof(int) * 8) + scan_multi_ws_bytes(nb + 1) +
+  return carve_size(sizeof(int) * 12) + scan_multi_ws_bytes(nb + 1) +
          2 * carve_size(sizeof(int) * ((size_t)nb + 1)) +
          4 * carve_size(sizeof(int) * (size_t)(nnz + 1));
 }
 
 // Column pointers of M_L and M_U and row pointers of the triangles of pattern
 // (row, col); h_nnz: blocks of M_L, M_U, the lower and the upper triangle;
-// h_longest: longest row of the pattern and of its triangles.  One host
-// synchronisation.
+// h_longest: longest row of the pattern and of its triangles, then their blocks in
+// long rows.  One host synchronisation.
 int isai_both_count(int nb, const int* row, const int* col, int* mL, int* mU, int* tL, int* tU,
                     int* h_nnz, int* h_longest, Carver& ws, cudaStream_t st) {
-  int* words = ws.take<int>(8);
+  int* words = ws.take<int>(12);
   if (!words) return BILU_ERR_WORKSPACE;
-  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * 8, st));
+  BILU_TRY_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * 12, st));
   BILU_TRY_CUDA(cudaMemsetAsync(mL, 0, sizeof(int) * nb, st));
   BILU_TRY_CUDA(cudaMemsetAsync(mU, 0, sizeof(int) * nb, st));
   k_isai_both_count<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, mL, mU, tL, tU, words);
   BILU_LAUNCH_CHECK();
   const ScanSets sets = {{mL, mU, tL, tU}, {nb, nb, nb, nb}};
   BILU_TRY(scan_exclusive_multi(4, sets, words + 4, ws, st));
-  int h[8];
+  int h[12];
   BILU_TRY_CUDA(cudaMemcpyAsync(h, words, sizeof(h), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
   if (h[0] != 0) return BILU_ERR_PATTERN;
   for (int i = 0; i < 4; ++i) h_nnz[i] = h[4 + i];
-  for (int i = 0; i < 3; ++i) h_longest[i] = h[1 + i];
+  for (int i = 0; i < 3; ++i) {
+    h_longest[i] = h[1 + i];
+    h_longest[3 + i] = h[8 + i];
+  }
   return BILU_OK;
 }
 

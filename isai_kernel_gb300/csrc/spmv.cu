@@ -150,23 +150,18 @@ __device__ __forceinline__ void load_entry(const VT* __restrict__ val,
     load_row<BS, VT, AccT>(val, p, r, a);
 }
 
-// Rows with more blocks than this are worth the CTA's help: power-law hub
-// rows hold up to ~2000 blocks, and a lane group alone runs one dependent
-// FMA chain over all of them while the rest of the GPU idles.
-constexpr int kLongSpmvRow = 64;
-
-// The CTA's long rows (slots in group order, -1 for none): its NG groups
+// The CTA's long rows (nslot slots, -1 for none): its NG groups
 // take the blocks g, g + NG, ... of each (two accumulators, even and odd
 // turns), the NG partials are added in group order.  Out of line so that
 // the short rows' loop keeps its registers.  Called by every thread.
-template <int BS, class VT, class XT, class YT, class AccT, int NSLOT, int NG>
-__device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __restrict__ row,
+template <int BS, class VT, class XT, class YT, class AccT, int NG>
+__device__ __noinline__ void spmv_long_rows(const int* long_rows, int nslot, const int* __restrict__ row,
                                             const int* __restrict__ col,
                                             const VT* __restrict__ val,
                                             const XT* __restrict__ x, YT* __restrict__ y,
                                             float* __restrict__ y32, AccT* red, bool in_group,
                                             int cg, int r) {
-  for (int i = 0; i < NSLOT; ++i) {
+  for (int i = 0; i < nslot; ++i) {
     const int br = long_rows[i];
     if (br < 0) continue;  // uniform across the CTA (shared memory)
     const int rs = __ldg(row + br), re = __ldg(row + br + 1);
@@ -240,7 +235,7 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, const int* __r
 // latencies at the start of the next (64^3 7-point, 4x4 blocks, the FP32 apply
 // 33.7 -> 28.9 us, FP64 71.2 -> 67.9; 128^3 FP32 249 -> 224).
 template <int BS, class VT, class XT, class YT, class AccT, int RPG, int U, int MINB, bool TR,
-          bool DEP>
+          bool DEP, bool HUBS>
 __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __restrict__ row,
                                                      const int* __restrict__ col,
                                                      const int* __restrict__ src,
@@ -256,11 +251,14 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
   const unsigned live = __ballot_sync(0xffffffffu, g < G && base < mb);
   if (g >= G || base >= mb) return;
   int s[RPG], e[RPG];
+  bool skip[RPG];
 #pragma unroll
   for (int q = 0; q < RPG; ++q) {
     bool ok = base + q < mb;
     s[q] = ok ? __ldg(row + base + q) : 0;
     e[q] = ok ? __ldg(row + base + q + 1) : 0;
+    skip[q] = HUBS && e[q] - s[q] > kLongSpmvRow;
+    if (skip[q]) e[q] = s[q];
   }
   AccT acc[RPG];
 #pragma unroll
@@ -339,10 +337,44 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv(int mb, const int* __res
   if constexpr (DEP) dependency_wait();  // rows without blocks
 #pragma unroll
   for (int q = 0; q < RPG; ++q)
-    if (base + q < mb) {
+    if (base + q < mb && !skip[q]) {
       y[(base + q) * BS + r] = (YT)acc[q];
       if (y32) y32[(base + q) * BS + r] = (float)acc[q];  // optional FP32 copy
     }
+}
+
+// The long rows of a product whose other rows are short and alike (k_bsr_spmv, HUBS,
+// leaves them out): a CTA each, its lane groups sharing the row's blocks.  The CTAs
+// look for them CH rows at a time.  Started by programmatic dependent launch beside
+// the other rows' kernel, it ends after that one (spmv_layout_word: when, and the
+// times).
+template <int BS, class VT, class XT, class YT>
+__global__ void __launch_bounds__(256) k_spmv_hubs(int mb, int ch, const int* __restrict__ row,
+                                                   const int* __restrict__ col,
+                                                   const VT* __restrict__ val,
+                                                   const XT* __restrict__ x, YT* __restrict__ y,
+                                                   float* __restrict__ y32) {
+  constexpr int G = 32 / BS;
+  __shared__ int list[256];
+  __shared__ int n_s;
+  __shared__ VT red[8 * G * BS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane / BS, r = lane - g * BS;
+  const int per = 256 / ch;
+  if (threadIdx.x == 0) n_s = 0;
+  __syncthreads();
+  for (long long t0 = 0; (t0 * gridDim.x + blockIdx.x) * ch < mb; t0 += per) {
+    const long long i =
+        ((t0 + threadIdx.x / ch) * gridDim.x + blockIdx.x) * ch + threadIdx.x % ch;
+    const bool hub = i < mb && __ldg(row + i + 1) - __ldg(row + i) > kLongSpmvRow;
+    if (hub) list[atomicAdd(&n_s, 1)] = (int)i;
+    if (!__syncthreads_or(hub)) continue;
+    spmv_long_rows<BS, VT, XT, YT, VT, 8 * G>(list, n_s, row, col, val, x, y, y32, red, g < G,
+                                              warp * G + g, r);
+    if (threadIdx.x == 0) n_s = 0;
+    __syncthreads();
+  }
+  dependency_wait();  // what follows in the stream comes after both kernels
 }
 
 // The same product with FP32 values for patterns with rows of more than
@@ -422,8 +454,8 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv_uneven(int mb, int rw,
   }
   // one CTA barrier, which also says whether the CTA holds a long row
   if (__syncthreads_or(skip != 0))
-    spmv_long_rows<BS, VT, XT, YT, AccT, NSLOT, 8 * G>(
-        long_slots, row, col, val, x, y, y32, reinterpret_cast<AccT*>(long_slots + NSLOT),
+    spmv_long_rows<BS, VT, XT, YT, AccT, 8 * G>(
+        long_slots, NSLOT, row, col, val, x, y, y32, reinterpret_cast<AccT*>(long_slots + NSLOT),
         g < G, warp * G + g, r);
 }
 
@@ -563,19 +595,56 @@ __global__ void __launch_bounds__(256, MINB) k_bsr_spmv_balanced(
 }
 
 // Layout word of a matrix for the SpMV: bit 0 = rows of more than
-// kLongSpmvRow blocks present (k_bsr_spmv_balanced, _uneven); bit 1 = more than
-// kWideSpmvRow blocks a row on average (FP32 values: one row per lane
-// group).
+// kLongSpmvRow blocks present; bit 1 = more than kWideSpmvRow blocks a row on
+// average (FP32 values: one row per lane group).  The other bits, for the choice of
+// the kernel alone (spmv_layout_word): the long rows hold few of the blocks and are
+// not too long (FP64, FP32); all rows are about as long; few and wide rows.
 constexpr int kLayoutLong = 1;
 constexpr int kLayoutWide = 2;
+constexpr int kLayoutHubs = 4;
+constexpr int kLayoutHubs32 = 8;
+constexpr int kLayoutAlike = 16;
+constexpr int kLayoutFew = 32;
+constexpr int kLayoutPublic = kLayoutLong | kLayoutWide;
 constexpr int kWideSpmvRow = 5;
+
+template <int BS, class VT, class XT, class YT>
+int launch_spmv_hubs(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
+                     cudaStream_t st, float* y32) {
+  // a row a CTA and turn, then runs of up to a sector of row pointers
+  constexpr int kCtas = 152 * 4;
+  int ch = 1;
+  while (ch < 8 && mb > ch * kCtas) ch *= 2;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min<unsigned>(ceil_div(mb, ch), kCtas));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  BILU_TRY_CUDA(cudaLaunchKernelEx(&cfg, k_spmv_hubs<BS, VT, XT, YT>, mb, ch, row, col, val, x, y,
+                                   y32));
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
+}
 
 template <int BS, class VT, class XT, class YT, int RPG, int U, int MINB, bool TR = false>
 int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
-                    cudaStream_t st, float* y32, bool dep, const int* src = nullptr) {
+                    cudaStream_t st, float* y32, bool dep, const int* src = nullptr,
+                    bool hubs = false) {
   constexpr int G = 32 / BS;
   long long groups = (mb + RPG - 1) / RPG;
   long long warps = (groups + G - 1) / G;
+  if constexpr (!TR) {
+    if (hubs) {  // a chain of its own: the hubs' kernel reads x when this one has started
+      k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, false, false, true>
+          <<<ceil_div(warps, 8), 256, 0, st>>>(mb, row, col, src, val, x, y, y32);
+      BILU_LAUNCH_CHECK();
+      return launch_spmv_hubs<BS, VT, XT, YT>(mb, row, col, val, x, y, st, y32);
+    }
+  }
   if constexpr (!TR && RPG == 1) {
     if (dep) {
       cudaLaunchAttribute at[1];
@@ -587,13 +656,13 @@ int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const
       cfg.stream = st;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      BILU_TRY_CUDA(cudaLaunchKernelEx(&cfg, k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR, true>,
+      BILU_TRY_CUDA(cudaLaunchKernelEx(&cfg, k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR, true, false>,
                                        mb, row, col, src, val, x, y, y32));
       BILU_LAUNCH_CHECK();
       return BILU_OK;
     }
   }
-  k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR, false><<<ceil_div(warps, 8), 256, 0, st>>>(
+  k_bsr_spmv<BS, VT, XT, YT, VT, RPG, U, MINB, TR, false, false><<<ceil_div(warps, 8), 256, 0, st>>>(
       mb, row, col, src, val, x, y, y32);
   BILU_LAUNCH_CHECK();
   return BILU_OK;
@@ -640,39 +709,51 @@ int launch_spmv_balanced(int mb, const int* row, const int* col, const int* src,
   return BILU_OK;
 }
 
-// The configurations measured faster on the stencil patterns (k_bsr_spmv)
-// apply to patterns without long rows.
+// The kernel and its configuration by the layout word; stencils and other patterns
+// of short rows take k_bsr_spmv.
 template <int BS, class VT, class XT, class YT>
 int launch_spmv(int mb, const int* row, const int* col, const VT* val, const XT* x, YT* y,
                 cudaStream_t st, int layout, float* y32, bool dep) {
   if (mb == 0) return BILU_OK;
-  if (layout & kLayoutLong) {
-    if constexpr (sizeof(VT) == 8)
+  const bool hubs = (layout & (sizeof(VT) == 8 ? kLayoutHubs : kLayoutHubs32)) != 0;
+  const int* none = nullptr;
+  // Long rows that are neither few of the blocks nor like the others; in FP64 also
+  // few wide rows, with or without long ones: a row a group leaves most of the
+  // chip idle, or runs one FMA chain per row (4000 rows of 41 blocks, a row a group /
+  // blocks split, us: 4x4 18.6 / 14.5, 8x8 41 / 33; 2000 of 201: 146 / 23, 187 / 62;
+  // 16,000 of 41: 35 / 40, 92 / 95).  Where all rows are about as long and many, a
+  // row a group it is (20,000 rows of 67: 4x4 64 / 70, 5x5 72 / 102, but 8x8
+  // 189 / 181; FP32 21 / 94, 35 / 147, 64 / 159).
+  if constexpr (sizeof(VT) == 8) {
+    if ((layout & kLayoutFew) || ((layout & kLayoutLong) && !hubs &&
+                                  !((layout & kLayoutAlike) && BS <= 5)))
       return launch_spmv_balanced<BS, 2, 4, false>(mb, row, col, nullptr, val, x, y, st, y32);
-    else
-      return launch_spmv_uneven<BS, XT, YT, BS == 4 ? 4 : 8, BS == 4 ? 4 : 2>(mb, row, col, val, x,
-                                                                             y, st, y32);
+  } else if ((layout & kLayoutLong) && !hubs && !(layout & kLayoutAlike)) {
+    return launch_spmv_uneven<BS, XT, YT, BS == 4 ? 4 : 8, BS == 4 ? 4 : 2>(mb, row, col, val, x, y,
+                                                                           st, y32);
   }
   if constexpr (sizeof(VT) == 8) {
-    if constexpr (BS <= 5)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 1, 6>(mb, row, col, val, x, y, st, y32, dep);
-    else
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 1, 5>(mb, row, col, val, x, y, st, y32, dep);
+    return launch_spmv_cfg<BS, VT, XT, YT, 1, 1, BS <= 5 ? 6 : 5>(mb, row, col, val, x, y, st, y32,
+                                                                  dep, none, hubs);
   } else if constexpr (BS == 8 && sizeof(XT) == 8) {
     // two rows of 8x8 blocks with FP64 x segments spill at 64 registers
-    return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
+    return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep, none,
+                                                    hubs);
   } else {
     // one row per group also where the first blocks are to wait in registers
     // for the launch before (two rows / one, the 512^2 5-point apply: bs 5 54.3
     // / 45.2 us, bs 8 80.4 / 68.9)
     if ((layout & kLayoutWide) || (BS != 4 && dep))
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 4>(mb, row, col, val, x, y, st, y32, dep, none,
+                                                      hubs);
     // bs 4 rows of ~4 blocks (the ISAI triangles of a 7-point pattern): one
     // row per group at 32 registers, 8 CTAs per SM (0.2214 -> 0.2185 ms
     // for the 128^3 inner apply)
     if constexpr (BS == 4)
-      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8>(mb, row, col, val, x, y, st, y32, dep);
-    return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4>(mb, row, col, val, x, y, st, y32, dep);
+      return launch_spmv_cfg<BS, VT, XT, YT, 1, 4, 8>(mb, row, col, val, x, y, st, y32, dep, none,
+                                                      hubs);
+    return launch_spmv_cfg<BS, VT, XT, YT, 2, 4, 4>(mb, row, col, val, x, y, st, y32, dep, none,
+                                                    hubs);
   }
 }
 
@@ -1023,13 +1104,19 @@ int spmv_f32_dual(int mb, const int* row, const int* col, const float* val, cons
   return launch_spmv<BS, float, float, double>(mb, row, col, val, x, y, st, lr, y32, dep);
 }
 
+// out[0] = the longest row, out[1] = the blocks in long rows
 __global__ void k_row_len_max(int mb, const int* __restrict__ row, int* out) {
-  int m = 0;
+  int m = 0, h = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < mb;
-       i += (long long)gridDim.x * blockDim.x)
-    m = max(m, __ldg(row + i + 1) - __ldg(row + i));
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+       i += (long long)gridDim.x * blockDim.x) {
+    const int n = __ldg(row + i + 1) - __ldg(row + i);
+    m = max(m, n);
+    if (n > kLongSpmvRow) h += n;
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  h = __reduce_add_sync(0xffffffffu, h);
   if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
+  if ((threadIdx.x & 31) == 0 && h > 0) atomicAdd(out + 1, h);
 }
 
 template <int BS>
@@ -1045,14 +1132,37 @@ int spmm_f32(int mb, int k, const int* row, const int* col, const float* val, co
 
 }  // namespace
 
-// The layout word of a pattern of mb rows and nnzb blocks, its longest row given.
-int spmv_layout_word(int mb, long long nnzb, int longest) {
-  return (longest > kLongSpmvRow ? kLayoutLong : 0) |
-         (nnzb > (long long)kWideSpmvRow * mb ? kLayoutWide : 0);
+// The layout word of a pattern of mb rows and nnzb blocks, its longest row and the
+// blocks in long rows given.  Long rows go apart (k_spmv_hubs) up to a length that
+// one SM gets through while the others do the rest, and to a share of the blocks
+// from which a split of all blocks is the better balance.  40^3 grids, rows apart /
+// balanced (FP64) or uneven (FP32), us, 4x4 and 8x8 --
+// FP64: 50 rows of 200 (2%) 23 / 32, 62 / 72; 1000 of 100 (16%) 42 / 37, 92 / 82;
+// 20 of 1000 (4%) 39 / 31, 106 / 71;
+// FP32: 50 of 200 9.5 / 12.4, 26 / 35; 1000 of 100 12.6 / 20.5, 37 / 45; 20 of 1000
+// 14.5 / 14.5, 46 / 36.
+// Hubs of 1000 are worth it again on 80^3 (5x5, FP32, 90 / 97), and a few hubs on
+// any small pattern (700 rows, 3 of 80, 4x4, FP64, 8.3 / 12.3).
+int spmv_layout_word(int mb, long long nnzb, int longest, long long hubs) {
+  int w = 0;
+  if (nnzb > (long long)kWideSpmvRow * mb) w |= kLayoutWide;
+  if ((long long)longest * mb <= 2 * nnzb) w |= kLayoutAlike;
+  if ((mb <= 8192 && nnzb >= 32ll * mb) || (mb <= 4096 && nnzb >= 24ll * mb)) w |= kLayoutFew;
+  if (longest > kLongSpmvRow) {
+    w |= kLayoutLong;
+    const bool fits = 2000ll * longest < nnzb;
+    if (!(w & kLayoutAlike)) {
+      if ((fits || longest <= 4 * kLongSpmvRow) && (10 * hubs < nnzb || hubs <= 4096))
+        w |= kLayoutHubs;
+      if ((fits || longest <= 8 * kLongSpmvRow) && (2 * hubs < nnzb || hubs <= 4096))
+        w |= kLayoutHubs32;
+    }
+  }
+  return w;
 }
 
 // SpMV layout word of a block pattern (see kLayoutLong): one reduction
-// over the row pointers into d_words (one device int), then a synchronising
+// over the row pointers into d_words (two device ints), then a synchronising
 // read of it and of the block count row[mb].  The engine calls it once per
 // matrix at setup.
 int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t st,
@@ -1060,22 +1170,22 @@ int spmv_layout_of(int mb, int bs, const int* row, void* d_words, cudaStream_t s
   (void)bs;
   *h_layout = 0;
   if (mb <= 0) return BILU_OK;
-  int h[2] = {0, 0};  // longest row, blocks
+  int h[3] = {0, 0, 0};  // longest row, blocks in long rows, blocks
   int* d = static_cast<int*>(d_words);
-  BILU_TRY_CUDA(cudaMemsetAsync(d, 0, sizeof(int), st));
+  BILU_TRY_CUDA(cudaMemsetAsync(d, 0, sizeof(int) * 2, st));
   k_row_len_max<<<(unsigned)std::min<long long>(ceil_div(mb, 256), 152 * 8), 256, 0, st>>>(
       mb, row, d);
   BILU_LAUNCH_CHECK();
-  BILU_TRY_CUDA(cudaMemcpyAsync(&h[0], d, sizeof(int), cudaMemcpyDeviceToHost, st));
-  BILU_TRY_CUDA(cudaMemcpyAsync(&h[1], row + mb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaMemcpyAsync(&h[0], d, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(cudaMemcpyAsync(&h[2], row + mb, sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
-  *h_layout = spmv_layout_word(mb, h[1], h[0]);
+  *h_layout = spmv_layout_word(mb, h[2], h[0], h[1]);
   return BILU_OK;
 }
 
 namespace {
 
-__device__ int g_layout_word;  // scratch of the cached check (under its lock)
+__device__ int g_layout_word[2];  // scratch of the cached check (under its lock)
 
 // The standalone entry points do not know the pattern: the answer is cached
 // per (row pointer array, block rows, block size), most recent first.  A
@@ -1198,11 +1308,13 @@ extern "C" int bilu_spmv_layout(int mb, int bs, const int* d_row, bilu_stream_t 
                                 int* h_layout) {
   if (mb < 0 || !h_layout || (mb > 0 && !d_row)) return BILU_ERR_ARG;
   if (!bs_supported(bs)) return BILU_ERR_UNSUPPORTED;
-  return layout_cached(mb, bs, d_row, S(stream), h_layout);
+  BILU_TRY(layout_cached(mb, bs, d_row, S(stream), h_layout));
+  *h_layout &= kLayoutPublic;
+  return BILU_OK;
 }
 
 extern "C" int bilu_debug_spmv_layout_set(int mb, int bs, const int* d_row, int layout) {
-  if (mb < 0 || (mb > 0 && !d_row) || layout < 0 || layout > (kLayoutLong | kLayoutWide))
+  if (mb < 0 || (mb > 0 && !d_row) || layout < 0 || layout > kLayoutPublic)
     return BILU_ERR_ARG;
   if (!bs_supported(bs)) return BILU_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lock(g_layout_mu);

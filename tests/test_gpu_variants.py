@@ -508,6 +508,46 @@ def test_uneven_rows_product(cuda, orc, name, bs):
 
 
 # ------------------------------------------------------------------ several right-hand sides
+@pytest.mark.parametrize("bs", [4, 5, 8])
+@pytest.mark.parametrize("mb, hubs, ln", [(80, 1, 65), (608, 3, 65), (609, 40, 66), (700, 3, 64),
+                                          (5000, 30, 250), (9000, 8, 300), (300, 300, 100),
+                                          (12000, 12000, 70), (5000, 5000, 33)])
+def test_products_of_few_long_rows(cuda, bs, mb, hubs, ln):
+    """Neighbouring rows of `ln` blocks among rows of two, and patterns of one row
+    length: the products of every combination of types, N terms of numbers in
+    [-1, 1] each within N^2 2^-53 (FP32 values: 2^-24) of the sum in 64 bits."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(mb + bs + ln)
+    n = np.full(mb, 2)
+    n[mb - hubs:] = ln
+    rp = np.zeros(mb + 1, np.int32)
+    np.cumsum(n, out=rp[1:])
+    rows = np.repeat(np.arange(mb), n)
+    col = rng.integers(0, mb, size=len(rows)).astype(np.int32)
+    val, x = rng.uniform(-1, 1, size=(len(col), bs, bs)), rng.uniform(-1, 1, size=mb * bs)
+    r, c, v, xd = T(rp, cuda), T(col, cuda), T(val, cuda), T(x, cuda)
+    bound = 2 * ((n * bs).astype(float) ** 2)[:, None]
+
+    def product(a, b):
+        ref = np.zeros((mb, bs))
+        np.add.at(ref, rows, np.einsum("pij,pj->pi", a, b.reshape(mb, bs)[col]))
+        return ref
+
+    y = N(api.bcsr_spmv(mb, bs, r, c, v, xd)).reshape(mb, bs)
+    assert np.all(np.abs(y - product(val, x)) <= bound * 2.0 ** -53)
+    v32 = v.float()
+    ref = product(N(v32).astype(np.float64), x.astype(np.float32).astype(np.float64))
+    for xt in (torch.float32, torch.float64):
+        for yt in (torch.float32, torch.float64):
+            out = torch.full((mb * bs,), float("nan"), dtype=yt, device=cuda)
+            y = N(api.bcsr_spmv(mb, bs, r, c, v32, xd.to(xt), out)).reshape(mb, bs)
+            # (an FP64 x is rounded where it is read)
+            assert np.all(np.abs(y - ref) <= bound * 2.0 ** -24)
+
+
 @pytest.mark.parametrize("k", [1, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 64])
 @pytest.mark.parametrize("bs", [4, 5, 8])
 def test_spmm_splits(cuda, orc, bs, k):
