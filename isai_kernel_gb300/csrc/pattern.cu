@@ -74,8 +74,10 @@ __global__ void k_isai_scatter(int nb, const int* __restrict__ row, const int* _
 }
 
 // out[ptr[s] + rank(key)] = key (and payload), keys distinct inside a segment:
-// 8 lanes per segment (most hold a handful of keys), the warp together on
-// segments of more than kSharedRow keys.
+// L lanes per segment (8: most hold a handful of keys), the warp together on
+// segments of more than kSharedRow keys.  A warp's segments are 8 apart, so that
+// neighbouring hubs go to different warps (three dense columns beside one another,
+// 5000 rows, the transposed product: 16.6 ms in one warp, 5.8 so).
 __device__ __forceinline__ void rank_one(int i, int s, int e, const int* __restrict__ key,
                                          const int* __restrict__ pay, int* __restrict__ key_out,
                                          int* __restrict__ pay_out) {
@@ -86,17 +88,20 @@ __device__ __forceinline__ void rank_one(int i, int s, int e, const int* __restr
   if (pay_out) pay_out[s + rank] = pay[i];
 }
 
+template <int L>
 __global__ void __launch_bounds__(kT) k_segment_rank_sort(int nseg, const int* __restrict__ ptr,
                                                           const int* __restrict__ key,
                                                           const int* __restrict__ pay,
                                                           int* __restrict__ key_out,
                                                           int* __restrict__ pay_out) {
-  const int lane = threadIdx.x & 31, l = lane & 7;
-  const long long sg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  constexpr int NW = kT / 32, PER = 32 / L;  // warps, segments of a warp
+  const int lane = threadIdx.x & 31, l = lane % L;
+  const long long sg =
+      ((long long)blockIdx.x * PER + lane / L) * NW + (int)(threadIdx.x >> 5);
   const int s = sg < nseg ? ptr[sg] : 0, e = sg < nseg ? ptr[sg + 1] : 0;
-  const bool shared = e - s > kSharedRow;
+  const bool shared = L < 32 && e - s > kSharedRow;
   if (!shared)
-    for (int i = s + l; i < e; i += 8) rank_one(i, s, e, key, pay, key_out, pay_out);
+    for (int i = s + l; i < e; i += L) rank_one(i, s, e, key, pay, key_out, pay_out);
   unsigned todo = __ballot_sync(0xffffffffu, shared && l == 0);
   while (todo) {
     const int from = __ffs(todo) - 1;
@@ -104,6 +109,19 @@ __global__ void __launch_bounds__(kT) k_segment_rank_sort(int nseg, const int* _
     const int a = __shfl_sync(0xffffffffu, s, from), b = __shfl_sync(0xffffffffu, e, from);
     for (int i = a + lane; i < b; i += 32) rank_one(i, a, b, key, pay, key_out, pay_out);
   }
+}
+
+// A warp per segment while the chip holds as many warps.
+int segment_rank_sort(int nseg, const int* ptr, const int* key, const int* pay, int* key_out,
+                      int* pay_out, cudaStream_t st) {
+  if (nseg <= 152 * 64)
+    k_segment_rank_sort<32><<<ceil_div(nseg, kT / 32), kT, 0, st>>>(nseg, ptr, key, pay, key_out,
+                                                                    pay_out);
+  else
+    k_segment_rank_sort<8><<<ceil_div(nseg, kT / 8), kT, 0, st>>>(nseg, ptr, key, pay, key_out,
+                                                                  pay_out);
+  BILU_LAUNCH_CHECK();
+  return BILU_OK;
 }
 
 // Rows of the lower (upper) triangle in their stored order: a thread per row,
@@ -612,9 +630,7 @@ int isai_pattern_fill_impl(int nb, const int* row, const int* col, int lower, co
   BILU_TRY_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * nb, st));
   k_isai_scatter<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, lower, Mptr, cursor, tmp);
   BILU_LAUNCH_CHECK();
-  k_segment_rank_sort<<<ceil_div((long long)nb * 8, kT), kT, 0, st>>>(nb, Mptr, tmp, nullptr, Mind, nullptr);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  return segment_rank_sort(nb, Mptr, tmp, nullptr, Mind, nullptr, st);
 }
 
 // --------------------------------------------------------------- both ISAI sides
@@ -665,12 +681,8 @@ int isai_both_fill(int nb, const int* row, const int* col, const int* mL, const 
   k_isai_both_fill<<<ceil_div(nb, kT), kT, 0, st>>>(nb, row, col, mL, mU, tL, tU, cur, cur + nb,
                                                     tcolL, tcolU, keyL, payL, keyU, payU);
   BILU_LAUNCH_CHECK();
-  const unsigned grid = ceil_div((long long)nb * 8, kT);
-  k_segment_rank_sort<<<grid, kT, 0, st>>>(nb, mL, keyL, payL, indL, mapL);
-  BILU_LAUNCH_CHECK();
-  k_segment_rank_sort<<<grid, kT, 0, st>>>(nb, mU, keyU, payU, indU, mapU);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  BILU_TRY(segment_rank_sort(nb, mL, keyL, payL, indL, mapL, st));
+  return segment_rank_sort(nb, mU, keyU, payU, indU, mapU, st);
 }
 
 // --------------------------------------------------------------- tri pattern
@@ -748,10 +760,7 @@ int transpose_fill(int mb, int nbcol, const int* cptr, const int* cind, long lon
   BILU_TRY_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * mb, st));
   k_csc_scatter<<<ceil_div(nbcol, kT), kT, 0, st>>>(nbcol, cptr, cind, rptr, cursor, key, pay);
   BILU_LAUNCH_CHECK();
-  k_segment_rank_sort<<<ceil_div((long long)mb * 8, kT), kT, 0, st>>>(mb, rptr, key, pay, rind,
-                                                                      src);
-  BILU_LAUNCH_CHECK();
-  return BILU_OK;
+  return segment_rank_sort(mb, rptr, key, pay, rind, src, st);
 }
 
 // Row pointer of the transpose of a square pattern, its block count and longest

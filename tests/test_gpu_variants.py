@@ -439,6 +439,26 @@ def test_transposed_product(cuda, name, bs):
         api.bcsr_spmv_transpose(nb, bs, T(rp, cuda), T(bad, cuda), T(val, cuda), T(x, cuda))
 
 
+@pytest.mark.parametrize("mb", [1, 31, 9727, 9728, 9729, 20000])
+def test_transposed_pattern_hub_columns(cuda, mb):
+    """Neighbouring dense columns (up to 9728 segments: a warp each) and short
+    ones: the transposed pattern and blocks."""
+    from isai_kernel_gb300 import api
+
+    rng = np.random.default_rng(mb)
+    hubs = {c for c in (0, 1, 2, 3, mb // 2, mb - 2, mb - 1) if 0 <= c < mb}
+    rp, col = pattern_of([hubs | {int(rng.integers(0, mb))} if i < 500 else {(7 * i) % mb}
+                          for i in range(mb)])
+    val = rng.uniform(-1, 1, size=(len(col), 4, 4))
+    tr, tc, tv = api.bsr_transpose(mb, 4, T(rp, cuda), T(col, cuda), T(val, cuda))
+    rows = np.repeat(np.arange(mb), np.diff(rp))
+    order = np.lexsort((rows, col))
+    want = np.zeros(mb + 1, np.int64)
+    np.cumsum(np.bincount(col, minlength=mb), out=want[1:])
+    assert np.array_equal(N(tr), want) and np.array_equal(N(tc), rows[order])
+    assert np.array_equal(N(tv), val[order].transpose(0, 2, 1))
+
+
 @pytest.mark.parametrize("scale", [1.0, -1.0, 2.5])
 @pytest.mark.parametrize("bs", [1, 2, 3, 4, 5, 6, 7, 8])
 @pytest.mark.parametrize("name", ["empty", "gaps", "hub column", "hub row"])
