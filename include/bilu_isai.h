@@ -572,8 +572,7 @@ int bilu_debug_spmv_layout_set(int mb, int bs, const int* d_row, int layout);
  * kernel (one cooperative launch): w is orthogonalised against the j+1
  * basis vectors V[0..j] (stride ldv elements, FP64, or FP32 when fp32 != 0)
  * by fused sweeps; d_h[0..j] receives h_i = v_i . w, d_h[j+1] = ||w||^2,
- * and d_vnext (optional) w / ||w||; w's own contents afterwards are
- * unspecified.  Vectors start on 16-byte boundaries;
+ * and d_vnext (optional) w / ||w||.  Vectors start on 16-byte boundaries;
  * workspace bilu_debug_mgs_step_ws_bytes().  Synchronises the stream;
  * returns BILU_ERR_TIMEOUT if a wait between sweeps gave up. */
 size_t bilu_debug_mgs_step_ws_bytes(void);

@@ -430,7 +430,7 @@ template <class T, int KR>
 __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     long long n, const T* __restrict__ V, long long ldv, int j, T* __restrict__ w,
     double* __restrict__ hout, int hstride, double* __restrict__ wwout,
-    unsigned* __restrict__ words, T* __restrict__ vnext, float* __restrict__ vnext32) {
+    unsigned* __restrict__ words, T* __restrict__ vnext, float* __restrict__ vnext32, int keep) {
   constexpr bool kResident = KR > 0;
   dependents_launch();  // the next product may read its matrix during the sweeps
   using M = MgsVec<T>;
@@ -661,6 +661,15 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       if (vnext32) vnext32[e] = (float)v;
     }
   }
+  if constexpr (kResident) {
+    if (keep) {
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        const long long e = tid + k * stride;
+        if (e < nv) wv[e] = wr[k];
+      }
+    }
+  }
   // every CTA has read the epoch before it arrives here: the last one leaves
   // the words as the next launch needs them
   if (threadIdx.x == 0 && atomicAdd(words + 1, 1u) == gridDim.x - 1u) {
@@ -719,11 +728,12 @@ int mgs_prepare(int* grid) {
 
 template <class T, int KR>
 int mgs_launch(int grid, long long n, const T* V, long long ldv, int j, T* w, double* hout,
-               int hstride, double* wwout, unsigned* words, T* vnext, float* vnext32,
+               int hstride, double* wwout, unsigned* words, T* vnext, float* vnext32, int keep,
                cudaStream_t st) {
   const size_t smem = KR > 0 ? (size_t)2 * KR * kStepThreads * 16
                              : (sizeof(T) == 8 ? kStepStageBytes : 0);
-  void* args[] = {&n, &V, &ldv, &j, &w, &hout, &hstride, &wwout, &words, &vnext, &vnext32};
+  void* args[] = {&n,     &V,     &ldv,   &j,       &w,   &hout, &hstride,
+                  &wwout, &words, &vnext, &vnext32, &keep};
   BILU_TRY_CUDA(cudaLaunchCooperativeKernel((const void*)k_mgs_step<T, KR>, dim3(grid),
                                             dim3(kStepThreads), args, smem, st));
   BILU_LAUNCH_CHECK();
@@ -732,7 +742,8 @@ int mgs_launch(int grid, long long n, const T* V, long long ldv, int j, T* w, do
 
 template <class T>
 int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout, int hstride,
-               double* wwout, unsigned* words, T* vnext, float* vnext32, cudaStream_t st) {
+               double* wwout, unsigned* words, T* vnext, float* vnext32, int keep,
+               cudaStream_t st) {
   static int grid = 0, resident = 0;
   if (!grid) {
     int g0 = 0, g2 = 0, g4 = 0, g6 = 0;
@@ -753,7 +764,7 @@ int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout
   const long long threads = (long long)grid * kStepThreads, nv = n / MgsVec<T>::W;
   const long long need = (nv + threads - 1) / threads;
 #define BILU_MGS(KR) \
-  mgs_launch<T, KR>(grid, n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, st)
+  mgs_launch<T, KR>(grid, n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, keep, st)
   if (need > resident) return BILU_MGS(0);
   if (need <= 2) return BILU_MGS(2);
   if (need <= 4) return BILU_MGS(4);
@@ -763,13 +774,16 @@ int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout
 
 int mgs_step(long long n, const double* V, long long ldv, int j, double* w, double* hout,
              int hstride, double* wwout, unsigned* words, double* vnext, float* vnext32,
-             cudaStream_t st) {
-  return mgs_step_t<double>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, st);
+             cudaStream_t st, int keep) {
+  return mgs_step_t<double>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, keep,
+                            st);
 }
 
 int mgs_step_f32(long long n, const float* V, long long ldv, int j, float* w, double* hout,
-                 int hstride, double* wwout, unsigned* words, float* vnext, cudaStream_t st) {
-  return mgs_step_t<float>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, nullptr, st);
+                 int hstride, double* wwout, unsigned* words, float* vnext, cudaStream_t st,
+                 int keep) {
+  return mgs_step_t<float>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, nullptr, keep,
+                           st);
 }
 
 int inner_lsq(int k, const double* H, const double* ww, double* y, cudaStream_t st) {
@@ -818,9 +832,9 @@ extern "C" int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long 
   unsigned* words = (unsigned*)(((uintptr_t)d_ws + 255) & ~(uintptr_t)255);
   BILU_TRY_CUDA(cudaMemsetAsync(words, 0, kStepWordsBytes, st));
   int rc = fp32 ? mgs_step_f32(n, (const float*)d_V, ldv, j, (float*)d_w, d_h, 1, d_h + j + 1,
-                               words, (float*)d_vnext, st)
+                               words, (float*)d_vnext, st, 1)
                 : mgs_step(n, (const double*)d_V, ldv, j, (double*)d_w, d_h, 1, d_h + j + 1,
-                           words, (double*)d_vnext, nullptr, st);
+                           words, (double*)d_vnext, nullptr, st, 1);
   if (rc != BILU_OK) return rc;
   int err = 0;
   BILU_TRY_CUDA(cudaMemcpyAsync(&err, words + kStepErrWord, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -808,6 +808,46 @@ def test_mgs_step_forms(cuda, fp32, per_thread):
         assert torch.all(vn[n:] == 0)
 
 
+def step_vectors(cuda, fp32, n, j):
+    """V (rows of ldv elements), w and the workspace of a Gram-Schmidt step."""
+    import torch
+
+    from isai_kernel_gb300 import _lib
+
+    g = torch.Generator(device=cuda).manual_seed(n)
+    dt = torch.float32 if fp32 else torch.float64
+    ldv = (n + 31) // 32 * 32
+    V = torch.zeros(j + 1, ldv, dtype=dt, device=cuda)
+    V[:, :n] = torch.linalg.qr(
+        torch.randn(n, j + 1, dtype=torch.float64, device=cuda, generator=g))[0].T.to(dt)
+    w = torch.zeros(ldv, dtype=dt, device=cuda)
+    w[:n] = torch.randn(n, dtype=torch.float64, device=cuda, generator=g).to(dt)
+    ws = torch.empty(_lib.lib().bilu_debug_mgs_step_ws_bytes(), dtype=torch.uint8, device=cuda)
+    return V, w, ws
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("n", [513, 300001, 1500002, 2500003, 4000001])
+def test_mgs_step_leaves_the_orthogonalised_vector(cuda, fp32, n):
+    """Every form of the step (up to 2, 4 and 6 vectors a thread, and more) leaves
+    w - sum h_i v_i in w: v_{j+1} is that over the square root of h_{j+1}, one
+    rounded product per element (root, quotient and product: 4 eps)."""
+    import torch
+
+    from isai_kernel_gb300 import _lib, api
+
+    j = 2
+    V, w, ws = step_vectors(cuda, fp32, n, j)
+    h = torch.empty(j + 2, dtype=torch.float64, device=cuda)
+    vn = torch.zeros_like(w)
+    assert _lib.lib().bilu_debug_mgs_step(n, fp32, api._p(V), V.shape[1], j, api._p(w), api._p(h),
+                                          api._p(vn), api._p(ws), ws.numel(), api._s()) == 0
+    eps = torch.finfo(w.dtype).eps
+    want = w[:n].double() / h[j + 1].sqrt()
+    assert torch.all((vn[:n].double() - want).abs() <= 4 * eps * want.abs())
+    assert abs(h[j + 1] - (w[:n].double() ** 2).sum()) <= eps * n ** 0.5 * h[j + 1]
+
+
 # ------------------------------------------------------------------ conversion
 @pytest.mark.parametrize("shift_in, shift_out", [(0, 0), (1, 0), (0, 1), (2, 4)])
 def test_values_to_fp32(cuda, shift_in, shift_out):
