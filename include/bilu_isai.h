@@ -554,6 +554,12 @@ int bilu_debug_sptrsv_withhold_flow(int nb, int nnzb, int bs, const int* d_row, 
                                     const double* d_val, int lower, const double* d_b,
                                     double* d_x, int withhold_row, long long spin_limit,
                                     void* d_ws, size_t ws_bytes, bilu_stream_t stream);
+/* bilu_sptrsv_analysis with block row withhold_row never publishing its level and
+ * waits that give up after spin_limit polls: BILU_ERR_TIMEOUT. */
+int bilu_debug_sptrsv_analysis_withhold(int nb, int nnzb, int bs, const int* d_row,
+                                        const int* d_col, int lower, int withhold_row,
+                                        long long spin_limit, void* d_info, void* d_ws,
+                                        size_t ws_bytes, bilu_stream_t stream);
 /* bilu_bsrilu0_ex with block row withhold_row never publishing (-1: every row
  * does) and a spin budget of spin_limit polls: the rows that depend on it give
  * up, BILU_ERR_TIMEOUT.  Workspace bilu_bsrilu0_ws_bytes(nb, nnzb).  The row
@@ -579,6 +585,13 @@ size_t bilu_debug_mgs_step_ws_bytes(void);
 int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long long ldv, int j, void* d_w,
                         double* d_h, void* d_vnext, void* d_ws, size_t ws_bytes,
                         bilu_stream_t stream);
+/* The same with the streaming form whatever n (streaming != 0; same bits), CTA
+ * withhold_cta never storing its sums (-1: every CTA does) and waits that give
+ * up after spin_limit polls: BILU_ERR_TIMEOUT, w, d_h and d_vnext unspecified. */
+int bilu_debug_mgs_step_ex(long long n, int fp32, const void* d_V, long long ldv, int j,
+                           void* d_w, double* d_h, void* d_vnext, int streaming,
+                           int withhold_cta, long long spin_limit, void* d_ws, size_t ws_bytes,
+                           bilu_stream_t stream);
 
 #ifdef __cplusplus
 }

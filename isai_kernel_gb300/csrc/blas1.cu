@@ -411,14 +411,14 @@ __device__ __forceinline__ bool load_tagged(const unsigned long long* p, unsigne
   v = __hiloint2double((int)(unsigned)hi, (int)(unsigned)lo);
   return (unsigned)(hi >> 32) == tag && (unsigned)(lo >> 32) == tag;
 }
-// Waits, kSpinLimit polls at most, for the tagged sum at p; false when the wait
+// Waits, spin polls at most, for the tagged sum at p; false when the wait
 // ran out here or elsewhere (the error word is set).
 template <class T>
 __device__ __forceinline__ bool wait_tagged(const unsigned long long* p, unsigned tag, int* err,
-                                            T& v) {
+                                            long long spin, T& v) {
   for (long long k = 0; !load_tagged(p, tag, v);) {
     if ((++k & 63) == 0 && ld_relaxed(err) != 0) return false;
-    if (k > kSpinLimit) {
+    if (k > spin) {
       atomicCAS(err, 0, (int)BILU_ERR_TIMEOUT);
       return false;
     }
@@ -430,7 +430,7 @@ template <class T, int KR>
 __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     long long n, const T* __restrict__ V, long long ldv, int j, T* __restrict__ w,
     double* __restrict__ hout, int hstride, double* __restrict__ wwout,
-    unsigned* __restrict__ words, T* __restrict__ vnext, float* __restrict__ vnext32, int keep) {
+    unsigned* __restrict__ words, T* __restrict__ vnext, float* __restrict__ vnext32, StepHook hook) {
   constexpr bool kResident = KR > 0;
   dependents_launch();  // the next product may read its matrix during the sweeps
   using M = MgsVec<T>;
@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     if constexpr (kResident) cp_async_wait<0>();
     return;
   }
+  const bool tells = lane == 0 && (int)blockIdx.x != hook.withhold;
   T h = T(0);
   for (int i = 0; i <= j + 1; ++i) {
     const T* vp = i > 0 ? V + (long long)(i - 1) * ldv : nullptr;
@@ -585,14 +586,15 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       for (int q = 1; q < kStepThreads / 32; ++q) t += red_s[lane + 32 * q];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) store_tagged(sums + (size_t)blockIdx.x * PW, tag, t);
+      if (tells)
+        store_tagged(sums + (size_t)blockIdx.x * PW, tag, t);
     }
     bool ok = true;
     if (blockIdx.x == 0) {
       T t = T(0);
       for (int c = threadIdx.x; c < G; c += kStepThreads) {
         T v = T(0);
-        ok = ok && wait_tagged(sums + (size_t)c * PW, tag, err, v);
+        ok = ok && wait_tagged(sums + (size_t)c * PW, tag, err, hook.spin, v);
         if constexpr (sizeof(T) == 8) sum_s[c] = v; else t += v;
       }
       __syncwarp();
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       }
     } else if (threadIdx.x == 0) {
       T v = T(0);
-      ok = wait_tagged(totals + (size_t)(blockIdx.x / kStepFan) * 16, tag, err, v);
+      ok = wait_tagged(totals + (size_t)(blockIdx.x / kStepFan) * 16, tag, err, hook.spin, v);
       h_s = v;
     }
     if (!__syncthreads_and(ok)) {
@@ -662,7 +664,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     }
   }
   if constexpr (kResident) {
-    if (keep) {
+    if (hook.keep) {
 #pragma unroll
       for (int k = 0; k < KR; ++k) {
         const long long e = tid + k * stride;
@@ -728,12 +730,12 @@ int mgs_prepare(int* grid) {
 
 template <class T, int KR>
 int mgs_launch(int grid, long long n, const T* V, long long ldv, int j, T* w, double* hout,
-               int hstride, double* wwout, unsigned* words, T* vnext, float* vnext32, int keep,
-               cudaStream_t st) {
+               int hstride, double* wwout, unsigned* words, T* vnext, float* vnext32,
+               StepHook hook, cudaStream_t st) {
   const size_t smem = KR > 0 ? (size_t)2 * KR * kStepThreads * 16
                              : (sizeof(T) == 8 ? kStepStageBytes : 0);
   void* args[] = {&n,     &V,     &ldv,   &j,       &w,   &hout, &hstride,
-                  &wwout, &words, &vnext, &vnext32, &keep};
+                  &wwout, &words, &vnext, &vnext32, &hook};
   BILU_TRY_CUDA(cudaLaunchCooperativeKernel((const void*)k_mgs_step<T, KR>, dim3(grid),
                                             dim3(kStepThreads), args, smem, st));
   BILU_LAUNCH_CHECK();
@@ -742,8 +744,8 @@ int mgs_launch(int grid, long long n, const T* V, long long ldv, int j, T* w, do
 
 template <class T>
 int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout, int hstride,
-               double* wwout, unsigned* words, T* vnext, float* vnext32, int keep,
-               cudaStream_t st) {
+               double* wwout, unsigned* words, T* vnext, float* vnext32,
+               StepHook hook, cudaStream_t st) {
   static int grid = 0, resident = 0;
   if (!grid) {
     int g0 = 0, g2 = 0, g4 = 0, g6 = 0;
@@ -764,8 +766,8 @@ int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout
   const long long threads = (long long)grid * kStepThreads, nv = n / MgsVec<T>::W;
   const long long need = (nv + threads - 1) / threads;
 #define BILU_MGS(KR) \
-  mgs_launch<T, KR>(grid, n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, keep, st)
-  if (need > resident) return BILU_MGS(0);
+  mgs_launch<T, KR>(grid, n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, hook, st)
+  if (need > resident || hook.streaming) return BILU_MGS(0);
   if (need <= 2) return BILU_MGS(2);
   if (need <= 4) return BILU_MGS(4);
   return BILU_MGS(6);
@@ -774,15 +776,15 @@ int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout
 
 int mgs_step(long long n, const double* V, long long ldv, int j, double* w, double* hout,
              int hstride, double* wwout, unsigned* words, double* vnext, float* vnext32,
-             cudaStream_t st, int keep) {
-  return mgs_step_t<double>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, keep,
+             cudaStream_t st, const StepHook& hook) {
+  return mgs_step_t<double>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, vnext32, hook,
                             st);
 }
 
 int mgs_step_f32(long long n, const float* V, long long ldv, int j, float* w, double* hout,
                  int hstride, double* wwout, unsigned* words, float* vnext, cudaStream_t st,
-                 int keep) {
-  return mgs_step_t<float>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, nullptr, keep,
+                 const StepHook& hook) {
+  return mgs_step_t<float>(n, V, ldv, j, w, hout, hstride, wwout, words, vnext, nullptr, hook,
                            st);
 }
 
@@ -818,11 +820,12 @@ extern "C" size_t bilu_debug_mgs_step_ws_bytes(void) {
   return kStepWordsBytes + 256;
 }
 
-extern "C" int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long long ldv, int j,
-                                   void* d_w, double* d_h, void* d_vnext, void* d_ws,
-                                   size_t ws_bytes, bilu_stream_t stream) {
+extern "C" int bilu_debug_mgs_step_ex(long long n, int fp32, const void* d_V, long long ldv,
+                                      int j, void* d_w, double* d_h, void* d_vnext, int streaming,
+                                      int withhold_cta, long long spin_limit, void* d_ws,
+                                      size_t ws_bytes, bilu_stream_t stream) {
   if (n < 1 || j < 0 || j >= kMaxVec || ldv < n || !d_V || !d_w || !d_h || !d_ws ||
-      ws_bytes < bilu_debug_mgs_step_ws_bytes())
+      spin_limit < 1 || spin_limit > kSpinLimit || ws_bytes < bilu_debug_mgs_step_ws_bytes())
     return BILU_ERR_ARG;
   // 16-byte vector accesses: every basis vector starts on a 16-byte boundary
   if ((ldv * (fp32 ? 4 : 8)) % 16 != 0 || ((uintptr_t)d_V | (uintptr_t)d_w) % 16 != 0 ||
@@ -831,13 +834,26 @@ extern "C" int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long 
   cudaStream_t st = S(stream);
   unsigned* words = (unsigned*)(((uintptr_t)d_ws + 255) & ~(uintptr_t)255);
   BILU_TRY_CUDA(cudaMemsetAsync(words, 0, kStepWordsBytes, st));
+  StepHook hook;
+  hook.keep = 1;
+  hook.streaming = streaming != 0;
+  hook.withhold = withhold_cta;
+  hook.spin = spin_limit;
   int rc = fp32 ? mgs_step_f32(n, (const float*)d_V, ldv, j, (float*)d_w, d_h, 1, d_h + j + 1,
-                               words, (float*)d_vnext, st, 1)
+                               words, (float*)d_vnext, st, hook)
                 : mgs_step(n, (const double*)d_V, ldv, j, (double*)d_w, d_h, 1, d_h + j + 1,
-                           words, (double*)d_vnext, nullptr, st, 1);
+                           words, (double*)d_vnext, nullptr, st, hook);
   if (rc != BILU_OK) return rc;
   int err = 0;
-  BILU_TRY_CUDA(cudaMemcpyAsync(&err, words + kStepErrWord, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BILU_TRY_CUDA(
+      cudaMemcpyAsync(&err, words + kStepErrWord, sizeof(int), cudaMemcpyDeviceToHost, st));
   BILU_TRY_CUDA(cudaStreamSynchronize(st));
   return err;
+}
+
+extern "C" int bilu_debug_mgs_step(long long n, int fp32, const void* d_V, long long ldv, int j,
+                                   void* d_w, double* d_h, void* d_vnext, void* d_ws,
+                                   size_t ws_bytes, bilu_stream_t stream) {
+  return bilu_debug_mgs_step_ex(n, fp32, d_V, ldv, j, d_w, d_h, d_vnext, 0, -1, kSpinLimit, d_ws,
+                                ws_bytes, stream);
 }

@@ -49,8 +49,8 @@ int combine_f32(long long n, const float* Q, long long ldq, int k, const double*
 // h_i = v_i . w; the last one w . w) with an exchange of tagged CTA sums
 // between them: h_i into hout[i * hstride]
 // (i <= j), ||w||^2 into *wwout, then vnext = w / ||w|| (and vnext32, its
-// FP32 copy, when given; zeros when ||w|| = 0).  w is used up, or with keep holds
-// the orthogonalised vector afterwards.  Sums are in the vectors' precision and in a
+// FP32 copy, when given; zeros when ||w|| = 0).  w is used up, or with hook.keep
+// holds the orthogonalised vector afterwards.  Sums are in the vectors' precision and in a
 // fixed order (CTA 0 adds the CTA sums by their index).  words holds
 // kStepWordsBytes: zero before the first launch; after a wait that ran out its
 // error word (kStepErrWord) holds BILU_ERR_TIMEOUT, launches return at once,
@@ -62,14 +62,20 @@ constexpr int kStepErrWord = 2;
 constexpr int kStepFan = 8;
 constexpr size_t kStepWordsBytes =
     128 + (size_t)kStepMaxCTAs * 16 + (size_t)kStepMaxCTAs / kStepFan * 128;
+// Test hook: keep w; the streaming form whatever n; polls before a wait gives up;
+// a CTA that never stores its sums (-1: none).
+struct StepHook {
+  int keep = 0, streaming = 0, withhold = -1;
+  long long spin = kSpinLimit;
+};
 int mgs_step(long long n, const double* V, long long ldv, int j, double* w, double* hout,
              int hstride, double* wwout, unsigned* words, double* vnext, float* vnext32,
-             cudaStream_t st, int keep = 0);
+             cudaStream_t st, const StepHook& hook = StepHook());
 // The FP32 form for the nested mode's inner solver: FP32 products and FP32
 // sums throughout (the CTA sums and their sum too; the FP64 pipe is
 // left alone), h and ||w||^2 written as FP64.
 int mgs_step_f32(long long n, const float* V, long long ldv, int j, float* w, double* hout,
                  int hstride, double* wwout, unsigned* words, float* vnext, cudaStream_t st,
-                 int keep = 0);
+                 const StepHook& hook = StepHook());
 
 }  // namespace bilu

@@ -415,10 +415,17 @@ struct LevelWords {
   int ticket, err;           // next 32 rows; 0 or a bilu_status
   int maxdeg, nlev;          // largest dependency count of a row; levels
   unsigned long long ndeps;  // dependencies of all rows
-  unsigned long long hubdeps;  // of the rows with more than kLongRow
+  unsigned long long hubdeps;  // k_bilu0_plan: of the rows with more than kLongRow
   int other;                 // k_bilu0_plan: the pattern is not one for the row flow
   int widest;                // rows of the widest level of at most kSortCap rows
   int blocks;                // k_bilu0_plan: the blocks the row pointers hold
+};
+
+// Test hook: a row that never publishes its level (-1: none), polls before a wait
+// gives up.
+struct LevelHook {
+  int withhold = -1;
+  long long spin = kSpinLimit;
 };
 
 __device__ __forceinline__ void st_relaxed(int* p, int v) {
@@ -448,11 +455,11 @@ constexpr int kLevelBatch = 4;
 constexpr int kLevelSpins = 64;      // polls of a waiting warp before it sleeps
 constexpr unsigned kLevelSleep = 32;  // ns between its polls then
 
-template <bool LOWER>
+template <bool LOWER, bool HOOK = false>
 __global__ void __launch_bounds__(256) k_levels(int nb, const int* __restrict__ row,
                                                 const int* __restrict__ col,
                                                 const int* __restrict__ diag, int* level,
-                                                LevelWords* w, long long spin) {
+                                                LevelWords* w, LevelHook hook) {
   const int lane = threadIdx.x & 31;
   while (true) {
     int t = 0;
@@ -472,14 +479,11 @@ __global__ void __launch_bounds__(256) k_levels(int nb, const int* __restrict__ 
       atomicMax(&w->maxdeg, deg);
       atomicAdd(&w->ndeps, (unsigned long long)deps);
     }
-    if (deg > kLongRow) {
-      const unsigned h = __reduce_add_sync(FULL, pe - p > kLongRow ? (unsigned)(pe - p) : 0u);
-      if (lane == 0) atomicAdd(&w->hubdeps, (unsigned long long)h);
-    }
     int c[kLevelBatch];
 #pragma unroll
     for (int u = 0; u < kLevelBatch; ++u) c[u] = -1;
     bool todo = mine;
+    const bool tells = !HOOK || I != hook.withhold;
     int lv = 0, own = 0;  // largest level seen; this row's, once known
     const int I0 = LOWER ? (int)k0 : nb - 1 - (int)k0;  // lane 0's row
     auto lane_of = [&](int r) { return LOWER ? r - I0 : I0 - r; };
@@ -538,8 +542,10 @@ __global__ void __launch_bounds__(256) k_levels(int nb, const int* __restrict__ 
           any |= c[u] >= 0;
         }
         if (todo && !any && p >= pe) {
-          own = lv + 1;
-          st_relaxed(level + I, own);
+          if (tells) {
+            own = lv + 1;
+            st_relaxed(level + I, own);
+          }
           todo = false;
           step = moved = true;
         }
@@ -564,7 +570,7 @@ __global__ void __launch_bounds__(256) k_levels(int nb, const int* __restrict__ 
       }
       long long n = 0;
       while (!__any_sync(FULL, wait >= 0 && ld_relaxed(level + max(wait, 0)) != 0)) {
-        if (++n > spin) {
+        if (++n > (HOOK ? hook.spin : kSpinLimit)) {
           if (lane == 0) atomicCAS(&w->err, 0, (int)BILU_ERR_TIMEOUT);
           return;
         }
@@ -2011,7 +2017,7 @@ __global__ void __launch_bounds__(kLvlThreads, 3) k_bilu0_blocks(
     for (int m = 0; m < PC; ++m)
       if (on[m]) blk[er[m] * BS + ec[m]] = a[m];
     __syncwarp();  // the warp's stores before lane 0's release
-    if (lane == 0) st_release(flags + p, 1);
+    if (lane == 0 && I != ss.withhold) st_release(flags + p, 1);
   }
 }
 
@@ -2112,7 +2118,8 @@ int sync_finish(const SyncState& ss, int* h_zp, cudaStream_t st) {
 // order[lvl[l]] .. order[lvl[l+1]-1]) and order[nb].  rec (optional): the
 // four words of the analysis record.  Returns the words' device copy.
 int level_sets(int nb, const int* row, const int* col, const int* diag, int lower, int* order,
-               int* lvl, int* rec, LevelWords** out, Carver& ws, cudaStream_t st) {
+               int* lvl, int* rec, LevelWords** out, Carver& ws, cudaStream_t st,
+               const LevelHook& hook = LevelHook()) {
   int* level = ws.take<int>((size_t)nb + 1);
   int* cnt = ws.take<int>((size_t)nb + 1);
   LevelWords* w = ws.take<LevelWords>(1);
@@ -2121,12 +2128,16 @@ int level_sets(int nb, const int* row, const int* col, const int* diag, int lowe
   // level, cnt and the words are neighbours: one fill
   BILU_TRY_CUDA(cudaMemsetAsync(level, 0, (char*)(w + 1) - (char*)level, st));
   if (nb == 0) return BILU_OK;
+  const bool hooked = hook.withhold >= 0 || hook.spin != kSpinLimit;
   const void* fn = lower ? (const void*)k_levels<true> : (const void*)k_levels<false>;
   const int grid = (int)std::min<long long>(occupancy_grid(fn, 256), (nb + 255) / 256);
-  if (lower)
-    k_levels<true><<<grid, 256, 0, st>>>(nb, row, col, diag, level, w, kSpinLimit);
-  else
-    k_levels<false><<<grid, 256, 0, st>>>(nb, row, col, diag, level, w, kSpinLimit);
+#define BILU_LEVELS(LOW, HK) \
+  k_levels<LOW, HK><<<grid, 256, 0, st>>>(nb, row, col, diag, level, w, hook)
+  if (hooked && lower) BILU_LEVELS(true, true);
+  else if (hooked) BILU_LEVELS(false, true);
+  else if (lower) BILU_LEVELS(true, false);
+  else BILU_LEVELS(false, false);
+#undef BILU_LEVELS
   BILU_LAUNCH_CHECK();
   k_level_count<<<ceil_div(nb, 256), 256, 0, st>>>(nb, level, cnt);
   BILU_LAUNCH_CHECK();
@@ -2293,6 +2304,7 @@ __global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
   const MatchLists m = match_lists(pk, nb, row, col, diag, I);
   const int dI = __ldg(diag + I);
   if (pk >= dI) return;
+  if (dI - __ldg(row + I) > kLongRow) atomicAdd(&w->hubdeps, 1ull);
   bool odd = m.ce - m.cs > kMatchSerial;
   int at = -1;
   for (int c = m.cs; c < m.ce && !odd; ++c) {
@@ -2399,7 +2411,7 @@ __global__ void __launch_bounds__(kLvlThreads, 3) k_bilu0_syncfree(
     if (__any_sync(FULL, ld_relaxed(ss.err) != 0)) return;
     if (!bilu0_wrow<BS, true>(I, row, col, diag, val, ss, stage)) return;
     __syncwarp();  // the warp's stores before lane 0's release
-    if (lane == 0) st_release(ss.flags + I, 1);
+    if (lane == 0 && I != ss.withhold) st_release(ss.flags + I, 1);
   }
 }
 
@@ -2574,7 +2586,7 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
                  long long ndeps_max, int* order, int* lvl_ptr, int* nlev_d, int* h_nlev,
                  Carver& ws, cudaStream_t st, int* h_sched = nullptr, int* h_maxdeg = nullptr,
                  int* h_fsched = nullptr, int2* plan = nullptr, long long nplan = 0, int bs = 0,
-                 LevelOut* out = nullptr) {
+                 LevelOut* out = nullptr, const LevelHook& hook = LevelHook()) {
   if (nb == 0) {
     BILU_TRY_CUDA(cudaMemsetAsync(nlev_d, 0, sizeof(int) * 4, st));
     BILU_TRY_CUDA(cudaMemsetAsync(lvl_ptr, 0, sizeof(int) * 2, st));
@@ -2583,7 +2595,7 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
     return BILU_OK;
   }
   LevelWords *w = nullptr, hw;
-  BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st));
+  BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st, hook));
   if (plan) {
     k_bilu0_plan<<<ceil_div(std::max(nplan, 1ll), 256), 256, 0, st>>>(nb, nplan, row, col, diag,
                                                                        plan, w);
@@ -2894,7 +2906,7 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
     // 15.6.)
     int* nmatch = keep.h_counted ? (int*)keep.plan : nullptr;  // the plan is not read any more
     SyncState ss;
-    BILU_TRY(sync_init(ss, nb, ws, st));
+    BILU_TRY(sync_init(ss, nb, ws, st, keep.spin, keep.withhold));
     ss.order = order;
     ss.rdiag = rdiag;
     ss.nmatch = nmatch;
@@ -2918,6 +2930,8 @@ int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
     if (!tcnt || !tptr) return BILU_ERR_WORKSPACE;
     SyncState ss;
     BILU_TRY(sync_init_words(ss, ws, st));
+    ss.spin = keep.spin;
+    ss.withhold = keep.withhold;
     ss.rdiag = rdiag;
     if (nb > 0) {
       const unsigned grid = ceil_div(nnzb, 256);
@@ -3277,6 +3291,27 @@ extern "C" int bilu_sptrsv_ex(int nb, int nnzb, int bs, const int* d_row, const 
   BILU_TRY(diag_positions(nb, d_row, d_col, diag, nullptr, ws, S(stream)));
   return sptrsv_level_impl(nb, nnzb, bs, d_row, d_col, diag, d_val, lower != 0, unit != 0, d_b,
                            d_x, ws, S(stream));
+}
+
+// Test hook: the level analysis with block row `withhold_row` never publishing its
+// level and a spin budget of spin_limit polls.
+extern "C" int bilu_debug_sptrsv_analysis_withhold(int nb, int nnzb, int bs, const int* d_row,
+                                                   const int* d_col, int lower, int withhold_row,
+                                                   long long spin_limit, void* d_info, void* d_ws,
+                                                   size_t ws_bytes, bilu_stream_t stream) {
+  if (nb < 1 || nnzb < nb || !d_info || !d_row || !d_col || spin_limit < 1 ||
+      spin_limit > kSpinLimit)
+    return BILU_ERR_ARG;
+  if (!bs_supported(bs)) return BILU_ERR_UNSUPPORTED;
+  AnalysisView a(d_info, nb);
+  Carver ws(d_ws, ws_bytes);
+  BILU_TRY(diag_positions(nb, d_row, d_col, a.diag, nullptr, ws, S(stream)));
+  LevelHook hook;
+  hook.withhold = withhold_row;
+  hook.spin = spin_limit;
+  return build_levels(nb, d_row, d_col, a.diag, lower != 0, (long long)nnzb - nb, a.order, a.lvl,
+                      a.nlev, nullptr, ws, S(stream), nullptr, nullptr, nullptr, nullptr, 0, 0,
+                      nullptr, hook);
 }
 
 // Test hook: BILU(0) (bilu_bsrilu0_ex) with block row `withhold_row` never

@@ -289,6 +289,43 @@ def withheld(cuda, A, schedule, row, polls):
     return st, N(lu)
 
 
+@pytest.mark.parametrize("name", ["7-point", "9-point", "dense", "hubs"])
+def test_bilu0_withheld_row_times_out(cuda, orc, name):
+    """Row flow, rows and blocks by ticket with a row that never publishes: the rows
+    that wait for it give up, the others leave, and the next call is right."""
+    rp, col = bilu_pattern(name)
+    nb = len(rp) - 1
+    rows = np.repeat(np.arange(nb), np.diff(rp))
+    val = np.random.default_rng(1).uniform(-1, 1, size=(len(col), 4, 4))
+    val[rows == col] += 8.0 * np.diff(rp)[:, None, None] * np.eye(4)
+    A = gen.BSRMatrix(nb, 4, rp, col, val)
+    ref, _ = orc.bsrilu0(nb, 4, rp, col, val)
+    for schedule in (-1, 1):
+        for row in (0, nb // 2):
+            assert withheld(cuda, A, schedule, row, 4000)[0] == _lib_status("BILU_ERR_TIMEOUT")
+        st, lu = withheld(cuda, A, schedule, -1, 1 << 20)
+        assert st == 0 and np.max(np.abs(lu - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("lower", [1, 0])
+@pytest.mark.parametrize("name", ["chain", "grid", "dense", "hubs"])
+def test_level_analysis_withheld_row_times_out(cuda, name, lower):
+    from isai_kernel_gb300 import _lib, api
+
+    rp, col = level_pattern(name)
+    nb, nnzb, L = len(rp) - 1, len(col), _lib.lib()
+    info = api._ws(L.bilu_sptrsv_analysis_bytes(nb), cuda)
+    ws = api._ws(L.bilu_sptrsv_analysis_ws_bytes(nb, nnzb), cuda)
+    r, c = T(rp, cuda), T(col, cuda)
+    for row in (nb // 3, nb // 2):
+        st = L.bilu_debug_sptrsv_analysis_withhold(nb, nnzb, 4, api._p(r), api._p(c), lower, row,
+                                                   4000, api._p(info), api._p(ws), ws.numel(),
+                                                   api._s())
+        assert st == _lib_status("BILU_ERR_TIMEOUT")
+    api.call("bilu_sptrsv_analysis", nb, nnzb, 4, api._p(r), api._p(c), lower, api._p(info),
+             api._p(ws), ws.numel(), api._s())
+
+
 @pytest.mark.parametrize("bs", [4, 8])
 def test_row_flow_waits_for_a_long_path(cuda, orc, bs):
     """A path of 3000 rows, walked by one warp, in front of 2000 rows that wait
@@ -846,6 +883,50 @@ def test_mgs_step_leaves_the_orthogonalised_vector(cuda, fp32, n):
     want = w[:n].double() / h[j + 1].sqrt()
     assert torch.all((vn[:n].double() - want).abs() <= 4 * eps * want.abs())
     assert abs(h[j + 1] - (w[:n].double() ** 2).sum()) <= eps * n ** 0.5 * h[j + 1]
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("n", [513, 300001, 1500002])
+def test_mgs_step_forms_give_the_same_bits(cuda, fp32, n):
+    """The streaming and the resident form: h, ||w||^2, v_{j+1} and w."""
+    import torch
+
+    from isai_kernel_gb300 import _lib, api
+
+    j, out = 3, []
+    for streaming in (1, 0):
+        V, w, ws = step_vectors(cuda, fp32, n, j)
+        h = torch.empty(j + 2, dtype=torch.float64, device=cuda)
+        vn = torch.zeros_like(w)
+        assert _lib.lib().bilu_debug_mgs_step_ex(
+            n, fp32, api._p(V), V.shape[1], j, api._p(w), api._p(h), api._p(vn), streaming, -1,
+            1 << 20, api._p(ws), ws.numel(), api._s()) == 0
+        out.append((h, vn, w))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("streaming", [0, 1])
+@pytest.mark.parametrize("cta", [0, 1, 200])
+def test_mgs_step_withheld_sum_times_out(cuda, fp32, streaming, cta):
+    """A CTA that never stores its sums: every wait gives up, the call says so,
+    and the next one on the same workspace is right."""
+    import torch
+
+    from isai_kernel_gb300 import _lib, api
+
+    n, j, L = 300001, 2, _lib.lib()
+    V, w, ws = step_vectors(cuda, fp32, n, j)
+    h = torch.empty(j + 2, dtype=torch.float64, device=cuda)
+    vn = torch.zeros_like(w)
+    st = L.bilu_debug_mgs_step_ex(n, fp32, api._p(V), V.shape[1], j, api._p(w.clone()), api._p(h),
+                                  api._p(vn), streaming, cta, 2000, api._p(ws), ws.numel(),
+                                  api._s())
+    assert st == _lib_status("BILU_ERR_TIMEOUT")
+    assert L.bilu_debug_mgs_step(n, fp32, api._p(V), V.shape[1], j, api._p(w), api._p(h),
+                                 api._p(vn), api._p(ws), ws.numel(), api._s()) == 0
+    eps = torch.finfo(w.dtype).eps
+    assert torch.all((V[:, :n].double() @ vn[:n].double()).abs() <= 50 * eps * n ** 0.5)
 
 
 # ------------------------------------------------------------------ conversion
