@@ -653,16 +653,18 @@ int autotune(bilu_batch* B, int r0, int r1, int k, double* X, double* Y, float* 
 
 template <int BS, int RM, int RA>
 int launch_batch_step_t(const BatchStepArgs& a, cudaStream_t st) {
-  static int grid = 0;
+  static PerDevice<int> grids;
   const void* fn = (const void*)k_batch_step<BS, RM, RA>;
-  if (!grid) {
+  int grid = 0;
+  BILU_TRY(per_device(grids, &grid, [&](int* g) -> int {
     int dev = 0, sms = 0, per = 0;
     BILU_TRY_CUDA(cudaGetDevice(&dev));
     BILU_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     BILU_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kStepT, 0));
     if (per < 1) return BILU_ERR_UNSUPPORTED;
-    grid = per * sms;
-  }
+    *g = per * sms;
+    return BILU_OK;
+  }));
   BatchStepArgs arg = a;
   void* args[] = {&arg};
   BILU_TRY_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kStepT), args, 0, st));

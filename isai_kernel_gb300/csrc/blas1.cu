@@ -746,17 +746,23 @@ template <class T>
 int mgs_step_t(long long n, const T* V, long long ldv, int j, T* w, double* hout, int hstride,
                double* wwout, unsigned* words, T* vnext, float* vnext32,
                StepHook hook, cudaStream_t st) {
-  static int grid = 0, resident = 0;
-  if (!grid) {
+  struct Plan {
+    int grid, resident;
+  };
+  static PerDevice<Plan> plans;
+  Plan plan{};
+  BILU_TRY(per_device(plans, &plan, [](Plan* p) -> int {
     int g0 = 0, g2 = 0, g4 = 0, g6 = 0;
     BILU_TRY((mgs_prepare<T, 0>(&g0)));
     BILU_TRY((mgs_prepare<T, 2>(&g2)));
     BILU_TRY((mgs_prepare<T, 4>(&g4)));
     BILU_TRY((mgs_prepare<T, 6>(&g6)));
     // a resident form whose CTAs do not all fit at once is not used
-    resident = g6 >= g0 ? 6 : g4 >= g0 ? 4 : g2 >= g0 ? 2 : 0;
-    grid = g0;
-  }
+    p->resident = g6 >= g0 ? 6 : g4 >= g0 ? 4 : g2 >= g0 ? 2 : 0;
+    p->grid = g0;
+    return BILU_OK;
+  }));
+  const int grid = plan.grid, resident = plan.resident;
   if (grid > kStepMaxCTAs) return BILU_ERR_UNSUPPORTED;
   // Vectors a thread has to hold: up to 6 of w fit its 64 registers, and twice
   // that two CTAs' shared memory (196 of 227 KB), i.e. n up to 1.87 M in FP64,

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "bilu_isai.h"
+#include "perdevice.cuh"
 
 namespace bilu {
 
@@ -49,6 +50,24 @@ inline bool bs_supported(int bs) { return bs == 4 || bs == 5 || bs == 8; }
                : BILU_ERR_UNSUPPORTED)
 
 inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
+
+// The current device's value in c (PerDevice::get).
+template <class V, class F>
+int per_device(PerDevice<V>& c, V* out, F make) {
+  int dev = 0;
+  BILU_TRY_CUDA(cudaGetDevice(&dev));
+  return c.get(dev, out, make);
+}
+
+// Dynamic shared memory above 48 KB for fn, allowed once per device.
+inline int allow_smem(PerDevice<int>& c, const void* fn, size_t bytes) {
+  int ok = 0;
+  return per_device(c, &ok, [&](int*) -> int {
+    BILU_TRY_CUDA(
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return BILU_OK;
+  });
+}
 
 // Workspace carving: aligned sub-allocations from a caller buffer.
 struct Carver {

@@ -333,12 +333,8 @@ int launch_isai(int nb, const double* Aval, const int* Mptr, const int* Mind, in
   using T = Team<BS>;
   constexpr int W = IsaiCfg<BS>::kWarps;
   size_t smem = (size_t)W * T::TPW * (IsaiCfg<BS>::kCache + 1) * T::BS2 * sizeof(double);
-  static bool attr_set = false;
-  if (!attr_set) {
-    BILU_TRY_CUDA(cudaFuncSetAttribute(k_isai<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-    attr_set = true;
-  }
+  static PerDevice<int> allowed;
+  BILU_TRY(allow_smem(allowed, (const void*)k_isai<BS>, smem));
   long long warps = (nb + T::TPW - 1) / T::TPW;
   k_isai<BS><<<ceil_div(warps, W), 32 * W, smem, st>>>(nb, Aval, Mptr, Mind, lower, pp, pl, ps,
                                                        Dinv, Mval, map, M32);

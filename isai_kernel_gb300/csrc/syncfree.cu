@@ -2065,14 +2065,15 @@ __global__ void __launch_bounds__(kLvlThreads, 2) k_bilu0_levels(
 
 
 int sm_count() {
-  static int sms = 0;
-  if (!sms) {
+  static PerDevice<int> c;
+  int sms = 1;
+  per_device(c, &sms, [](int* n) -> int {
     int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 1;
-  }
-  return sms;
+    BILU_TRY_CUDA(cudaGetDevice(&dev));
+    BILU_TRY_CUDA(cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev));
+    return BILU_OK;
+  });
+  return std::max(sms, 1);
 }
 
 int occupancy_per_sm(const void* fn, int threads, size_t smem = 0) {
@@ -2619,13 +2620,8 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
     out->h_blocks = counted && rec[1] > kLongRow && blocks_instead(bs, nplan, hw.hubdeps);
   }
   if (hw.widest > 1) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      BILU_TRY_CUDA(cudaFuncSetAttribute((const void*)k_sort_levels,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sort_smem(kSortCap)));
-      attr_set = true;
-    }
+    static PerDevice<int> allowed;
+    BILU_TRY(allow_smem(allowed, (const void*)k_sort_levels, sort_smem(kSortCap)));
     int bits = 1;
     while (bits < 31 && (nb - 1) >> bits) ++bits;
     k_sort_levels<<<(unsigned)rec[0], kSortThreads, sort_smem(hw.widest), st>>>(order, lvl_ptr,
@@ -2701,12 +2697,8 @@ int launch_bilu0_syncfree(int nb, const int* row, const int* col, const int* dia
                           SyncState ss, cudaStream_t st) {
   const void* fn = (const void*)k_bilu0_syncfree<BS>;
   const size_t smem = (size_t)(kLvlThreads / 32) * kRowStage * sizeof(int);
-  static bool attr_set = false;
-  if (!attr_set) {
-    BILU_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-    attr_set = true;
-  }
+  static PerDevice<int> allowed;
+  BILU_TRY(allow_smem(allowed, fn, smem));
   // every warp resident at once is not required (tickets), but more warps
   // than rows would only spin
   int grid = std::min<long long>(occupancy_grid(fn, kLvlThreads, smem),
