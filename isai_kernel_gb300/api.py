@@ -28,15 +28,17 @@ def _p(t):
     return None if t is None else t.data_ptr()
 
 
-_raw_stream = torch._C._cuda_getCurrentRawStream if torch.backends.cuda.is_built() else None
+# torch's own shortcuts past the Stream object; without them, the public call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _s(stream=None):
     if stream is not None:
         return stream.cuda_stream
-    if _raw_stream is None or not torch.cuda.is_initialized():
+    if _raw_stream is None or _raw_device is None or not torch.cuda.is_initialized():
         return torch.cuda.current_stream().cuda_stream  # initialises CUDA, or says why not
-    return _raw_stream(torch._C._cuda_getDevice())
+    return _raw_stream(_raw_device())
 
 
 def _ws(nbytes: int, dev):
