@@ -181,7 +181,6 @@ struct bilu_ctx {
   double *partial = nullptr, *dscal = nullptr, *dcoef = nullptr;
   double* hpin = nullptr;  // pinned host mirror of dscal
   cudaEvent_t ev = nullptr;
-  unsigned* counter = nullptr;  // arrival counter of the MGS sweep reductions
   unsigned* step_words = nullptr;  // kStepWordsBytes of mgs_step: error word, tagged sums
   long long steps = 0, restarts = 0;  // Arnoldi steps and cycles of the last solve
   // nested (GMRES-IR) mode: FP32 inner GMRES of inner_k steps per outer
@@ -210,8 +209,7 @@ struct bilu_ctx {
   }
   void free_solver() {
     for (void* p : {(void*)V, (void*)Z, (void*)w, (void*)r, (void*)tmp, (void*)v32, (void*)z32,
-                    (void*)partial, (void*)dscal, (void*)dcoef, (void*)counter,
-                    (void*)step_words, (void*)U32,
+                    (void*)partial, (void*)dscal, (void*)dcoef, (void*)step_words, (void*)U32,
                     (void*)Q32, (void*)w32, (void*)inner_small})
       if (p) cudaFreeAsync(p, st);
     U32 = Q32 = w32 = nullptr;
@@ -219,7 +217,6 @@ struct bilu_ctx {
     inner_alloc = 0;
     v32 = nullptr;
     z32 = nullptr;
-    counter = nullptr;
     step_words = nullptr;
     if (hpin) cudaFreeHost(hpin);
     if (ev) cudaEventDestroy(ev);
@@ -666,8 +663,6 @@ int ensure_solver(bilu_ctx* c, int m) {
   BILU_TRY_CUDA(get(&c->dscal, sizeof(double) * 6 * kPartStride));
   BILU_TRY_CUDA(get(&c->dcoef, sizeof(double) * kPartStride));
   BILU_TRY_CUDA(cudaMallocHost(&c->hpin, sizeof(double) * 6 * kPartStride));
-  BILU_TRY_CUDA(get(&c->counter, sizeof(unsigned)));
-  BILU_TRY_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->st));
   BILU_TRY_CUDA(get(&c->step_words, kStepWordsBytes));
   BILU_TRY_CUDA(cudaMemsetAsync(c->step_words, 0, kStepWordsBytes, c->st));
   c->m_alloc = m;

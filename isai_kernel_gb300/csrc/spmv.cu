@@ -645,7 +645,8 @@ int launch_spmv_cfg(int mb, const int* row, const int* col, const VT* val, const
       return launch_spmv_hubs<BS, VT, XT, YT>(mb, row, col, val, x, y, st, y32);
     }
   }
-  if constexpr (!TR && RPG == 1) {
+  // early starts follow a kernel that wrote x in the product's precision
+  if constexpr (!TR && RPG == 1 && sizeof(XT) == sizeof(VT)) {
     if (dep) {
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
