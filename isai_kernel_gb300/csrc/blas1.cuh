@@ -21,7 +21,7 @@ int multidot(long long n, const double* V, long long ldv, int nv, const double* 
 int multiaxpy_norm(long long n, const double* V, long long ldv, int nv, const double* coef,
                    double sign, double* w, double* partial, const int* skip_flag,
                    cudaStream_t st);
-// out[i] = sum_cta partial[cta*kPartStride + i], i < nout (one thread each).
+// out[i] = sum_cta partial[cta*kPartStride + i], i < nout (a warp each).
 int reduce_partials(const double* partial, int nout, double* out, cudaStream_t st);
 // y = x * (1/sqrt(*nrm2)) with *nrm2 a device scalar; y32 (optional)
 // receives the same vector rounded to FP32 (input of the FP32 apply).
@@ -32,7 +32,7 @@ int residual_norm(long long n, const double* b, const double* ax, double* r, dou
                   cudaStream_t st);
 
 // ---- FP32 inner solver of the nested (GMRES-IR) mode ----
-// Least squares of the inner Arnoldi steps on the device (one thread): H
+// Least squares of the inner Arnoldi steps on the device (one warp): H
 // holds (k+1) x k entries H[i*k + j] with the raw column entries h_ij
 // (i <= j) and, in ww[j], ||w_j||^2 (the subdiagonal squared); Givens
 // rotations in FP64 reduce H to triangular form against beta e_1 (beta = 1)

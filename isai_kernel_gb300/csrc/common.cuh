@@ -107,7 +107,6 @@ __device__ __forceinline__ T warp_sum(T v, unsigned mask = 0xffffffffu) {
   return v;
 }
 
-// Streaming (evict-first) 16-byte loads for values read exactly once.
 // Programmatic dependent launch (k_bsr_spmv, DEP): the launch before this one
 // in the stream has finished and its writes are visible / the next one may start.
 __device__ __forceinline__ void dependency_wait() {
@@ -117,6 +116,7 @@ __device__ __forceinline__ void dependents_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Streaming (evict-first) loads for values read exactly once.
 __device__ __forceinline__ double2 ld_stream(const double2* p) {
   double2 v;
   asm volatile("ld.global.cs.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));

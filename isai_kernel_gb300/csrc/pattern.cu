@@ -278,7 +278,7 @@ __global__ void k_gather_blocks(long long nnzb, int bs2, const int* __restrict__
 //
 // The merge needs block columns that never decrease along a scalar row.  A
 // lane that sees one decrease marks its block row, which the whole warp then
-// does over again with the searches below (quadratic in the row's entries;
+// does over again with the searches below (up to cubic in the row's entries;
 // only files with unsorted rows come here).
 template <int BS>
 struct C2b {

@@ -215,8 +215,8 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, int nslot, con
 // all the groups have reached is issued, and the warps of a full SM cover the
 // latency (two rows a group of the 4- and 5-blocks, two blocks a batch of the
 // 8-blocks before; the apply, before -> now: 64^3 7-point 4x4 67.8 -> 63.7 us,
-// 47x43x41 5x5 41.3 -> 38.9, 512^2 5-point 5x5 81.8 -> 77.9, 8x8 249 -> 172 of
-// 174 at 0.58 TDFMA/s).
+// 47x43x41 5x5 41.3 -> 38.9, 512^2 5-point 5x5 81.8 -> 77.9, 8x8 249 -> 172, 161
+// of them DFMA at 1.25 TFLOP/s).
 // FP32: bound by memory.  A group handles RPG consecutive block rows and issues
 // the loads of the next U blocks of all of them before any arithmetic, so a warp
 // keeps RPG*U independent block loads per lane in flight; each row's sum runs in
@@ -224,8 +224,9 @@ __device__ __noinline__ void spmv_long_rows(const int* long_rows, int nslot, con
 // measurements on the 128^3 7-point pattern (7 blocks a row) and its triangle (4
 // a row): U = 4 with RPG = 1 for wider rows (0.199 -> 0.176 ms on the operator),
 // RPG = 1 at 8 CTAs per SM for bs 4 rows of ~4 blocks, else RPG = 2.
-// Patterns with rows of more than kLongSpmvRow blocks take
-// k_bsr_spmv_balanced (FP64) or k_bsr_spmv_uneven (FP32).
+// Patterns with rows of more than kLongSpmvRow blocks take k_bsr_spmv_balanced
+// (FP64) or k_bsr_spmv_uneven (FP32), unless the rows are alike or the long ones
+// few (launch_spmv); HUBS leaves those few to k_spmv_hubs.
 // DEP, for a product whose x is the result of the launch before it (U after L,
 // A after U): started by programmatic dependent launch while that one drains,
 // it reads its row pointers, columns and first blocks, none of which the launch
@@ -1191,7 +1192,7 @@ __device__ int g_layout_word[2];  // scratch of the cached check (under its lock
 // The standalone entry points do not know the pattern: the answer is cached
 // per (row pointer array, block rows, block size), most recent first.  A
 // stale entry (a buffer reused for another pattern) can only cost speed:
-// both kernels are exact for any row length.
+// every kernel is exact for any row length.
 struct LayoutEntry {
   const int* row;
   int mb, bs, layout;

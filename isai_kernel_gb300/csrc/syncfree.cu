@@ -4,15 +4,20 @@
 //                                                            k_bilu0_blocks,
 //                                                            k_bilu0_levels,
 //                                                            k_bilu0_syncfree
-//   spTrSolveL / spTrSolveU (cape_sptrsv.h:8,55)         -> k_sptrsv_levels,
+//   spTrSolveL / spTrSolveU (cape_sptrsv.h:8,55)         -> k_sptrsv_flow,
+//                                                            k_sptrsv_levels,
 //                                                            k_sptrsv (sync-free)
 //
-// Level schedule (default): the block rows are grouped by dependency level
-// (k_levels); one cooperative launch then processes a level with a group of
-// bs lanes per row and meets at a bounded grid barrier.
+// Every schedule starts from the dependency levels of the rows (k_levels).
 //
-// Sync-free schedule (the reference's design, kept for the solve): a warp
-// owns one block row at a time.  Rows are handed out by an atomic ticket
+// Level order, flow (default of both, k_sptrsv_flow, k_bilu0_rowflow): resident
+// warps take their rows in level order and wait for what a row reads.
+//
+// Level order, barrier (wide levels of BILU(0), long rows of the solves): one
+// cooperative launch processes a level and meets at a bounded grid barrier.
+//
+// Sync-free (the reference's design): a warp owns one block row, or one block
+// (k_bilu0_blocks), at a time.  They are handed out by an atomic ticket
 // counter in level order, so every row a warp waits on was taken by a warp
 // that is already running (the reference maps rows to threads statically and
 // relies on scheduling order).  A finished row publishes its flag with
@@ -2812,12 +2817,9 @@ int sync_init_words(SyncState& ss, Carver& ws, cudaStream_t st) {
 
 }  // namespace
 
-// BILU(0) in place, level scheduled (one cooperative launch, one grid
-// barrier per dependency level of the lower DAG) or sync-free.  rdiag
-// (nb x bs) receives the reciprocal pivots; null: carved from ws.  keep
-// (optional): where the level analysis of the lower DAG is built and kept.
-// Level analysis of BILU(0)'s lower DAG into keep (order, lvl, nlev on the
-// device; level count, schedules and largest dependency count on the host).
+// Level analysis of BILU(0)'s lower DAG into keep (order, lvl, nlev and the row
+// flow's plan on the device; level count, schedules and largest dependency count
+// on the host).
 // Structure only: it may run before the values are on the device.
 int bilu0_analyze(int nb, long long nnzb, int bs, const int* row, const int* col, const int* diag,
                   LevelOut& keep, Carver& ws, cudaStream_t st) {
@@ -2868,8 +2870,10 @@ int bilu0_match_fill(int nb, long long nnzb, const int* row, const int* col, con
   return BILU_OK;
 }
 
-// BILU(0) on an analysis from bilu0_analyze (with the match lists when
-// keep has them and the level-order kernel runs).
+// BILU(0) in place on an analysis from bilu0_analyze: the row flow, the barrier
+// kernel (with the match lists when keep has them), or sync-free over rows or over
+// blocks, as the analysis or the caller's schedule says.  rdiag (nb x bs) receives
+// the reciprocal pivots; null: carved from ws.
 int bilu0_factor(int nb, long long nnzb, int bs, const int* row, const int* col,
                  const int* diag, double* val, int* h_zp, Carver& ws, cudaStream_t st,
                  int schedule, double* rdiag, const LevelOut& keep) {
