@@ -426,7 +426,7 @@ __device__ __forceinline__ bool wait_tagged(const unsigned long long* p, unsigne
   return true;
 }
 
-template <class T, int KR>
+template <class T, int KR, bool HOOK>
 __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     long long n, const T* __restrict__ V, long long ldv, int j, T* __restrict__ w,
     double* __restrict__ hout, int hstride, double* __restrict__ wwout,
@@ -493,7 +493,8 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
     if constexpr (kResident) cp_async_wait<0>();
     return;
   }
-  const bool tells = lane == 0 && (int)blockIdx.x != hook.withhold;
+  const bool tells = lane == 0 && (!HOOK || (int)blockIdx.x != hook.withhold);
+  const long long spin = HOOK ? hook.spin : kSpinLimit;
   T h = T(0);
   for (int i = 0; i <= j + 1; ++i) {
     const T* vp = i > 0 ? V + (long long)(i - 1) * ldv : nullptr;
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       T t = T(0);
       for (int c = threadIdx.x; c < G; c += kStepThreads) {
         T v = T(0);
-        ok = ok && wait_tagged(sums + (size_t)c * PW, tag, err, hook.spin, v);
+        ok = ok && wait_tagged(sums + (size_t)c * PW, tag, err, spin, v);
         if constexpr (sizeof(T) == 8) sum_s[c] = v; else t += v;
       }
       __syncwarp();
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       }
     } else if (threadIdx.x == 0) {
       T v = T(0);
-      ok = wait_tagged(totals + (size_t)(blockIdx.x / kStepFan) * 16, tag, err, hook.spin, v);
+      ok = wait_tagged(totals + (size_t)(blockIdx.x / kStepFan) * 16, tag, err, spin, v);
       h_s = v;
     }
     if (!__syncthreads_and(ok)) {
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepPerSM) k_mgs_step(
       if (vnext32) vnext32[e] = (float)v;
     }
   }
-  if constexpr (kResident) {
+  if constexpr (kResident && HOOK) {
     if (hook.keep) {
 #pragma unroll
       for (int k = 0; k < KR; ++k) {
@@ -713,18 +714,27 @@ int scale_rsqrt(long long n, const double* x, const double* nrm2, double* y, cud
 // The grid of the k_mgs_step forms: one CTA count for all of them, so that a
 // vector is cut alike whichever form runs.
 template <class T, int KR>
+constexpr size_t mgs_smem() {
+  return KR > 0 ? (size_t)2 * KR * kStepThreads * 16 : (sizeof(T) == 8 ? kStepStageBytes : 0);
+}
+
+template <class T, int KR, bool HOOK = false>
 int mgs_prepare(int* grid) {
-  const size_t smem = KR > 0 ? (size_t)2 * KR * kStepThreads * 16
-                             : (sizeof(T) == 8 ? kStepStageBytes : 0);
+  constexpr size_t smem = mgs_smem<T, KR>();
   int per = 0, dev = 0, sms = 0;
   BILU_TRY_CUDA(cudaGetDevice(&dev));
   BILU_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (smem)
-    BILU_TRY_CUDA(cudaFuncSetAttribute(k_mgs_step<T, KR>,
+    BILU_TRY_CUDA(cudaFuncSetAttribute(k_mgs_step<T, KR, HOOK>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  BILU_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mgs_step<T, KR>,
+  BILU_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mgs_step<T, KR, HOOK>,
                                                               kStepThreads, smem));
   *grid = std::max(1, std::min(per, kStepPerSM)) * sms;
+  if constexpr (!HOOK) {  // the entry points' instance, on the same grid
+    int hooked = 0;
+    BILU_TRY((mgs_prepare<T, KR, true>(&hooked)));
+    *grid = std::min(*grid, hooked);
+  }
   return BILU_OK;
 }
 
@@ -732,12 +742,14 @@ template <class T, int KR>
 int mgs_launch(int grid, long long n, const T* V, long long ldv, int j, T* w, double* hout,
                int hstride, double* wwout, unsigned* words, T* vnext, float* vnext32,
                StepHook hook, cudaStream_t st) {
-  const size_t smem = KR > 0 ? (size_t)2 * KR * kStepThreads * 16
-                             : (sizeof(T) == 8 ? kStepStageBytes : 0);
+  // (the streaming form leaves w as keep wants it anyway)
+  const bool hooked = (hook.keep && KR > 0) || hook.withhold >= 0 || hook.spin != kSpinLimit;
+  const void* fn = hooked ? (const void*)k_mgs_step<T, KR, true>
+                          : (const void*)k_mgs_step<T, KR, false>;
   void* args[] = {&n,     &V,     &ldv,   &j,       &w,   &hout, &hstride,
                   &wwout, &words, &vnext, &vnext32, &hook};
-  BILU_TRY_CUDA(cudaLaunchCooperativeKernel((const void*)k_mgs_step<T, KR>, dim3(grid),
-                                            dim3(kStepThreads), args, smem, st));
+  BILU_TRY_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kStepThreads), args,
+                                            mgs_smem<T, KR>(), st));
   BILU_LAUNCH_CHECK();
   return BILU_OK;
 }
