@@ -218,6 +218,8 @@ def rule_pattern(name):
     if name == "wide, a triangle":
         return pattern_of([[] if i < 8192 else [0, 1, i - 8192] if i > 16383 else [i - 8192]
                            for i in range(16385)] + [[8192, 0]])
+    if name == "parallel long rows":  # one level of them: no chain to cut
+        return pattern_of([range(i % 50, 2000, 50) if i >= 2000 else [] for i in range(2200)])
     A = gen.laplace2d(30, bs=4)
     rows = [set(A.colind[A.rowptr[i]:A.rowptr[i + 1]].tolist()) for i in range(A.nb)]
     n = {"one row of 33": 1, "long rows, 2%": 2, "long rows, 10%": 12}[name]
@@ -230,7 +232,8 @@ def rule_pattern(name):
 @pytest.mark.parametrize("bs", [4, 5, 8])
 @pytest.mark.parametrize("name", ["two wide levels", "a little narrower",
                                   "wide, six dependencies", "wide, a triangle",
-                                  "one row of 33", "long rows, 2%", "long rows, 10%"])
+                                  "parallel long rows", "one row of 33", "long rows, 2%",
+                                  "long rows, 10%"])
 def test_bilu0_rule_between_schedules(cuda, orc, name, bs):
     """As test_bilu0_schedules, on both sides of each line of the rule."""
     from isai_kernel_gb300 import api
@@ -798,6 +801,66 @@ def test_apply_starts_before_the_first_product_ends(cuda, name, bs, fp32):
         b.add_(1.0)
         graph.replay()
         assert torch.equal(got, both()[1])
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("bs", [4, 5, 8])
+def test_hub_kernels_keep_the_stream_order(cuda, bs, fp32):
+    """The hub rows' kernels start beside the other rows' one: what is written right
+    before a product is read by both, what follows sees both, on the current and a
+    side stream and replayed from a graph; the bits are those of a product on its
+    own."""
+    import torch
+
+    from isai_kernel_gb300 import api
+
+    mb, k = 7000, 9
+    n = np.full(mb, 3)
+    n[1000:1012] = 200
+    rp = np.zeros(mb + 1, np.int32)
+    np.cumsum(n, out=rp[1:])
+    g = torch.Generator(device=cuda).manual_seed(bs)
+    rand = lambda *s: torch.randn(*s, dtype=torch.float64, device=cuda, generator=g)
+    col = np.random.default_rng(bs).integers(0, mb, size=rp[-1]).astype(np.int32)
+    dt = torch.float32 if fp32 else torch.float64
+    r, c, v = T(rp, cuda), T(col, cuda), rand(len(col), bs, bs).to(dt)
+    X, x = rand(mb * bs, k), rand(mb * bs).to(dt)
+
+    def chain():
+        Y = api.bcsr_spmm(mb, bs, r, c, v, X)
+        y = api.bcsr_spmv(mb, bs, r, c, v, x)
+        # each result goes straight into the next product
+        return Y, api.bcsr_spmm(mb, bs, r, c, v, Y), y, api.bcsr_spmv(mb, bs, r, c, v, y)
+
+    def apart():
+        out = []
+        for f, a in ((api.bcsr_spmm, X), (api.bcsr_spmv, x)):
+            for _ in range(2):
+                torch.cuda.synchronize()
+                a = f(mb, bs, r, c, v, a)
+                torch.cuda.synchronize()
+                out.append(a)
+        return out
+
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for _ in range(8):
+                v.mul_(-0.5)
+                X.add_(0.25)
+                x.neg_()
+                got = chain()
+                assert all(torch.equal(a, b) for a, b in zip(got, apart()))
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain()
+    for _ in range(3):
+        v.mul_(-1.5)
+        X.neg_()
+        x.add_(1.0)
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, apart()))
 
 
 # ------------------------------------------------------------------ orthogonalisation
