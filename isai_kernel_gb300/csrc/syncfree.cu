@@ -2580,12 +2580,13 @@ int launch_coop(const void* fn, int grid, int threads, void** args, cudaStream_t
 // of a half or whole warp.  Rows per level, dependencies a row: barrier / row flow
 // in us, block sizes 4, 5 and 8 --
 // 8000, 1: 484 / 508, 598 / 1048, 1052 / 1717; 8000, 3: 831 / 670, 990 / 1227,
-// 1827 / 2168; 16000, 1: 660 / 835, 999 / 1939, 1772 / 3264; 32000, 3 (bs 4):
-// 1631 / 1619; 16000, 12 (bs 4): 3972 / 2581; no dependencies at all, 300,000 rows:
-// 261 / 458, 328 / 972, 640 / 1767.
+// 1827 / 2168; 5000, 1: -, 507 / 766, 808 / 1202; 5000, 3: -, 906 / 893, 1399 / 1496;
+// 128^3 (5490, 3): -, 12.7 / 15.3 ms, 28.0 / 28.0; 16000, 1: 660 / 835, 999 / 1939,
+// 1772 / 3264; 32000, 3 (bs 4): 1631 / 1619; 16000, 12 (bs 4): 3972 / 2581; no
+// dependencies at all, 300,000 rows: 261 / 458, 328 / 972, 640 / 1767.
 bool barrier_instead(int bs, int nb, int nlev, unsigned long long ndeps) {
   if (bs == 4) return nb >= 2ll * kFactorLevelWidth * nlev && 2 * ndeps < 5ull * nb;
-  return 2ll * nb >= 3ll * kFactorLevelWidth * nlev;
+  return nb >= (long long)kFactorLevelWidth * nlev;
 }
 
 // Block tasks cost each block a few microseconds of a warp (2.1 ns a block of the
