@@ -421,7 +421,6 @@ struct LevelWords {
   int maxdeg, nlev;          // largest dependency count of a row; levels
   unsigned long long ndeps;  // dependencies of all rows
   unsigned long long hubdeps;  // k_bilu0_plan: of the rows with more than kLongRow
-  unsigned long long hubspan;  // k_hub_span: the largest such row of every level, added up
   int other;                 // k_bilu0_plan: the pattern is not one for the row flow
   int widest;                // rows of the widest level of at most kSortCap rows
   int blocks;                // k_bilu0_plan: the blocks the row pointers hold
@@ -1880,7 +1879,7 @@ __global__ void __launch_bounds__(kLvlThreads, BS == 4 ? 2 : 1) k_bilu0_rowflow(
 // path.  Tasks are dealt by ticket, rows in level order and a row's blocks in
 // column order, so every block a task reads belongs to an earlier ticket and
 // its warp is running.  tcnt[p] is the number of updates of block p
-// (structure only, k_bilu0_tcount): most blocks have none and search for
+// (structure only, k_bilu0_nmatch<true>): most blocks have none and search for
 // none; the others look J up in the rows K of the row's earlier blocks, 32 at a
 // time, until they have found tcnt.  The operations per element and their
 // order are those of bilu0_grow.  What bounds it is the chain of dependent
@@ -2123,19 +2122,15 @@ int sync_finish(const SyncState& ss, int* h_zp, cudaStream_t st) {
 
 // Launches of a level analysis: the levels, their sizes, lvl[nb+1] (level l is
 // order[lvl[l]] .. order[lvl[l+1]-1]) and order[nb].  rec (optional): the
-// four words of the analysis record.  Returns the words' device copy, the rows'
-// levels (from 1) and nb + 1 zeros.
+// four words of the analysis record.  Returns the words' device copy.
 int level_sets(int nb, const int* row, const int* col, const int* diag, int lower, int* order,
                int* lvl, int* rec, LevelWords** out, Carver& ws, cudaStream_t st,
-               const LevelHook& hook = LevelHook(), int** levels = nullptr,
-               int** zeros = nullptr) {
+               const LevelHook& hook = LevelHook()) {
   int* level = ws.take<int>((size_t)nb + 1);
   int* cnt = ws.take<int>((size_t)nb + 1);
   LevelWords* w = ws.take<LevelWords>(1);
   if (!level || !cnt || !w) return BILU_ERR_WORKSPACE;
   *out = w;
-  if (levels) *levels = level;
-  if (zeros) *zeros = cnt;
   // level, cnt and the words are neighbours: one fill
   BILU_TRY_CUDA(cudaMemsetAsync(level, 0, (char*)(w + 1) - (char*)level, st));
   if (nb == 0) return BILU_OK;
@@ -2307,9 +2302,7 @@ __global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
                                                     const int* __restrict__ row,
                                                     const int* __restrict__ col,
                                                     const int* __restrict__ diag,
-                                                    int2* __restrict__ plan, LevelWords* w,
-                                                    const int* __restrict__ level,
-                                                    int* __restrict__ most) {
+                                                    int2* __restrict__ plan, LevelWords* w) {
   const long long pk = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (pk == 0) w->blocks = __ldg(row + nb);
   if (pk >= nnzb) return;
@@ -2317,10 +2310,9 @@ __global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
   const MatchLists m = match_lists(pk, nb, row, col, diag, I);
   const int dI = __ldg(diag + I);
   if (pk >= dI) return;
-  if (const int s = __ldg(row + I); dI - s > kLongRow) {
-    atomicAdd(&w->hubdeps, 1ull);
-    if (pk == s) atomicMax(most + level[I] - 1, dI - s);
-  }
+  // (once a row: atomics on one address take some 15 ns each)
+  if (const int n = dI - (int)pk; n > kLongRow && pk == __ldg(row + I))
+    atomicAdd(&w->hubdeps, (unsigned long long)n);
   bool odd = m.ce - m.cs > kMatchSerial;
   int at = -1;
   for (int c = m.cs; c < m.ce && !odd; ++c) {
@@ -2331,16 +2323,6 @@ __global__ void __launch_bounds__(256) k_bilu0_plan(int nb, long long nnzb,
   }
   plan[pk] = make_int2(__ldg(diag + __ldg(col + pk)), at);
   if (odd) w->other = 1;
-}
-
-// w->hubspan from the levels' largest long rows (zero for levels without one).
-__global__ void __launch_bounds__(256) k_hub_span(const int* __restrict__ most, LevelWords* w) {
-  if (w->maxdeg <= kLongRow) return;
-  int s = 0;
-  for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < w->nlev; l += gridDim.x * blockDim.x)
-    s += most[l];
-  s = __reduce_add_sync(FULL, s);
-  if ((threadIdx.x & 31) == 0 && s > 0) atomicAdd(&w->hubspan, (unsigned long long)s);
 }
 
 // Total of the match counts in 64 bits (the caller decides from it whether
@@ -2591,20 +2573,21 @@ bool barrier_instead(int bs, int nb, int nlev, unsigned long long ndeps) {
 
 // Block tasks cost each block a few microseconds of a warp (2.1 ns a block of the
 // whole chip more than rows do), and cut the chain through long rows into its
-// blocks.  They pay where that chain is long -- the largest long row of every level,
-// added up, at 0.08 us a dependency (8x8 blocks 0.3) -- and where enough of the
-// blocks are dependencies of long rows, so that it is not the levels' count that
-// sets the time.  Rows / blocks in ms, block sizes 4 and 8:
+// blocks.  They pay where that chain is long -- taken as half the longest row in every
+// level, at most all of the long rows one after the other, at 0.08 us a dependency
+// (8x8 blocks 0.3) -- and where enough of the blocks are dependencies of long rows,
+// so that it is not the levels' count that sets the time.  (The largest long row of
+// every level added up is 0.5 to 1.2 times that estimate on these patterns.)  Rows / blocks in ms, block sizes 4 and 8:
 //   power law, 3000 rows 2.8 / 0.4, 5.4 / 0.5; 20,000 2.7 / 1.1, 5.8 / 1.3; 50,000
 //   3.0 / 2.0, 5.6 / 2.5; 100,000 3.0 / 3.6, 6.6 / 4.5; 500,000 5.0 / 15.3, 11 / 20;
 //   40^3 grids with long rows (128^2: *), share of all blocks 0.1%* 2.4 / 5.6,
 //   3.2 / 4.0; 0.2% 2.2 / 4.2, 3.6 / 4.1; 0.4% 4.4 / 7.5, 7.2 / 6.3; 1.1%* 7.0 / 8.6,
 //   11.3 / 7.9; 3.8% 17.9 / 23.9, 28 / 17; 8.4%* 18.8 / 11.1, 33 / 10; 8.7% 26 / 27,
 //   42 / 27; 60,000 rows, 600 of 100 among rows of 3: 0.48 / 0.82, 0.84 / 1.01.
-bool blocks_instead(int bs, long long nnzb, unsigned long long hubdeps,
-                    unsigned long long hubspan) {
+bool blocks_instead(int bs, long long nnzb, int nlev, int maxdeg, unsigned long long hubdeps) {
   const unsigned long long n = (unsigned long long)nnzb;
-  return hubdeps * (bs <= 5 ? 20 : 400) > n && hubspan * (bs <= 5 ? 38 : 143) > n;
+  const unsigned long long chain = std::min(hubdeps, (unsigned long long)nlev * maxdeg / 2);
+  return hubdeps * (bs <= 5 ? 20 : 400) > n && chain * (bs <= 5 ? 38 : 143) > n;
 }
 
 // Level analysis of the lower (or upper) dependency DAG: order[nb] (ascending
@@ -2628,14 +2611,10 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
     return BILU_OK;
   }
   LevelWords *w = nullptr, hw;
-  int *level = nullptr, *most = nullptr;
-  BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st, hook, &level,
-                      &most));
+  BILU_TRY(level_sets(nb, row, col, diag, lower, order, lvl_ptr, nlev_d, &w, ws, st, hook));
   if (plan) {
     k_bilu0_plan<<<ceil_div(std::max(nplan, 1ll), 256), 256, 0, st>>>(nb, nplan, row, col, diag,
-                                                                       plan, w, level, most);
-    BILU_LAUNCH_CHECK();
-    k_hub_span<<<16, 256, 0, st>>>(most, w);
+                                                                       plan, w);
     BILU_LAUNCH_CHECK();
   }
   int rec[4];
@@ -2653,7 +2632,7 @@ int build_levels(int nb, const int* row, const int* col, const int* diag, int lo
     out->h_counted = counted;
     out->h_rowflow = counted && !hw.other && rec[1] <= kLongRow &&
                      !barrier_instead(bs, nb, rec[0], hw.ndeps);
-    out->h_blocks = counted && rec[1] > kLongRow && blocks_instead(bs, nplan, hw.hubdeps, hw.hubspan);
+    out->h_blocks = counted && rec[1] > kLongRow && blocks_instead(bs, nplan, rec[0], rec[1], hw.hubdeps);
   }
   if (hw.widest > 1) {
     static PerDevice<int> allowed;
