@@ -2577,7 +2577,7 @@ bool barrier_instead(int bs, int nb, int nlev, unsigned long long ndeps) {
 // level, at most all of the long rows one after the other, at 0.08 us a dependency
 // (8x8 blocks 0.3) -- and where enough of the blocks are dependencies of long rows,
 // so that it is not the levels' count that sets the time.  (The largest long row of
-// every level added up is 0.6 to 1.2 times that estimate on these patterns, 2 on
+// every level added up is 0.6 to 1.5 times that estimate on these patterns, 2 on
 // bands.)  Rows / blocks in ms, block sizes 4 and 8:
 //   power law, 3000 rows 2.8 / 0.4, 5.4 / 0.5; 20,000 2.7 / 1.1, 5.8 / 1.3; 50,000
 //   3.0 / 2.0, 5.6 / 2.5; 100,000 3.0 / 3.6, 6.6 / 4.5; 500,000 5.0 / 15.3, 11 / 20;
